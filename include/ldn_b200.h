@@ -119,6 +119,17 @@ LDN_API int ldn_mean_shift_rows(const float* x, int B, int C, float* running_mea
                         float* mean_out, ldn_stream_t stream);
 
 /*
+ * Patches of x[B][C][H][W] as columns cols[B][C * kh * kw][OH * OW] (zero outside the image), and the adjoint: x = sum of
+ * the columns' elements that come from each pixel.  OH = (H + 2 pad - dil (kh - 1) - 1) / stride + 1, OW alike.  The
+ * reference calls torch's unfold (core/modules/norm_dist.py:84-97).  Both write every element of their output.
+ * Status 1 for sizes that are not positive, an empty output plane, or a plane's columns beyond 2^30 elements.
+ */
+LDN_API int ldn_unfold(const float* x, int B, int C, int H, int W, int kh, int kw, int stride, int pad, int dil, float* cols,
+                       ldn_stream_t stream);
+LDN_API int ldn_fold(const float* cols, int B, int C, int H, int W, int kh, int kw, int stride, int pad, int dil, float* x,
+                     ldn_stream_t stream);
+
+/*
  * Pipe-throughput probe for roofline denominators (no counterpart in the reference).  kind 0 runs a loop
  * of independent FFMA chains, kind 2 the same chains issued as packed fma.rn.f32x2, kind 1 a loop of
  * independent ex2(lg2(x)) chains, kind 3 eight such MUFU chains beside eight packed-FMA chains (16 FMAs per step;

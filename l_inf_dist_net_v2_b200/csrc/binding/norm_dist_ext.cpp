@@ -157,6 +157,24 @@ void bound_inf_dist_backward_input_weight(Tensor& grad_outputL, Tensor& grad_out
           "bound_inf_dist_backward_input_weight");
 }
 
+// not part of the reference's extension module: patches as columns and the adjoint (ldn_unfold / ldn_fold)
+void unfold(Tensor& x, Tensor& cols, std::pair<int, int> kernel, int stride, int padding, int dilation) {
+    const float* a = fptr(x, "x");
+    float* c = fptr_mut(cols, "cols");
+    const c10::cuda::CUDAGuard guard(x.device());
+    check(ldn_unfold(a, x.size(0), x.size(1), x.size(2), x.size(3), kernel.first, kernel.second, stride, padding, dilation,
+                     c, stream()),
+          "unfold");
+}
+void fold(Tensor& cols, Tensor& x, std::pair<int, int> kernel, int stride, int padding, int dilation) {
+    const float* c = fptr(cols, "cols");
+    float* a = fptr_mut(x, "x");
+    const c10::cuda::CUDAGuard guard(x.device());
+    check(ldn_fold(c, x.size(0), x.size(1), x.size(2), x.size(3), kernel.first, kernel.second, stride, padding, dilation, a,
+                   stream()),
+          "fold");
+}
+
 void check_status() { check(ldn_check_status(stream()), "device status check"); }
 
 }  // namespace
@@ -174,5 +192,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("bound_inf_dist_forward_nograd", &bound_inf_dist_forward_nograd);
     m.def("bound_inf_dist_backward_input", &bound_inf_dist_backward_input);
     m.def("bound_inf_dist_backward_input_weight", &bound_inf_dist_backward_input_weight);
+    m.def("unfold", &unfold);
+    m.def("fold", &fold);
     m.def("check_status", &check_status);
 }

@@ -37,6 +37,41 @@ class _MeanShiftRowsF(torch.autograd.Function):
         return grad_input, None, None
 
 
+class _UnfoldF(torch.autograd.Function):
+    """F.unfold of (B, C, H, W) images in one launch, and its gradient in one launch (csrc/ldn_unfold.cu)."""
+
+    @staticmethod
+    def forward(ctx, x, positions, kernel_size, stride, padding, dilation):
+        ctx.geometry = kernel_size, stride, padding, dilation
+        ctx.image = x.shape
+        cols = torch.empty(x.size(0), x.size(1) * kernel_size[0] * kernel_size[1], positions, device=x.device,
+                           dtype=torch.float32)
+        _C.unfold(x, cols, *ctx.geometry)
+        return cols
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, grad_cols):
+        grad_cols = grad_cols.contiguous()
+        grad_x = torch.empty(ctx.image, device=grad_cols.device, dtype=torch.float32)
+        _C.fold(grad_cols, grad_x, *ctx.geometry)
+        return grad_x, None, None, None, None, None
+
+
+def _unfold(x, kernel_size, dilation, padding, stride):
+    """F.unfold(x, kernel_size, dilation, padding, stride); contiguous float32 CUDA images with one stride, padding and
+    dilation for both axes take this package's kernel, everything else (and every error) torch's."""
+    plain = (all(isinstance(v, int) for v in (dilation, padding, stride)) and dilation > 0 and padding >= 0 and stride > 0
+             and x.is_cuda and x.dtype == torch.float32 and x.dim() == 4 and x.is_contiguous() and x.numel() > 0
+             and min(kernel_size) > 0)
+    if plain:
+        out = [(s + 2 * padding - dilation * (k - 1) - 1) // stride + 1 for s, k in zip(x.shape[2:], kernel_size)]
+        columns = out[0] * out[1] * kernel_size[0] * kernel_size[1]
+        if min(out) > 0 and max(columns, x.size(2) * x.size(3), *(s + 2 * padding for s in x.shape[2:])) < 1 << 30:
+            return _UnfoldF.apply(x, out[0] * out[1], kernel_size, stride, padding, dilation)
+    return F.unfold(x, kernel_size, dilation, padding, stride)
+
+
 class MeanShift(nn.Module):
     """Subtracts the per-channel batch mean (training; running mean updated with `momentum`) or the running
     mean (eval) from x and from both bounds."""
@@ -186,11 +221,11 @@ class NormDistConv(NormDistBase):
         h, w = 0, 0
         if x is not None:
             h, w = x.size(2), x.size(3)
-            x = F.unfold(x, *unfold_paras)
+            x = _unfold(x, *unfold_paras)
         if lower is not None and upper is not None:
             h, w = lower.size(2), lower.size(3)
-            lower = F.unfold(lower, *unfold_paras)
-            upper = F.unfold(upper, *unfold_paras)
+            lower = _unfold(lower, *unfold_paras)
+            upper = _unfold(upper, *unfold_paras)
         x, lower, upper = super().forward(x, lower, upper)
         # as in the reference, the output size ignores dilation
         h, w = [(s + 2 * self.padding - k) // self.stride + 1 for s, k in zip((h, w), self.kernel_size)]

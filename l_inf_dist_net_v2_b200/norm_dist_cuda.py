@@ -161,6 +161,21 @@ def mean_shift_rows(x, running_mean, momentum, out):
         check(lib.ldn_mean_shift_rows(a, B, C, rm, float(momentum), y, None, _stream()), "mean_shift_rows")
 
 
+def unfold(x, cols, kernel_size, stride, padding, dilation):
+    """Not part of the reference's extension module: the patches of the images x (B, C, H, W) as columns, in one launch
+    (see ldn_unfold); cols has room for (B, C * kh * kw, OH * OW)."""
+    a, c = _f(x, "x"), _f(cols, "cols")
+    with torch.cuda.device(x.device):
+        check(lib.ldn_unfold(a, *x.shape, *kernel_size, stride, padding, dilation, c, _stream()), "unfold")
+
+
+def fold(cols, x, kernel_size, stride, padding, dilation):
+    """Not part of the reference's extension module: the adjoint of `unfold`, written to x (B, C, H, W)."""
+    c, a = _f(cols, "cols"), _f(x, "x")
+    with torch.cuda.device(x.device):
+        check(lib.ldn_fold(c, *x.shape, *kernel_size, stride, padding, dilation, a, _stream()), "fold")
+
+
 def norm_dist_backward_channels(grad_output, input, weight, output, grad_input, grad_weight, p, co_begin, co_count,
                                 accumulate_input):
     """Not part of the reference's extension module: the finite-p backward pass of an ungrouped layer restricted to the
@@ -213,6 +228,6 @@ try:
 except ImportError:
     _ext = None
 if _ext is not None:
-    for _name in __all__ + ["check_status"]:
+    for _name in __all__ + ["unfold", "fold", "check_status"]:
         globals()[_name] = getattr(_ext, _name)
     BINDING = "pybind11"
