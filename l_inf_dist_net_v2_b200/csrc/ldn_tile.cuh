@@ -493,7 +493,7 @@ tile_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ 
                 float* dst = P.partials +
                              (static_cast<size_t>(blockIdx.x) * 2 + slot) * (size_t)(NF + NI) * TELEMS;
 #pragma unroll
-                for (int i = 0; i < kRegM; ++i)
+                for (int i = 0; i < RM; ++i)
 #pragma unroll
                     for (int j = 0; j < RN; ++j) {
                         const int e = (i * RN + j) * kThreads + tid;
@@ -518,67 +518,127 @@ tile_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ 
     }
 }
 
-// Folds the partial accumulators of every tile that was shared between CTAs, in k order, and
-// finalises it.  Launched with kRegM CTAs per tile (CTA r of a tile handles register-row r of every
-// thread's block, i.e. 8 outputs per thread) and the grid size of the main kernel as an argument; CTAs
-// of unshared tiles return at once.
-template <class Op>
+// Folds the partial accumulators of every tile that was shared between CTAs, in k order, and finalises it.  The CTAs that
+// share a tile are consecutive, and only the first of them can have begun in an earlier tile (its second slot then holds
+// this tile's partial).  A work item is J neighbouring register columns of register row i of every thread of a tile's CTA,
+// so J outputs per thread; the fold is bound by the latency of its loads and its index arithmetic, not by bytes, so kBatch
+// partials are in flight per thread before the first is combined.  Two forms, chosen by launch_tile:
+//   MANY:  tiles shared by many CTAs each (small problems): J = 2 and an item for every part of every tile, so that the
+//          few tiles still spread over the chip;
+//   !MANY: tiles shared by two or three CTAs (large problems): J = REG_N, so that the index arithmetic serves 8 outputs,
+//          and the shared tiles are found from the boundaries between neighbouring CTAs' ranges (at most main_grid - 1,
+//          however many tiles there are): the first boundary inside a tile stands for it.
+// `rows` = register rows the main kernel computed and stored.
+// (8 outputs per thread, one partial in flight, 64-bit divisions per partial: 16.8 us for 8 tiles of 18.5 partials each,
+// 31 us for 4 tiles of 37, 18 us for 147 of 160 tiles shared by two or three.)
+template <class Op, bool MANY>
 __global__ void __launch_bounds__(kThreads)
-tile_fixup_kernel(const TileParams P, const int main_grid) {
+tile_fixup_kernel(const TileParams P, const int main_grid, const int rows) {
     constexpr int NF = Op::NF;
     constexpr int NI = Op::NI;
     constexpr int NIA = NI > 0 ? NI : 1;
     constexpr int RN = Op::REG_N;
     constexpr int TN = 16 * RN;
     constexpr int TELEMS = kTileM * TN;
+    constexpr int J = MANY ? 2 : RN;
+    constexpr int kBatch = !MANY ? 2 : (NF + NI > 3 ? 4 : 8);
+    constexpr size_t SLOT = static_cast<size_t>(NF + NI) * TELEMS;
     if (P.gate != nullptr && (*P.gate != 0) == (P.gate_invert != 0)) return;
-    const long long tile = blockIdx.x / kRegM;
-    const int i = blockIdx.x % kRegM;
-    const int KT = P.kt;
-    const long long t0 = tile * KT, t1 = t0 + KT;
-    // CTA whose range contains iteration t0
-    int c = static_cast<int>(((t0 + 1) * main_grid - 1) / P.total_iters);
-    if (range_begin(P.total_iters, main_grid, c + 1) >= t1) return;  // owned whole by one CTA
-
     const int tid = threadIdx.x;
     const int tn = thread_col<Op>(tid);
     const int tm = thread_row<Op>(tid);
-    const TileCoord tc = tile_coord(P, tile, TN);
-    float accf[RN][NF];
-    int acci[RN][NIA];
-#pragma unroll
-    for (int j = 0; j < RN; ++j) Op::init(accf[j], acci[j]);
-
-    for (; c < main_grid; ++c) {
-        const long long b0 = range_begin(P.total_iters, main_grid, c);
-        const long long b1 = range_begin(P.total_iters, main_grid, c + 1);
-        if (b0 >= t1) break;
-        if (b1 <= b0) continue;
-        const int slot = (b0 / KT == tile) ? 0 : 1;
-        const float* src = P.partials + (static_cast<size_t>(c) * 2 + slot) * (size_t)(NF + NI) * TELEMS;
-        float pf[RN][NF];
-        int pn[RN][NIA];
-#pragma unroll
-        for (int j = 0; j < RN; ++j) {
-            const int e = (i * RN + j) * kThreads + tid;
-#pragma unroll
-            for (int a = 0; a < NF; ++a) pf[j][a] = src[a * TELEMS + e];
-#pragma unroll
-            for (int a = 0; a < NI; ++a) pn[j][a] = __float_as_int(src[(NF + a) * TELEMS + e]);
+    const int per_tile = rows * (RN / J);
+    const int items = (MANY ? P.G * P.tiles_m * P.tiles_n : main_grid - 1) * per_tile;
+    // the same index arithmetic in 32 bits wherever it fits (64-bit divisions took longer than the loads of an item)
+    const bool narrow = P.total_iters * main_grid < 0x7fffffffLL;
+    for (int item = blockIdx.x; item < items; item += static_cast<int>(gridDim.x)) {
+        const int unit = item / per_tile;  // MANY: the tile; else: the boundary behind the range of CTA `unit`
+        const int part_of_tile = item - unit * per_tile;
+        int c0, c1;   // the CTAs that share the tile
+        bool second;  // c0 began in an earlier tile
+        TileCoord tc;
+        if (narrow) {
+            const unsigned total = static_cast<unsigned>(P.total_iters), kt = P.kt, grid = main_grid;
+            unsigned t = unit, t0 = t * kt;
+            if constexpr (MANY) {
+                c0 = static_cast<int>(((t0 + 1) * grid - 1) / total);
+            } else {
+                c0 = unit;
+                const unsigned begin = total * static_cast<unsigned>(unit + 1) / grid;
+                t = begin / kt;
+                t0 = t * kt;
+                if (begin == t0) continue;  // no tile is cut here
+            }
+            const unsigned before = total * static_cast<unsigned>(c0) / grid;
+            if (!MANY && before > t0) continue;  // an earlier boundary stands for this tile
+            second = before < t0;
+            c1 = static_cast<int>(((t0 + kt) * grid - 1) / total);
+            const unsigned tiles_m = P.tiles_m, per_group = tiles_m * P.tiles_n;
+            const unsigned g = t / per_group, r = t - g * per_group, col = r / tiles_m;
+            tc = TileCoord{static_cast<int>(g), static_cast<int>((r - col * tiles_m) * kTileM), static_cast<int>(col * TN)};
+        } else {
+            long long t = unit, t0 = t * P.kt;
+            if constexpr (MANY) {
+                c0 = static_cast<int>(((t0 + 1) * main_grid - 1) / P.total_iters);
+            } else {
+                c0 = unit;
+                const long long begin = range_begin(P.total_iters, main_grid, unit + 1);
+                t = begin / P.kt;
+                t0 = t * P.kt;
+                if (begin == t0) continue;
+            }
+            const long long before = range_begin(P.total_iters, main_grid, c0);
+            if (!MANY && before > t0) continue;
+            second = before < t0;
+            c1 = static_cast<int>(((t0 + P.kt) * main_grid - 1) / P.total_iters);
+            tc = tile_coord(P, t, TN);
         }
+        if (MANY && c0 == c1) continue;  // owned whole by one CTA
+        const int i = part_of_tile / (RN / J), j0 = J * (part_of_tile % (RN / J));
+        const float* src = P.partials + static_cast<size_t>(c0) * 2 * SLOT + (i * RN + j0) * kThreads + tid;
+        float accf[J][NF];
+        int acci[J][NIA];
 #pragma unroll
-        for (int j = 0; j < RN; ++j) Op::combine(accf[j], acci[j], pf[j], pn[j]);
-    }
+        for (int j = 0; j < J; ++j) Op::init(accf[j], acci[j]);
+        for (int cc = c0; cc <= c1; cc += kBatch) {
+            float pf[kBatch][J][NF];
+            int pn[kBatch][J][NIA];
 #pragma unroll
-    for (int j = 0; j < RN; ++j) {
+            for (int u = 0; u < kBatch; ++u) {
+                if (cc + u <= c1) {
+                    const float* part = src + static_cast<size_t>(cc + u - c0) * 2 * SLOT + ((second && cc + u == c0) ? SLOT : 0);
+#pragma unroll
+                    for (int j = 0; j < J; ++j) {
+#pragma unroll
+                        for (int a = 0; a < NF; ++a) pf[u][j][a] = part[a * TELEMS + j * kThreads];
+#pragma unroll
+                        for (int a = 0; a < NI; ++a)
+                            pn[u][j][a] = __float_as_int(part[(NF + a) * TELEMS + j * kThreads]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u)
+                if (cc + u <= c1) {
+#pragma unroll
+                    for (int j = 0; j < J; ++j) Op::combine(accf[j], acci[j], pf[u][j], pn[u][j]);
+                }
+        }
         const int m = tc.m0 + own_index<Op::LA>(tm, i);
-        const int n = tc.n0 + own_index<Op::LB, RN>(tn, j);
-        if (m < P.M && n < P.N) {
-            const float pr = Op::HAS_P ? Op::load_pres(P, m, n, tc.g) : 0.0f;
-            Op::finalize(accf[j], acci[j], pr, m, n, tc.g, P);
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int n = tc.n0 + own_index<Op::LB, RN>(tn, j0 + j);
+            if (m < P.M && n < P.N) {
+                const float pr = Op::HAS_P ? Op::load_pres(P, m, n, tc.g) : 0.0f;
+                Op::finalize(accf[j], acci[j], pr, m, n, tc.g, P);
+            }
         }
     }
 }
+
+// Most CTAs of a gated fold, which usually returns at once: 8 per SM of a 148-SM chip stay cheap to launch, the
+// grid-stride loop covers the rest when it runs.  (An ungated fold has a CTA per item.)
+constexpr int kGatedFixupCtas = 148 * 8;
 
 // Host launcher (ldn_launch.cuh provides the definition used by the .cu files).
 struct TileLaunch {
@@ -606,7 +666,8 @@ int launch_tile(const TileLaunch& L, cudaStream_t stream) {
     // (a gated launch usually returns at once: the optional timing brackets the ungated kernels only)
     const bool timed = L.params.gate == nullptr;
     if (timed) timing_before(stream);
-    if (HALF && L.params.M <= kTileM / 2)
+    const bool half = HALF && L.params.M <= kTileM / 2;
+    if (half)
         tile_kernel<Op, (HALF ? kRegM / 2 : kRegM)><<<L.grid, kThreads, SMEM, stream>>>(L.map_a0, L.map_a1, L.map_b,
                                                                                       L.params);
     else
@@ -618,7 +679,16 @@ int launch_tile(const TileLaunch& L, cudaStream_t stream) {
     const long long tiles = L.params.total_iters / L.params.kt;
     // a tile can only be shared when the ranges do not fall on tile boundaries
     if (L.params.total_iters % L.grid != 0 || (L.params.total_iters / L.grid) % L.params.kt != 0) {
-        tile_fixup_kernel<Op><<<static_cast<unsigned>(tiles * kRegM), kThreads, 0, stream>>>(L.params, L.grid);
+        const int rows = half ? kRegM / 2 : kRegM;
+        // up to two CTAs per tile: 147 shared tiles of 160 (512 x 3072 -> 5120, p = 8) take 14.0 us in the boundary form
+        // and 24.4 in the other; beyond, 8 tiles of 18.5 partials take 3.9 us in the tile form and 7.3 with the boundary
+        // form's items
+        const bool many = L.grid > 2 * tiles;
+        long long blocks = many ? tiles * rows * (Op::REG_N / 2) : static_cast<long long>(L.grid - 1) * rows;
+        if (L.params.gate && blocks > kGatedFixupCtas) blocks = kGatedFixupCtas;
+        const unsigned n = static_cast<unsigned>(blocks);
+        if (many) tile_fixup_kernel<Op, true><<<n, kThreads, 0, stream>>>(L.params, L.grid, rows);
+        else tile_fixup_kernel<Op, false><<<n, kThreads, 0, stream>>>(L.params, L.grid, rows);
         e = cudaGetLastError();
         count_launches(1);
     }
