@@ -5,7 +5,9 @@ namespace ldn {
 namespace {
 constexpr int kBlock = 256;
 constexpr int kRescanInplaceMaxSmem = 200 * 1024;  // input slab of rescan_inplace_kernel
-constexpr int kRescanChunk = 1024;  // outputs a block of rescan_kernel handles in one pass (a multiple of kBlock / 8)
+constexpr int kRescanIlp = 4;                         // outputs in flight per lane group of rescan_kernel
+constexpr int kRescanStep = kRescanIlp * kBlock / 4;  // outputs a block of rescan_kernel handles in one step
+constexpr long long kRescanBlocks = 148 * 32;         // its blocks beyond which each takes several steps of one input row
 // grid of a kernel that usually returns at once (gated): small, the grid-stride loops cover the rest when it runs
 inline unsigned gated_blocks(unsigned blocks, const int* gate) { return (gate && blocks > 592u) ? 592u : blocks; }
 inline unsigned blocks_for(long long n) {
@@ -175,82 +177,101 @@ __global__ void coef_gen_kernel(const float* __restrict__ go, const float* __res
     }
 }
 
-// Eight lanes per output element: lane q of a group loads the q-th 16-byte piece of the recorded 32-channel stage of
-// each operand row (one full 128-byte line per group and operand: operand views are 16-byte aligned with row
-// pitches that are multiples of 4 floats), finds the lowest matching channel among its four, and a minimum over the
-// group's lanes keeps the lowest channel of the stage -- the index a strictly-greater scan in ascending order ends with.
-// blockIdx.x = (sample, group); blockIdx.y walks that pair's CO/G * HW outputs in chunks, so the index arithmetic
-// per output is one division by HW (none for fully connected layers) and, for those, a block keeps rereading one
-// input row, which stays in the L1 cache: only the weight pieces come from L2.
+// Four lanes per output element, kRescanIlp outputs per lane group in flight: lane q of a group loads the 16-byte pieces q
+// and q + 4 of the recorded 32-channel stage of each operand row (one full 128-byte line per output and operand: operand
+// views are 16-byte aligned with row pitches that are multiples of 4 floats), finds the lowest matching channel among its
+// eight, and a minimum over the group's lanes keeps the lowest channel of the stage -- the index a strictly-greater scan in
+// ascending order ends with.  The search is a chain of two dependent loads (stage id, then the pieces), so it is bound by
+// their latency unless several outputs are in flight per lane, and then by the L2 reads of the weight pieces (128 bytes
+// per output) and by its instructions (hence four lanes with two pieces rather than eight with one).
+// (512 x 5120 -> 5120 forward + backward 1149 -> 1116 us, of which the search was 99 with one output in flight.)
+// blockIdx.x = (sample, group); blockIdx.y walks that pair's CO/G * HW outputs in steps of kRescanStep, so the index
+// arithmetic per output is one division by HW (none for fully connected layers) and, for those, a block keeps rereading
+// one input row, which stays in the L1 cache: only the weight pieces come from L2.
 template <int mode>
-__global__ void rescan_kernel(Operand a0, Operand a1, Operand b, const float* __restrict__ y,
-                              int* __restrict__ pos, Shape s, long long a_stride_k) {
+__global__ void __launch_bounds__(kBlock) rescan_kernel(Operand a0, Operand a1, Operand b, const float* __restrict__ y,
+                                                        int* __restrict__ pos, Shape s, long long a_stride_k) {
+    constexpr int U = kRescanIlp;
     const int kpad = (s.CIg + 3) & ~3;
-    const int q = threadIdx.x & 7;
-    const int group_in_block = threadIdx.x >> 3;
+    const int q = threadIdx.x & 3;
+    const int group_in_block = threadIdx.x >> 2;
     const unsigned cohw = static_cast<unsigned>(s.COg) * static_cast<unsigned>(s.HW);  // < 2^31, checked by the launcher
     const long long bg = blockIdx.x;
     const int bi = static_cast<int>(bg / s.G), g = static_cast<int>(bg - static_cast<long long>(bi) * s.G);
     const float* arow = a0.ptr + g * a0.stride_group;
     const float* urow = a1.ptr + g * a1.stride_group;
     const float* brow = b.ptr + g * b.stride_group;
-    // (the trip counts are the same for all lanes of a warp: its four groups handle consecutive outputs)
-    for (unsigned j0 = blockIdx.y * kRescanChunk; j0 < cohw; j0 += gridDim.y * kRescanChunk)
-        for (unsigned step = 0; step < kRescanChunk && j0 + step < cohw; step += kBlock / 8) {
-            const unsigned j = j0 + step + group_in_block;
+    // (the trip counts are the same for all lanes of a warp: its eight groups handle consecutive outputs)
+    for (unsigned j0 = blockIdx.y * kRescanStep; j0 < cohw; j0 += gridDim.y * kRescanStep) {
+        int stage[U];
+        float yv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const unsigned j = j0 + u * (kBlock / 4) + group_in_block;
             const bool valid = j < cohw;
-            const long long i = bg * cohw + j;
-            const int stage = valid ? pos[i] : -1;
-            int best = 0x7fffffff;
-            if (stage >= 0) {
+            stage[u] = valid ? pos[bg * cohw + j] : -1;
+            yv[u] = valid ? y[bg * cohw + j] : 0.0f;
+        }
+        int best[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            best[u] = 0x7fffffff;
+            const unsigned j = j0 + u * (kBlock / 4) + group_in_block;
+            if (stage[u] >= 0) {
                 const unsigned o = s.HW == 1 ? j : j / static_cast<unsigned>(s.HW);
                 const unsigned hw = j - o * s.HW;
                 const long long m = static_cast<long long>(bi) * s.HW + hw;
-                const int k = stage * 32 + 4 * q;
-                if (k < kpad) {
-                    float4 av;
-                    if (a_stride_k == 1) {
-                        av = *reinterpret_cast<const float4*>(arow + m * a0.stride_row + k);
-                    } else {
-                        // input read in place (channels HW apart, no padding behind the last one)
-                        const float* ap = a0.ptr + bg * a0.stride_group + hw * a0.stride_row + k * a_stride_k;
-                        av.x = ap[0];
-                        av.y = k + 1 < s.CIg ? ap[a_stride_k] : 0.0f;
-                        av.z = k + 2 < s.CIg ? ap[2 * a_stride_k] : 0.0f;
-                        av.w = k + 3 < s.CIg ? ap[3 * a_stride_k] : 0.0f;
-                    }
-                    const float4 bv = *reinterpret_cast<const float4*>(brow + o * b.stride_row + k);
-                    float4 uv = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (mode != 0) uv = *reinterpret_cast<const float4*>(urow + m * a1.stride_row + k);
-                    const float yv = y[i];
-                    const float ae[4] = {av.x, av.y, av.z, av.w};
-                    const float be[4] = {bv.x, bv.y, bv.z, bv.w};
-                    const float ue[4] = {uv.x, uv.y, uv.z, uv.w};
 #pragma unroll
-                    for (int e = 3; e >= 0; --e) {
-                        bool hit, flag;
-                        if (mode == 0) {
-                            const float d = ae[e] - be[e];
-                            hit = fabsf(d) == yv;
-                            flag = d < 0.0f;
+                for (int h = 1; h >= 0; --h) {
+                    const int k = stage[u] * 32 + 16 * h + 4 * q;
+                    if (k < kpad) {
+                        float4 av;
+                        if (a_stride_k == 1) {
+                            av = *reinterpret_cast<const float4*>(arow + m * a0.stride_row + k);
                         } else {
-                            const float t1 = be[e] - ae[e], t2v = ue[e] - be[e];
-                            hit = (mode == 1) ? (fminf(t1, t2v) == -yv) : (fmaxf(t1, t2v) == yv);
-                            flag = !(t1 <= t2v);
+                            // input read in place (channels HW apart, no padding behind the last one)
+                            const float* ap = a0.ptr + bg * a0.stride_group + hw * a0.stride_row + k * a_stride_k;
+                            av.x = ap[0];
+                            av.y = k + 1 < s.CIg ? ap[a_stride_k] : 0.0f;
+                            av.z = k + 2 < s.CIg ? ap[2 * a_stride_k] : 0.0f;
+                            av.w = k + 3 < s.CIg ? ap[3 * a_stride_k] : 0.0f;
                         }
-                        if (hit && k + e < s.CIg) best = ((k + e) << 1) | (flag ? 1 : 0);
+                        const float4 bv = *reinterpret_cast<const float4*>(brow + o * b.stride_row + k);
+                        float4 uv = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (mode != 0) uv = *reinterpret_cast<const float4*>(urow + m * a1.stride_row + k);
+                        const float ae[4] = {av.x, av.y, av.z, av.w};
+                        const float be[4] = {bv.x, bv.y, bv.z, bv.w};
+                        const float ue[4] = {uv.x, uv.y, uv.z, uv.w};
+#pragma unroll
+                        for (int e = 3; e >= 0; --e) {
+                            bool hit, flag;
+                            if (mode == 0) {
+                                const float d = ae[e] - be[e];
+                                hit = fabsf(d) == yv[u];
+                                flag = d < 0.0f;
+                            } else {
+                                const float t1 = be[e] - ae[e], t2v = ue[e] - be[e];
+                                hit = (mode == 1) ? (fminf(t1, t2v) == -yv[u]) : (fmaxf(t1, t2v) == yv[u]);
+                                flag = !(t1 <= t2v);
+                            }
+                            if (hit && k + e < s.CIg) best[u] = ((k + e) << 1) | (flag ? 1 : 0);
+                        }
                     }
                 }
             }
-            best = min(best, __shfl_xor_sync(0xffffffffu, best, 1));
-            best = min(best, __shfl_xor_sync(0xffffffffu, best, 2));
-            best = min(best, __shfl_xor_sync(0xffffffffu, best, 4));
-            if (valid && q == 0) {
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            best[u] = min(best[u], __shfl_xor_sync(0xffffffffu, best[u], 1));
+            best[u] = min(best[u], __shfl_xor_sync(0xffffffffu, best[u], 2));
+            const unsigned j = j0 + u * (kBlock / 4) + group_in_block;
+            if (j < cohw && q == 0) {
                 int result = (mode == 1) ? static_cast<int>(0xffffffffu) : 0;
-                if (best != 0x7fffffff) result = (best >> 1) | ((best & 1) ? static_cast<int>(0x80000000u) : 0);
-                pos[i] = result;
+                if (best[u] != 0x7fffffff) result = (best[u] >> 1) | ((best[u] & 1) ? static_cast<int>(0x80000000u) : 0);
+                pos[bg * cohw + j] = result;
             }
         }
+    }
 }
 
 // The same search for inputs read in place (x[B, C, HW]: the channels of an output are HW floats apart, so the
@@ -510,8 +531,10 @@ int launch_rescan(int mode, Operand a0, Operand a1, Operand b, const float* y, i
             if (row * 8 <= limit) return launch_rescan_inplace<8>(a0, b, y, pos, s, st);
         }
     }
-    long long chunks = (cohw + kRescanChunk - 1) / kRescanChunk;
-    if (chunks > 65535) chunks = 65535;  // the kernel strides over the rest
+    long long chunks = (cohw + kRescanStep - 1) / kRescanStep;
+    const long long most = kRescanBlocks / bg > 1 ? kRescanBlocks / bg : 1;
+    if (chunks > most) chunks = most;  // the kernel strides over the rest
+    if (chunks > 65535) chunks = 65535;
     const dim3 grid(static_cast<unsigned>(bg), static_cast<unsigned>(chunks));
     if (mode == 0) rescan_kernel<0><<<grid, kBlock, 0, st>>>(a0, a1, b, y, pos, s, a_stride_k);
     else if (mode == 1) rescan_kernel<1><<<grid, kBlock, 0, st>>>(a0, a1, b, y, pos, s, a_stride_k);
