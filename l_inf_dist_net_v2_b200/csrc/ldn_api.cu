@@ -320,8 +320,9 @@ int norm_dist_backward_part(const float* go, const float* x, const float* w, con
 
     // the kernels of one arithmetic form (fam: 0..8 integer q, -1 / -2 general p) on coefficient views cv0 / cv1.
     // gate: run only if *gate != 0 (the guard's second form); the weight-gradient reduction of the fast form is
-    // gated the other way round, so exactly one of the two forms touches grad_weight.
-    auto run_family = [&](int fam, const View& cv0, const View& cv1, const int* gate) -> int {
+    // gated the other way round, so exactly one of the two forms touches grad_weight.  next (fused form only, may be null):
+    // coefficients of the following form, computed in the launch behind this form's tile kernel.
+    auto run_family = [&](int fam, const View& cv0, const View& cv1, const int* gate, const CoefJob* next) -> int {
         auto plan_rows = [&](TileLaunch& L, const OpGeom geom) -> int {
             int e = fill_plan(c, &L, s.M, s.CIg, s.COg, s.G, 1, geom);
             if (e != kOk) return e;
@@ -349,9 +350,10 @@ int norm_dist_backward_part(const float* go, const float* x, const float* w, con
             TileLaunch L;
             if ((e = plan_rows(L, bwd_fused_geom(fam))) != kOk) return e;
             L.params.side_out = side;
-            if ((e = launch_bwd_fused(fam, L, c.st)) != kOk) return e;
-            return launch_side_reduce(side, gw, static_cast<long long>(s.CO) * s.CIg, static_cast<int>(tiles_m),
-                                      accumulate_gw, gate ? gate : flag, gate != nullptr, c.st);
+            L.post.side = side_reduce_job(side, gw, static_cast<long long>(s.CO) * s.CIg, static_cast<int>(tiles_m),
+                                          accumulate_gw, gate ? gate : flag, gate != nullptr);
+            if (next) L.post.coef = *next;
+            return launch_bwd_fused(fam, L, c.st);
         }
         if (gx) {
             TileLaunch L;
@@ -389,26 +391,27 @@ int norm_dist_backward_part(const float* go, const float* x, const float* w, con
         if (!c0) return kWorkspace;
         const View cv = View{c0, s.COg, s.M, s.G, int_pitch, s.M * int_pitch, 1};
         if ((r = launch_coef_int(go, y, c0, s, static_cast<int>(int_pitch), iq, flag, c.st)) != kOk) return r;
-        if ((r = run_family(iq, cv, cv, nullptr)) != kOk) return r;
-        if (!guarded) return kOk;
+        if (!guarded) return run_family(iq, cv, cv, nullptr, nullptr);
         // second form, gated by the flag: 1 / y and g as coefficients, 2^(q lg2(|t| / y)) per pair
         float* r0 = c.bump.take<float>(gen_floats);
         float* r1 = c.bump.take<float>(gen_floats);
         if (!r0 || !r1) return kWorkspace;
         View v0, v1;
         gen_views(r0, r1, &v0, &v1);
-        if ((r = launch_coef_gen(go, y, r0, r1, s, static_cast<int>(gen_pitch), gen_rows, p - 1.0f, false, flag, c.st)) != kOk)
-            return r;
-        return run_family(-2, v0, v1, flag);
+        const CoefJob second = coef_gen_job(go, y, r0, r1, s, static_cast<int>(gen_pitch), gen_rows, p - 1.0f, false, flag);
+        if ((r = run_family(iq, cv, cv, nullptr, &second)) != kOk) return r;
+        if (!fused && (r = launch_coef_gen(second, c.st)) != kOk) return r;
+        return run_family(-2, v0, v1, flag, nullptr);
     }
     float* c0 = c.bump.take<float>(gen_floats);
     float* c1 = c.bump.take<float>(gen_floats);
     if (!c0 || !c1) return kWorkspace;
     View v0, v1;
     gen_views(c0, c1, &v0, &v1);
-    if ((r = launch_coef_gen(go, y, c0, c1, s, static_cast<int>(gen_pitch), gen_rows, p - 1.0f, iq == -1, nullptr, c.st)) != kOk)
+    if ((r = launch_coef_gen(coef_gen_job(go, y, c0, c1, s, static_cast<int>(gen_pitch), gen_rows, p - 1.0f, iq == -1, nullptr),
+                             c.st)) != kOk)
         return r;
-    return run_family(iq, v0, v1, nullptr);
+    return run_family(iq, v0, v1, nullptr, nullptr);
 }
 
 int norm_dist_backward(const float* go, const float* x, const float* w, const float* y, const Shape& s, float* gx,

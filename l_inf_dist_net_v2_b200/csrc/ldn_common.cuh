@@ -49,6 +49,15 @@ struct Operand {
     long long stride_group;
 };
 
+struct Shape {
+    int B, CO, CI, G, HW;
+    int CIg, COg;
+    long long M;  // B * HW
+    // A range of output channels of a wider layer (G == 1 only): grad_output / output rows are co_src channels long and
+    // this problem's channel o is their channel co_off + o.  co_src == CO, co_off == 0: the whole layer.
+    int co_src, co_off;
+};
+
 // Output addressing shared by all kernels:
 //   offset(m, n, g) = (m / hw_div) * s_b + (m % hw_div) * s_hw + g * s_g + n * s_n
 struct OutAddr {

@@ -3,7 +3,7 @@
 namespace ldn {
 
 namespace {
-constexpr int kBlock = 256;
+constexpr int kBlock = kPostBlock;
 constexpr int kRescanInplaceMaxSmem = 200 * 1024;  // input slab of rescan_inplace_kernel
 constexpr int kRescanIlp = 4;                         // outputs in flight per lane group of rescan_kernel
 constexpr int kRescanStep = kRescanIlp * kBlock / 4;  // outputs a block of rescan_kernel handles in one step
@@ -15,21 +15,6 @@ inline unsigned blocks_for(long long n) {
     if (b < 1) b = 1;
     if (b > 1184 * 8) b = 1184 * 8;  // grid-stride beyond this
     return static_cast<unsigned>(b);
-}
-
-// index helpers -------------------------------------------------------------------------------
-// canonical arrays are [g][m][pitch]; thread index runs over (g, m, c) with c fastest
-struct CanonIdx {
-    int g, c;
-    long long m;
-};
-__device__ __forceinline__ CanonIdx canon_idx(long long i, int inner, long long M) {
-    CanonIdx r;
-    r.c = static_cast<int>(i % inner);
-    const long long t = i / inner;
-    r.m = t % M;
-    r.g = static_cast<int>(t / M);
-    return r;
 }
 
 __global__ void canon_x_kernel(const float* __restrict__ x, float* __restrict__ xc, Shape s, int pitch) {
@@ -98,13 +83,6 @@ __global__ void canon_w_kernel(const float* __restrict__ w, float* __restrict__ 
     }
 }
 
-// thread index runs over (g, m, o) with o fastest; source offset in output layout
-__device__ __forceinline__ long long y_offset(const Shape& s, const CanonIdx& q) {
-    const long long b = q.m / s.HW, hw = q.m % s.HW;
-    if (s.co_src != s.CO) return (b * s.co_src + s.co_off + q.c) * s.HW + hw;  // channel range, G == 1
-    return ((b * s.G + q.g) * s.COg + q.c) * s.HW + hw;
-}
-
 // Range guard of the integer-q coefficient g / y^q: *flag is raised when some y^-q is outside [kRqMin, kRqMax]
 // (beyond: y^-q overflows or |t|^q <= y^q goes denormal; below: the coefficient loses its bits).  The caller clears
 // the word beforehand; flag may be null (q = 0).
@@ -144,38 +122,7 @@ __global__ void coef_int_flat_kernel(const float4* __restrict__ go, const float4
     }
     if (flag && bad) *flag = 1;
 }
-__global__ void coef_gen_flat_kernel(const float4* __restrict__ go, const float4* __restrict__ y,
-                                     float4* __restrict__ rinv, float4* __restrict__ gcp, long long n4, float q, bool fold,
-                                     const int* gate) {
-    if (gate && *gate == 0) return;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-        const float4 yv = y[i];
-        rinv[i] = fold ? make_float4(-q * log2f(yv.x), -q * log2f(yv.y), -q * log2f(yv.z), -q * log2f(yv.w))
-                       : make_float4(1.0f / yv.x, 1.0f / yv.y, 1.0f / yv.z, 1.0f / yv.w);
-        gcp[i] = go[i];
-    }
-}
-
-// The general-p coefficient arrays are padded to whole tiles (rows to a multiple of 128, the inner extent to the
-// pitch, a multiple of 32): padding gets the offset -1e30 (folded form) or the factor 0 (1 / y form), which sends
-// the power to (almost) zero whatever |t| the zero-filled partner operand produces, and a zero gradient factor.
-__global__ void coef_gen_kernel(const float* __restrict__ go, const float* __restrict__ y, float* __restrict__ rinv,
-                                float* __restrict__ gcp, Shape s, int pitch, long long rows_pad, float q, bool fold,
-                                const int* gate) {
-    if (gate && *gate == 0) return;
-    const long long total = static_cast<long long>(s.G) * rows_pad * pitch;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const CanonIdx ci = canon_idx(i, pitch, rows_pad);
-        float off = fold ? -1e30f : 0.0f, gv = 0.0f;
-        if (ci.m < s.M && ci.c < s.COg) {
-            const long long src = y_offset(s, ci);
-            off = fold ? -q * log2f(y[src]) : 1.0f / y[src];
-            gv = go[src];
-        }
-        rinv[i] = off;
-        gcp[i] = gv;
-    }
-}
+__global__ void __launch_bounds__(kBlock) coef_gen_kernel(const CoefJob job) { coef_gen_block(job, blockIdx.x, gridDim.x); }
 
 // Four lanes per output element, kRescanIlp outputs per lane group in flight: lane q of a group loads the 16-byte pieces q
 // and q + 4 of the recorded 32-channel stage of each operand row (one full 128-byte line per output and operand: operand
@@ -386,17 +333,6 @@ __global__ void row_absmax_strided_kernel(Operand v, long long rows, int inner, 
     }
 }
 
-// gate (may be null): the kernel runs only if (*gate != 0) == run_if_nonzero
-__global__ void side_reduce_kernel(const float* __restrict__ part, float* __restrict__ gw, long long count, int tiles,
-                                   bool accumulate, const int* gate, bool run_if_nonzero) {
-    if (gate && (*gate != 0) != run_if_nonzero) return;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        for (int t = 0; t < tiles; ++t) s += part[t * count + i];
-        gw[i] = accumulate ? gw[i] - s : -s;
-    }
-}
-
 // One thread per output element, in output-layout order (coalesced reads of go / pos).
 __global__ void inf_scatter_kernel(const float* __restrict__ go, const int* __restrict__ pos, float* gx, float* gw,
                                    Shape s) {
@@ -498,18 +434,15 @@ int launch_coef_int(const float* go, const float* y, float* coef, const Shape& s
     coef_int_kernel<<<blocks_for((long long)s.G * s.M * s.COg), kBlock, 0, st>>>(go, y, coef, s, pitch, iq, flag);
     LDN_LAUNCH_RET();
 }
-int launch_coef_gen(const float* go, const float* y, float* rinv, float* gcp, const Shape& s, int pitch,
-                    long long rows_pad, float q, bool fold, const int* gate, cudaStream_t st) {
-    if (flat_ok(s, pitch, go, y) && rows_pad == s.M) {
-        const long long n4 = static_cast<long long>(s.M) * s.COg / 4;
-        coef_gen_flat_kernel<<<gated_blocks(blocks_for(n4), gate), kBlock, 0, st>>>(reinterpret_cast<const float4*>(go),
-                                                              reinterpret_cast<const float4*>(y),
-                                                              reinterpret_cast<float4*>(rinv),
-                                                              reinterpret_cast<float4*>(gcp), n4, q, fold, gate);
-        LDN_LAUNCH_RET();
-    }
-    coef_gen_kernel<<<gated_blocks(blocks_for((long long)s.G * rows_pad * pitch), gate), kBlock, 0, st>>>(
-        go, y, rinv, gcp, s, pitch, rows_pad, q, fold, gate);
+CoefJob coef_gen_job(const float* go, const float* y, float* rinv, float* gcp, const Shape& s, int pitch,
+                     long long rows_pad, float q, bool fold, const int* gate) {
+    const bool flat = flat_ok(s, pitch, go, y) && rows_pad == s.M;
+    const long long items = flat ? s.M * s.COg / 4 : static_cast<long long>(s.G) * rows_pad * pitch;
+    return CoefJob{go, y, rinv, gcp, s, pitch, rows_pad, q, fold, flat, gate,
+                   static_cast<int>(gated_blocks(blocks_for(items), gate))};
+}
+int launch_coef_gen(const CoefJob& job, cudaStream_t st) {
+    coef_gen_kernel<<<job.blocks, kBlock, 0, st>>>(job);
     LDN_LAUNCH_RET();
 }
 
@@ -552,11 +485,11 @@ int launch_row_absmax(Operand v, long long rows, int inner, int groups, long lon
     LDN_LAUNCH_RET();
 }
 
-int launch_side_reduce(const float* part, float* gw, long long count, int tiles, bool accumulate, const int* gate,
-                       bool run_if_nonzero, cudaStream_t st) {
-    side_reduce_kernel<<<gated_blocks(blocks_for(count), run_if_nonzero ? gate : nullptr), kBlock, 0, st>>>(
-        part, gw, count, tiles, accumulate, gate, run_if_nonzero);
-    LDN_LAUNCH_RET();
+SideJob side_reduce_job(const float* part, float* gw, long long count, int tiles, bool accumulate, const int* gate,
+                        bool run_if_nonzero) {
+    const bool vec = (count & 3) == 0 && ((reinterpret_cast<uintptr_t>(part) | reinterpret_cast<uintptr_t>(gw)) & 15u) == 0;
+    return SideJob{part, gw, count, tiles, accumulate, vec, gate, run_if_nonzero,
+                   static_cast<int>(gated_blocks(blocks_for(vec ? count / 4 : count), run_if_nonzero ? gate : nullptr))};
 }
 
 int launch_inf_scatter(const float* go, const int* pos, float* gx, float* gw, const Shape& s, cudaStream_t st) {

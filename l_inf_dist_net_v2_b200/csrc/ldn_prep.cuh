@@ -1,17 +1,8 @@
 // Memory-bound helper kernels: canonical operand copies, backward coefficients, p = inf scatters.
 #pragma once
-#include "ldn_common.cuh"
+#include "ldn_post.cuh"
 
 namespace ldn {
-
-struct Shape {
-    int B, CO, CI, G, HW;
-    int CIg, COg;
-    long long M;  // B * HW
-    // A range of output channels of a wider layer (G == 1 only): grad_output / output rows are co_src channels long and
-    // this problem's channel o is their channel co_off + o.  co_src == CO, co_off == 0: the whole layer.
-    int co_src, co_off;
-};
 
 // xc[g][m][pitch] <- x[((b G + g) CIg + c) HW + hw],  m = b HW + hw
 int launch_canon_x(const float* x, float* xc, const Shape& s, int pitch, cudaStream_t st);
@@ -24,12 +15,11 @@ int launch_canon_w(const float* w, float* wc, const Shape& s, int pitch, cudaStr
 // some y^-iq is outside the range in which that coefficient times |t|^iq is accurate (cleared by the caller before).
 int launch_coef_int(const float* go, const float* y, float* coef, const Shape& s, int pitch, int iq, int* flag,
                     cudaStream_t st);
-// general p: rinv[g][rows_pad][pitch] <- -q lg2 y (fold: the exponent offset of (|t| / y)^q) or 1 / y,
-// gcp[g][rows_pad][pitch] <- go; rows beyond M and columns beyond CO / G are padding (offset -1e30 resp. factor 0,
-// gradient factor 0)
-int launch_coef_gen(const float* go, const float* y, float* rinv, float* gcp, const Shape& s, int pitch,
-                    long long rows_pad, float q, bool fold, const int* gate,
-                    cudaStream_t st);  // gate (may be null): the kernel does nothing unless *gate != 0
+// general p: the coefficient job of ldn_post.cuh with its `flat` and `blocks` filled in, and the same as a launch of its
+// own.  rinv, gcp: [g][rows_pad][pitch]
+CoefJob coef_gen_job(const float* go, const float* y, float* rinv, float* gcp, const Shape& s, int pitch,
+                     long long rows_pad, float q, bool fold, const int* gate);
+int launch_coef_gen(const CoefJob& job, cudaStream_t st);
 
 // Second step of the forward kernels that save an index: `pos` holds, per output, the id of the 32-channel
 // stage in which the extremum was first reached (or -1); replace it by the channel index | flag.
@@ -47,10 +37,9 @@ int launch_rescan(int mode, Operand a0, Operand a1, Operand b, const float* y, i
 int launch_row_absmax(Operand v, long long rows, int inner, int groups, long long stride_k, float* out, int* clear,
                       cudaStream_t st);
 
-// grad_weight of the fused backward: gw[i] = -sum_t part[t * count + i], t < tiles
-// gate (may be null): the kernel runs only if (*gate != 0) == run_if_nonzero
-int launch_side_reduce(const float* part, float* gw, long long count, int tiles, bool accumulate, const int* gate,
-                       bool run_if_nonzero, cudaStream_t st);
+// grad_weight of the fused backward: the reduction job of ldn_post.cuh with its `blocks` filled in
+SideJob side_reduce_job(const float* part, float* gw, long long count, int tiles, bool accumulate, const int* gate,
+                        bool run_if_nonzero);
 
 // p = inf backward: gx[b, idx] += v, gw[o, idx] -= v with v = pos >= 0 ? go : -go.  gx / gw may be null.
 int launch_inf_scatter(const float* go, const int* pos, float* gx, float* gw, const Shape& s, cudaStream_t st);

@@ -17,7 +17,7 @@
 // operand its rows are t + 16 r (conflict-free with the swizzle), with a KMajor operand its columns
 // are 4 t .. 4 t + 3 and 64 + 4 t .. 64 + 4 t + 3 (conflict-free 128-bit reads).
 #pragma once
-#include "ldn_common.cuh"
+#include "ldn_post.cuh"
 
 namespace ldn {
 
@@ -138,6 +138,7 @@ tile_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ 
     constexpr int RN = Op::REG_N;          // output columns per thread
     constexpr int TN = 16 * RN;            // output columns per tile
     constexpr int TELEMS = kTileM * TN;    // outputs per tile
+    static_assert(kThreads == kPostBlock, "the jobs beside a fold run in its blocks");
     static_assert(RN == 8 || RN == 4 || RN == 2, "a thread owns 8, 4 or 2 output columns");
 
     extern __shared__ char smem_raw[];
@@ -518,6 +519,12 @@ tile_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ 
     }
 }
 
+// Jobs that share the fold's launch (see tile_fixup_kernel).
+struct PostJobs {
+    SideJob side;
+    CoefJob coef;
+};
+
 // Folds the partial accumulators of every tile that was shared between CTAs, in k order, and finalises it.  The CTAs that
 // share a tile are consecutive, and only the first of them can have begun in an earlier tile (its second slot then holds
 // this tile's partial).  A work item is J neighbouring register columns of register row i of every thread of a tile's CTA,
@@ -529,11 +536,13 @@ tile_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ 
 //          and the shared tiles are found from the boundaries between neighbouring CTAs' ranges (at most main_grid - 1,
 //          however many tiles there are): the first boundary inside a tile stands for it.
 // `rows` = register rows the main kernel computed and stored.
+// The first blocks run the jobs that follow the tile kernel beside the fold (ldn_post.cuh; fused backward only): they are
+// bound by memory, the longest first, and each saves a launch.
 // (8 outputs per thread, one partial in flight, 64-bit divisions per partial: 16.8 us for 8 tiles of 18.5 partials each,
 // 31 us for 4 tiles of 37, 18 us for 147 of 160 tiles shared by two or three.)
 template <class Op, bool MANY>
 __global__ void __launch_bounds__(kThreads)
-tile_fixup_kernel(const TileParams P, const int main_grid, const int rows) {
+tile_fixup_kernel(const TileParams P, const int main_grid, const int rows, const PostJobs jobs) {
     constexpr int NF = Op::NF;
     constexpr int NI = Op::NI;
     constexpr int NIA = NI > 0 ? NI : 1;
@@ -543,15 +552,26 @@ tile_fixup_kernel(const TileParams P, const int main_grid, const int rows) {
     constexpr int J = MANY ? 2 : RN;
     constexpr int kBatch = !MANY ? 2 : (NF + NI > 3 ? 4 : 8);
     constexpr size_t SLOT = static_cast<size_t>(NF + NI) * TELEMS;
+    if constexpr (Op::FUSED_W) {
+        if (static_cast<int>(blockIdx.x) < jobs.side.blocks) {
+            side_reduce_block(jobs.side, blockIdx.x, jobs.side.blocks);
+            return;
+        }
+        if (static_cast<int>(blockIdx.x) < jobs.side.blocks + jobs.coef.blocks) {
+            coef_gen_block(jobs.coef, blockIdx.x - jobs.side.blocks, jobs.coef.blocks);
+            return;
+        }
+    }
     if (P.gate != nullptr && (*P.gate != 0) == (P.gate_invert != 0)) return;
     const int tid = threadIdx.x;
     const int tn = thread_col<Op>(tid);
     const int tm = thread_row<Op>(tid);
+    const int first_block = jobs.side.blocks + jobs.coef.blocks;
     const int per_tile = rows * (RN / J);
     const int items = (MANY ? P.G * P.tiles_m * P.tiles_n : main_grid - 1) * per_tile;
     // the same index arithmetic in 32 bits wherever it fits (64-bit divisions took longer than the loads of an item)
     const bool narrow = P.total_iters * main_grid < 0x7fffffffLL;
-    for (int item = blockIdx.x; item < items; item += static_cast<int>(gridDim.x)) {
+    for (int item = static_cast<int>(blockIdx.x) - first_block; item < items; item += static_cast<int>(gridDim.x) - first_block) {
         const int unit = item / per_tile;  // MANY: the tile; else: the boundary behind the range of CTA `unit`
         const int part_of_tile = item - unit * per_tile;
         int c0, c1;   // the CTAs that share the tile
@@ -645,6 +665,7 @@ struct TileLaunch {
     CUtensorMap map_a0, map_a1, map_b;
     TileParams params;
     int grid;
+    PostJobs post;  // all zero: none
 };
 
 template <class Op>
@@ -677,18 +698,19 @@ int launch_tile(const TileLaunch& L, cudaStream_t stream) {
     if (e != cudaSuccess) return cuda_status(e);
     count_launches(1);
     const long long tiles = L.params.total_iters / L.params.kt;
+    const int rows = half ? kRegM / 2 : kRegM;
     // a tile can only be shared when the ranges do not fall on tile boundaries
-    if (L.params.total_iters % L.grid != 0 || (L.params.total_iters / L.grid) % L.params.kt != 0) {
-        const int rows = half ? kRegM / 2 : kRegM;
-        // up to two CTAs per tile: 147 shared tiles of 160 (512 x 3072 -> 5120, p = 8) take 14.0 us in the boundary form
-        // and 24.4 in the other; beyond, 8 tiles of 18.5 partials take 3.9 us in the tile form and 7.3 with the boundary
-        // form's items
-        const bool many = L.grid > 2 * tiles;
-        long long blocks = many ? tiles * rows * (Op::REG_N / 2) : static_cast<long long>(L.grid - 1) * rows;
-        if (L.params.gate && blocks > kGatedFixupCtas) blocks = kGatedFixupCtas;
+    const bool shared = L.params.total_iters % L.grid != 0 || (L.params.total_iters / L.grid) % L.params.kt != 0;
+    // up to two CTAs per tile: 147 shared tiles of 160 (512 x 3072 -> 5120, p = 8) take 14.0 us in the boundary form and
+    // 24.4 in the other; beyond, 8 tiles of 18.5 partials take 3.9 us in the tile form and 7.3 with the boundary form's items
+    const bool many = L.grid > 2 * tiles;
+    long long fold = shared ? (many ? tiles * rows * (Op::REG_N / 2) : static_cast<long long>(L.grid - 1) * rows) : 0;
+    if (L.params.gate && fold > kGatedFixupCtas) fold = kGatedFixupCtas;
+    const long long blocks = fold + L.post.side.blocks + L.post.coef.blocks;
+    if (blocks > 0) {
         const unsigned n = static_cast<unsigned>(blocks);
-        if (many) tile_fixup_kernel<Op, true><<<n, kThreads, 0, stream>>>(L.params, L.grid, rows);
-        else tile_fixup_kernel<Op, false><<<n, kThreads, 0, stream>>>(L.params, L.grid, rows);
+        if (many) tile_fixup_kernel<Op, true><<<n, kThreads, 0, stream>>>(L.params, L.grid, rows, L.post);
+        else tile_fixup_kernel<Op, false><<<n, kThreads, 0, stream>>>(L.params, L.grid, rows, L.post);
         e = cudaGetLastError();
         count_launches(1);
     }
