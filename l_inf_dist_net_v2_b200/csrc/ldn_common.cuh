@@ -146,6 +146,17 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
         : "memory");
 }
 
+// Start of every kernel that is launched with launch_after(): lets the next kernel of the stream be set up while this one
+// runs, and waits until everything in front of it on the stream is complete and visible.  Nothing may be read or written
+// before it, and every block executes it: a grid that was complete before its predecessor would let its successor run too
+// early.  (Pointers of these kernels carry no __restrict__: a load that is known not to change could be moved up across it.)
+// A launch behind another costs 1 us less: 200 x 1001 -> 777, p = 3, forward + input gradient (10 launches) 121 -> 107 us,
+// 128 x 64 x 16 x 16 convolution step at p = inf 400 -> 391, 512 x 3072 -> 5120 certification 1982 -> 1972.
+__device__ __forceinline__ void stream_order_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ unsigned long long global_timer_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -219,5 +230,25 @@ unsigned long long* trace_buffer();
 void count_launches(int n);
 
 inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? kOk : kCudaBase + static_cast<int>(e); }
+
+// Launches a kernel that begins with stream_order_begin(): its blocks may be placed on the SMs that the kernel in front of it
+// on the stream leaves, instead of after that kernel's end and a launch's latency.
+template <class... P, class... A>
+int launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e == cudaSuccess) count_launches(1);
+    else cudaGetLastError();
+    return cuda_status(e);
+}
 
 }  // namespace ldn

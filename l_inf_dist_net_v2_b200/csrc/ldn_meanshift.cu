@@ -13,8 +13,9 @@ constexpr int kRowLanes = 32;  // row groups per CTA (1024 threads: 8 of them to
 // x, out: [B][C] row-major.  Thread (lane = channel in the CTA's 32, rl = row group) sums rows rl, rl + 8, ...;
 // the 8 partial sums of a channel are folded in shared memory in a fixed order, so the result is deterministic.
 __global__ void __launch_bounds__(kCols * kRowLanes)
-mean_shift_rows_kernel(const float* __restrict__ x, float* __restrict__ out, float* __restrict__ running_mean,
-                       float* __restrict__ mean_out, float momentum, int B, int C) {
+mean_shift_rows_kernel(const float* x, float* out, float* running_mean,
+                       float* mean_out, float momentum, int B, int C) {
+    stream_order_begin();
     __shared__ float part[kRowLanes][kCols];
     const int lane = threadIdx.x & (kCols - 1);
     const int rl = threadIdx.x / kCols;
@@ -61,8 +62,6 @@ extern "C" LDN_API int ldn_mean_shift_rows(const float* x, int B, int C, float* 
     int r = get_device_ctx(&ctx);
     if (r != kOk) return r;
     const unsigned blocks = static_cast<unsigned>((C + kCols - 1) / kCols);
-    mean_shift_rows_kernel<<<blocks, kCols * kRowLanes, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        x, out, running_mean, mean_out, momentum, B, C);
-    count_launches(1);
-    return cuda_status(cudaGetLastError());
+    return launch_after(mean_shift_rows_kernel, blocks, kCols * kRowLanes, 0, reinterpret_cast<cudaStream_t>(stream),
+                        x, out, running_mean, mean_out, momentum, B, C);
 }

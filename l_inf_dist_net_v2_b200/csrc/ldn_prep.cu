@@ -17,7 +17,8 @@ inline unsigned blocks_for(long long n) {
     return static_cast<unsigned>(b);
 }
 
-__global__ void canon_x_kernel(const float* __restrict__ x, float* __restrict__ xc, Shape s, int pitch) {
+__global__ void canon_x_kernel(const float* x, float* xc, Shape s, int pitch) {
+    stream_order_begin();
     const long long total = static_cast<long long>(s.G) * s.M * s.CIg;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const CanonIdx q = canon_idx(i, s.CIg, s.M);
@@ -26,8 +27,9 @@ __global__ void canon_x_kernel(const float* __restrict__ x, float* __restrict__ 
     }
 }
 
-__global__ void canon_bounds_kernel(const float* __restrict__ xl, const float* __restrict__ xu, float* __restrict__ lc,
-                                    float* __restrict__ uc, Shape s, int pitch) {
+__global__ void canon_bounds_kernel(const float* xl, const float* xu, float* lc,
+                                    float* uc, Shape s, int pitch) {
+    stream_order_begin();
     const long long total = static_cast<long long>(s.G) * s.M * s.CIg;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const CanonIdx q = canon_idx(i, s.CIg, s.M);
@@ -44,8 +46,9 @@ __global__ void canon_bounds_kernel(const float* __restrict__ xl, const float* _
 // HW > 1: tiled transpose through shared memory.  Source rows (b, g, c, :) are contiguous in hw, destination
 // rows (g, m = b HW + hw, :) are contiguous in c; a 32 x 32 tile makes both sides coalesced.  grid = (ceil(HW/32),
 // ceil(CIg/32), B*G).  With `second` non-null the pair (x, second) is treated as interval bounds and sanitised.
-__global__ void canon_transpose_kernel(const float* __restrict__ x, const float* __restrict__ second,
-                                       float* __restrict__ xc, float* __restrict__ sc, Shape s, int pitch) {
+__global__ void canon_transpose_kernel(const float* x, const float* second,
+                                       float* xc, float* sc, Shape s, int pitch) {
+    stream_order_begin();
     __shared__ float t0[32][33], t1[32][33];
     const int bg = blockIdx.z, b = bg / s.G, g = bg % s.G;
     const int hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -74,7 +77,8 @@ __global__ void canon_transpose_kernel(const float* __restrict__ x, const float*
     }
 }
 
-__global__ void canon_w_kernel(const float* __restrict__ w, float* __restrict__ wc, Shape s, int pitch) {
+__global__ void canon_w_kernel(const float* w, float* wc, Shape s, int pitch) {
+    stream_order_begin();
     const long long total = static_cast<long long>(s.CO) * s.CIg;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long row = i / s.CIg;
@@ -89,8 +93,9 @@ __global__ void canon_w_kernel(const float* __restrict__ w, float* __restrict__ 
 constexpr float kRqMin = 1e-30f, kRqMax = 1e24f;
 __device__ __forceinline__ bool rq_unsafe(float rq) { return !(rq >= kRqMin && rq <= kRqMax); }
 
-__global__ void coef_int_kernel(const float* __restrict__ go, const float* __restrict__ y, float* __restrict__ coef,
+__global__ void coef_int_kernel(const float* go, const float* y, float* coef,
                                 Shape s, int pitch, int iq, int* flag) {
+    stream_order_begin();
     const long long total = static_cast<long long>(s.G) * s.M * s.COg;
     bool bad = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -106,8 +111,9 @@ __global__ void coef_int_kernel(const float* __restrict__ go, const float* __res
 }
 
 // flat fast paths (HW == 1, G == 1, pitch == COg: source and destination have the same element order)
-__global__ void coef_int_flat_kernel(const float4* __restrict__ go, const float4* __restrict__ y,
-                                     float4* __restrict__ coef, long long n4, int iq, int* flag) {
+__global__ void coef_int_flat_kernel(const float4* go, const float4* y,
+                                     float4* coef, long long n4, int iq, int* flag) {
+    stream_order_begin();
     bool bad = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
         const float4 yv = y[i];
@@ -122,7 +128,10 @@ __global__ void coef_int_flat_kernel(const float4* __restrict__ go, const float4
     }
     if (flag && bad) *flag = 1;
 }
-__global__ void __launch_bounds__(kBlock) coef_gen_kernel(const CoefJob job) { coef_gen_block(job, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(kBlock) coef_gen_kernel(const CoefJob job) {
+    stream_order_begin();
+    coef_gen_block(job, blockIdx.x, gridDim.x);
+}
 
 // Four lanes per output element, kRescanIlp outputs per lane group in flight: lane q of a group loads the 16-byte pieces q
 // and q + 4 of the recorded 32-channel stage of each operand row (one full 128-byte line per output and operand: operand
@@ -136,8 +145,9 @@ __global__ void __launch_bounds__(kBlock) coef_gen_kernel(const CoefJob job) { c
 // arithmetic per output is one division by HW (none for fully connected layers) and, for those, a block keeps rereading
 // one input row, which stays in the L1 cache: only the weight pieces come from L2.
 template <int mode>
-__global__ void __launch_bounds__(kBlock) rescan_kernel(Operand a0, Operand a1, Operand b, const float* __restrict__ y,
-                                                        int* __restrict__ pos, Shape s, long long a_stride_k) {
+__global__ void __launch_bounds__(kBlock) rescan_kernel(Operand a0, Operand a1, Operand b, const float* y,
+                                                        int* pos, Shape s, long long a_stride_k) {
+    stream_order_begin();
     constexpr int U = kRescanIlp;
     const int kpad = (s.CIg + 3) & ~3;
     const int q = threadIdx.x & 3;
@@ -228,8 +238,9 @@ __global__ void __launch_bounds__(kBlock) rescan_kernel(Operand a0, Operand a1, 
 // positions of 32 / P outputs, so y / pos are read and written coalesced and the shared-memory reads are
 // conflict-free whatever the lanes' stages.  The weight pieces (one 128-byte run per output and stage) come from L1 / L2.
 template <int P>
-__global__ void __launch_bounds__(kBlock) rescan_inplace_kernel(Operand a0, Operand b, const float* __restrict__ y,
-                                                                int* __restrict__ pos, Shape s) {
+__global__ void __launch_bounds__(kBlock) rescan_inplace_kernel(Operand a0, Operand b, const float* y,
+                                                                int* pos, Shape s) {
+    stream_order_begin();
     extern __shared__ float4 xs4[];
     float* xs = reinterpret_cast<float*>(xs4);  // [CI/G][P]
     constexpr int V = P / 4;
@@ -298,14 +309,13 @@ int launch_rescan_inplace(Operand a0, Operand b, const float* y, int* pos, const
         if (dev < 64) configured[dev] = true;
     }
     const dim3 grid(static_cast<unsigned>(static_cast<long long>(s.B) * s.G), static_cast<unsigned>((s.HW + P - 1) / P));
-    rescan_inplace_kernel<P><<<grid, kBlock, smem, st>>>(a0, b, y, pos, s);
-    count_launches(1);
-    return cuda_status(cudaGetLastError());
+    return launch_after(rescan_inplace_kernel<P>, grid, kBlock, smem, st, a0, b, y, pos, s);
 }
 
 // out[g * rows + r] = max_k |v[g][r][k]|.  Contiguous k: one warp per row; k `stride_k` apart with neighbouring rows
 // contiguous (inputs read in place): one thread per row.  clear (may be null): a flag word the first thread resets.
-__global__ void row_absmax_kernel(Operand v, long long rows, int inner, int groups, float* __restrict__ out, int* clear) {
+__global__ void row_absmax_kernel(Operand v, long long rows, int inner, int groups, float* out, int* clear) {
+    stream_order_begin();
     if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
     const int lane = threadIdx.x & 31;
     const long long warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
@@ -321,7 +331,8 @@ __global__ void row_absmax_kernel(Operand v, long long rows, int inner, int grou
     }
 }
 __global__ void row_absmax_strided_kernel(Operand v, long long rows, int inner, int groups, long long stride_k,
-                                          float* __restrict__ out, int* clear) {
+                                          float* out, int* clear) {
+    stream_order_begin();
     if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
     const long long total = rows * groups;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -334,8 +345,9 @@ __global__ void row_absmax_strided_kernel(Operand v, long long rows, int inner, 
 }
 
 // One thread per output element, in output-layout order (coalesced reads of go / pos).
-__global__ void inf_scatter_kernel(const float* __restrict__ go, const int* __restrict__ pos, float* gx, float* gw,
+__global__ void inf_scatter_kernel(const float* go, const int* pos, float* gx, float* gw,
                                    Shape s) {
+    stream_order_begin();
     const long long total = static_cast<long long>(s.B) * s.CO * s.HW;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int hw = static_cast<int>(i % s.HW);
@@ -352,9 +364,10 @@ __global__ void inf_scatter_kernel(const float* __restrict__ go, const int* __re
     }
 }
 
-__global__ void bound_scatter_kernel(const float* __restrict__ gol, const float* __restrict__ gou,
-                                     const int* __restrict__ posl, const int* __restrict__ posu, float* gxl, float* gxu,
+__global__ void bound_scatter_kernel(const float* gol, const float* gou,
+                                     const int* posl, const int* posu, float* gxl, float* gxu,
                                      float* gw, Shape s) {
+    stream_order_begin();
     const long long total = static_cast<long long>(s.B) * s.CO * s.HW;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int hw = static_cast<int>(i % s.HW);
@@ -381,11 +394,7 @@ __global__ void bound_scatter_kernel(const float* __restrict__ gol, const float*
 }
 }  // namespace
 
-#define LDN_LAUNCH_RET() \
-    do {                  \
-        count_launches(1); \
-        return cuda_status(cudaGetLastError()); \
-    } while (0)
+
 
 static bool transpose_grid(const Shape& s, dim3* grid) {
     const long long bg = static_cast<long long>(s.B) * s.G;
@@ -397,25 +406,21 @@ static bool transpose_grid(const Shape& s, dim3* grid) {
 int launch_canon_x(const float* x, float* xc, const Shape& s, int pitch, cudaStream_t st) {
     dim3 grid;
     if (transpose_grid(s, &grid)) {
-        canon_transpose_kernel<<<grid, dim3(32, 8), 0, st>>>(x, nullptr, xc, nullptr, s, pitch);
-        LDN_LAUNCH_RET();
+        return launch_after(canon_transpose_kernel, grid, dim3(32, 8), 0, st, x, nullptr, xc, nullptr, s, pitch);
     }
-    canon_x_kernel<<<blocks_for((long long)s.G * s.M * s.CIg), kBlock, 0, st>>>(x, xc, s, pitch);
-    LDN_LAUNCH_RET();
+    return launch_after(canon_x_kernel, blocks_for((long long)s.G * s.M * s.CIg), kBlock, 0, st, x, xc, s, pitch);
 }
 int launch_canon_bounds(const float* xl, const float* xu, float* lc, float* uc, const Shape& s, int pitch,
                         cudaStream_t st) {
     dim3 grid;
     if (transpose_grid(s, &grid)) {
-        canon_transpose_kernel<<<grid, dim3(32, 8), 0, st>>>(xl, xu, lc, uc, s, pitch);
-        LDN_LAUNCH_RET();
+        return launch_after(canon_transpose_kernel, grid, dim3(32, 8), 0, st, xl, xu, lc, uc, s, pitch);
     }
-    canon_bounds_kernel<<<blocks_for((long long)s.G * s.M * s.CIg), kBlock, 0, st>>>(xl, xu, lc, uc, s, pitch);
-    LDN_LAUNCH_RET();
+    return launch_after(canon_bounds_kernel, blocks_for((long long)s.G * s.M * s.CIg), kBlock, 0, st, xl, xu, lc, uc,
+                        s, pitch);
 }
 int launch_canon_w(const float* w, float* wc, const Shape& s, int pitch, cudaStream_t st) {
-    canon_w_kernel<<<blocks_for((long long)s.CO * s.CIg), kBlock, 0, st>>>(w, wc, s, pitch);
-    LDN_LAUNCH_RET();
+    return launch_after(canon_w_kernel, blocks_for((long long)s.CO * s.CIg), kBlock, 0, st, w, wc, s, pitch);
 }
 static bool flat_ok(const Shape& s, int pitch, const void* a, const void* b) {
     return s.HW == 1 && s.G == 1 && s.co_src == s.CO && pitch == s.COg && (s.COg & 3) == 0 &&
@@ -426,13 +431,11 @@ int launch_coef_int(const float* go, const float* y, float* coef, const Shape& s
                     cudaStream_t st) {
     if (flat_ok(s, pitch, go, y)) {
         const long long n4 = static_cast<long long>(s.M) * s.COg / 4;
-        coef_int_flat_kernel<<<blocks_for(n4), kBlock, 0, st>>>(reinterpret_cast<const float4*>(go),
-                                                              reinterpret_cast<const float4*>(y),
-                                                              reinterpret_cast<float4*>(coef), n4, iq, flag);
-        LDN_LAUNCH_RET();
+        return launch_after(coef_int_flat_kernel, blocks_for(n4), kBlock, 0, st, reinterpret_cast<const float4*>(go),
+                            reinterpret_cast<const float4*>(y), reinterpret_cast<float4*>(coef), n4, iq, flag);
     }
-    coef_int_kernel<<<blocks_for((long long)s.G * s.M * s.COg), kBlock, 0, st>>>(go, y, coef, s, pitch, iq, flag);
-    LDN_LAUNCH_RET();
+    return launch_after(coef_int_kernel, blocks_for((long long)s.G * s.M * s.COg), kBlock, 0, st, go, y, coef, s,
+                        pitch, iq, flag);
 }
 CoefJob coef_gen_job(const float* go, const float* y, float* rinv, float* gcp, const Shape& s, int pitch,
                      long long rows_pad, float q, bool fold, const int* gate) {
@@ -442,8 +445,7 @@ CoefJob coef_gen_job(const float* go, const float* y, float* rinv, float* gcp, c
                    static_cast<int>(gated_blocks(blocks_for(items), gate))};
 }
 int launch_coef_gen(const CoefJob& job, cudaStream_t st) {
-    coef_gen_kernel<<<job.blocks, kBlock, 0, st>>>(job);
-    LDN_LAUNCH_RET();
+    return launch_after(coef_gen_kernel, job.blocks, kBlock, 0, st, job);
 }
 
 int launch_rescan(int mode, Operand a0, Operand a1, Operand b, const float* y, int* pos, const Shape& s,
@@ -469,20 +471,18 @@ int launch_rescan(int mode, Operand a0, Operand a1, Operand b, const float* y, i
     if (chunks > most) chunks = most;  // the kernel strides over the rest
     if (chunks > 65535) chunks = 65535;
     const dim3 grid(static_cast<unsigned>(bg), static_cast<unsigned>(chunks));
-    if (mode == 0) rescan_kernel<0><<<grid, kBlock, 0, st>>>(a0, a1, b, y, pos, s, a_stride_k);
-    else if (mode == 1) rescan_kernel<1><<<grid, kBlock, 0, st>>>(a0, a1, b, y, pos, s, a_stride_k);
-    else rescan_kernel<2><<<grid, kBlock, 0, st>>>(a0, a1, b, y, pos, s, a_stride_k);
-    LDN_LAUNCH_RET();
+    if (mode == 0) return launch_after(rescan_kernel<0>, grid, kBlock, 0, st, a0, a1, b, y, pos, s, a_stride_k);
+    if (mode == 1) return launch_after(rescan_kernel<1>, grid, kBlock, 0, st, a0, a1, b, y, pos, s, a_stride_k);
+    return launch_after(rescan_kernel<2>, grid, kBlock, 0, st, a0, a1, b, y, pos, s, a_stride_k);
 }
 
 int launch_row_absmax(Operand v, long long rows, int inner, int groups, long long stride_k, float* out, int* clear,
                       cudaStream_t st) {
     if (stride_k == 1)
-        row_absmax_kernel<<<blocks_for(rows * groups * 32), kBlock, 0, st>>>(v, rows, inner, groups, out, clear);
-    else
-        row_absmax_strided_kernel<<<blocks_for(rows * groups), kBlock, 0, st>>>(v, rows, inner, groups, stride_k, out,
-                                                                               clear);
-    LDN_LAUNCH_RET();
+        return launch_after(row_absmax_kernel, blocks_for(rows * groups * 32), kBlock, 0, st, v, rows, inner, groups, out,
+                            clear);
+    return launch_after(row_absmax_strided_kernel, blocks_for(rows * groups), kBlock, 0, st, v, rows, inner, groups,
+                        stride_k, out, clear);
 }
 
 SideJob side_reduce_job(const float* part, float* gw, long long count, int tiles, bool accumulate, const int* gate,
@@ -497,8 +497,7 @@ int launch_inf_scatter(const float* go, const int* pos, float* gx, float* gw, co
     if (gx) e = cudaMemsetAsync(gx, 0, sizeof(float) * (size_t)s.B * s.CI * s.HW, st);
     if (e == cudaSuccess && gw) e = cudaMemsetAsync(gw, 0, sizeof(float) * (size_t)s.CO * s.CIg, st);
     if (e != cudaSuccess) return cuda_status(e);
-    inf_scatter_kernel<<<blocks_for((long long)s.B * s.CO * s.HW), kBlock, 0, st>>>(go, pos, gx, gw, s);
-    LDN_LAUNCH_RET();
+    return launch_after(inf_scatter_kernel, blocks_for((long long)s.B * s.CO * s.HW), kBlock, 0, st, go, pos, gx, gw, s);
 }
 
 int launch_bound_scatter(const float* gol, const float* gou, const int* posl, const int* posu, float* gxl, float* gxu,
@@ -507,9 +506,8 @@ int launch_bound_scatter(const float* gol, const float* gou, const int* posl, co
     if (e == cudaSuccess) e = cudaMemsetAsync(gxu, 0, sizeof(float) * (size_t)s.B * s.CI * s.HW, st);
     if (e == cudaSuccess && gw) e = cudaMemsetAsync(gw, 0, sizeof(float) * (size_t)s.CO * s.CIg, st);
     if (e != cudaSuccess) return cuda_status(e);
-    bound_scatter_kernel<<<blocks_for((long long)s.B * s.CO * s.HW), kBlock, 0, st>>>(gol, gou, posl, posu, gxl, gxu,
-                                                                                     gw, s);
-    LDN_LAUNCH_RET();
+    return launch_after(bound_scatter_kernel, blocks_for((long long)s.B * s.CO * s.HW), kBlock, 0, st, gol, gou, posl,
+                        posu, gxl, gxu, gw, s);
 }
 
 }  // namespace ldn

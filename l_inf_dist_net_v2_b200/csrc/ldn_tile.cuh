@@ -147,6 +147,7 @@ tile_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ 
     int* ints = reinterpret_cast<int*>(smem + STAGES * STAGE + TileSmem<Op>::kSide);  // N_IN_SMEM ops
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE + TileSmem<Op>::kSide + TileSmem<Op>::kInts);
 
+    stream_order_begin();
     if (P.gate != nullptr && (*P.gate != 0) == (P.gate_invert != 0)) return;
     const int tid = threadIdx.x;
     const int tn = thread_col<Op>(tid);
@@ -552,6 +553,7 @@ tile_fixup_kernel(const TileParams P, const int main_grid, const int rows, const
     constexpr int J = MANY ? 2 : RN;
     constexpr int kBatch = !MANY ? 2 : (NF + NI > 3 ? 4 : 8);
     constexpr size_t SLOT = static_cast<size_t>(NF + NI) * TELEMS;
+    stream_order_begin();
     if constexpr (Op::FUSED_W) {
         if (static_cast<int>(blockIdx.x) < jobs.side.blocks) {
             side_reduce_block(jobs.side, blockIdx.x, jobs.side.blocks);
@@ -688,15 +690,14 @@ int launch_tile(const TileLaunch& L, cudaStream_t stream) {
     const bool timed = L.params.gate == nullptr;
     if (timed) timing_before(stream);
     const bool half = HALF && L.params.M <= kTileM / 2;
+    int r;
     if (half)
-        tile_kernel<Op, (HALF ? kRegM / 2 : kRegM)><<<L.grid, kThreads, SMEM, stream>>>(L.map_a0, L.map_a1, L.map_b,
-                                                                                      L.params);
+        r = launch_after(tile_kernel<Op, (HALF ? kRegM / 2 : kRegM)>, L.grid, kThreads, SMEM, stream, L.map_a0, L.map_a1,
+                         L.map_b, L.params);
     else
-        tile_kernel<Op><<<L.grid, kThreads, SMEM, stream>>>(L.map_a0, L.map_a1, L.map_b, L.params);
+        r = launch_after(tile_kernel<Op>, L.grid, kThreads, SMEM, stream, L.map_a0, L.map_a1, L.map_b, L.params);
     if (timed) timing_after(stream);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_status(e);
-    count_launches(1);
+    if (r != kOk) return r;
     const long long tiles = L.params.total_iters / L.params.kt;
     const int rows = half ? kRegM / 2 : kRegM;
     // a tile can only be shared when the ranges do not fall on tile boundaries
@@ -709,12 +710,10 @@ int launch_tile(const TileLaunch& L, cudaStream_t stream) {
     const long long blocks = fold + L.post.side.blocks + L.post.coef.blocks;
     if (blocks > 0) {
         const unsigned n = static_cast<unsigned>(blocks);
-        if (many) tile_fixup_kernel<Op, true><<<n, kThreads, 0, stream>>>(L.params, L.grid, rows, L.post);
-        else tile_fixup_kernel<Op, false><<<n, kThreads, 0, stream>>>(L.params, L.grid, rows, L.post);
-        e = cudaGetLastError();
-        count_launches(1);
+        return many ? launch_after(tile_fixup_kernel<Op, true>, n, kThreads, 0, stream, L.params, L.grid, rows, L.post)
+                    : launch_after(tile_fixup_kernel<Op, false>, n, kThreads, 0, stream, L.params, L.grid, rows, L.post);
     }
-    return cuda_status(e);
+    return kOk;
 }
 
 }  // namespace ldn

@@ -40,8 +40,9 @@ struct Patches {
 
 // Thread = V neighbouring positions of one row of `cols`; blockIdx.y splits the planes so that every index fits 31 bits.
 template <int V>
-__global__ void __launch_bounds__(kBlock) unfold_kernel(const float* __restrict__ x, float* __restrict__ cols, Patches P,
+__global__ void __launch_bounds__(kBlock) unfold_kernel(const float* x, float* cols, Patches P,
                                                         long long planes, unsigned planes_per_slice) {
+    stream_order_begin();
     const long long plane0 = static_cast<long long>(blockIdx.y) * planes_per_slice;
     const unsigned here = static_cast<unsigned>(planes - plane0 < planes_per_slice ? planes - plane0 : planes_per_slice);
     const unsigned n = here * P.by_khkw.d * P.by_row.d;
@@ -74,8 +75,9 @@ __global__ void __launch_bounds__(kBlock) unfold_kernel(const float* __restrict_
 }
 
 // Thread = one pixel of one plane (b, c).
-__global__ void __launch_bounds__(kBlock) fold_kernel(const float* __restrict__ cols, float* __restrict__ x, Patches P,
+__global__ void __launch_bounds__(kBlock) fold_kernel(const float* cols, float* x, Patches P,
                                                       long long planes, unsigned planes_per_slice) {
+    stream_order_begin();
     const long long plane0 = static_cast<long long>(blockIdx.y) * planes_per_slice;
     const unsigned n =
         static_cast<unsigned>(planes - plane0 < planes_per_slice ? planes - plane0 : planes_per_slice) * P.by_row.d;
@@ -160,10 +162,8 @@ LDN_API int ldn_unfold(const float* x, int B, int C, int H, int W, int kh, int k
     if ((r = slice(planes, P.by_khkw.d * P.by_row.d, &s)) != kOk) return r;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const dim3 grid(s.blocks, s.count);
-    if (vec) unfold_kernel<4><<<grid, kBlock, 0, st>>>(x, cols, P, planes, s.per_slice);
-    else unfold_kernel<1><<<grid, kBlock, 0, st>>>(x, cols, P, planes, s.per_slice);
-    count_launches(1);
-    return cuda_status(cudaGetLastError());
+    if (vec) return launch_after(unfold_kernel<4>, grid, kBlock, 0, st, x, cols, P, planes, s.per_slice);
+    return launch_after(unfold_kernel<1>, grid, kBlock, 0, st, x, cols, P, planes, s.per_slice);
 }
 
 LDN_API int ldn_fold(const float* cols, int B, int C, int H, int W, int kh, int kw, int stride, int pad, int dil, float* x,
@@ -177,10 +177,8 @@ LDN_API int ldn_fold(const float* cols, int B, int C, int H, int W, int kh, int 
     const long long planes = static_cast<long long>(B) * C;
     Slices s;
     if ((r = slice(planes, P.by_row.d, &s)) != kOk) return r;
-    fold_kernel<<<dim3(s.blocks, s.count), kBlock, 0, reinterpret_cast<cudaStream_t>(stream)>>>(cols, x, P, planes,
-                                                                                              s.per_slice);
-    count_launches(1);
-    return cuda_status(cudaGetLastError());
+    return launch_after(fold_kernel, dim3(s.blocks, s.count), kBlock, 0, reinterpret_cast<cudaStream_t>(stream), cols,
+                        x, P, planes, s.per_slice);
 }
 
 }  // extern "C"
