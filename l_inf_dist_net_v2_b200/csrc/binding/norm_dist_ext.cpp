@@ -5,7 +5,10 @@
 // current stream of the tensors' device (with a device guard) and a non-zero status raises.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
+
+#include <cmath>
 
 #include "ldn_b200.h"
 
@@ -175,6 +178,200 @@ void fold(Tensor& cols, Tensor& x, std::pair<int, int> kernel, int stride, int p
           "fold");
 }
 
+// ---- the operators as autograd functions ---------------------------------------------------------------------------
+//
+// The Python autograd functions (norm_dist.py, modules.py) restated in C++: the same steps in the same order.  A forward and
+// backward pass of a Python autograd function costs 55 us on the host before it does anything (the engine's thread takes
+// the interpreter lock and runs the Python backward), more than the kernels of a small layer; here it is 25 us.  The
+// entry points return None for whatever the Python functions should see instead (other devices, types and layouts, shapes
+// that do not fit): those raise or handle it.
+
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+bool plain(const Tensor& t, int64_t dim) {
+    return t.is_cuda() && t.scalar_type() == at::kFloat && t.layout() == at::kStrided && t.dim() == dim && t.is_contiguous() &&
+           t.numel() > 0;
+}
+bool fits(const Tensor& x, const Tensor& w, int64_t G) {
+    return plain(x, 3) && plain(w, 2) && x.device() == w.device() && G > 0 && G <= w.size(0) && w.size(1) * G == x.size(1);
+}
+Tensor output_of(const Tensor& x, const Tensor& w) { return at::empty({x.size(0), w.size(0), x.size(2)}, x.options()); }
+
+struct NormDistFn : public torch::autograd::Function<NormDistFn> {
+    static Tensor forward(AutogradContext* ctx, Tensor x, Tensor w, int64_t G, double p, bool need_grad) {
+        Tensor y = output_of(x, w);
+        ctx->saved_data["G"] = G;
+        ctx->saved_data["p"] = p;
+        const int g = static_cast<int>(G);
+        if (std::isinf(p)) {
+            if (!need_grad) {
+                inf_dist_forward_nograd(x, w, y, g);
+            } else {
+                Tensor pos = at::empty(y.sizes(), y.options().dtype(at::kInt));
+                inf_dist_forward(x, w, y, pos, g);
+                ctx->save_for_backward({x, w, pos});
+            }
+        } else {
+            norm_dist_forward(x, w, y, g, static_cast<float>(p));
+            ctx->save_for_backward({x, w, y});
+        }
+        return y;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        Tensor go = grads[0].contiguous();
+        const int g = static_cast<int>(ctx->saved_data["G"].toInt());
+        const double p = ctx->saved_data["p"].toDouble();
+        const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+        variable_list saved = ctx->get_saved_variables();
+        Tensor &x = saved[0], &w = saved[1], &third = saved[2];
+        Tensor gx, gw;
+        c10::optional<Tensor> maybe_gx;
+        if (need_x) maybe_gx = gx = at::empty_like(x);
+        if (need_w) {
+            gw = at::empty_like(w);
+            if (std::isinf(p)) inf_dist_backward_input_weight(go, third, maybe_gx, gw, g);
+            else norm_dist_backward_input_weight(go, x, w, third, maybe_gx, gw, g, static_cast<float>(p));
+        } else if (need_x) {
+            if (std::isinf(p)) inf_dist_backward_input(go, third, gx, g);
+            else norm_dist_backward_input(go, x, w, third, gx, g, static_cast<float>(p));
+        }
+        return {gx, gw, Tensor(), Tensor(), Tensor()};
+    }
+};
+
+struct BoundInfDistFn : public torch::autograd::Function<BoundInfDistFn> {
+    static variable_list forward(AutogradContext* ctx, Tensor xl, Tensor xu, Tensor w, int64_t G, bool need_grad) {
+        Tensor yl = output_of(xl, w), yu = at::empty_like(yl);
+        ctx->saved_data["G"] = G;
+        const int g = static_cast<int>(G);
+        if (!need_grad) {
+            bound_inf_dist_forward_nograd(xl, xu, w, yl, yu, g);
+        } else {
+            Tensor pl = at::empty(yl.sizes(), yl.options().dtype(at::kInt)), pu = at::empty_like(pl);
+            bound_inf_dist_forward(xl, xu, w, yl, yu, pl, pu, g);
+            ctx->save_for_backward({xl, xu, w, pl, pu});
+        }
+        return {yl, yu};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        Tensor gl = grads[0].contiguous(), gu = grads[1].contiguous();
+        const int g = static_cast<int>(ctx->saved_data["G"].toInt());
+        variable_list saved = ctx->get_saved_variables();
+        Tensor &xl = saved[0], &xu = saved[1], &w = saved[2], &pl = saved[3], &pu = saved[4];
+        const bool need_l = ctx->needs_input_grad(0), need_u = ctx->needs_input_grad(1), need_w = ctx->needs_input_grad(2);
+        Tensor gxl, gxu, gw;
+        if (need_w || (need_l && need_u)) {
+            gxl = at::empty_like(xl);
+            gxu = at::empty_like(xu);
+            if (need_w) {
+                gw = at::empty_like(w);
+                bound_inf_dist_backward_input_weight(gl, gu, pl, pu, gxl, gxu, gw, g);
+            } else {
+                bound_inf_dist_backward_input(gl, gu, pl, pu, gxl, gxu, g);
+            }
+        } else {
+            gxl = at::zeros_like(xl);
+            gxu = at::zeros_like(xu);
+        }
+        return {need_l ? gxl : Tensor(), need_u ? gxu : Tensor(), gw, Tensor(), Tensor()};
+    }
+};
+
+// x - mean over the batch; running_mean may be undefined
+void mean_shift_rows(const Tensor& x, const Tensor& running_mean, double momentum, Tensor& out) {
+    const float* a = fptr(x, "x");
+    float* rm = running_mean.defined() ? const_cast<float*>(fptr(running_mean, "running_mean")) : nullptr;
+    float* y = fptr_mut(out, "out");
+    const c10::cuda::CUDAGuard guard(x.device());
+    const int64_t B = x.size(0);
+    check(ldn_mean_shift_rows(a, B, x.numel() / std::max<int64_t>(B, 1), rm, static_cast<float>(momentum), y, nullptr,
+                              stream()),
+          "mean_shift_rows");
+}
+
+struct MeanShiftRowsFn : public torch::autograd::Function<MeanShiftRowsFn> {
+    static Tensor forward(AutogradContext*, Tensor x, Tensor running_mean, double momentum) {
+        Tensor out = at::empty_like(x);
+        mean_shift_rows(x, running_mean, momentum, out);
+        return out;
+    }
+    static variable_list backward(AutogradContext*, variable_list grads) {
+        Tensor go = grads[0].contiguous(), gx = at::empty_like(go);
+        mean_shift_rows(go, Tensor(), 0.0, gx);
+        return {gx, Tensor(), Tensor()};
+    }
+};
+
+struct UnfoldFn : public torch::autograd::Function<UnfoldFn> {
+    static Tensor forward(AutogradContext* ctx, Tensor x, int64_t positions, int64_t kh, int64_t kw, int64_t stride,
+                          int64_t padding, int64_t dilation) {
+        ctx->saved_data["image"] = x.sizes().vec();
+        ctx->saved_data["geometry"] = std::vector<int64_t>{kh, kw, stride, padding, dilation};
+        Tensor cols = at::empty({x.size(0), x.size(1) * kh * kw, positions}, x.options());
+        unfold(x, cols, {static_cast<int>(kh), static_cast<int>(kw)}, static_cast<int>(stride), static_cast<int>(padding),
+               static_cast<int>(dilation));
+        return cols;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        Tensor go = grads[0].contiguous();
+        const std::vector<int64_t> n = ctx->saved_data["geometry"].toIntVector();
+        Tensor gx = at::empty(ctx->saved_data["image"].toIntVector(), go.options());
+        fold(go, gx, {static_cast<int>(n[0]), static_cast<int>(n[1])}, static_cast<int>(n[2]), static_cast<int>(n[3]),
+             static_cast<int>(n[4]));
+        return {gx, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+c10::optional<Tensor> norm_dist(const Tensor& x, const Tensor& w, double p, int64_t G) {
+    if (!fits(x, w, G) || !(p > 0.0) || torch::jit::tracer::isTracing()) return c10::nullopt;
+    const bool need_grad = at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad());
+    return NormDistFn::apply(x, w, G, p, need_grad);
+}
+
+c10::optional<std::tuple<Tensor, Tensor>> bound_inf_dist(const Tensor& xl, const Tensor& xu, const Tensor& w, int64_t G) {
+    if (!fits(xl, w, G) || !fits(xu, w, G) || xl.sizes() != xu.sizes() || torch::jit::tracer::isTracing()) return c10::nullopt;
+    const bool need_grad = at::GradMode::is_enabled() && (xl.requires_grad() || xu.requires_grad() || w.requires_grad());
+    variable_list y = BoundInfDistFn::apply(xl, xu, w, G, need_grad);
+    return std::make_tuple(y[0], y[1]);
+}
+
+c10::optional<Tensor> mean_shift(const Tensor& x, const Tensor& running_mean, double momentum) {
+    if (!plain(x, 3) || !plain(running_mean, 1) || x.device() != running_mean.device() || running_mean.requires_grad() ||
+        running_mean.size(0) != x.size(1) || x.size(2) != 1 || torch::jit::tracer::isTracing())
+        return c10::nullopt;
+    return MeanShiftRowsFn::apply(x, running_mean, momentum);
+}
+
+c10::optional<Tensor> unfold_columns(const Tensor& x, int64_t positions, std::pair<int64_t, int64_t> kernel, int64_t stride,
+                                     int64_t padding, int64_t dilation) {
+    if (!plain(x, 4) || torch::jit::tracer::isTracing()) return c10::nullopt;
+    return UnfoldFn::apply(x, positions, kernel.first, kernel.second, stride, padding, dilation);
+}
+
+// eval-mode layers (not part of the reference's extension module): (y - sub[o]) + add[o] applied in the store
+void inf_dist_forward_nograd_shifted(Tensor& input, Tensor& weight, Tensor& output, c10::optional<Tensor> sub,
+                                     c10::optional<Tensor> add, int G) {
+    const float *x = fptr(input, "input"), *w = fptr(weight, "weight");
+    float* y = fptr_mut(output, "output");
+    const float *s = opt_fptr(sub, "sub"), *a = opt_fptr(add, "add");
+    const c10::cuda::CUDAGuard guard(input.device());
+    check(ldn_inf_dist_forward_nograd_shifted(x, w, input.size(0), output.size(1), input.size(1), G, input.size(2), y, s, a,
+                                              stream()),
+          "inf_dist_forward_nograd_shifted");
+}
+
+void bound_inf_dist_forward_nograd_shifted(Tensor& inputL, Tensor& inputU, Tensor& weight, Tensor& outputL, Tensor& outputU,
+                                           c10::optional<Tensor> sub, c10::optional<Tensor> add, int G) {
+    const float *xl = fptr(inputL, "inputL"), *xu = fptr(inputU, "inputU"), *w = fptr(weight, "weight");
+    float *yl = fptr_mut(outputL, "outputL"), *yu = fptr_mut(outputU, "outputU");
+    const float *s = opt_fptr(sub, "sub"), *a = opt_fptr(add, "add");
+    const c10::cuda::CUDAGuard guard(inputL.device());
+    check(ldn_bound_inf_dist_forward_nograd_shifted(xl, xu, w, inputL.size(0), outputL.size(1), inputL.size(1), G,
+                                                    inputL.size(2), yl, yu, s, a, stream()),
+          "bound_inf_dist_forward_nograd_shifted");
+}
+
 void check_status() { check(ldn_check_status(stream()), "device status check"); }
 
 }  // namespace
@@ -194,5 +391,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("bound_inf_dist_backward_input_weight", &bound_inf_dist_backward_input_weight);
     m.def("unfold", &unfold);
     m.def("fold", &fold);
+    m.def("norm_dist", &norm_dist);
+    m.def("bound_inf_dist", &bound_inf_dist);
+    m.def("mean_shift", &mean_shift);
+    m.def("unfold_columns", &unfold_columns);
+    m.def("inf_dist_forward_nograd_shifted", &inf_dist_forward_nograd_shifted);
+    m.def("bound_inf_dist_forward_nograd_shifted", &bound_inf_dist_forward_nograd_shifted);
     m.def("check_status", &check_status);
 }

@@ -68,7 +68,9 @@ def _unfold(x, kernel_size, dilation, padding, stride):
         out = [(s + 2 * padding - dilation * (k - 1) - 1) // stride + 1 for s, k in zip(x.shape[2:], kernel_size)]
         columns = out[0] * out[1] * kernel_size[0] * kernel_size[1]
         if min(out) > 0 and max(columns, x.size(2) * x.size(3), *(s + 2 * padding for s in x.shape[2:])) < 1 << 30:
-            return _UnfoldF.apply(x, out[0] * out[1], kernel_size, stride, padding, dilation)
+            ext = _C.native()
+            cols = None if ext is None else ext.unfold_columns(x, out[0] * out[1], kernel_size, stride, padding, dilation)
+            return cols if cols is not None else _UnfoldF.apply(x, out[0] * out[1], kernel_size, stride, padding, dilation)
     return F.unfold(x, kernel_size, dilation, padding, stride)
 
 
@@ -98,7 +100,11 @@ class MeanShift(nn.Module):
             if (lower is None and upper is None and self.bias is None and x.is_cuda and x.dtype == torch.float32
                     and x.dim() == 3 and x.size(2) == 1 and x.is_contiguous() and self.fused):
                 # fully connected layer: mean, running-mean update and subtraction in one kernel
-                return _MeanShiftRowsF.apply(x, self.running_mean, self.momentum), None, None
+                ext = _C.native()
+                out = None if ext is None else ext.mean_shift(x, self.running_mean, self.momentum)
+                if out is None:
+                    out = _MeanShiftRowsF.apply(x, self.running_mean, self.momentum)
+                return out, None, None
             mean = x.mean(dim=[0, 2])
             with torch.no_grad():
                 self.running_mean.mul_(1 - self.momentum).add_(mean, alpha=self.momentum)

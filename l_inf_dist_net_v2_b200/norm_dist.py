@@ -118,6 +118,11 @@ class BoundInfDistF(torch.autograd.Function):
 def norm_dist(input, weight, p, groups=1, use_custom_cuda_func=True, tag=None):
     if not use_custom_cuda_func:
         raise NotImplementedError("this package has no non-CUDA path (use_custom_cuda_func=False)")
+    ext = _C.native()
+    if ext is not None and type(p) in (float, int) and type(groups) is int:
+        output = ext.norm_dist(input, weight, p, groups)
+        if output is not None:
+            return output
     need_grad = torch.is_grad_enabled() and (input.requires_grad or weight.requires_grad)
     return NormDistF.apply(input, weight, groups, p, need_grad, tag)
 
@@ -125,5 +130,10 @@ def norm_dist(input, weight, p, groups=1, use_custom_cuda_func=True, tag=None):
 def bound_inf_dist(x_lower, x_upper, weight, groups=1, use_custom_cuda_func=True, tag=None):
     if not use_custom_cuda_func:
         raise NotImplementedError("this package has no non-CUDA path (use_custom_cuda_func=False)")
+    ext = _C.native()
+    if ext is not None and type(groups) is int:
+        bounds = ext.bound_inf_dist(x_lower, x_upper, weight, groups)
+        if bounds is not None:
+            return bounds
     need_grad = torch.is_grad_enabled() and (x_lower.requires_grad or x_upper.requires_grad or weight.requires_grad)
     return BoundInfDistF.apply(x_lower, x_upper, weight, groups, need_grad, tag)

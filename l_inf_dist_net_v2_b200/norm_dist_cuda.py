@@ -228,6 +228,15 @@ try:
 except ImportError:
     _ext = None
 if _ext is not None:
-    for _name in __all__ + ["unfold", "fold", "check_status"]:
+    for _name in __all__ + ["unfold", "fold", "inf_dist_forward_nograd_shifted", "bound_inf_dist_forward_nograd_shifted",
+                            "check_status"]:
         globals()[_name] = getattr(_ext, _name)
     BINDING = "pybind11"
+
+
+def native():
+    """The compiled binding when its C++ autograd functions may stand in for the Python ones, else None: it was not built,
+    or a function transform (vmap, grad, jvp) or torch.compile is at work, which the Python functions refuse or handle."""
+    if _ext is None or torch._C._are_functorch_transforms_active() or torch.compiler.is_compiling():
+        return None
+    return _ext
