@@ -87,6 +87,8 @@ struct TileParams {
     const float* col_add;       //   stored value = (result - col_sub[channel]) + col_add[channel]; either may be null
     const int* gate;            // not null: the kernel returns at once unless (*gate != 0) == (gate_invert == 0)
     int gate_invert;
+    int pres_vec;               // backward kernels: elements n .. n + 3 (n a multiple of 4) of a row of the resident operand,
+                                //   which has the output's layout, are one aligned 16-byte piece
     int accumulate_out;         // backward kernels: add to the output instead of overwriting it
     float* side_out;            // fused backward: per-row-tile column sums [tile_m][g][k][n] (else null)
     float* partials;            // stream-K scratch: [grid][2][arrays][kTileElems]

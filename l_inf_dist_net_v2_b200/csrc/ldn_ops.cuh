@@ -198,6 +198,8 @@ struct FwdLayout {
     static constexpr bool N_IN_SMEM = false;     // integer accumulators live in shared memory, not registers
     static constexpr bool ROLLED_EPILOGUE = true;  // finalise a tile row by row in a rolled loop (small code)
     static constexpr bool ROLLED_PRES = true;      // the same for loading the resident per-output operand
+    static constexpr bool PRES_ROWS = false;       // the resident operand lies like the output: loaded by rows
+    static constexpr bool PRES_VEC = false;        // ... in 16-byte pieces where they are whole
     static constexpr int STAGES = kStages;
     static constexpr int REG_N = 8;        // output columns per thread: 8 (128 x 128 tile) or 4 (128 x 64)
     static constexpr int CTAS_PER_SM = 1;  // 2 needs REG_N = 4 (registers) and at most 113 KB of shared memory
@@ -616,12 +618,15 @@ struct BwdLayout {
     static constexpr bool N_IN_SMEM = false;
     static constexpr bool ROLLED_EPILOGUE = false;  // measured: no gain for the backward kernels (160-stage tiles)
     static constexpr bool ROLLED_PRES = false;
+    static constexpr bool PRES_ROWS = true;
+    static constexpr bool PRES_VEC = true;
     static constexpr int STAGES = kStages;
     static constexpr int REG_N = 8;
     static constexpr int CTAS_PER_SM = 1;
     static constexpr bool HAS_P = true;
+    // the resident operand (x or w as the caller laid it out) has the layout of the gradient
     __device__ static float load_pres(const TileParams& P, int m, int n, int g) {
-        return P.pres.ptr[n + m * P.pres.stride_row + g * P.pres.stride_group];
+        return P.pres.ptr[out_offset(P.out, m, n, g)];
     }
     __device__ static float diff(float pres, float b) { return WEIGHT ? b - pres : pres - b; }
     __device__ static void store(float v, int m, int n, int g, const TileParams& P) {
@@ -681,6 +686,7 @@ struct BwdPowGen : BwdLayout<WEIGHT> {
     using L = BwdLayout<WEIGHT>;
     static constexpr int NUM_A = 2, NF = 1, NI = 0;
     static constexpr bool PACKED = true;
+    static constexpr bool PRES_VEC = false;
     // two CTAs of the 128 x 64 tile per SM (see BwdFusedGen)
     static constexpr int UNROLL = 4;
     static constexpr int STAGES = 2;
@@ -751,6 +757,7 @@ struct BwdFusedGen : BwdLayout<false> {
     static constexpr int NUM_A = 2, NF = 1, NI = 0;
     static constexpr bool PACKED = true;
     static constexpr bool FUSED_W = true;
+    static constexpr bool PRES_VEC = false;  // (0.5 % slower with it at 512 x 3072 -> 5120)
     // two CTAs of the 128 x 64 tile per SM: twice the warps to cover the MUFU / polynomial dependency chains
     static constexpr int UNROLL = 2;
     static constexpr int STAGES = 2;

@@ -260,7 +260,7 @@ tile_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ 
 #pragma unroll
                 for (int j = 0; j < RN; ++j) {
                     Op::init(accf[i][j], iacc(i, j));
-                    if (Op::HAS_P && !Op::ROLLED_PRES) {
+                    if (Op::HAS_P && !Op::ROLLED_PRES && !Op::PRES_ROWS) {
                         const int m = tc.m0 + own_index<Op::LA>(tm, i);
                         const int n = tc.n0 + own_index<Op::LB, RN>(tn, j);
                         pres[i][j] = (m < P.M && n < P.N) ? Op::load_pres(P, m, n, tc.g) : 0.0f;
@@ -268,6 +268,34 @@ tile_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ 
                         pres[i][j] = 0.0f;
                     }
                 }
+            if constexpr (Op::PRES_ROWS) {
+                // The resident operand is the caller's array and has the output's layout.  A thread's columns come in fours:
+                // where rows are whole 16-byte pieces one load serves four outputs (PRES_VEC ops), otherwise (convolutions:
+                // positions contiguous, neighbouring threads read neighbouring rows) one each.  All are in flight together.
+#pragma unroll
+                for (int i = 0; i < kRegM; ++i) {
+                    const int m = tc.m0 + own_index<Op::LA>(tm, i);
+                    const float* row = P.pres.ptr + out_offset(P.out, m, 0, tc.g);
+                    if (Op::PRES_VEC && P.pres_vec) {
+#pragma unroll
+                        for (int j = 0; j < RN; j += 4) {
+                            const int n = tc.n0 + own_index<Op::LB, RN>(tn, j);
+                            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            if (m < P.M && n < P.N) v = *reinterpret_cast<const float4*>(row + n);
+                            pres[i][j] = v.x;
+                            pres[i][j + 1] = v.y;
+                            pres[i][j + 2] = v.z;
+                            pres[i][j + 3] = v.w;
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < RN; ++j) {
+                            const int n = tc.n0 + own_index<Op::LB, RN>(tn, j);
+                            pres[i][j] = (m < P.M && n < P.N) ? row[n * P.out.s_n] : 0.0f;
+                        }
+                    }
+                }
+            }
             if constexpr (Op::HAS_P && Op::ROLLED_PRES) {
                 // one register row per trip of a rolled loop (see the epilogue below): the rows move down one
                 // slot per trip, the row loaded in trip i ends in slot i
