@@ -119,6 +119,12 @@ LDN_API int ldn_mean_shift_rows(const float* x, int B, int C, float* running_mea
                         float* mean_out, ldn_stream_t stream);
 
 /*
+ * The same for a convolution layer: x and out are [B][C][HW], the mean of a channel runs over samples and positions.
+ */
+LDN_API int ldn_mean_shift_planes(const float* x, int B, int C, int HW, float* running_mean, float momentum, float* out,
+                                  ldn_stream_t stream);
+
+/*
  * Patches of x[B][C][H][W] as columns cols[B][C * kh * kw][OH * OW] (zero outside the image), and the adjoint: x = sum of
  * the columns' elements that come from each pixel.  OH = (H + 2 pad - dil (kh - 1) - 1) / stride + 1, OW alike.  The
  * reference calls torch's unfold (core/modules/norm_dist.py:84-97).  Both write every element of their output.

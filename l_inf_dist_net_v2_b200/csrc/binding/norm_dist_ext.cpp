@@ -278,27 +278,27 @@ struct BoundInfDistFn : public torch::autograd::Function<BoundInfDistFn> {
     }
 };
 
-// x - mean over the batch; running_mean may be undefined
-void mean_shift_rows(const Tensor& x, const Tensor& running_mean, double momentum, Tensor& out) {
+// x - mean over the batch and the positions; running_mean may be undefined
+void subtract_mean(const Tensor& x, const Tensor& running_mean, double momentum, Tensor& out) {
     const float* a = fptr(x, "x");
     float* rm = running_mean.defined() ? const_cast<float*>(fptr(running_mean, "running_mean")) : nullptr;
     float* y = fptr_mut(out, "out");
     const c10::cuda::CUDAGuard guard(x.device());
-    const int64_t B = x.size(0);
-    check(ldn_mean_shift_rows(a, B, x.numel() / std::max<int64_t>(B, 1), rm, static_cast<float>(momentum), y, nullptr,
-                              stream()),
-          "mean_shift_rows");
+    const int B = x.size(0), C = x.size(1), HW = x.size(2);
+    const float m = static_cast<float>(momentum);
+    if (HW == 1) check(ldn_mean_shift_rows(a, B, C, rm, m, y, nullptr, stream()), "mean_shift_rows");
+    else check(ldn_mean_shift_planes(a, B, C, HW, rm, m, y, stream()), "mean_shift_planes");
 }
 
-struct MeanShiftRowsFn : public torch::autograd::Function<MeanShiftRowsFn> {
+struct MeanShiftFn : public torch::autograd::Function<MeanShiftFn> {
     static Tensor forward(AutogradContext*, Tensor x, Tensor running_mean, double momentum) {
         Tensor out = at::empty_like(x);
-        mean_shift_rows(x, running_mean, momentum, out);
+        subtract_mean(x, running_mean, momentum, out);
         return out;
     }
     static variable_list backward(AutogradContext*, variable_list grads) {
         Tensor go = grads[0].contiguous(), gx = at::empty_like(go);
-        mean_shift_rows(go, Tensor(), 0.0, gx);
+        subtract_mean(go, Tensor(), 0.0, gx);
         return {gx, Tensor(), Tensor()};
     }
 };
@@ -338,9 +338,9 @@ c10::optional<std::tuple<Tensor, Tensor>> bound_inf_dist(const Tensor& xl, const
 
 c10::optional<Tensor> mean_shift(const Tensor& x, const Tensor& running_mean, double momentum) {
     if (!plain(x, 3) || !plain(running_mean, 1) || x.device() != running_mean.device() || running_mean.requires_grad() ||
-        running_mean.size(0) != x.size(1) || x.size(2) != 1 || torch::jit::tracer::isTracing())
+        running_mean.size(0) != x.size(1) || torch::jit::tracer::isTracing())
         return c10::nullopt;
-    return MeanShiftRowsFn::apply(x, running_mean, momentum);
+    return MeanShiftFn::apply(x, running_mean, momentum);
 }
 
 c10::optional<Tensor> unfold_columns(const Tensor& x, int64_t positions, std::pair<int64_t, int64_t> kernel, int64_t stride,

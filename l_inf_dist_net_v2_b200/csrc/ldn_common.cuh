@@ -236,21 +236,29 @@ inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? kOk : kCudaBas
 // Launches a kernel that begins with stream_order_begin(): its blocks may be placed on the SMs that the kernel in front of it
 // on the stream leaves, instead of after that kernel's end and a launch's latency.
 template <class... P, class... A>
-int launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+int launch_after_in_clusters(void (*kernel)(P...), unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                             A&&... args) {
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
     if (e == cudaSuccess) count_launches(1);
     else cudaGetLastError();
     return cuda_status(e);
+}
+template <class... P, class... A>
+int launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    return launch_after_in_clusters(kernel, 1, grid, block, smem, st, args...);
 }
 
 }  // namespace ldn

@@ -18,6 +18,7 @@ struct SideJob {
     long long count;
     int tiles;
     bool accumulate, vec;  // vec: count is a multiple of 4 and both arrays are 16-byte aligned
+    bool wide;             // vec only: the warps of a block share the row tiles
     const int* gate;
     bool run_if_nonzero;
     int blocks;  // 0: no such job
@@ -64,6 +65,36 @@ __device__ __forceinline__ long long y_offset(const Shape& s, const CanonIdx& q)
 __device__ __forceinline__ void side_reduce_block(const SideJob& J, unsigned block, unsigned blocks) {
     if (J.gate && (*J.gate != 0) != J.run_if_nonzero) return;
     const long long first = block * (long long)kPostBlock + threadIdx.x, step = (long long)blocks * kPostBlock;
+    if (J.wide) {
+        __shared__ float4 sums[kPostBlock];
+        const long long n4 = J.count / 4;
+        const float4* part = reinterpret_cast<const float4*>(J.part);
+        float4* gw = reinterpret_cast<float4*>(J.gw);
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        for (long long i0 = block * 32LL; i0 < n4; i0 += blocks * 32LL) {
+            const long long i = i0 + lane;
+            float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (i < n4) {
+#pragma unroll 4
+                for (int t = w; t < J.tiles; t += kPostBlock / 32) {
+                    const float4 v = part[t * n4 + i];
+                    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+                }
+            }
+            sums[threadIdx.x] = s;
+            __syncthreads();
+            if (w == 0 && i < n4) {
+                for (int k = 1; k < kPostBlock / 32; ++k) {
+                    const float4 v = sums[k * 32 + lane];
+                    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+                }
+                const float4 o = J.accumulate ? gw[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                gw[i] = make_float4(o.x - s.x, o.y - s.y, o.z - s.z, o.w - s.w);
+            }
+            __syncthreads();
+        }
+        return;
+    }
     if (J.vec) {
         // bound by HBM / L2 reads: 16-byte loads, four row tiles in flight
         const long long n4 = J.count / 4;

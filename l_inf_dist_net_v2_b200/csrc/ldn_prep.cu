@@ -110,6 +110,40 @@ __global__ void coef_int_kernel(const float* go, const float* y, float* coef,
     if (flag && bad) *flag = 1;
 }
 
+// HW > 1: the same through shared memory.  Rows (b, g, o, :) of go / y are contiguous in hw, rows (g, m, :) of the coefficients
+// contiguous in o; a 32 x 32 tile makes both sides coalesced (one thread per coefficient read 4 bytes from every 4 HW).  grid =
+// (ceil(HW/32), ceil(COg/32), B*G).
+__global__ void __launch_bounds__(kBlock) coef_int_transpose_kernel(const float* go, const float* y, float* coef, Shape s,
+                                                                    int pitch, int iq, int* flag) {
+    stream_order_begin();
+    __shared__ float tile[32][33];
+    const int bg = blockIdx.z, b = bg / s.G, g = bg - b * s.G;
+    const int hw0 = blockIdx.x * 32, o0 = blockIdx.y * 32;
+    const long long src = s.co_src != s.CO ? (static_cast<long long>(b) * s.co_src + s.co_off) * s.HW
+                                           : static_cast<long long>(bg) * s.COg * s.HW;
+    bool bad = false;
+#pragma unroll
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int o = o0 + r, hw = hw0 + threadIdx.x;
+        if (o < s.COg && hw < s.HW) {
+            const long long i = src + static_cast<long long>(o) * s.HW + hw;
+            const float inv = 1.0f / y[i];
+            float rq = 1.0f;
+            for (int k = 0; k < iq; ++k) rq *= inv;
+            bad |= rq_unsafe(rq);
+            tile[r][threadIdx.x] = go[i] * rq;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int hw = hw0 + r, o = o0 + threadIdx.x;
+        if (o < s.COg && hw < s.HW)
+            coef[(g * s.M + static_cast<long long>(b) * s.HW + hw) * pitch + o] = tile[threadIdx.x][r];
+    }
+    if (flag && bad) *flag = 1;
+}
+
 // flat fast paths (HW == 1, G == 1, pitch == COg: source and destination have the same element order)
 __global__ void coef_int_flat_kernel(const float4* go, const float4* y,
                                      float4* coef, long long n4, int iq, int* flag) {
@@ -396,16 +430,16 @@ __global__ void bound_scatter_kernel(const float* gol, const float* gou,
 
 
 
-static bool transpose_grid(const Shape& s, dim3* grid) {
+static bool transpose_grid(const Shape& s, int channels, dim3* grid) {
     const long long bg = static_cast<long long>(s.B) * s.G;
-    if (s.HW < 8 || bg > 65535 || (s.CIg + 31) / 32 > 65535) return false;
-    *grid = dim3((s.HW + 31) / 32, (s.CIg + 31) / 32, static_cast<unsigned>(bg));
+    if (s.HW < 8 || bg > 65535 || (channels + 31) / 32 > 65535) return false;
+    *grid = dim3((s.HW + 31) / 32, (channels + 31) / 32, static_cast<unsigned>(bg));
     return true;
 }
 
 int launch_canon_x(const float* x, float* xc, const Shape& s, int pitch, cudaStream_t st) {
     dim3 grid;
-    if (transpose_grid(s, &grid)) {
+    if (transpose_grid(s, s.CIg, &grid)) {
         return launch_after(canon_transpose_kernel, grid, dim3(32, 8), 0, st, x, nullptr, xc, nullptr, s, pitch);
     }
     return launch_after(canon_x_kernel, blocks_for((long long)s.G * s.M * s.CIg), kBlock, 0, st, x, xc, s, pitch);
@@ -413,7 +447,7 @@ int launch_canon_x(const float* x, float* xc, const Shape& s, int pitch, cudaStr
 int launch_canon_bounds(const float* xl, const float* xu, float* lc, float* uc, const Shape& s, int pitch,
                         cudaStream_t st) {
     dim3 grid;
-    if (transpose_grid(s, &grid)) {
+    if (transpose_grid(s, s.CIg, &grid)) {
         return launch_after(canon_transpose_kernel, grid, dim3(32, 8), 0, st, xl, xu, lc, uc, s, pitch);
     }
     return launch_after(canon_bounds_kernel, blocks_for((long long)s.G * s.M * s.CIg), kBlock, 0, st, xl, xu, lc, uc,
@@ -434,6 +468,9 @@ int launch_coef_int(const float* go, const float* y, float* coef, const Shape& s
         return launch_after(coef_int_flat_kernel, blocks_for(n4), kBlock, 0, st, reinterpret_cast<const float4*>(go),
                             reinterpret_cast<const float4*>(y), reinterpret_cast<float4*>(coef), n4, iq, flag);
     }
+    dim3 grid;
+    if (transpose_grid(s, s.COg, &grid))
+        return launch_after(coef_int_transpose_kernel, grid, dim3(32, 8), 0, st, go, y, coef, s, pitch, iq, flag);
     return launch_after(coef_int_kernel, blocks_for((long long)s.G * s.M * s.COg), kBlock, 0, st, go, y, coef, s,
                         pitch, iq, flag);
 }
@@ -488,8 +525,13 @@ int launch_row_absmax(Operand v, long long rows, int inner, int groups, long lon
 SideJob side_reduce_job(const float* part, float* gw, long long count, int tiles, bool accumulate, const int* gate,
                         bool run_if_nonzero) {
     const bool vec = (count & 3) == 0 && ((reinterpret_cast<uintptr_t>(part) | reinterpret_cast<uintptr_t>(gw)) & 15u) == 0;
-    return SideJob{part, gw, count, tiles, accumulate, vec, gate, run_if_nonzero,
-                   static_cast<int>(gated_blocks(blocks_for(vec ? count / 4 : count), run_if_nonzero ? gate : nullptr))};
+    // many row tiles of a small weight (convolutions): with a thread per piece 512 blocks' worth of threads would not exist,
+    // so the 8 warps of a block share the tiles of 32 pieces (256 tiles of 128 x 576: 40 us with a thread per piece; with this
+    // and the coefficients by tiles, 46 us before, the fold by rows and the mean by planes the step went 1377 -> 1242 us)
+    const bool wide = vec && tiles >= 32 && count / 4 < 512LL * kPostBlock;
+    const long long threads = (vec ? count / 4 : count) * (wide ? 8 : 1);
+    return SideJob{part, gw, count, tiles, accumulate, vec, wide, gate, run_if_nonzero,
+                   static_cast<int>(gated_blocks(blocks_for(threads), run_if_nonzero ? gate : nullptr))};
 }
 
 int launch_inf_scatter(const float* go, const int* pos, float* gx, float* gw, const Shape& s, cudaStream_t st) {

@@ -106,6 +106,37 @@ __global__ void __launch_bounds__(kBlock) fold_kernel(const float* cols, float* 
     }
 }
 
+// The same at stride 1 for rows of whole 16-byte pieces: a thread sums four neighbouring pixels, so the index arithmetic of a
+// patch offset serves four loads, which are in flight together (32 x 64 x 32 x 32, 3 x 3: 17 us instead of 52).
+__global__ void __launch_bounds__(kBlock) fold_row_kernel(const float* cols, float* x, Patches P, long long planes,
+                                                          unsigned planes_per_slice) {
+    stream_order_begin();
+    const long long plane0 = static_cast<long long>(blockIdx.y) * planes_per_slice;
+    const unsigned n =
+        static_cast<unsigned>(planes - plane0 < planes_per_slice ? planes - plane0 : planes_per_slice) * P.by_row.d;
+    const int L = P.OH * P.OW;
+    for (unsigned i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
+        const unsigned pl = quotient(i, P.by_row);
+        const unsigned pix = (i - pl * P.by_row.d) * 4;
+        const int h = static_cast<int>(quotient(pix, P.by_w)), w = static_cast<int>(pix) - h * P.W;
+        const float* src = cols + (plane0 + pl) * (static_cast<long long>(P.kh) * P.kw * L);
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int ki = P.kh - 1; ki >= 0; --ki) {
+            const int oh = h + P.pad - ki * P.dil;
+            if (oh < 0 || oh >= P.OH) continue;
+#pragma unroll 3
+            for (int kj = P.kw - 1; kj >= 0; --kj) {
+                const int ow = w + P.pad - kj * P.dil;
+                const float* row = src + static_cast<long long>(ki * P.kw + kj) * L + oh * P.OW + ow;
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (ow + e >= 0 && ow + e < P.OW) s[e] += row[e];
+            }
+        }
+        *reinterpret_cast<float4*>(x + (plane0 + pl) * P.by_row.d * 4 + pix) = make_float4(s[0], s[1], s[2], s[3]);
+    }
+}
+
 // Checks the geometry and fills it in.
 int fill(Patches* P, int B, int C, int H, int W, int kh, int kw, int stride, int pad, int dil) {
     if (B < 0 || C <= 0 || H <= 0 || W <= 0 || kh <= 0 || kw <= 0 || stride <= 0 || pad < 0 || dil <= 0) return kBadArgument;
@@ -173,12 +204,15 @@ LDN_API int ldn_fold(const float* cols, int B, int C, int H, int W, int kh, int 
     if (r != kOk) return r;
     if (B == 0) return kOk;
     if (!x || !cols) return kBadArgument;
-    P.by_row = make_divider(static_cast<unsigned>(H * W));
+    const bool vec = stride == 1 && (W & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    P.by_row = make_divider(static_cast<unsigned>(vec ? H * W / 4 : H * W));
     const long long planes = static_cast<long long>(B) * C;
     Slices s;
     if ((r = slice(planes, P.by_row.d, &s)) != kOk) return r;
-    return launch_after(fold_kernel, dim3(s.blocks, s.count), kBlock, 0, reinterpret_cast<cudaStream_t>(stream), cols,
-                        x, P, planes, s.per_slice);
+    const dim3 grid(s.blocks, s.count);
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (vec) return launch_after(fold_row_kernel, grid, kBlock, 0, st, cols, x, P, planes, s.per_slice);
+    return launch_after(fold_kernel, grid, kBlock, 0, st, cols, x, P, planes, s.per_slice);
 }
 
 }  // extern "C"

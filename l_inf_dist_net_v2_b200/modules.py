@@ -98,13 +98,14 @@ class MeanShift(nn.Module):
         if self.training:
             assert x is not None, "Currently not supported"
             if (lower is None and upper is None and self.bias is None and x.is_cuda and x.dtype == torch.float32
-                    and x.dim() == 3 and x.size(2) == 1 and x.is_contiguous() and self.fused):
-                # fully connected layer: mean, running-mean update and subtraction in one kernel
+                    and x.dim() == 3 and x.is_contiguous() and self.fused):
+                # mean, running-mean update and subtraction in one kernel
                 ext = _C.native()
                 out = None if ext is None else ext.mean_shift(x, self.running_mean, self.momentum)
-                if out is None:
+                if out is None and x.size(2) == 1:
                     out = _MeanShiftRowsF.apply(x, self.running_mean, self.momentum)
-                return out, None, None
+                if out is not None:
+                    return out, None, None
             mean = x.mean(dim=[0, 2])
             with torch.no_grad():
                 self.running_mean.mul_(1 - self.momentum).add_(mean, alpha=self.momentum)
