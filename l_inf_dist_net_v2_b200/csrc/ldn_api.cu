@@ -6,6 +6,7 @@
 #include <mutex>
 
 #include "ldn_b200.h"
+#include "ldn_extreme.cuh"
 #include "ldn_launch.cuh"
 #include "ldn_prep.cuh"
 
@@ -451,6 +452,21 @@ int norm_dist_backward(const float* go, const float* x, const float* w, const fl
     return norm_dist_backward_part(go, x, w, y, s, gx, gw, p, stream, false, accumulate_gx);
 }
 
+// Whether `bytes` of scratch can be had on this stream: an arena that is large enough, or may grow (not during a capture).
+// Paths that need more scratch than the general one are taken only then, so that a reservation made for that one suffices.
+bool scratch_available(ldn_stream_t stream, size_t bytes) {
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    Arena* arena;
+    if (find_arena(st, &arena) != kOk) return false;
+    std::lock_guard<std::mutex> lock(*static_cast<std::mutex*>(arena->call_mutex));
+    return ensure_arena(arena, st, bytes) == kOk;
+}
+
+// Large fully connected p = inf problems on the whole chip start from the extreme channels (ldn_extreme.cu).
+bool extreme_path(const DeviceCtx* ctx, const Shape& s, bool bound) {
+    return s.G == 1 && s.HW == 1 && cap_for(ctx) == ctx->sm_count && extreme_applies(s.M, s.CO, s.CI, bound);
+}
+
 int inf_forward(const float* x, const float* w, const Shape& s, float* y, int* pos, ldn_stream_t stream,
                 const float* col_sub = nullptr, const float* col_add = nullptr) {
     if (!x || !w || !y) return kBadArgument;
@@ -461,6 +477,9 @@ int inf_forward(const float* x, const float* w, const Shape& s, float* y, int* p
     const bool inplace = x_inplace_kmajor(x, s);
     size_t need = (inplace ? 0 : x_scratch_bytes(x, s)) + w_scratch_bytes(w, s) +
                   partial_bytes(cap_for(ctx), fwd_acc_arrays(kind));
+    const bool extreme = extreme_path(ctx, s, false) &&
+                         scratch_available(stream, need + extreme_scratch_bytes(s.M, s.CO, false));
+    if (extreme) need += extreme_scratch_bytes(s.M, s.CO, false);
     Call c;
     if ((r = begin_call(&c, stream, need)) != kOk) return r;
     c.col_sub = col_sub;
@@ -469,15 +488,22 @@ int inf_forward(const float* x, const float* w, const Shape& s, float* y, int* p
     if (inplace) xv = x_kmajor_view(x, s);
     else if ((r = get_x_view(c, x, s, &xv)) != kOk) return r;
     if ((r = get_w_view(c, w, s, &wv)) != kOk) return r;
+    if (extreme) {
+        ExtremeScratch t;
+        if (!extreme_take_scratch(&c.bump, s.M, s.CO, false, &t)) return kWorkspace;
+        r = launch_extreme(as_operand(xv), as_operand(xv), as_operand(wv), s.M, s.CO, s.CI, false, y, nullptr, pos, col_sub,
+                           col_add, t, &c.gate, c.st);
+        if (r != kOk) return r;
+    }
     r = run_forward(c, kind, 0, xv, nullptr, wv, s, y, nullptr, pos, nullptr, nullptr, INFINITY, inplace);
     if (r != kOk || !pos) return r;
     if (inplace) {
         // the input as the index search addresses it: element (sample-group bg, position hw, channel k) at
         // bg * stride_group + hw * stride_row + k * HW
         const Operand xin{x, 1, static_cast<long long>(s.CIg) * s.HW};
-        return launch_rescan(0, xin, xin, as_operand(wv), y, pos, s, c.st, s.HW);
+        return launch_rescan(0, xin, xin, as_operand(wv), y, pos, s, c.st, s.HW, nullptr);
     }
-    return launch_rescan(0, as_operand(xv), as_operand(xv), as_operand(wv), y, pos, s, c.st, 1);
+    return launch_rescan(0, as_operand(xv), as_operand(xv), as_operand(wv), y, pos, s, c.st, 1, c.gate);
 }
 
 int bound_forward(const float* xl, const float* xu, const float* w, const Shape& s, float* yl, float* yu, int* pl,
@@ -488,6 +514,9 @@ int bound_forward(const float* xl, const float* xu, const float* w, const Shape&
     if (r != kOk) return r;
     const size_t xfloats = canonical_floats(s.CIg, s.M, s.G);
     size_t need = 2 * pad256(xfloats * sizeof(float)) + w_scratch_bytes(w, s) + 2 * partial_bytes(cap_for(ctx), 5);
+    const bool extreme = !pl && extreme_path(ctx, s, true) &&
+                         scratch_available(stream, need + extreme_scratch_bytes(s.M, s.CO, true));
+    if (extreme) need += extreme_scratch_bytes(s.M, s.CO, true);
     Call c;
     if ((r = begin_call(&c, stream, need)) != kOk) return r;
     c.col_sub = col_sub;
@@ -500,20 +529,27 @@ int bound_forward(const float* xl, const float* xu, const float* w, const Shape&
     if ((r = launch_canon_bounds(xl, xu, lc, uc, s, static_cast<int>(lv.stride_row), c.st)) != kOk) return r;
     View wv;
     if ((r = get_w_view(c, w, s, &wv)) != kOk) return r;
+    if (extreme) {
+        ExtremeScratch t;
+        if (!extreme_take_scratch(&c.bump, s.M, s.CO, true, &t)) return kWorkspace;
+        r = launch_extreme(as_operand(lv), as_operand(uv), as_operand(wv), s.M, s.CO, s.CI, true, yl, yu, nullptr, col_sub,
+                           col_add, t, &c.gate, c.st);
+        if (r != kOk) return r;
+    }
     if (!pl) return run_forward(c, FwdKind::Bound, 0, lv, &uv, wv, s, yl, yu, nullptr, nullptr, nullptr, INFINITY);
     if ((s.CIg + kTileK - 1) / kTileK <= g_bound_one_pass_stages) {
         // one pass: both bounds and the stage of each extremum, then the two index searches
         r = run_forward(c, FwdKind::BoundPosBoth, 0, lv, &uv, wv, s, yl, yu, pl, pu, nullptr, INFINITY);
         if (r != kOk) return r;
-        if ((r = launch_rescan(1, as_operand(lv), as_operand(uv), as_operand(wv), yl, pl, s, c.st, 1)) != kOk) return r;
-        return launch_rescan(2, as_operand(lv), as_operand(uv), as_operand(wv), yu, pu, s, c.st, 1);
+        if ((r = launch_rescan(1, as_operand(lv), as_operand(uv), as_operand(wv), yl, pl, s, c.st, 1, nullptr)) != kOk) return r;
+        return launch_rescan(2, as_operand(lv), as_operand(uv), as_operand(wv), yu, pu, s, c.st, 1, nullptr);
     }
     r = run_forward(c, FwdKind::BoundPosLower, 0, lv, &uv, wv, s, yl, yu, pl, pu, nullptr, INFINITY);
     if (r != kOk) return r;
-    if ((r = launch_rescan(1, as_operand(lv), as_operand(uv), as_operand(wv), yl, pl, s, c.st, 1)) != kOk) return r;
+    if ((r = launch_rescan(1, as_operand(lv), as_operand(uv), as_operand(wv), yl, pl, s, c.st, 1, nullptr)) != kOk) return r;
     r = run_forward(c, FwdKind::BoundPosUpper, 0, lv, &uv, wv, s, yl, yu, pl, pu, nullptr, INFINITY);
     if (r != kOk) return r;
-    return launch_rescan(2, as_operand(lv), as_operand(uv), as_operand(wv), yu, pu, s, c.st, 1);
+    return launch_rescan(2, as_operand(lv), as_operand(uv), as_operand(wv), yu, pu, s, c.st, 1, nullptr);
 }
 
 }  // namespace

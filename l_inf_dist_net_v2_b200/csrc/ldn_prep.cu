@@ -180,8 +180,9 @@ __global__ void __launch_bounds__(kBlock) coef_gen_kernel(const CoefJob job) {
 // one input row, which stays in the L1 cache: only the weight pieces come from L2.
 template <int mode>
 __global__ void __launch_bounds__(kBlock) rescan_kernel(Operand a0, Operand a1, Operand b, const float* y,
-                                                        int* pos, Shape s, long long a_stride_k) {
+                                                        int* pos, Shape s, long long a_stride_k, const int* gate) {
     stream_order_begin();
+    if (gate && *gate == 0) return;
     constexpr int U = kRescanIlp;
     const int kpad = (s.CIg + 3) & ~3;
     const int q = threadIdx.x & 3;
@@ -486,7 +487,7 @@ int launch_coef_gen(const CoefJob& job, cudaStream_t st) {
 }
 
 int launch_rescan(int mode, Operand a0, Operand a1, Operand b, const float* y, int* pos, const Shape& s,
-                  cudaStream_t st, long long a_stride_k) {
+                  cudaStream_t st, long long a_stride_k, const int* gate) {
     if (a_stride_k != 1 && mode != 0) return kBadArgument;
     const long long cohw = static_cast<long long>(s.COg) * s.HW;
     const long long bg = static_cast<long long>(s.B) * s.G;
@@ -508,9 +509,9 @@ int launch_rescan(int mode, Operand a0, Operand a1, Operand b, const float* y, i
     if (chunks > most) chunks = most;  // the kernel strides over the rest
     if (chunks > 65535) chunks = 65535;
     const dim3 grid(static_cast<unsigned>(bg), static_cast<unsigned>(chunks));
-    if (mode == 0) return launch_after(rescan_kernel<0>, grid, kBlock, 0, st, a0, a1, b, y, pos, s, a_stride_k);
-    if (mode == 1) return launch_after(rescan_kernel<1>, grid, kBlock, 0, st, a0, a1, b, y, pos, s, a_stride_k);
-    return launch_after(rescan_kernel<2>, grid, kBlock, 0, st, a0, a1, b, y, pos, s, a_stride_k);
+    if (mode == 0) return launch_after(rescan_kernel<0>, grid, kBlock, 0, st, a0, a1, b, y, pos, s, a_stride_k, gate);
+    if (mode == 1) return launch_after(rescan_kernel<1>, grid, kBlock, 0, st, a0, a1, b, y, pos, s, a_stride_k, gate);
+    return launch_after(rescan_kernel<2>, grid, kBlock, 0, st, a0, a1, b, y, pos, s, a_stride_k, gate);
 }
 
 int launch_row_absmax(Operand v, long long rows, int inner, int groups, long long stride_k, float* out, int* clear,

@@ -30,7 +30,7 @@ int launch_coef_gen(const CoefJob& job, cudaStream_t st);
 // a_stride_k != 1 (mode 0 only) a0 is an input read in place: element (sample-group bg, position hw, channel k) at
 // a0.ptr + bg * a0.stride_group + hw * a0.stride_row + k * a_stride_k.
 int launch_rescan(int mode, Operand a0, Operand a1, Operand b, const float* y, int* pos, const Shape& s,
-                  cudaStream_t st, long long a_stride_k);
+                  cudaStream_t st, long long a_stride_k, const int* gate);  // gate (a_stride_k == 1; may be null): as above
 
 // out[g * rows + r] = max_k |v[g][r][k]| for an operand view with `inner` reduction elements per row, stride_k apart
 // (1: contiguous).  clear (may be null): a device word that the kernel resets to 0.
