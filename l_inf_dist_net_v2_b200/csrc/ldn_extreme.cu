@@ -13,13 +13,15 @@
 // N(0, 1) about 60 of 3072 channels are visited for images in [0, 1], 170 of 5120 for activations of deviation 0.5.  Where
 // the lists would not be a small part of a row, anything is not finite, or too many outputs turn out hard, a device word
 // makes the dense kernels behind it run instead.
-// 512 x 5120 -> 5120 forward + backward 1105 -> 567 us, certification of 512 x 3072 -> 5120 (value and bounds) 1971 -> 443.
+// 512 x 5120 -> 5120 forward + backward: dense 1105 us, this path 505; certification of 512 x 3072 -> 5120 (value and bounds):
+// 1971 and 335.
 //
 // What bounds it: the gathers x[b, c] for a list's channels.  A block keeps S rows of one operand in shared memory as
-// [channel][S], so a lane gathers four rows' values of a channel with one 16-byte read; a warp holds 32 / (S / 4) lists at
-// once, whose entries lie [entry][list] in groups of 16 so that one step reads whole 128-byte lines.  Random channels meet
-// bank conflicts of about two, i.e. 16 pairs per clock and SM.  The maximum is taken over batches of 8 entries and compared
-// once per batch (2.4 instructions per pair); the channel is found at the end in the batch that last raised it.
+// [channel][S]; a lane owns a list, gathers four rows' values of a channel with one 16-byte read, and a warp's 32 lists lie
+// [entry][list] in groups of 16, so that a step reads whole 128-byte lines, in an order that keeps the lists of a step on
+// different banks (extreme_lists_kernel).  The maximum is taken over batches of 8 entries and compared once per batch; the
+// channel is found at the end in the batch that last raised it, or in the whole list where a later batch reached the same
+// value.
 #include <float.h>
 
 #include "ldn_extreme.cuh"
@@ -34,10 +36,11 @@ constexpr int kGroup = 16;         // lists whose entries are interleaved
 constexpr int kListThreads = 256;
 constexpr int kMaxChannels = 6144;
 constexpr int kListKeep = kMaxChannels / kListThreads;  // channels a thread of extreme_lists_kernel holds
-constexpr int kScanThreads = 1024;
+constexpr int kScanThreads = 512;
+constexpr int kBatch = 8;          // entries a scan works on at a time (lists are whole batches long)
 constexpr int kSampleBlocks = 148;
 constexpr int kSamples = kSampleBlocks * 8;
-constexpr int kQuantile = 4;       // tau + sigma: this smallest of the samples' maxima (0.3 %)
+constexpr int kQuantile = 2;       // tau + sigma: this smallest of the samples' maxima (0.2 %)
 constexpr int kMaxTile = 224 * 1024;
 // a gathered pair costs about 4 of the dense kernel's, and the samples' lists another pass over the weights
 constexpr int kDenseShare = 8;     // dense where the lists hold more than 1 / kDenseShare of a row
@@ -89,69 +92,105 @@ __device__ __forceinline__ float block_max(float v, float* warps, int n_warps) {
     return v;
 }
 
-// One block per row: the channels whose magnitude reaches the threshold, in ascending order; the row is read once, into
-// registers, with all loads in flight.  Channels beyond `cap` entries count as not listed.
-template <bool PAIR>
-__global__ void __launch_bounds__(kListThreads)
+// One block per row: the channels whose magnitude reaches the threshold; the row is read once, into registers, with all loads
+// in flight (KEEP channels per thread), and magnitudes are compared as integers (a sign bit less, not-a-numbers on top).
+//
+// Order of a list.  A scan step reads one channel of each of a warp's lists from shared memory, 32 bytes at bank
+// 8 (channel % 4) (tiles of 8 rows), so four neighbouring lists read without conflicts if their channels differ modulo 4.
+// Entry k of row r's list therefore has channel % 4 == (k + r) % 4: four interleaved sub-lists, the shorter ones filled up
+// with entries that change nothing (NaN), so that a list is a whole number of batches, at least one.  A lane's channels are
+// all of class lane % 4, so places come from one count per lane.  Channels beyond `cap` entries count as not listed.
+template <bool PAIR, int KEEP>
+__global__ void __launch_bounds__(kListThreads, KEEP <= 12 ? 3 : 2)
 extreme_lists_kernel(Operand v, Operand second, int C, int cap, const float* threshold, typename EntryOf<PAIR>::type* list,
                      int* len, float* rest, int* words) {
     stream_order_begin();
     // (one decision per block: another block of this very kernel may set the word between two threads' reads)
     if (__syncthreads_or(words[0] != 0)) return;
-    __shared__ float warps[kListThreads / 32];
-    __shared__ int counts[kListThreads / 32];
+    using E = typename EntryOf<PAIR>::type;
+    constexpr int WARPS = kListThreads / 32;
+    __shared__ int counts[WARPS][4], lefts[WARPS];
     const long long row = blockIdx.x;
-    const float* src = v.ptr + row * v.stride_row;
-    const float* src2 = second.ptr + row * second.stride_row;
-    const float limit = *threshold;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // a warp takes a run of channels
-    const int per = (C + kListThreads - 1) / kListThreads * 32;
-    const int c0 = warp * per, c1 = min(C, c0 + per);
-    float a[kListKeep], b[PAIR ? kListKeep : 1];
+    const int limit = __float_as_int(*threshold);
+    const float* src = v.ptr + row * v.stride_row + threadIdx.x;
+    const float* src2 = second.ptr + row * second.stride_row + threadIdx.x;
+    float a[KEEP], b[PAIR ? KEEP : 1];
+    const int mine_n = C - static_cast<int>(threadIdx.x);  // this thread's channels: threadIdx.x + 256 k < C
 #pragma unroll
-    for (int k = 0; k < kListKeep; ++k) {
-        const int c = c0 + 32 * k + lane;
-        a[k] = c < c1 ? src[c] : 0.0f;
-        if (PAIR) b[k] = c < c1 ? src2[c] : 0.0f;
+    for (int k = 0; k < KEEP; ++k) {
+        a[k] = kListThreads * k < mine_n ? src[kListThreads * k] : 0.0f;
+        if (PAIR) b[k] = kListThreads * k < mine_n ? src2[kListThreads * k] : 0.0f;
     }
-    int n = 0;
-    bool finite = true;
+    auto magnitude = [&](int k) {
+        const int m = __float_as_int(a[k]) & 0x7fffffff;
+        return PAIR ? max(m, __float_as_int(b[k]) & 0x7fffffff) : m;
+    };
+    int n = 0, top = 0;
 #pragma unroll
-    for (int k = 0; k < kListKeep; ++k) {
-        const float m = PAIR ? fmaxf(fabsf(a[k]), fabsf(b[k])) : fabsf(a[k]);
-        finite &= fabsf(a[k]) <= FLT_MAX && (!PAIR || fabsf(b[k]) <= FLT_MAX);
-        n += __popc(__ballot_sync(0xffffffffu, c0 + 32 * k + lane < c1 && m >= limit));
+    for (int k = 0; k < KEEP; ++k) {
+        const int m = magnitude(k);
+        top = max(top, m);
+        n += m >= limit ? 1 : 0;  // (the threshold is above 0, padding is not)
     }
-    if (!finite) words[0] = 1;  // dense
-    if (lane == 0) counts[warp] = n;
+    if (top >= 0x7f800000) words[0] = 1;  // infinite or not a number: dense
+    // places: exclusive sums over the lanes of a class, then over the warps
+    int at = n;
+#pragma unroll
+    for (int d = 4; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, at, d);
+        if (lane >= d) at += o;
+    }
+    if (lane >= 28) counts[warp][lane & 3] = at;
+    at -= n;
     __syncthreads();
-    int at = 0, total = 0;
+    int longest = 0, here = 0;
 #pragma unroll
-    for (int k = 0; k < kListThreads / 32; ++k) {
-        if (k < warp) at += counts[k];
-        total += counts[k];
-    }
-    float left = 0.0f;
+    for (int q = 0; q < 4; ++q) {
+        int total = 0;
 #pragma unroll
-    for (int k = 0; k < kListKeep; ++k) {
-        const int c = c0 + 32 * k + lane;
-        const float m = PAIR ? fmaxf(fabsf(a[k]), fabsf(b[k])) : fabsf(a[k]);
-        const bool in = c < c1 && m >= limit;
-        const unsigned who = __ballot_sync(0xffffffffu, in);
-        const int slot = at + __popc(who & ((1u << lane) - 1));
-        if (in && slot < cap) {
-            if constexpr (PAIR) list[entry_index(row, slot, cap)] = Entry2{a[k], b[k], c, 0};
-            else list[entry_index(row, slot, cap)] = Entry1{a[k], c};
-        } else {
-            left = fmaxf(left, m);
+        for (int k = 0; k < WARPS; ++k) {
+            if (q == (lane & 3) && k < warp) at += counts[k][q];
+            total += counts[k][q];
         }
-        at += __popc(who);
+        longest = max(longest, total);
+        if (q == (lane & 3)) here = total;
     }
-    left = block_max(left, warps, kListThreads / 32);
+    longest = min(longest, cap / 4);
+    const int slots = max((longest + 1) & ~1, 2);  // of a sub-list, fillers included: kBatch entries are two slots
+    static_assert(kBatch == 8 && kListW % kBatch == 0 && kListX % kBatch == 0, "lists are whole batches");
+    // entry of class lane % 4 at sub-list position `slot`
+    E* dst = list + entry_index(row, ((lane & 3) - static_cast<int>(row & 3)) & 3, cap);
+    int left = 0;
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int m = magnitude(k);
+        if (m >= limit && at < cap / 4) {
+            const int c = static_cast<int>(threadIdx.x) + kListThreads * k;
+            E e;
+            if constexpr (PAIR) e = E{a[k], b[k], c, 0};
+            else e = E{a[k], c};
+            dst[at * 4 * kGroup] = e;
+            ++at;
+        } else {
+            left = max(left, m);
+        }
+    }
+    if (threadIdx.x < 4) {
+        const float none = __int_as_float(0x7fc00000);
+        E e;
+        if constexpr (PAIR) e = E{none, none, static_cast<int>(threadIdx.x), 0};
+        else e = E{none, static_cast<int>(threadIdx.x)};
+        for (int slot = here; slot < slots; ++slot) dst[slot * 4 * kGroup] = e;
+    }
+    left = __reduce_max_sync(0xffffffffu, left);
+    if (lane == 0) lefts[warp] = left;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        len[row] = min(total, cap);
-        rest[row] = left;
+#pragma unroll
+        for (int k = 1; k < WARPS; ++k) left = max(left, lefts[k]);
+        len[row] = longest > 0 ? 4 * slots : 0;
+        rest[row] = __int_as_float(left);
     }
 }
 
@@ -201,7 +240,7 @@ __global__ void __launch_bounds__(256) extreme_sample_kernel(const Problem P) {
         const float* urow = P.xu.ptr + b * P.xu.stride_row;
         const float* wrow = P.w.ptr + o * P.w.stride_row;
         float lo = kFloor, up = kFloor;
-#pragma unroll 4
+#pragma unroll 8
         for (int c = 4 * lane; c < P.C; c += 128) {
             const float4 x4 = *reinterpret_cast<const float4*>(xrow + c);  // (rows are whole 16-byte pieces)
             const float4 u4 = BOUND ? *reinterpret_cast<const float4*>(urow + c) : x4;
@@ -303,16 +342,18 @@ __global__ void __launch_bounds__(256) extreme_sample_kernel(const Problem P) {
 
 // The maximum over one operand's lists.  WSIDE: S samples in shared memory, the weight rows' lists walked (sets y and pos);
 // else: S weight rows in shared memory, the samples' lists walked (merged into y and pos).
+//
+// A lane owns a list and S outputs.  What bounds the walk is the load / store pipe: a step of 32 lists costs 4 S / 4 wavefronts
+// of shared memory and about 4.5 of list entries, hence as many rows per list as fit (S = 8) where the lists are long; the
+// samples' lists are short, and four rows leave room for two blocks, one filling its tile while the other walks.
 template <bool BOUND, bool WSIDE, int S>
-__global__ void __launch_bounds__(kScanThreads) extreme_scan_kernel(const Problem P, int splits) {
+__global__ void __launch_bounds__(kScanThreads, S == 4 ? 2 : 1) extreme_scan_kernel(const Problem P, int splits) {
     stream_order_begin();
     if (P.t.words[0] != 0) return;
     extern __shared__ float4 tile4[];
-    constexpr int Q = S / 4;           // lanes that share a list
-    constexpr int LISTS = 32 / Q;      // lists of a warp
+    constexpr int H = S / 4;
     constexpr bool PAIR_TILE = BOUND && WSIDE, PAIR_LIST = BOUND && !WSIDE;
     constexpr int CAP = WSIDE ? kListW : kListX;
-    constexpr int kBatch = PAIR_LIST ? 4 : 8;  // entries in flight beside those being worked on
     using E = typename EntryOf<PAIR_LIST>::type;
     const int C4 = (P.C + 3) / 4;      // (rows of the operands are whole 16-byte pieces)
     const long long block = blockIdx.x / splits;
@@ -331,118 +372,143 @@ __global__ void __launch_bounds__(kScanThreads) extreme_scan_kernel(const Proble
         if (!__syncthreads_or(any)) return;
     }
     auto fill = [&](const Operand& v, float* dst) {
+#pragma unroll 5
         for (int i = threadIdx.x; i < C4 * S; i += kScanThreads) {
             const int r = i % S, c = i / S;
-            float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (row0 + r < tile_rows) q = *reinterpret_cast<const float4*>(v.ptr + (row0 + r) * v.stride_row + 4 * c);
-            dst[(4 * c + 0) * S + r] = q.x;
-            dst[(4 * c + 1) * S + r] = q.y;
-            dst[(4 * c + 2) * S + r] = q.z;
-            dst[(4 * c + 3) * S + r] = q.w;
+            float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (row0 + r < tile_rows) t = *reinterpret_cast<const float4*>(v.ptr + (row0 + r) * v.stride_row + 4 * c);
+            // the four stores of neighbouring pieces start at different channels: no two lanes of a store on one bank
+            if (c & 1) t = make_float4(t.y, t.z, t.w, t.x);
+            if (c & 2) t = make_float4(t.z, t.w, t.x, t.y);
+            dst[(4 * c + (c & 3)) * S + r] = t.x;
+            dst[(4 * c + ((c + 1) & 3)) * S + r] = t.y;
+            dst[(4 * c + ((c + 2) & 3)) * S + r] = t.z;
+            dst[(4 * c + ((c + 3) & 3)) * S + r] = t.w;
         }
     };
     fill(WSIDE ? P.x : P.w, tile);
     if (PAIR_TILE) fill(P.xu, tile_up);
     __syncthreads();
-    const int q = lane % Q;
-    const long long chunks = (list_rows + LISTS - 1) / LISTS;
+    // of a channel's two 16-byte halves a lane reads first the one that its neighbours four lists on do not (H = 2)
+    const int swap = H == 2 ? (lane >> 2) & 1 : 0;
+    const long long chunks = (list_rows + 31) / 32;
     for (long long chunk = static_cast<long long>(split) * (kScanThreads / 32) + warp; chunk < chunks;
          chunk += static_cast<long long>(splits) * (kScanThreads / 32)) {
-        const long long l = chunk * LISTS + lane / Q;
-        const int n = l < list_rows ? len[l] : 0;
-        int most = n;
+        const long long l = chunk * 32 + lane;
+        const long long row = l < list_rows ? l : list_rows - 1;  // (lanes beyond the last list repeat it)
+        const int n = max(len[row], kBatch);
+        const int most = __reduce_max_sync(0xffffffffu, n);
+        float best[S], best_up[S];
+        int batch[S];  // first entry of the batch that last raised the maximum; kTie: a later batch reached it too
+        constexpr int kTie = 1 << 30;
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, d));
-        float best[4], best_up[4];
-        int batch[4];  // first entry of the batch that last raised the maximum
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < S; ++e) {
             best[e] = best_up[e] = kFloor;
-            batch[e] = -1;
+            batch[e] = 0;
         }
-        const E* entries = list + (l / kGroup * CAP) * kGroup + l % kGroup;
-        auto load = [&](E (&en)[kBatch], int k0) {
+        const E* entries = list + (row / kGroup * CAP) * kGroup + row % kGroup;
+        auto gather = [&](const float* from, int c, float (&v)[S]) {
 #pragma unroll
-            for (int u = 0; u < kBatch; ++u) {
-                en[u] = E{};
-                if (k0 + u < n) en[u] = entries[(k0 + u) * kGroup];
+            for (int h = 0; h < H; ++h) {
+                const float4 t = *reinterpret_cast<const float4*>(from + c * S + 4 * (h ^ swap));
+                v[4 * h] = t.x; v[4 * h + 1] = t.y; v[4 * h + 2] = t.z; v[4 * h + 3] = t.w;
             }
         };
-        auto gather = [&](const float* from, int c, float (&v)[4]) {
-            const float4 t = *reinterpret_cast<const float4*>(from + c * S + 4 * q);
-            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-        };
-        E now[kBatch];
-        load(now, 0);
-        for (int k0 = 0; k0 < most; k0 += kBatch) {
-            E next[kBatch];
-            load(next, k0 + kBatch);
-            float top[4];
+        // (lanes whose list has ended keep their last batch and work on it again without taking the result)
+        auto load = [&](E (&en)[kBatch], int k0) {
+            if (k0 < n) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) top[e] = 0.0f;
+                for (int u = 0; u < kBatch; ++u) en[u] = entries[(k0 + u) * kGroup];
+            }
+        };
+        auto work = [&](const E (&en)[kBatch], int k0) {
+            float top[S];
+#pragma unroll
+            for (int e = 0; e < S; ++e) top[e] = 0.0f;
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
-                if (k0 + u < n) {
-                    float tv[4], sv[4];
-                    gather(tile, now[u].c, tv);
-                    if constexpr (PAIR_TILE) gather(tile_up, now[u].c, sv);
+                float tv[S], sv[S];
+                gather(tile, en[u].c, tv);
+                if constexpr (PAIR_TILE) gather(tile_up, en[u].c, sv);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        if constexpr (PAIR_TILE) visit<true>(tv[e], sv[e], now[u].v, best[e], best_up[e]);
-                        else if constexpr (PAIR_LIST) visit<true>(now[u].lo, now[u].up, tv[e], best[e], best_up[e]);
-                        else top[e] = fmaxf(top[e], fabsf(now[u].v - tv[e]));
-                    }
+                for (int e = 0; e < S; ++e) {
+                    if constexpr (PAIR_TILE) visit<true>(tv[e], sv[e], en[u].v, best[e], best_up[e]);
+                    else if constexpr (PAIR_LIST) visit<true>(en[u].lo, en[u].up, tv[e], best[e], best_up[e]);
+                    else top[e] = fmaxf(top[e], fabsf(en[u].v - tv[e]));
                 }
             }
             if constexpr (!BOUND) {
+                if (k0 < n) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (top[e] > best[e]) {  // channels ascend: the first batch of equal ones stays
-                        best[e] = top[e];
-                        batch[e] = k0;
-                    }
-            }
-#pragma unroll
-            for (int u = 0; u < kBatch; ++u) now[u] = next[u];
-        }
-        int at[4] = {0, 0, 0, 0};
-        if (!BOUND && P.pos) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (batch[e] >= 0) {
-#pragma unroll
-                    for (int u = kBatch - 1; u >= 0; --u) {
-                        if (batch[e] + u < n) {
-                            const E en = entries[(batch[e] + u) * kGroup];
-                            float lv, tv = tile[en.c * S + 4 * q + e];
-                            if constexpr (PAIR_LIST) lv = en.lo;
-                            else lv = en.v;
-                            const float d = WSIDE ? tv - lv : lv - tv;  // x - w
-                            if (fabsf(d) == best[e]) at[e] = en.c | (d < 0.0f ? static_cast<int>(0x80000000u) : 0);
+                    for (int e = 0; e < S; ++e)
+                        if (top[e] >= best[e]) {
+                            batch[e] = top[e] > best[e] ? k0 : batch[e] | kTie;
+                            best[e] = top[e];
                         }
-                    }
                 }
+            }
+        };
+        if constexpr (S == 4) {
+            E en[kBatch];
+            for (int k0 = 0; k0 < most; k0 += kBatch) {
+                load(en, k0);
+                work(en, k0);
+            }
+        } else {
+            E even[kBatch], odd[kBatch];
+            load(even, 0);
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) odd[u] = even[u];
+            for (int k0 = 0; k0 < most; k0 += 2 * kBatch) {
+                load(odd, k0 + kBatch);
+                work(even, k0);
+                load(even, k0 + 2 * kBatch);
+                if (k0 + kBatch < most) work(odd, k0 + kBatch);
             }
         }
         if (l >= list_rows) continue;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const long long r = row0 + 4 * q + e;
+        for (int e = 0; e < S; ++e) {
+            const int in_tile = 4 * ((e / 4) ^ swap) + e % 4;
+            const long long r = row0 + in_tile;
             if (r >= tile_rows) continue;
             const long long i = WSIDE ? r * P.CO + l : l * P.CO + r;
-            if (BOUND) {
+            if constexpr (BOUND) {
                 P.y[i] = WSIDE ? best[e] : fmaxf(P.y[i], best[e]);
                 P.yu[i] = WSIDE ? best_up[e] : fmaxf(P.yu[i], best_up[e]);
-            } else if (WSIDE) {
-                P.y[i] = best[e];
-                if (P.pos) P.pos[i] = at[e];
             } else {
-                const float old = P.y[i];
-                if (P.pos) {
-                    const int c = at[e] & 0x7fffffff;
-                    if (best[e] > old || (best[e] == old && best[e] > kFloor && c < (P.pos[i] & 0x7fffffff))) P.pos[i] = at[e];
+                const float old = WSIDE ? kFloor : P.y[i];
+                int at = 0;
+                if (P.pos && best[e] > kFloor && best[e] >= old) {
+                    // the lowest channel that attains the maximum: in the batch that raised it, or anywhere after a tie
+                    const bool tie = (batch[e] & kTie) != 0;
+                    const int from = tie ? 0 : batch[e], to = tie ? n : from + kBatch;
+                    int first = 0x7fffffff;
+                    for (int k = from; k < to; k += kBatch) {
+                        E en[kBatch];
+#pragma unroll
+                        for (int u = 0; u < kBatch; ++u) en[u] = entries[(k + u) * kGroup];
+#pragma unroll
+                        for (int u = 0; u < kBatch; ++u) {
+                            float lv;
+                            const float tv = tile[en[u].c * S + in_tile];
+                            if constexpr (PAIR_LIST) lv = en[u].lo;
+                            else lv = en[u].v;
+                            const float d = WSIDE ? tv - lv : lv - tv;  // x - w
+                            if (fabsf(d) == best[e] && en[u].c < first) {
+                                first = en[u].c;
+                                at = en[u].c | (d < 0.0f ? static_cast<int>(0x80000000u) : 0);
+                            }
+                        }
+                    }
+                    if (!WSIDE && (best[e] > old || first < (P.pos[i] & 0x7fffffff))) P.pos[i] = at;
                 }
-                if (best[e] > old) P.y[i] = best[e];
+                if (WSIDE) {
+                    P.y[i] = best[e];
+                    if (P.pos) P.pos[i] = at;
+                } else if (best[e] > old) {
+                    P.y[i] = best[e];
+                }
             }
         }
     }
@@ -460,15 +526,25 @@ __global__ void __launch_bounds__(256) extreme_check_kernel(const Problem P, uns
     stream_order_begin();
     if (P.t.words[0] != 0) return;
     const bool shift = P.sub != nullptr || P.add != nullptr;
-    for (long long b = blockIdx.y; b < P.B; b += gridDim.y) {
-        const float rest_b = P.t.x_rest[b];
-        for (int o = blockIdx.x * 256 + threadIdx.x; o < P.CO; o += gridDim.x * 256) {
-            const long long i = b * P.CO + o;
-            const float lo = P.y[i], up = BOUND ? P.yu[i] : lo;
-            if (proven(fminf(lo, up), P.t.w_rest[o], rest_b)) {
+    for (long long b0 = blockIdx.y * 4LL; b0 < P.B; b0 += gridDim.y * 4LL) {
+        const int o = blockIdx.x * 256 + threadIdx.x;
+        if (o >= P.CO) continue;
+        const float rest_o = P.t.w_rest[o];
+        float lo[4], up[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (b0 + k < P.B) {
+                lo[k] = P.y[(b0 + k) * P.CO + o];
+                up[k] = BOUND ? P.yu[(b0 + k) * P.CO + o] : lo[k];
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (b0 + k >= P.B) break;
+            const long long i = (b0 + k) * P.CO + o;
+            if (proven(fminf(lo[k], up[k]), rest_o, P.t.x_rest[b0 + k])) {
                 if (shift) {
-                    P.y[i] = epilogue(lo, o, P);
-                    if (BOUND) P.yu[i] = epilogue(up, o, P);
+                    P.y[i] = epilogue(lo[k], o, P);
+                    if (BOUND) P.yu[i] = epilogue(up[k], o, P);
                 }
             } else {
                 const unsigned h = atomicAdd(reinterpret_cast<unsigned*>(&P.t.words[2]), 1u);
@@ -537,9 +613,6 @@ unsigned most_hard_of(long long B, int CO) {
 }
 
 int round4(int c) { return (c + 3) & ~3; }
-// samples (weight rows) a scan block holds: 8 where they fit, else 4
-int tile_rows_of(int C, int arrays) { return static_cast<long long>(round4(C)) * 8 * 4 * arrays <= kMaxTile ? 8 : 4; }
-
 template <class K>
 int allow_smem(K kernel, bool (&configured)[64], int bytes) {
     int dev = 0;
@@ -558,9 +631,9 @@ int launch_scan_s(const Problem& P, cudaStream_t st) {
     if (r != kOk) return r;
     const int smem = round4(P.C) * S * 4 * (BOUND && WSIDE ? 2 : 1);
     const long long tiles = ((WSIDE ? P.B : P.CO) + S - 1) / S;
-    const long long chunks = ((WSIDE ? P.CO : P.B) + 32 / (S / 4) - 1) / (32 / (S / 4));
+    const long long chunks = ((WSIDE ? P.CO : P.B) + 31) / 32;
     // blocks that share a tile's lists: as few as fill the chip's last wave well (each fills its own tile)
-    const int resident = 148 * (2 * (smem + 1024) <= 227 * 1024 ? 2 : 1);
+    const int resident = 148 * (S == 4 && 2 * (smem + 1024) <= 227 * 1024 ? 2 : 1);
     int splits = 1;
     double best = 0.0;
     for (int k = 1; k <= 16 && k * (kScanThreads / 32) <= chunks + kScanThreads / 32 - 1; ++k) {
@@ -577,8 +650,24 @@ int launch_scan_s(const Problem& P, cudaStream_t st) {
 }
 template <bool BOUND, bool WSIDE>
 int launch_scan(const Problem& P, cudaStream_t st) {
-    return tile_rows_of(P.C, BOUND && WSIDE ? 2 : 1) == 8 ? launch_scan_s<BOUND, WSIDE, 8>(P, st)
-                                                          : launch_scan_s<BOUND, WSIDE, 4>(P, st);
+    if constexpr (WSIDE)
+        if (static_cast<long long>(round4(P.C)) * 8 * 4 * (BOUND ? 2 : 1) <= kMaxTile) return launch_scan_s<BOUND, WSIDE, 8>(P, st);
+    return launch_scan_s<BOUND, WSIDE, 4>(P, st);
+}
+
+template <bool PAIR>
+int launch_lists(const Operand& v, const Operand& second, long long rows, int C, int cap, const float* threshold,
+                 typename EntryOf<PAIR>::type* list, int* len, float* rest, int* words, cudaStream_t st) {
+    const unsigned grid = static_cast<unsigned>(rows);
+    if (C <= 12 * kListThreads)
+        return launch_after(extreme_lists_kernel<PAIR, 12>, grid, kListThreads, 0, st, v, second, C, cap, threshold, list, len,
+                            rest, words);
+    if (C <= 20 * kListThreads)
+        return launch_after(extreme_lists_kernel<PAIR, 20>, grid, kListThreads, 0, st, v, second, C, cap, threshold, list, len,
+                            rest, words);
+    static_assert(kListKeep == 24, "the longest row");
+    return launch_after(extreme_lists_kernel<PAIR, 24>, grid, kListThreads, 0, st, v, second, C, cap, threshold, list, len,
+                        rest, words);
 }
 
 template <bool BOUND>
@@ -589,15 +678,16 @@ int run(const Problem& P, cudaStream_t st) {
     const float* thresholds = reinterpret_cast<const float*>(P.t.words + kThresholdWord);
     int r = launch_after(extreme_sample_kernel<BOUND>, kSampleBlocks, 256, 0, st, P);
     if (r == kOk)
-        r = launch_after(extreme_lists_kernel<false>, static_cast<unsigned>(P.CO), kListThreads, 0, st, P.w, P.w, P.C, kListW,
-                         thresholds, static_cast<Entry1*>(P.t.w_list), P.t.w_len, P.t.w_rest, P.t.words);
+        r = launch_lists<false>(P.w, P.w, P.CO, P.C, kListW, thresholds, static_cast<Entry1*>(P.t.w_list), P.t.w_len, P.t.w_rest,
+                                P.t.words, st);
     if (r == kOk)
-        r = launch_after(extreme_lists_kernel<BOUND>, static_cast<unsigned>(P.B), kListThreads, 0, st, P.x, P.xu, P.C, kListX,
-                         thresholds + 1, static_cast<EX*>(P.t.x_list), P.t.x_len, P.t.x_rest, P.t.words);
+        r = launch_lists<BOUND>(P.x, P.xu, P.B, P.C, kListX, thresholds + 1, static_cast<EX*>(P.t.x_list), P.t.x_len,
+                                P.t.x_rest, P.t.words, st);
     if (r == kOk) r = launch_scan<BOUND, true>(P, st);
     if (r == kOk) r = launch_scan<BOUND, false>(P, st);
     if (r == kOk) {
-        const dim3 grid(static_cast<unsigned>((P.CO + 255) / 256), static_cast<unsigned>(P.B < 65535 ? P.B : 65535));
+        const long long rows4 = (P.B + 3) / 4;
+        const dim3 grid(static_cast<unsigned>((P.CO + 255) / 256), static_cast<unsigned>(rows4 < 65535 ? rows4 : 65535));
         r = launch_after(extreme_check_kernel<BOUND>, grid, 256, 0, st, P, most_hard_of(P.B, P.CO));
     }
     if (r == kOk) r = launch_after(extreme_resolve_kernel<BOUND>, 148 * 8, 256, 0, st, P);
