@@ -379,6 +379,26 @@ __global__ void row_absmax_strided_kernel(Operand v, long long rows, int inner, 
     }
 }
 
+// The gradients a scatter adds into, cleared in one launch (a memset per gradient costs a launch each, and the scatter could
+// not be set up behind it: 128 x 64 x 16 x 16 convolution step at p = inf 313 -> 306 us, bounds of
+// 100 x 1023 -> 500, forward + backward, 100 -> 95).
+struct ZeroArgs {
+    float* p[3];
+    long long n[3];
+};
+__global__ void __launch_bounds__(kBlock) zero_kernel(const ZeroArgs A) {
+    stream_order_begin();
+    const long long first = blockIdx.x * (long long)kBlock + threadIdx.x, step = (long long)gridDim.x * kBlock;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float* p = A.p[k];
+        if (p == nullptr) continue;
+        const long long n4 = (reinterpret_cast<uintptr_t>(p) & 15u) == 0 ? A.n[k] / 4 : 0;
+        for (long long i = first; i < n4; i += step) reinterpret_cast<float4*>(p)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (long long i = 4 * n4 + first; i < A.n[k]; i += step) p[i] = 0.0f;
+    }
+}
+
 // One thread per output element, in output-layout order (coalesced reads of go / pos).
 __global__ void inf_scatter_kernel(const float* go, const int* pos, float* gx, float* gw,
                                    Shape s) {
@@ -535,20 +555,25 @@ SideJob side_reduce_job(const float* part, float* gw, long long count, int tiles
                    static_cast<int>(gated_blocks(blocks_for(threads), run_if_nonzero ? gate : nullptr))};
 }
 
+static int launch_zero(const ZeroArgs& A, cudaStream_t st) {
+    long long most = 0;
+    for (int k = 0; k < 3; ++k)
+        if (A.p[k] && A.n[k] > most) most = A.n[k];
+    return most > 0 ? launch_after(zero_kernel, blocks_for(most / 4), kBlock, 0, st, A) : kOk;
+}
+
 int launch_inf_scatter(const float* go, const int* pos, float* gx, float* gw, const Shape& s, cudaStream_t st) {
-    cudaError_t e = cudaSuccess;
-    if (gx) e = cudaMemsetAsync(gx, 0, sizeof(float) * (size_t)s.B * s.CI * s.HW, st);
-    if (e == cudaSuccess && gw) e = cudaMemsetAsync(gw, 0, sizeof(float) * (size_t)s.CO * s.CIg, st);
-    if (e != cudaSuccess) return cuda_status(e);
+    const long long nx = static_cast<long long>(s.B) * s.CI * s.HW, nw = static_cast<long long>(s.CO) * s.CIg;
+    const int r = launch_zero(ZeroArgs{{gx, gw, nullptr}, {nx, nw, 0}}, st);
+    if (r != kOk) return r;
     return launch_after(inf_scatter_kernel, blocks_for((long long)s.B * s.CO * s.HW), kBlock, 0, st, go, pos, gx, gw, s);
 }
 
 int launch_bound_scatter(const float* gol, const float* gou, const int* posl, const int* posu, float* gxl, float* gxu,
                          float* gw, const Shape& s, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(gxl, 0, sizeof(float) * (size_t)s.B * s.CI * s.HW, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(gxu, 0, sizeof(float) * (size_t)s.B * s.CI * s.HW, st);
-    if (e == cudaSuccess && gw) e = cudaMemsetAsync(gw, 0, sizeof(float) * (size_t)s.CO * s.CIg, st);
-    if (e != cudaSuccess) return cuda_status(e);
+    const long long nx = static_cast<long long>(s.B) * s.CI * s.HW, nw = static_cast<long long>(s.CO) * s.CIg;
+    const int r = launch_zero(ZeroArgs{{gxl, gxu, gw}, {nx, nx, nw}}, st);
+    if (r != kOk) return r;
     return launch_after(bound_scatter_kernel, blocks_for((long long)s.B * s.CO * s.HW), kBlock, 0, st, gol, gou, posl,
                         posu, gxl, gxu, gw, s);
 }
