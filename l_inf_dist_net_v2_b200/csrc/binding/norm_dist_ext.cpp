@@ -184,14 +184,17 @@ void fold(Tensor& cols, Tensor& x, std::pair<int, int> kernel, int stride, int p
 // backward pass of a Python autograd function costs 55 us on the host before it does anything (the engine's thread takes
 // the interpreter lock and runs the Python backward), more than the kernels of a small layer; here it is 25 us.  The
 // entry points return None for whatever the Python functions should see instead (other devices, types and layouts, shapes
-// that do not fit): those raise or handle it.
+// that do not fit, tensors that carry a forward-mode tangent or intercept operators): those raise or handle it.
+//
+// The linear maps (mean shift, unfold) replace torch operators that can be differentiated and transformed in any way, so
+// where a gradient is itself to be differentiated, or is not plain memory, their backward steps are those operators.
 
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 bool plain(const Tensor& t, int64_t dim) {
     return t.is_cuda() && t.scalar_type() == at::kFloat && t.layout() == at::kStrided && t.dim() == dim && t.is_contiguous() &&
-           t.numel() > 0;
+           t.numel() > 0 && t.has_storage() && !t._fw_grad(0).defined() && !t.unsafeGetTensorImpl()->is_python_dispatch();
 }
 bool fits(const Tensor& x, const Tensor& w, int64_t G) {
     return plain(x, 3) && plain(w, 2) && x.device() == w.device() && G > 0 && G <= w.size(0) && w.size(1) * G == x.size(1);
@@ -290,6 +293,11 @@ void subtract_mean(const Tensor& x, const Tensor& running_mean, double momentum,
     else check(ldn_mean_shift_planes(a, B, C, HW, rm, m, y, stream()), "mean_shift_planes");
 }
 
+// whether a kernel of this package may compute a linear map's gradient from this one
+bool plain_gradient(const Tensor& grad, int64_t dim) {
+    return plain(grad, dim) && !(at::GradMode::is_enabled() && grad.requires_grad());
+}
+
 struct MeanShiftFn : public torch::autograd::Function<MeanShiftFn> {
     static Tensor forward(AutogradContext*, Tensor x, Tensor running_mean, double momentum) {
         Tensor out = at::empty_like(x);
@@ -297,7 +305,9 @@ struct MeanShiftFn : public torch::autograd::Function<MeanShiftFn> {
         return out;
     }
     static variable_list backward(AutogradContext*, variable_list grads) {
-        Tensor go = grads[0].contiguous(), gx = at::empty_like(go);
+        Tensor go = grads[0].contiguous();
+        if (!plain_gradient(go, 3)) return {go - go.mean(at::IntArrayRef({0, 2}), true), Tensor(), Tensor()};
+        Tensor gx = at::empty_like(go);
         subtract_mean(go, Tensor(), 0.0, gx);
         return {gx, Tensor(), Tensor()};
     }
@@ -314,11 +324,16 @@ struct UnfoldFn : public torch::autograd::Function<UnfoldFn> {
         return cols;
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
-        Tensor go = grads[0].contiguous();
+        Tensor go = grads[0].contiguous(), gx;
         const std::vector<int64_t> n = ctx->saved_data["geometry"].toIntVector();
-        Tensor gx = at::empty(ctx->saved_data["image"].toIntVector(), go.options());
-        fold(go, gx, {static_cast<int>(n[0]), static_cast<int>(n[1])}, static_cast<int>(n[2]), static_cast<int>(n[3]),
-             static_cast<int>(n[4]));
+        const std::vector<int64_t> image = ctx->saved_data["image"].toIntVector();
+        if (plain_gradient(go, 3)) {
+            gx = at::empty(image, go.options());
+            fold(go, gx, {static_cast<int>(n[0]), static_cast<int>(n[1])}, static_cast<int>(n[2]), static_cast<int>(n[3]),
+                 static_cast<int>(n[4]));
+        } else {
+            gx = at::col2im(go, {image[2], image[3]}, {n[0], n[1]}, {n[4], n[4]}, {n[3], n[3]}, {n[2], n[2]});
+        }
         return {gx, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };

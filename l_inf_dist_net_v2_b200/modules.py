@@ -19,6 +19,13 @@ def apply_if_not_none(paras, func):
     return [None if x is None else func(x) for x in paras]
 
 
+def _plain_backward(grad):
+    """Whether a kernel of this package may compute a linear map's gradient from this one: it is plain memory and nothing
+    differentiates or transforms the result."""
+    return not (torch.is_grad_enabled() or _C.transformed() or torch.autograd.forward_ad._current_level >= 0
+                or not torch._C._has_storage(grad))
+
+
 class _MeanShiftRowsF(torch.autograd.Function):
     """x - (mean of x over the batch) for (B, C, 1) inputs, with the running-mean update, as one kernel per pass.
     d(out)/d(x) = I - (1/B) 1 1^T, so the backward pass is the same kernel on the incoming gradient."""
@@ -31,6 +38,8 @@ class _MeanShiftRowsF(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_output):
+        if not _plain_backward(grad_output):
+            return grad_output - grad_output.mean(0, keepdim=True), None, None
         grad_output = grad_output.contiguous()
         grad_input = torch.empty_like(grad_output)
         _C.mean_shift_rows(grad_output, None, 0.0, grad_input)
@@ -50,8 +59,10 @@ class _UnfoldF(torch.autograd.Function):
         return cols
 
     @staticmethod
-    @torch.autograd.function.once_differentiable
     def backward(ctx, grad_cols):
+        if not _plain_backward(grad_cols):
+            kernel_size, stride, padding, dilation = ctx.geometry
+            return F.fold(grad_cols, ctx.image[2:], kernel_size, dilation, padding, stride), None, None, None, None, None
         grad_cols = grad_cols.contiguous()
         grad_x = torch.empty(ctx.image, device=grad_cols.device, dtype=torch.float32)
         _C.fold(grad_cols, grad_x, *ctx.geometry)
@@ -60,7 +71,8 @@ class _UnfoldF(torch.autograd.Function):
 
 def _unfold(x, kernel_size, dilation, padding, stride):
     """F.unfold(x, kernel_size, dilation, padding, stride); contiguous float32 CUDA images with one stride, padding and
-    dilation for both axes take this package's kernel, everything else (and every error) torch's."""
+    dilation for both axes take this package's kernel, everything else (and every error, and what differentiates or traces
+    operators in another way than reverse mode) torch's."""
     plain = (all(isinstance(v, int) for v in (dilation, padding, stride)) and dilation > 0 and padding >= 0 and stride > 0
              and x.is_cuda and x.dtype == torch.float32 and x.dim() == 4 and x.is_contiguous() and x.numel() > 0
              and min(kernel_size) > 0)
@@ -68,9 +80,12 @@ def _unfold(x, kernel_size, dilation, padding, stride):
         out = [(s + 2 * padding - dilation * (k - 1) - 1) // stride + 1 for s, k in zip(x.shape[2:], kernel_size)]
         columns = out[0] * out[1] * kernel_size[0] * kernel_size[1]
         if min(out) > 0 and max(columns, x.size(2) * x.size(3), *(s + 2 * padding for s in x.shape[2:])) < 1 << 30:
-            ext = _C.native()
-            cols = None if ext is None else ext.unfold_columns(x, out[0] * out[1], kernel_size, stride, padding, dilation)
-            return cols if cols is not None else _UnfoldF.apply(x, out[0] * out[1], kernel_size, stride, padding, dilation)
+            if _C.native() is not None:
+                cols = _C.native().unfold_columns(x, out[0] * out[1], kernel_size, stride, padding, dilation)
+                if cols is not None:
+                    return cols
+            elif not _C.transformed() and torch.autograd.forward_ad._current_level < 0:
+                return _UnfoldF.apply(x, out[0] * out[1], kernel_size, stride, padding, dilation)
     return F.unfold(x, kernel_size, dilation, padding, stride)
 
 

@@ -131,3 +131,80 @@ def test_what_was_refused_stays_refused():
     xr = x.clone().requires_grad_()
     grad, = torch.autograd.grad(ldn.norm_dist(xr, w, 8.0).sum(), xr, create_graph=True)
     assert not grad.requires_grad
+
+
+def _twice(fn, x, c):
+    """The gradient of a cubic of fn(x), and the gradient of that gradient's square."""
+    g, = torch.autograd.grad((fn(x) ** 3 * c).sum(), x, create_graph=True)
+    assert g.requires_grad
+    return g.detach(), torch.autograd.grad(g.square().sum(), x)[0]
+
+
+@pytest.mark.parametrize("shape", [(9, 6, 1), (5, 6, 4), (5, 6, 7)])
+def test_mean_shift_differentiates_twice(both, shape):
+    import l_inf_dist_net_v2_b200 as ldn
+    torch.manual_seed(0)
+    layer = ldn.MeanShift(shape[1], affine=False).cuda()
+    x = torch.randn(shape, device="cuda", requires_grad=True)
+    c = torch.randn(shape, device="cuda")
+    got = both(lambda: _twice(lambda t: layer(t)[0], x, c))
+    layer.fused = False
+    want = _twice(lambda t: layer(t)[0], x, c)
+    for result in got:
+        for a, b in zip(result, want):
+            assert torch.allclose(a, b, rtol=1e-5, atol=1e-5 * b.abs().max().item())
+
+
+@pytest.mark.parametrize("geometry", [((3, 3), 1, 1, 1), ((3, 2), 1, 0, 2), ((2, 2), 2, 1, 1)])
+def test_unfold_differentiates_twice(both, geometry):
+    from l_inf_dist_net_v2_b200.modules import _unfold
+    torch.manual_seed(0)
+    x = torch.randn(3, 4, 8, 8, device="cuda", requires_grad=True)
+    c = torch.randn_like(torch.nn.functional.unfold(x, *geometry))
+    want = _twice(lambda t: torch.nn.functional.unfold(t, *geometry), x, c)
+    for result in both(lambda: _twice(lambda t: _unfold(t, *geometry), x, c)):
+        for a, b in zip(result, want):
+            assert torch.allclose(a, b, rtol=1e-5, atol=1e-5 * b.abs().max().item())
+
+
+def test_what_sees_operators_sees_them(both):
+    """Forward-mode tangents and traced graphs of what torch operators computed before there was a kernel for it."""
+    import l_inf_dist_net_v2_b200 as ldn
+    from l_inf_dist_net_v2_b200.modules import _unfold
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils._python_dispatch import TorchDispatchMode
+    torch.manual_seed(0)
+    layer = ldn.MeanShift(6, affine=False).cuda()
+    plain = ldn.MeanShift(6, affine=False).cuda()
+    plain.fused = False
+    cases = [(lambda t: layer(t)[0], lambda t: plain(t)[0], (5, 6, 4)),
+             (lambda t: _unfold(t, (3, 3), 1, 1, 1), lambda t: torch.nn.functional.unfold(t, (3, 3), 1, 1, 1), (2, 3, 6, 6))]
+
+    class Seen(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.names.append(func.name())
+            return func(*args, **(kwargs or {}))
+
+    def check():
+        for fn, reference, shape in cases:
+            x, v = torch.randn(shape, device="cuda"), torch.randn(shape, device="cuda")
+            with torch.autograd.forward_ad.dual_level():
+                got, want = (torch.autograd.forward_ad.unpack_dual(f(torch.autograd.forward_ad.make_dual(x, v)))
+                             for f in (fn, reference))
+            assert torch.allclose(got.tangent, want.tangent, rtol=1e-5, atol=1e-5)
+            names = []
+            for f in (fn, reference):
+                with Seen() as mode:
+                    mode.names = []
+                    f(x)
+                names.append(mode.names)
+            assert names[0] == names[1]
+            # gradients in batches, which vmap the backward step
+            x.requires_grad_()
+            ups = torch.randn(3, *reference(x).shape, device="cuda")
+            got, want = (torch.autograd.grad(f(x), x, ups, is_grads_batched=True)[0] for f in (fn, reference))
+            assert torch.allclose(got, want, rtol=1e-5, atol=1e-5)
+    both(check)
+    graph = make_fx(cases[1][0])(torch.randn(2, 3, 6, 6, device="cuda"))
+    x = torch.randn(2, 3, 6, 6, device="cuda")
+    assert torch.equal(graph(x), cases[1][1](x))
