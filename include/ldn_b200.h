@@ -63,7 +63,9 @@ LDN_API int ldn_release_scratch(void);
  * find it large enough (no counterpart in the reference).  Scratch cannot grow while the stream is being captured
  * into a CUDA graph -- a call that would need to returns status 6 -- so before a capture either run the same calls
  * once eagerly or reserve here.  Once a capture has used an arena, a later growth keeps the earlier blocks until
- * ldn_release_scratch, so graphs captured before stay valid.
+ * ldn_release_scratch, so graphs captured before stay valid.  A reserved arena grows only for a call that cannot run
+ * without: calls that have a faster path with more scratch (large p = inf layers, about 12 MB more) take it when the
+ * reservation has room for it, and otherwise the path that the scratch suffices for.
  */
 LDN_API int ldn_reserve_scratch(ldn_stream_t stream, unsigned long long bytes);
 

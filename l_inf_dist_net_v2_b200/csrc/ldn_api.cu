@@ -102,7 +102,8 @@ struct Call {
     std::unique_lock<std::mutex> lock;  // the arena's call mutex, released when the entry point returns
 };
 
-int begin_call(Call* c, ldn_stream_t stream, size_t scratch_bytes) {
+// `more` bytes beyond scratch_bytes, which the call can do without, are there if *granted says so.
+int begin_call(Call* c, ldn_stream_t stream, size_t scratch_bytes, size_t more = 0, bool* granted = nullptr) {
     int r = get_device_ctx(&c->ctx);
     if (r != kOk) return r;
     c->st = reinterpret_cast<cudaStream_t>(stream);
@@ -110,7 +111,9 @@ int begin_call(Call* c, ldn_stream_t stream, size_t scratch_bytes) {
     r = find_arena(c->st, &c->arena);
     if (r != kOk) return r;
     c->lock = std::unique_lock<std::mutex>(*static_cast<std::mutex*>(c->arena->call_mutex));
-    if ((r = ensure_arena(c->arena, c->st, scratch_bytes)) != kOk) return r;
+    const bool extended = more > 0 && extend_arena(c->arena, c->st, scratch_bytes + more);
+    if (granted) *granted = extended;
+    if (!extended && (r = ensure_arena(c->arena, c->st, scratch_bytes)) != kOk) return r;
     c->bump = Bump{c->arena->base, 0, c->arena->capacity};
     return kOk;
 }
@@ -452,19 +455,13 @@ int norm_dist_backward(const float* go, const float* x, const float* w, const fl
     return norm_dist_backward_part(go, x, w, y, s, gx, gw, p, stream, false, accumulate_gx);
 }
 
-// Whether `bytes` of scratch can be had on this stream: an arena that is large enough, or may grow (not during a capture).
-// Paths that need more scratch than the general one are taken only then, so that a reservation made for that one suffices.
-bool scratch_available(ldn_stream_t stream, size_t bytes) {
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    Arena* arena;
-    if (find_arena(st, &arena) != kOk) return false;
-    std::lock_guard<std::mutex> lock(*static_cast<std::mutex*>(arena->call_mutex));
-    return ensure_arena(arena, st, bytes) == kOk;
-}
-
-// Large fully connected p = inf problems on the whole chip start from the extreme channels (ldn_extreme.cu).
-bool extreme_path(const DeviceCtx* ctx, const Shape& s, bool bound) {
-    return s.G == 1 && s.HW == 1 && cap_for(ctx) == ctx->sm_count && extreme_applies(s.M, s.CO, s.CI, bound);
+// Large fully connected p = inf problems on the whole chip start from the extreme channels (ldn_extreme.cu): the scratch
+// that takes, 0 for all others.  A call that cannot have it takes the general path alone.
+constexpr size_t kExtremeMaxScratch = size_t(1) << 30;
+size_t extreme_path_bytes(const DeviceCtx* ctx, const Shape& s, bool bound) {
+    if (s.G != 1 || s.HW != 1 || cap_for(ctx) != ctx->sm_count || !extreme_applies(s.M, s.CO, s.CI, bound)) return 0;
+    const size_t bytes = extreme_scratch_bytes(s.M, s.CO, bound);
+    return bytes <= kExtremeMaxScratch ? bytes : 0;
 }
 
 int inf_forward(const float* x, const float* w, const Shape& s, float* y, int* pos, ldn_stream_t stream,
@@ -477,11 +474,9 @@ int inf_forward(const float* x, const float* w, const Shape& s, float* y, int* p
     const bool inplace = x_inplace_kmajor(x, s);
     size_t need = (inplace ? 0 : x_scratch_bytes(x, s)) + w_scratch_bytes(w, s) +
                   partial_bytes(cap_for(ctx), fwd_acc_arrays(kind));
-    const bool extreme = extreme_path(ctx, s, false) &&
-                         scratch_available(stream, need + extreme_scratch_bytes(s.M, s.CO, false));
-    if (extreme) need += extreme_scratch_bytes(s.M, s.CO, false);
+    bool extreme = false;
     Call c;
-    if ((r = begin_call(&c, stream, need)) != kOk) return r;
+    if ((r = begin_call(&c, stream, need, extreme_path_bytes(ctx, s, false), &extreme)) != kOk) return r;
     c.col_sub = col_sub;
     c.col_add = col_add;
     View xv, wv;
@@ -514,11 +509,9 @@ int bound_forward(const float* xl, const float* xu, const float* w, const Shape&
     if (r != kOk) return r;
     const size_t xfloats = canonical_floats(s.CIg, s.M, s.G);
     size_t need = 2 * pad256(xfloats * sizeof(float)) + w_scratch_bytes(w, s) + 2 * partial_bytes(cap_for(ctx), 5);
-    const bool extreme = !pl && extreme_path(ctx, s, true) &&
-                         scratch_available(stream, need + extreme_scratch_bytes(s.M, s.CO, true));
-    if (extreme) need += extreme_scratch_bytes(s.M, s.CO, true);
+    bool extreme = false;
     Call c;
-    if ((r = begin_call(&c, stream, need)) != kOk) return r;
+    if ((r = begin_call(&c, stream, need, pl ? 0 : extreme_path_bytes(ctx, s, true), &extreme)) != kOk) return r;
     c.col_sub = col_sub;
     c.col_add = col_add;
     float* lc = c.bump.take<float>(xfloats);
@@ -596,7 +589,8 @@ LDN_API int ldn_reserve_scratch(ldn_stream_t stream, unsigned long long bytes) {
     int r = find_arena(st, &arena);
     if (r != kOk) return r;
     std::lock_guard<std::mutex> lock(*static_cast<std::mutex*>(arena->call_mutex));
-    return ensure_arena(arena, st, static_cast<size_t>(bytes));
+    if ((r = ensure_arena(arena, st, static_cast<size_t>(bytes))) == kOk) arena->reserved = true;
+    return r;
 }
 
 LDN_API int ldn_check_status(ldn_stream_t stream) {

@@ -198,9 +198,13 @@ struct Arena {
                        // use the same stream cannot interleave launches that share the scratch block
     bool graph_used;   // a call was issued on this arena while its stream was being captured
     void* retired;     // std::vector<void*>*: earlier blocks that captured graphs may still refer to
+    bool reserved = false;  // the caller chose the size (ldn_reserve_scratch): it grows only for what a call cannot do without
+    size_t refused = 0;     // not 0: the smallest size that could not be had for a growth that a call can do without
 };
 int find_arena(cudaStream_t stream, Arena** out);
 int ensure_arena(Arena* arena, cudaStream_t stream, size_t bytes);  // caller holds call_mutex
+// The same for scratch that a call can do without: false leaves the arena as it is.
+bool extend_arena(Arena* arena, cudaStream_t stream, size_t bytes);
 
 // Bump allocator over an arena (256-byte granularity).
 struct Bump {

@@ -79,11 +79,8 @@ int find_arena(cudaStream_t stream, Arena** out) {
     return kOk;
 }
 
-// Makes the arena's block at least `bytes` large.  The caller holds the arena's call mutex, so no other host thread
-// is enqueueing kernels that use the block.  While the stream is being captured nothing may be allocated or waited
-// for, so a growth is refused then; and once a capture has used the arena, earlier blocks are kept (a captured
-// graph replays with the addresses it was recorded with) until ldn_release_scratch.
-int ensure_arena(Arena* arena, cudaStream_t stream, size_t bytes) {
+// Whether the stream is being captured; notes in the arena that a graph refers to its block then.
+static bool note_capture(Arena* arena, cudaStream_t stream) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
         cudaGetLastError();
@@ -91,21 +88,38 @@ int ensure_arena(Arena* arena, cudaStream_t stream, size_t bytes) {
     }
     const bool capturing = cs != cudaStreamCaptureStatusNone;
     if (capturing) arena->graph_used = true;
-    if (bytes <= arena->capacity) return kOk;
-    if (capturing) return kCaptureGrowth;
-    // kernels already queued on the stream may still use the old block
+    return capturing;
+}
+
+// What to ask for when the block has to hold `bytes`.
+static size_t growth(const Arena* arena, size_t bytes) {
+    size_t want = bytes + bytes / 8;
+    // kept blocks add up: grow geometrically then, so that they stay below twice the final size
+    if (arena->graph_used && want < arena->capacity + arena->capacity / 2) want = arena->capacity + arena->capacity / 2;
+    return (want + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
+}
+
+// Gives the arena's block up (kernels already queued on the stream may still use it, captured graphs for good).
+static void drop_block(Arena* arena, cudaStream_t stream) {
     cudaStreamSynchronize(stream);
     if (arena->base) {
         if (arena->graph_used) static_cast<std::vector<void*>*>(arena->retired)->push_back(arena->base);
         else cudaFree(arena->base);
     }
     arena->base = nullptr;
-    const size_t old_cap = arena->capacity;
     arena->capacity = 0;
-    size_t want = bytes + bytes / 8;
-    // kept blocks add up: grow geometrically then, so that they stay below twice the final size
-    if (arena->graph_used && want < old_cap + old_cap / 2) want = old_cap + old_cap / 2;
-    want = (want + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
+}
+
+// Makes the arena's block at least `bytes` large.  The caller holds the arena's call mutex, so no other host thread
+// is enqueueing kernels that use the block.  While the stream is being captured nothing may be allocated or waited
+// for, so a growth is refused then; and once a capture has used the arena, earlier blocks are kept (a captured
+// graph replays with the addresses it was recorded with) until ldn_release_scratch.
+int ensure_arena(Arena* arena, cudaStream_t stream, size_t bytes) {
+    const bool capturing = note_capture(arena, stream);
+    if (bytes <= arena->capacity) return kOk;
+    if (capturing) return kCaptureGrowth;
+    size_t want = growth(arena, bytes);
+    drop_block(arena, stream);
     void* p = nullptr;
     if (cudaMalloc(&p, want) != cudaSuccess) {
         cudaGetLastError();
@@ -118,6 +132,30 @@ int ensure_arena(Arena* arena, cudaStream_t stream, size_t bytes) {
     arena->base = static_cast<char*>(p);
     arena->capacity = want;
     return kOk;
+}
+
+// The new block is there before the old one goes, so a device without room for it costs the call nothing but the faster
+// path; and it is not asked for again.  (Relaxed capture mode: another stream's capture, which an allocation in the default
+// mode would end, is none of this call's business.)
+bool extend_arena(Arena* arena, cudaStream_t stream, size_t bytes) {
+    const bool capturing = note_capture(arena, stream);
+    if (bytes <= arena->capacity) return true;
+    if (capturing || arena->reserved || (arena->refused != 0 && bytes >= arena->refused)) return false;
+    const size_t want = growth(arena, bytes);
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    const bool there = cudaMalloc(&p, want) == cudaSuccess;
+    if (there) {
+        drop_block(arena, stream);
+        arena->base = static_cast<char*>(p);
+        arena->capacity = want;
+    } else {
+        cudaGetLastError();
+        arena->refused = bytes;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return there;
 }
 
 int release_arenas() {
