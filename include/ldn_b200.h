@@ -97,8 +97,10 @@ LDN_API unsigned long long ldn_kernel_launches(void);
 
 /*
  * Per-kernel timing (no counterpart in the reference): while enabled, every launch of a tile kernel is bracketed by
- * a CUDA-event pair on its stream; ldn_last_tile_kernel_ms waits for the latest pair and returns the duration of that
- * one kernel in milliseconds (-1 if nothing was recorded).  One pair per process: use from one thread, one device.
+ * a CUDA-event pair on its stream, but for launches that run or return at once by a word in device memory;
+ * ldn_last_tile_kernel_ms waits for the latest pair and returns the duration of that one kernel in milliseconds.  It
+ * returns -1 if nothing was recorded since timing was enabled, or after a large p = inf call that starts from the
+ * extreme channels, whose tile kernels are of that kind.  One pair per process: use from one thread, one device.
  */
 LDN_API void ldn_enable_kernel_timing(int enabled);
 LDN_API float ldn_last_tile_kernel_ms(void);

@@ -486,6 +486,7 @@ int inf_forward(const float* x, const float* w, const Shape& s, float* y, int* p
     if (extreme) {
         ExtremeScratch t;
         if (!extreme_take_scratch(&c.bump, s.M, s.CO, false, &t)) return kWorkspace;
+        timing_forget();  // (the tile kernels behind it are gated, their launches not bracketed)
         r = launch_extreme(as_operand(xv), as_operand(xv), as_operand(wv), s.M, s.CO, s.CI, false, y, nullptr, pos, col_sub,
                            col_add, t, &c.gate, c.st);
         if (r != kOk) return r;
@@ -525,6 +526,7 @@ int bound_forward(const float* xl, const float* xu, const float* w, const Shape&
     if (extreme) {
         ExtremeScratch t;
         if (!extreme_take_scratch(&c.bump, s.M, s.CO, true, &t)) return kWorkspace;
+        timing_forget();  // (the tile kernels behind it are gated, their launches not bracketed)
         r = launch_extreme(as_operand(lv), as_operand(uv), as_operand(wv), s.M, s.CO, s.CI, true, yl, yu, nullptr, col_sub,
                            col_add, t, &c.gate, c.st);
         if (r != kOk) return r;

@@ -230,6 +230,7 @@ int make_tensor_map(CUtensorMap* map, const float* base, const unsigned long lon
 // optional CUDA-event pair around the most recent tile-kernel launch (ldn_diag.cu); no-ops unless enabled
 void timing_before(cudaStream_t st);
 void timing_after(cudaStream_t st);
+void timing_forget();  // there is no launch to report until the next pair
 
 // host-side launch counter and optional per-CTA trace buffer (ldn_diag.cu)
 unsigned long long* trace_buffer();

@@ -16,6 +16,7 @@ unsigned long long* trace_buffer() { return g_trace; }
 
 // Event pair around the latest tile-kernel launch, for per-kernel roofline numbers.
 bool g_timing = false;
+bool g_timed = false;  // the events hold a pair that ldn_last_tile_kernel_ms may report
 cudaEvent_t g_ev0 = nullptr, g_ev1 = nullptr;
 void timing_before(cudaStream_t st) {
     if (!g_timing) return;
@@ -26,8 +27,11 @@ void timing_before(cudaStream_t st) {
     cudaEventRecord(g_ev0, st);
 }
 void timing_after(cudaStream_t st) {
-    if (g_timing && g_ev1) cudaEventRecord(g_ev1, st);
+    if (!g_timing || !g_ev1) return;
+    cudaEventRecord(g_ev1, st);
+    g_timed = true;
 }
+void timing_forget() { g_timed = false; }
 
 namespace {
 constexpr int kProbeThreads = 256;
@@ -129,10 +133,13 @@ extern "C" {
 
 LDN_API void ldn_set_trace_buffer(unsigned long long* device_buffer) { g_trace = device_buffer; }
 
-LDN_API void ldn_enable_kernel_timing(int enabled) { g_timing = enabled != 0; }
+LDN_API void ldn_enable_kernel_timing(int enabled) {
+    g_timing = enabled != 0;
+    if (g_timing) g_timed = false;
+}
 
 LDN_API float ldn_last_tile_kernel_ms(void) {
-    if (!g_ev0 || !g_ev1) return -1.0f;
+    if (!g_timed) return -1.0f;
     if (cudaEventSynchronize(g_ev1) != cudaSuccess) return -1.0f;
     float ms = -1.0f;
     if (cudaEventElapsedTime(&ms, g_ev0, g_ev1) != cudaSuccess) return -1.0f;

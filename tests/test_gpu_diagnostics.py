@@ -105,6 +105,27 @@ def test_kernel_timing_hook(lib):
     assert 0.0 < ms < 50.0
 
 
+def test_kernel_timing_hook_reports_no_earlier_call(lib):
+    from l_inf_dist_net_v2_b200 import norm_dist_cuda as C
+    x, w = torch.rand(512, 2560, 1, device="cuda"), torch.randn(5200, 2560, device="cuda")
+    y, y2 = torch.empty(512, 5200, 1, device="cuda"), torch.empty(512, 5200, 1, device="cuda")
+    lib.ldn_enable_kernel_timing(1)
+    try:
+        for large in (lambda: C.inf_dist_forward_nograd(x, w, y, 1),  # start from the extreme channels
+                      lambda: C.bound_inf_dist_forward_nograd(x, x, w, y, y2, 1)):
+            C.norm_dist_forward(x, w, y, 1, 8.0)
+            assert lib.ldn_last_tile_kernel_ms() > 0.0
+            large()
+            assert lib.ldn_last_tile_kernel_ms() == -1.0
+        C.norm_dist_forward(x, w, y, 1, 8.0)
+        lib.ldn_enable_kernel_timing(0)
+        assert lib.ldn_last_tile_kernel_ms() > 0.0
+        lib.ldn_enable_kernel_timing(1)
+        assert lib.ldn_last_tile_kernel_ms() == -1.0
+    finally:
+        lib.ldn_enable_kernel_timing(0)
+
+
 def test_two_host_threads_on_one_stream(lib):
     """Calls from two host threads that use the same stream share one scratch block; the library serialises such
     calls, so each one's helper kernels and tile kernel stay together in stream order."""
