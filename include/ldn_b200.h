@@ -106,6 +106,14 @@ LDN_API void ldn_enable_kernel_timing(int enabled);
 LDN_API float ldn_last_tile_kernel_ms(void);
 
 /*
+ * How the last call on the stream went, if it was a large p = inf call that starts from the extreme channels of both
+ * operands (no counterpart in the reference): waits for the stream and writes outcome[0] = 1 if the device chose the
+ * dense kernels (else 0), outcome[1] = the number of outputs that the lists left to a full search.  Status 1 if the
+ * last call was another one.  Not during a capture.
+ */
+LDN_API int ldn_last_extreme_outcome(ldn_stream_t stream, int outcome[2]);
+
+/*
  * Tracing hook (no counterpart in the reference): while a non-null device buffer is set, every CTA of every
  * tile-engine launch writes four 64-bit words at buffer[4 * cta]: SM id, start and end time (globaltimer, ns)
  * and its number of k-steps.  The buffer must hold 4 * (number of SMs) words; pass NULL to switch it off.

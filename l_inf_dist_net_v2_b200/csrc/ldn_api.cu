@@ -115,6 +115,7 @@ int begin_call(Call* c, ldn_stream_t stream, size_t scratch_bytes, size_t more =
     if (granted) *granted = extended;
     if (!extended && (r = ensure_arena(c->arena, c->st, scratch_bytes)) != kOk) return r;
     c->bump = Bump{c->arena->base, 0, c->arena->capacity};
+    c->arena->extreme_words = nullptr;  // (the scratch that held them is this call's now)
     return kOk;
 }
 
@@ -490,6 +491,7 @@ int inf_forward(const float* x, const float* w, const Shape& s, float* y, int* p
         r = launch_extreme(as_operand(xv), as_operand(xv), as_operand(wv), s.M, s.CO, s.CI, false, y, nullptr, pos, col_sub,
                            col_add, t, &c.gate, c.st);
         if (r != kOk) return r;
+        c.arena->extreme_words = t.words;
     }
     r = run_forward(c, kind, 0, xv, nullptr, wv, s, y, nullptr, pos, nullptr, nullptr, INFINITY, inplace);
     if (r != kOk || !pos) return r;
@@ -530,6 +532,7 @@ int bound_forward(const float* xl, const float* xu, const float* w, const Shape&
         r = launch_extreme(as_operand(lv), as_operand(uv), as_operand(wv), s.M, s.CO, s.CI, true, yl, yu, nullptr, col_sub,
                            col_add, t, &c.gate, c.st);
         if (r != kOk) return r;
+        c.arena->extreme_words = t.words;
     }
     if (!pl) return run_forward(c, FwdKind::Bound, 0, lv, &uv, wv, s, yl, yu, nullptr, nullptr, nullptr, INFINITY);
     if ((s.CIg + kTileK - 1) / kTileK <= g_bound_one_pass_stages) {
@@ -607,6 +610,22 @@ LDN_API int ldn_check_status(ldn_stream_t stream) {
     const int v = *arena->status_host;
     *arena->status_host = 0;
     return v;
+}
+
+LDN_API int ldn_last_extreme_outcome(ldn_stream_t stream, int* outcome) {
+    if (!outcome) return kBadArgument;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    Arena* arena;
+    int r = find_arena(st, &arena);
+    if (r != kOk) return r;
+    std::lock_guard<std::mutex> lock(*static_cast<std::mutex*>(arena->call_mutex));
+    if (!arena->extreme_words) return kBadArgument;
+    int words[kExtremeOutcomeWords];
+    cudaError_t e = cudaMemcpyAsync(words, arena->extreme_words, sizeof(words), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_status(e);
+    extreme_outcome(words, outcome);
+    return kOk;
 }
 
 LDN_API int ldn_norm_dist_forward(const float* input, const float* weight, int B, int CO, int CI, int G, int HW,

@@ -199,6 +199,7 @@ struct Arena {
     bool graph_used;   // a call was issued on this arena while its stream was being captured
     void* retired;     // std::vector<void*>*: earlier blocks that captured graphs may still refer to
     bool reserved = false;  // the caller chose the size (ldn_reserve_scratch): it grows only for what a call cannot do without
+    const int* extreme_words = nullptr;  // device words of the last call, if that started from the extreme channels
     size_t refused = 0;     // not 0: the smallest size that could not be had for a growth that a call can do without
 };
 int find_arena(cudaStream_t stream, Arena** out);

@@ -108,6 +108,7 @@ static void drop_block(Arena* arena, cudaStream_t stream) {
     }
     arena->base = nullptr;
     arena->capacity = 0;
+    arena->extreme_words = nullptr;
 }
 
 // Makes the arena's block at least `bytes` large.  The caller holds the arena's call mutex, so no other host thread

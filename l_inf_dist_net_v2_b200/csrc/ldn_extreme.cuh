@@ -31,4 +31,12 @@ bool extreme_take_scratch(Bump* bump, long long B, int CO, bool bound, ExtremeSc
 int launch_extreme(Operand x, Operand xu, Operand w, long long B, int CO, int C, bool bound, float* y, float* yu, int* pos,
                    const float* sub, const float* add, const ExtremeScratch& t, const int** dense_gate, cudaStream_t st);
 
+// What a call's first words say once it is done: whether the dense kernels computed the outputs, and how many the lists left
+// to be searched in full.
+constexpr int kExtremeOutcomeWords = 3;
+inline void extreme_outcome(const int (&words)[kExtremeOutcomeWords], int outcome[2]) {
+    outcome[0] = words[0] != 0 ? 1 : 0;
+    outcome[1] = words[2];
+}
+
 }  // namespace ldn

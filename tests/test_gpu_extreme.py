@@ -117,3 +117,50 @@ def test_unaligned_rows_streams_and_capture(dense):
     C.inf_dist_forward_nograd(x2, w, out[3], 1)
     assert torch.equal(out[2], out[3])
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[3].flip(0))
+
+
+def _outcome():
+    """(whether the device chose the dense kernels, outputs searched in full) of the last call on the current stream."""
+    import ctypes
+
+    from l_inf_dist_net_v2_b200._lib import check, lib
+    out = (ctypes.c_int * 2)()
+    check(lib.ldn_last_extreme_outcome(torch.cuda.current_stream().cuda_stream, out), "last_extreme_outcome")
+    return out[0], out[1]
+
+
+# what each kind of data is there to reach; the others may go either way
+CHOICE = {"images": 0, "hidden": 0, "hard rows": 0, "identity": 0, "flat": 1, "nan": 1, "inf": 1}
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_which_kernels_gave_the_result(shape):
+    """The bits above are the dense kernels' whichever ran: here, that the lists gave them where they should, and that some
+    outputs were left to the full search."""
+    from l_inf_dist_net_v2_b200 import norm_dist_cuda as C
+    B, CO, CI = shape
+    y, pos, yu = torch.empty(B, CO, 1, device="cuda"), torch.empty(B, CO, 1, device="cuda", dtype=torch.int32), \
+        torch.empty(B, CO, 1, device="cuda")
+    searched = 0
+    for kind, dense in CHOICE.items():
+        x, w = _operands(kind, B, CO, CI)
+        for call in (lambda: C.inf_dist_forward(x, w, y, pos, 1), lambda: C.inf_dist_forward_nograd(x, w, y, 1),
+                     lambda: C.bound_inf_dist_forward_nograd(x - 8 / 255, x + 8 / 255, w, y, yu, 1)):
+            call()
+            chosen, hard = _outcome()
+            assert chosen == dense, kind
+            if not dense:
+                searched += hard
+    assert searched > 0
+
+
+def test_no_outcome_of_another_call():
+    from l_inf_dist_net_v2_b200 import norm_dist_cuda as C
+    B, CO, CI = SHAPES[0]
+    x, w = _operands("images", B, CO, CI)
+    y = torch.empty(B, CO, 1, device="cuda")
+    C.inf_dist_forward_nograd(x, w, y, 1)
+    assert _outcome()[0] == 0
+    C.norm_dist_forward(x[:8].contiguous(), w[:64].contiguous(), y.view(-1)[:512].view(8, 64, 1), 1, 8.0)
+    with pytest.raises(RuntimeError, match="status 1"):
+        _outcome()
