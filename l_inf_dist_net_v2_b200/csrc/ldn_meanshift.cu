@@ -55,7 +55,9 @@ mean_shift_rows_kernel(const float* x, float* out, float* running_mean,
 // x, out: [B][C][HW].  Bound by the bytes of x and out, so x is read once: a cluster of 8 CTAs owns a channel, every CTA
 // sums its eighth of the channel's B HW elements and keeps them in registers (up to kKeep 16-byte pieces per thread, 64 K
 // elements per channel; what lies beyond is read again), the eight sums are exchanged through distributed shared memory and
-// added in rank order (deterministic).  V = elements per piece: 4 where planes are whole aligned pieces, else 1.
+// added in rank order (deterministic).  Sums are 64 bits wide beyond a thread's 16-byte piece: in 32 bits the mean of a
+// channel of 32768 elements was further off than torch's, by up to 1.6 times behind the subtraction, which takes most of the
+// value away.  V = elements per piece: 4 where planes are whole aligned pieces, else 1.
 // (Mean, running mean and subtraction by torch operators were five launches forward and four backward, 50 us of a
 // 128 x 64 x 16 x 16 layer step; with this kernel and the fold by rows that step takes 310 us instead of 388.)
 constexpr int kCluster = 8;
@@ -68,8 +70,8 @@ mean_shift_planes_kernel(const float* x, float* out, float* running_mean, float 
     stream_order_begin();
     namespace cg = cooperative_groups;
     const cg::cluster_group cluster = cg::this_cluster();
-    __shared__ float warp_sums[kPlaneThreads / 32];
-    __shared__ float total;
+    __shared__ double warp_sums[kPlaneThreads / 32];
+    __shared__ double total;
     const int c = blockIdx.x / kCluster, rank = blockIdx.x % kCluster;
     const long long row = HW / V, n = B * row;  // pieces per plane and per channel
     const long long first = n * rank / kCluster + threadIdx.x, last = n * (rank + 1) / kCluster;
@@ -78,7 +80,7 @@ mean_shift_planes_kernel(const float* x, float* out, float* running_mean, float 
         return (b * C + c) * HW + (t - b * row) * V;
     };
     float keep[kKeep][V];
-    float s = 0.0f;
+    double s = 0.0;
 #pragma unroll
     for (int k = 0; k < kKeep; ++k) {
         const long long t = first + k * kPlaneThreads;
@@ -93,27 +95,24 @@ mean_shift_planes_kernel(const float* x, float* out, float* running_mean, float 
             }
         }
     }
+    auto piece_sum = [](const float* v) { return V == 4 ? (v[0] + v[1]) + (v[2] + v[3]) : v[0]; };
 #pragma unroll
-    for (int k = 0; k < kKeep; ++k)
-#pragma unroll
-        for (int e = 0; e < V; ++e) s += keep[k][e];
-    for (long long t = first + kKeep * kPlaneThreads; t < last; t += kPlaneThreads)
-#pragma unroll
-        for (int e = 0; e < V; ++e) s += x[offset(t) + e];
+    for (int k = 0; k < kKeep; ++k) s += piece_sum(keep[k]);
+    for (long long t = first + kKeep * kPlaneThreads; t < last; t += kPlaneThreads) s += piece_sum(x + offset(t));
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
     if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x / 32] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
-        s = 0.0f;
+        s = 0.0;
         for (int w = 0; w < kPlaneThreads / 32; ++w) s += warp_sums[w];
         total = s;
     }
     cluster.sync();
-    float mean = 0.0f;
+    s = 0.0;
 #pragma unroll
-    for (int q = 0; q < kCluster; ++q) mean += *cluster.map_shared_rank(&total, q);
-    mean /= static_cast<float>(B) * static_cast<float>(HW);
+    for (int q = 0; q < kCluster; ++q) s += *cluster.map_shared_rank(&total, q);
+    const float mean = static_cast<float>(s / (static_cast<double>(B) * HW));
     cluster.sync();  // every rank has read the others' sums before one of them may exit
     if (running_mean && rank == 0 && threadIdx.x == 0)
         running_mean[c] = running_mean[c] * (1.0f - momentum) + momentum * mean;

@@ -49,3 +49,15 @@ def test_convolution_shaped_backward(shape, p):
     tol = 1e-5 if p == int(p) else 1e-4
     for got, want in ((gx, ex), (gw, ew)):
         assert float((got.cpu().double().view(-1) - want.reshape(-1)).abs().max()) <= tol * float(want.abs().max())
+
+
+@pytest.mark.parametrize("shape", [(32, 128, 1024), (40, 2, 2500), (33, 3, 2501), (700, 2, 2304)])
+def test_mean_of_planes_is_rounded_once(shape):
+    """The sum of n < 2^29 equal fp32 terms is exact in 64 bits, so a constant channel's mean is the constant."""
+    import l_inf_dist_net_v2_b200 as ldn
+    ms = ldn.MeanShift(shape[1], affine=False).cuda().train()
+    for value in (0.1, 7.3, -1 / 3):
+        x = torch.full(shape, value, device="cuda", requires_grad=True)
+        out, _, _ = ms(x)
+        grad, = torch.autograd.grad(out, x, torch.full_like(x, value))
+        assert not out.any() and not grad.any()
