@@ -1,20 +1,30 @@
 // p = inf forward of large fully connected layers: max_c |x[b, c] - w[o, c]| without visiting most channels.
 //
 // A channel can only be the maximum of output (b, o) where |x| or |w| is large.  So every row of either operand gets a list
-// of its extreme channels (|w| >= tau, |x| >= sigma) and the largest magnitude that is NOT in the list, rest_o and rest_b.
-// The maximum over the two lists' channels, M, is compared with fl(rest_o + rest_b): a channel in neither list has
-// |w| <= rest_o and |x| <= rest_b, hence |fl(x - w)| <= fl(rest_o + rest_b) (rounding is monotonic), so
-// M > fl(rest_o + rest_b) proves that M is the maximum over all channels and that no other channel equals it: value and
-// first channel are those of the dense kernel, bit for bit.  Outputs without the proof ("hard") are searched over all
-// channels.  All arithmetic is the dense kernel's fp32 subtraction and comparison.
+// of its extreme channels and the largest magnitude that is NOT in the list, rest_o and rest_b.  The maximum over the two
+// lists' channels, M, is compared with fl(rest_o + rest_b): a channel in neither list has |w| <= rest_o and |x| <= rest_b, hence
+// |fl(x - w)| <= fl(rest_o + rest_b) (rounding is monotonic), so M > fl(rest_o + rest_b) proves that M is the maximum over all
+// channels and that no other channel equals it: value and first channel are those of the dense kernel, bit for bit.  Outputs
+// without the proof ("hard") are searched over all channels.  All arithmetic is the dense kernel's fp32 subtraction and
+// comparison.
 //
-// tau and sigma come from the data: a sample of outputs is searched in full, tau + sigma is a low quantile of their maxima,
-// and the split between the two is the one with the fewest list entries by the magnitudes' histograms.  With weights
-// N(0, 1) about 60 of 3072 channels are visited for images in [0, 1], 170 of 5120 for activations of deviation 0.5.  Where
-// the lists would not be a small part of a row, anything is not finite, or too many outputs turn out hard, a device word
-// makes the dense kernels behind it run instead.
-// 512 x 5120 -> 5120 forward + backward: dense 1105 us, this path 505; certification of 512 x 3072 -> 5120 (value and bounds):
-// 1971 and 335.
+// A list holds the same number of channels in every row, the row's own largest ones, so rows may have any scale and a list
+// never overflows (with one threshold for all rows, rows whose scales differ by a tenth overflowed their lists: the walks ran
+// for nothing in front of the dense kernels).  The two lengths are chosen by trial on 592 outputs: their full maxima, and
+// what the rests of their two rows would be after lists of any length, tell how many of them each pair of lengths leaves
+// hard; the cheapest pair is taken, before anything is listed or walked.  Where no pair is cheaper than the dense kernels, or
+// anything is not finite, or far more outputs turn out hard than the samples said, a device word makes the dense kernels behind
+// run instead.
+// Forward with index / bounds in us, against the dense kernels' 1048 / 2349 (512 x 5120 -> 5120) and 677 / 1426 (512 x 3072 ->
+// 5120), w = N(0, 1) with rows scaled by exp(s N(0, 1)); one threshold for all rows in parentheses (+: dense behind the walks):
+//                           s = 0                    s = 0.05                 s = 0.1                   s = 0.4
+//   5120, x = N(0, 0.5^2)   373 / 701 (429 / 780)    359 / 696 (1531+/3240+)  369 / 699 (1091 / 2392)   416 / 768 (1091 / 2389)
+//   5120, x in [0, 1)       203 / 262 (220 / 326)    201 / 263 (308 / 556)    195 / 271 (1089 / 2392)   206 / 339 (1089 / 2393)
+//   3072, x = N(0, 0.5^2)   293 / 500 (341 / 541)    297 / 512 (396 / 637)    297 / 523 (1206+/1468)    344 / 543 (716 / 1468)
+//   3072, x in [0, 1)       162 / 209 (183 / 205)    162 / 211 (218 / 264)    162 / 187 (978+/1804+)    175 / 228 (715 / 1468)
+// Signs (w, x = +-1: nothing can be proven, the samples choose dense) 1083 / 2378 and 709 / 1461.  512 x 5120 -> 5120 layer,
+// forward + backward: dense 1105 us, one threshold 496, now 430; certification of 512 x 3072 -> 5120 (value and bounds): 1971,
+// 335 and 298.
 //
 // What bounds it: the gathers x[b, c] for a list's channels.  A block keeps S rows of one operand in shared memory as
 // [channel][S]; a lane owns a list, gathers four rows' values of a channel with one 16-byte read, and a warp's 32 lists lie
@@ -34,30 +44,43 @@ constexpr int kListW = 256;        // entries of a weight row's list, at most
 constexpr int kListX = 128;        // of a sample's
 constexpr int kGroup = 16;         // lists whose entries are interleaved
 constexpr int kListThreads = 256;
+constexpr int kListWarps = kListThreads / 32;
 constexpr int kMaxChannels = 6144;
-constexpr int kListKeep = kMaxChannels / kListThreads;  // channels a thread of extreme_lists_kernel holds
 constexpr int kScanThreads = 512;
 constexpr int kBatch = 8;          // entries a scan works on at a time (lists are whole batches long)
-constexpr int kSampleBlocks = 148;
-constexpr int kSamples = kSampleBlocks * 8;
-constexpr int kQuantile = 2;       // tau + sigma: this smallest of the samples' maxima (0.2 %)
+constexpr int kSamples = 148 * 4;
 constexpr int kMaxTile = 224 * 1024;
-// a gathered pair costs about 4 of the dense kernel's, and the samples' lists another pass over the weights
-constexpr int kDenseShare = 8;     // dense where the lists hold more than 1 / kDenseShare of a row
-constexpr int kSecondPass = 60;    // entries that pass costs
+
+// Lengths that are tried: kBatch (a + 1) entries of the weights' lists, kBatch b of the samples' (none at b = 0).
+constexpr int kLevelsW = kListW / kBatch, kLevelsX = kListX / kBatch + 1;
+// What a pair of lengths costs, in the walk of one entry of the weights' lists in tiles of eight rows (0.5 us of
+// 512 x 5120 -> 5120, bounds 0.8), fitted to lengths of 40 to 256 and 0 to 128 at 3072 and 5120 channels:
+//   the samples' lists at all, another pass over the weights and over the outputs: 52 - 54 us there, bounds 240;
+//   an entry of theirs (four rows per step of a list instead of eight) 1.0 us, bounds 1.2;
+//   one output in a hundred hard: 75 - 87 us at 5120 channels, 49 at 3072, bounds 100 and 63;
+//   filling the tiles and reading the outputs 45 us, and the lists themselves 56 us (in proportion to rows, not to outputs).
+// The dense kernels take a channel in 0.17 us there (without index), bounds 0.46.
+struct Costs {
+    float second_pass, second_entry, hard_channel, dense_channel;
+};
+template <bool BOUND>
+__device__ constexpr Costs costs() {
+    return BOUND ? Costs{290.0f, 1.7f, 2.5f, 1.0f / 2.5f} : Costs{100.0f, 2.0f, 3.2f, 1.0f / 3.5f};
+}
+constexpr float kFixedCost = 90.0f, kListCost = 11.0f;  // the latter per channel and row of the weights
+constexpr int kMostFailed = 6;  // hard samples, at most: 1 % (3 % of the outputs are more than can be searched in full)
+
+__host__ __device__ constexpr int round4(int c) { return (c + 3) & ~3; }
+// whether a tile of the weights' lists' walk holds eight samples (with both bounds), not four
+template <bool BOUND>
+__host__ __device__ constexpr bool eight_rows(int C) {
+    return round4(C) * 8 * 4 * (BOUND ? 2 : 1) <= kMaxTile;
+}
 
 // device words (cleared by every call): 0 dense gate, 1 finished sampling blocks, 2 hard outputs
-constexpr int kThresholdWord = 4;  // tau, sigma
-constexpr int kHistWord = 8;
-
-// magnitude histograms: 32 bins per octave from 2^-10 to 2^6 (what lies outside counts in the first / last bin)
-constexpr int kBins = 512;
-constexpr int kBinShift = 18;
-constexpr int kBinBase = (127 - 10) << (23 - kBinShift);
-__device__ __forceinline__ int bin_of(float m) {
-    return min(kBins - 1, max(0, (__float_as_int(m) >> kBinShift) - kBinBase));
-}
-__device__ __forceinline__ float bin_edge(int i) { return __int_as_float((i + kBinBase) << kBinShift); }
+constexpr int kLengthWord = 4;  // entries of a weight row's list, of a sample's
+constexpr int kTrialWord = 8;   // [level a][first level b that proves the sample, kLevelsX: none], counts of samples
+static_assert(kTrialWord + kLevelsW * (kLevelsX + 1) == kExtremeWords, "");
 
 // an entry: the value (bounds: lower and upper) and its channel
 struct Entry1 {
@@ -81,115 +104,161 @@ __host__ __device__ inline long long groups_of(long long rows) { return (rows + 
 __device__ __forceinline__ long long entry_index(long long row, int k, int cap) {
     return (row / kGroup * cap + k) * kGroup + row % kGroup;
 }
-__device__ __forceinline__ float block_max(float v, float* warps, int n_warps) {
+__device__ __forceinline__ float block_max(float v, float* warps) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = v;
     __syncthreads();
     v = warps[0];
-    for (int k = 1; k < n_warps; ++k) v = fmaxf(v, warps[k]);
+    for (int k = 1; k < kListWarps; ++k) v = fmaxf(v, warps[k]);
     return v;
 }
 
-// One block per row: the channels whose magnitude reaches the threshold; the row is read once, into registers, with all loads
-// in flight (KEEP channels per thread), and magnitudes are compared as integers (a sign bit less, not-a-numbers on top).
+// Magnitudes in order.  A block holds a row, thread t channels t + 256 k, magnitudes as integers (a sign bit less,
+// not-a-numbers on top); padding has magnitude 0.  The channels of a class (channel % 4, so lane % 4) are put in the order of
+// the bins of a histogram, 64 per octave and two octaves from half of a magnitude near the row's top (the fourth largest of
+// the warps' maxima: outliers do not move it, nor runs of zeros), higher ones first, any order within a bin.  emit(k, m, place)
+// is called for the places below `keep`; the return value is the largest magnitude of this thread's that got none, `top` the
+// largest of all.  Magnitudes below the last bin get no place.
+constexpr int kBins = 128;
+constexpr int kBinShift = 23 - 6;
+struct RankShared {
+    int bins[4 * kBins];  // [bin][class]: counts, then the next place
+    int warps[kListWarps];
+    int upper[4], stop[4], total[4];
+};
+template <int KEEP, class Magnitude, class Emit>
+__device__ __forceinline__ int rank_row(RankShared& sh, int keep, Magnitude magnitude, int& top, Emit emit) {
+    static_assert(kListThreads == 2 * kBins, "a thread scans two bins of a class");
+    const int t = threadIdx.x, lane = t & 31;
+    top = 0;
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) top = max(top, magnitude(k));
+    const int mine = __reduce_max_sync(0xffffffffu, top);
+    __syncthreads();  // (the arrays may still be read from an earlier call)
+    if (lane == 0) sh.warps[t >> 5] = mine;
+    sh.bins[t] = sh.bins[t + kListThreads] = 0;
+    __syncthreads();
+    const int v = sh.warps[lane & 7];
+    int above = 0;
+#pragma unroll
+    for (int j = 0; j < kListWarps; ++j) {
+        const int o = sh.warps[j];
+        above += (o > v || (o == v && j < (lane & 7))) ? 1 : 0;
+    }
+    const int near_top = __shfl_sync(0xffffffffu, v, __ffs(__ballot_sync(0xffffffffu, above == 3)) - 1);
+    // (finite: then no sum below overflows; rows with infinities go to the dense kernels)
+    const int cut = max(min(near_top, 0x7f7fffff) - (1 << 23), 1);
+    auto bin_of = [&](int m) { return min((m - cut) >> kBinShift, kBins - 1) * 4 + (lane & 3); };
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int m = magnitude(k);
+        if (m >= cut) atomicAdd(&sh.bins[bin_of(m)], 1);
+    }
+    __syncthreads();
+    // places: of class q, 64 threads with two bins each
+    const int q = t >> 6, lower_bin = 2 * (t & 63);
+    const int n0 = sh.bins[lower_bin * 4 + q], n1 = sh.bins[(lower_bin + 1) * 4 + q];
+    int sum = n0 + n1;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_down_sync(0xffffffffu, sum, d);
+        if (lane + d < 32) sum += o;
+    }
+    if ((t & 63) == 32) sh.upper[q] = sum;
+    __syncthreads();
+    if ((t & 32) == 0) sum += sh.upper[q];  // magnitudes in these two bins and above
+    const int first1 = sum - n0 - n1, first0 = first1 + n1;
+    sh.bins[(lower_bin + 1) * 4 + q] = first1;
+    sh.bins[lower_bin * 4 + q] = first0;
+    if (lower_bin == 0) sh.total[q] = sum;
+    // the lowest bin that has a place below `keep`
+    if (first0 < keep ? (lower_bin == 0 || sum >= keep) : first1 < keep) sh.stop[q] = first0 < keep ? lower_bin : lower_bin + 1;
+    __syncthreads();
+    const int limit = keep > 0 ? cut + (sh.stop[lane & 3] << kBinShift) : 0x7fffffff;
+    int left = 0;
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int m = magnitude(k);
+        bool listed = false;
+        if (m >= limit) {
+            const int place = atomicAdd(&sh.bins[bin_of(m)], 1);
+            if (place < keep) {
+                emit(k, m, place);
+                listed = true;
+            }
+        }
+        if (!listed) left = max(left, m);
+    }
+    return left;
+}
+__device__ __forceinline__ int magnitude_of(float v) { return __float_as_int(v) & 0x7fffffff; }
+constexpr int kInfinite = 0x7f800000;
+
+// One block per row: its list and its rest; the row is read once, into registers, with all loads in flight (KEEP channels per
+// thread).
 //
 // Order of a list.  A scan step reads one channel of each of a warp's lists from shared memory, 32 bytes at bank
 // 8 (channel % 4) (tiles of 8 rows), so four neighbouring lists read without conflicts if their channels differ modulo 4.
-// Entry k of row r's list therefore has channel % 4 == (k + r) % 4: four interleaved sub-lists, the shorter ones filled up
-// with entries that change nothing (NaN), so that a list is a whole number of batches, at least one.  A lane's channels are
-// all of class lane % 4, so places come from one count per lane.  Channels beyond `cap` entries count as not listed.
+// Entry k of row r's list therefore has channel % 4 == (k + r) % 4: four interleaved sub-lists with a quarter of the entries
+// each, filled up with entries that change nothing (NaN) where a class has fewer magnitudes near the row's top.
 template <bool PAIR, int KEEP>
-__global__ void __launch_bounds__(kListThreads, KEEP <= 12 ? 3 : 2)
-extreme_lists_kernel(Operand v, Operand second, int C, int cap, const float* threshold, typename EntryOf<PAIR>::type* list,
-                     int* len, float* rest, int* words) {
+__global__ void __launch_bounds__(kListThreads, KEEP <= 12 ? 4 : (PAIR && KEEP > 20 ? 2 : 3))
+extreme_lists_kernel(Operand v, Operand second, int C, int cap, int length_word, typename EntryOf<PAIR>::type* list,
+                     float* rest, int* words) {
     stream_order_begin();
     // (one decision per block: another block of this very kernel may set the word between two threads' reads)
     if (__syncthreads_or(words[0] != 0)) return;
     using E = typename EntryOf<PAIR>::type;
-    constexpr int WARPS = kListThreads / 32;
-    __shared__ int counts[WARPS][4], lefts[WARPS];
+    __shared__ RankShared sh;
     const long long row = blockIdx.x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int limit = __float_as_int(*threshold);
-    const float* src = v.ptr + row * v.stride_row + threadIdx.x;
-    const float* src2 = second.ptr + row * second.stride_row + threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31;
+    const int keep = words[length_word] / 4;
+    const float* src = v.ptr + row * v.stride_row + t;
+    const float* src2 = second.ptr + row * second.stride_row + t;
     float a[KEEP], b[PAIR ? KEEP : 1];
-    const int mine_n = C - static_cast<int>(threadIdx.x);  // this thread's channels: threadIdx.x + 256 k < C
+    const int mine_n = C - t;  // this thread's channels: t + 256 k < C
 #pragma unroll
     for (int k = 0; k < KEEP; ++k) {
         a[k] = kListThreads * k < mine_n ? src[kListThreads * k] : 0.0f;
         if (PAIR) b[k] = kListThreads * k < mine_n ? src2[kListThreads * k] : 0.0f;
     }
     auto magnitude = [&](int k) {
-        const int m = __float_as_int(a[k]) & 0x7fffffff;
-        return PAIR ? max(m, __float_as_int(b[k]) & 0x7fffffff) : m;
+        if constexpr (PAIR) return max(magnitude_of(a[k]), magnitude_of(b[k]));
+        else return magnitude_of(a[k]);
     };
-    int n = 0, top = 0;
+    int left = 0, top = 0;
+    if (keep == 0) {
 #pragma unroll
-    for (int k = 0; k < KEEP; ++k) {
-        const int m = magnitude(k);
-        top = max(top, m);
-        n += m >= limit ? 1 : 0;  // (the threshold is above 0, padding is not)
-    }
-    if (top >= 0x7f800000) words[0] = 1;  // infinite or not a number: dense
-    // places: exclusive sums over the lanes of a class, then over the warps
-    int at = n;
-#pragma unroll
-    for (int d = 4; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, at, d);
-        if (lane >= d) at += o;
-    }
-    if (lane >= 28) counts[warp][lane & 3] = at;
-    at -= n;
-    __syncthreads();
-    int longest = 0, here = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        int total = 0;
-#pragma unroll
-        for (int k = 0; k < WARPS; ++k) {
-            if (q == (lane & 3) && k < warp) at += counts[k][q];
-            total += counts[k][q];
-        }
-        longest = max(longest, total);
-        if (q == (lane & 3)) here = total;
-    }
-    longest = min(longest, cap / 4);
-    const int slots = max((longest + 1) & ~1, 2);  // of a sub-list, fillers included: kBatch entries are two slots
-    static_assert(kBatch == 8 && kListW % kBatch == 0 && kListX % kBatch == 0, "lists are whole batches");
-    // entry of class lane % 4 at sub-list position `slot`
-    E* dst = list + entry_index(row, ((lane & 3) - static_cast<int>(row & 3)) & 3, cap);
-    int left = 0;
-#pragma unroll
-    for (int k = 0; k < KEEP; ++k) {
-        const int m = magnitude(k);
-        if (m >= limit && at < cap / 4) {
-            const int c = static_cast<int>(threadIdx.x) + kListThreads * k;
+        for (int k = 0; k < KEEP; ++k) top = max(top, magnitude(k));
+        left = top;
+    } else {
+        // entry of class q at place `p`
+        auto entry_at = [&](int q, int p) { return list + entry_index(row, ((q - static_cast<int>(row & 3)) & 3) + 4 * p, cap); };
+        left = rank_row<KEEP>(sh, keep, magnitude, top, [&](int k, int, int place) {
+            const int c = t + kListThreads * k;
             E e;
             if constexpr (PAIR) e = E{a[k], b[k], c, 0};
             else e = E{a[k], c};
-            dst[at * 4 * kGroup] = e;
-            ++at;
-        } else {
-            left = max(left, m);
+            *entry_at(lane & 3, place) = e;
+        });
+        const int q = t >> 6;
+        for (int p = sh.total[q] + (t & 63); p < keep; p += 64) {
+            const float none = __int_as_float(0x7fc00000);
+            E e;
+            if constexpr (PAIR) e = E{none, none, q, 0};
+            else e = E{none, q};
+            *entry_at(q, p) = e;
         }
     }
-    if (threadIdx.x < 4) {
-        const float none = __int_as_float(0x7fc00000);
-        E e;
-        if constexpr (PAIR) e = E{none, none, static_cast<int>(threadIdx.x), 0};
-        else e = E{none, static_cast<int>(threadIdx.x)};
-        for (int slot = here; slot < slots; ++slot) dst[slot * 4 * kGroup] = e;
-    }
+    if (top >= kInfinite) words[0] = 1;  // infinite or not a number: dense
     left = __reduce_max_sync(0xffffffffu, left);
-    if (lane == 0) lefts[warp] = left;
+    if (lane == 0) sh.warps[t >> 5] = left;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (t == 0) {
 #pragma unroll
-        for (int k = 1; k < WARPS; ++k) left = max(left, lefts[k]);
-        len[row] = longest > 0 ? 4 * slots : 0;
+        for (int k = 1; k < kListWarps; ++k) left = max(left, sh.warps[k]);
         rest[row] = __int_as_float(left);
     }
 }
@@ -220,123 +289,96 @@ __device__ __forceinline__ void visit(float lo, float up, float w, float& best_l
     }
 }
 
-// A warp per sampled output: its maximum over all channels, and every fourth magnitude of its two rows into the histograms.
-// The last block to finish chooses tau and sigma, or the dense kernels.
-template <bool BOUND>
-__global__ void __launch_bounds__(256) extreme_sample_kernel(const Problem P) {
+// A block per sampled output: its maximum over all channels, and for every length of the weights' list the shortest list of
+// the sample's that would prove it.  The last block to finish chooses the two lengths, or the dense kernels.
+template <bool BOUND, int KEEP>
+__global__ void __launch_bounds__(kListThreads, KEEP <= 12 ? 3 : 2) extreme_sample_kernel(const Problem P) {
     stream_order_begin();
-    __shared__ int hist[2 * kBins];  // weights, inputs
-    __shared__ float warps[8];
+    __shared__ RankShared sh;
+    __shared__ float warps[kListWarps];
+    __shared__ int level_w[kLevelsW + 1], level_x[kLevelsX];  // largest magnitude among the places of a batch; last: without
+    __shared__ int trials[kLevelsW * (kLevelsX + 1)];
+    __shared__ unsigned long long best;
     __shared__ bool last;
-    const int tid = threadIdx.x, lane = tid & 31;
-    for (int i = tid; i < 2 * kBins; i += 256) hist[i] = 0;
-    __syncthreads();
-    const unsigned id = blockIdx.x * 8 + (tid >> 5);
-    {
-        // samples on a lattice that visits rows and outputs evenly (fractions of the golden ratio and of the square root of 2)
-        const long long b = static_cast<long long>((static_cast<unsigned long long>(id * 2654435769u) * P.B) >> 32);
-        const int o = static_cast<int>((static_cast<unsigned long long>(id * 1779033703u) * P.CO) >> 32);
-        const float* xrow = P.x.ptr + b * P.x.stride_row;
-        const float* urow = P.xu.ptr + b * P.xu.stride_row;
-        const float* wrow = P.w.ptr + o * P.w.stride_row;
-        float lo = kFloor, up = kFloor;
-#pragma unroll 8
-        for (int c = 4 * lane; c < P.C; c += 128) {
-            const float4 x4 = *reinterpret_cast<const float4*>(xrow + c);  // (rows are whole 16-byte pieces)
-            const float4 u4 = BOUND ? *reinterpret_cast<const float4*>(urow + c) : x4;
-            const float4 w4 = *reinterpret_cast<const float4*>(wrow + c);
-            const float xv[4] = {x4.x, x4.y, x4.z, x4.w}, uv[4] = {u4.x, u4.y, u4.z, u4.w}, wv[4] = {w4.x, w4.y, w4.z, w4.w};
+    const int t = threadIdx.x, lane = t & 31;
+    const unsigned id = blockIdx.x;
+    // samples on a lattice that visits rows and outputs evenly (fractions of the golden ratio and of the square root of 2)
+    const long long b = static_cast<long long>((static_cast<unsigned long long>(id * 2654435769u) * P.B) >> 32);
+    const int o = static_cast<int>((static_cast<unsigned long long>(id * 1779033703u) * P.CO) >> 32);
+    const float* xrow = P.x.ptr + b * P.x.stride_row + t;
+    const float* urow = P.xu.ptr + b * P.xu.stride_row + t;
+    const float* wrow = P.w.ptr + o * P.w.stride_row + t;
+    float x[KEEP], u[BOUND ? KEEP : 1], w[KEEP];
+    const int mine_n = P.C - t;
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (c + e < P.C) visit<BOUND>(xv[e], uv[e], wv[e], lo, up);
-            atomicAdd(&hist[bin_of(fabsf(w4.x))], 1);
-            atomicAdd(&hist[kBins + bin_of(BOUND ? fmaxf(fabsf(x4.x), fabsf(u4.x)) : fabsf(x4.x))], 1);
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, d));
-            up = fmaxf(up, __shfl_xor_sync(0xffffffffu, up, d));
-        }
-        if (lane == 0) P.t.samples[id] = BOUND ? fminf(lo, up) : lo;
+    for (int k = 0; k < KEEP; ++k) {
+        const bool in = kListThreads * k < mine_n;
+        x[k] = in ? xrow[kListThreads * k] : 0.0f;
+        if (BOUND) u[k] = in ? urow[kListThreads * k] : 0.0f;
+        w[k] = in ? wrow[kListThreads * k] : 0.0f;
     }
+    if (t <= kLevelsW) level_w[t] = 0;
+    if (t < kLevelsX) level_x[t] = 0;
+    float lo = kFloor, up = kFloor;
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) visit<BOUND>(x[k], BOUND ? u[k] : x[k], w[k], lo, up);
+    lo = block_max(lo, warps);
+    if (BOUND) up = block_max(up, warps);
+    const float value = BOUND ? fminf(lo, up) : lo;
+    auto put = [&](int* level) { return [=](int, int m, int place) { atomicMax(&level[4 * place / kBatch], m); }; };
+    int top_w, top_x;
+    const int left_w = rank_row<KEEP>(sh, kListW / 4, [&](int k) { return magnitude_of(w[k]); }, top_w, put(level_w));
+    const int left_x = rank_row<KEEP>(sh, kListX / 4, [&](int k) {
+        return BOUND ? max(magnitude_of(x[k]), magnitude_of(u[k])) : magnitude_of(x[k]);
+    }, top_x, put(level_x));
+    const int worst_w = __reduce_max_sync(0xffffffffu, left_w), worst_x = __reduce_max_sync(0xffffffffu, left_x);
+    if (lane == 0) {
+        atomicMax(&level_w[kLevelsW], worst_w);
+        atomicMax(&level_x[kLevelsX - 1], worst_x);
+    }
+    if (max(top_w, top_x) >= kInfinite) P.t.words[0] = 1;
     __syncthreads();
-    for (int i = tid; i < 2 * kBins; i += 256)
-        if (hist[i]) atomicAdd(&P.t.words[kHistWord + i], hist[i]);
+    if (t < kLevelsW) {
+        int rest_o = 0, rest_b = 0, tries = 0;
+        for (int k = t + 1; k <= kLevelsW; ++k) rest_o = max(rest_o, level_w[k]);
+        for (int k = kLevelsX - 1; k >= 0; --k) {
+            rest_b = max(rest_b, level_x[k]);
+            tries += proven(value, __int_as_float(rest_o), __int_as_float(rest_b)) ? 0 : 1;
+        }
+        atomicAdd(&P.t.words[kTrialWord + t * (kLevelsX + 1) + tries], 1);
+    }
     __threadfence();
     __syncthreads();
-    if (tid == 0) last = atomicAdd(&P.t.words[1], 1) == kSampleBlocks - 1;
+    if (t == 0) {
+        last = atomicAdd(&P.t.words[1], 1) == kSamples - 1;
+        best = ~0ull;
+    }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    // the kQuantile-th smallest maximum
-    float mine[(kSamples + 255) / 256];
-#pragma unroll
-    for (int k = 0; k < (kSamples + 255) / 256; ++k)
-        mine[k] = tid + 256 * k < kSamples ? __ldcg(&P.t.samples[tid + 256 * k]) : FLT_MAX;
-    float total = 0.0f;
-    for (int round = 0; round < kQuantile; ++round) {
-        float low = FLT_MAX;
-#pragma unroll
-        for (int k = 0; k < (kSamples + 255) / 256; ++k) low = fminf(low, mine[k]);
-        total = -block_max(-low, warps, 8);
-        // one thread that holds it drops one copy
-        __syncthreads();
-        if (tid == 0) hist[0] = 256;
-        __syncthreads();
-        if (low == total) atomicMin(&hist[0], tid);
-        __syncthreads();
-        if (tid == hist[0]) {
-            bool dropped = false;
-#pragma unroll
-            for (int k = 0; k < (kSamples + 255) / 256; ++k)
-                if (!dropped && mine[k] == total) {
-                    mine[k] = FLT_MAX;
-                    dropped = true;
-                }
-        }
-        __syncthreads();
-    }
-    for (int i = tid; i < 2 * kBins; i += 256) hist[i] = __ldcg(&P.t.words[kHistWord + i]);
+    for (int i = t; i < kLevelsW * (kLevelsX + 1); i += kListThreads) trials[i] = __ldcg(&P.t.words[kTrialWord + i]);
     __syncthreads();
-    // suffix sums: values in this bin and above
-    for (int d = 1; d < kBins; d <<= 1) {
-        int add[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = tid + 256 * k;
-            add[k] = i % kBins + d < kBins ? hist[i + d] : 0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 4; ++k) hist[tid + 256 * k] += add[k];
-        __syncthreads();
+    constexpr Costs unit = costs<BOUND>();
+    const float entry = BOUND && !eight_rows<BOUND>(P.C) ? 2.0f : 1.0f;
+    const float most = unit.dense_channel * P.C - kFixedCost - kListCost * P.C / P.B;
+    for (int i = t; i < kLevelsW * kLevelsX; i += kListThreads) {
+        const int lw = i / kLevelsX, lx = i % kLevelsX;
+        int failed = 0;
+        for (int k = lx + 1; k <= kLevelsX; ++k) failed += trials[lw * (kLevelsX + 1) + k];
+        const float cost = entry * kBatch * (lw + 1) +
+                           (lx > 0 ? unit.second_pass + unit.second_entry * kBatch * lx : 0.0f) +
+                           unit.hard_channel * P.C / kSamples * failed;
+        if (failed <= kMostFailed && cost <= most)
+            atomicMin(&best, (static_cast<unsigned long long>(__float_as_int(cost)) << 32) | i);
     }
-    const float per_row = 4.0f / kSamples;
-    float best = FLT_MAX, tau = 0.0f, sigma = 0.0f;
-    for (int i = tid; i < kBins; i += 256) {
-        const float t = bin_edge(i);
-        if (!(t < total)) continue;
-        const int j = bin_of(total - t);
-        const float nw = hist[i] * per_row, nx = hist[kBins + j] * per_row;
-        // (bin 0 holds everything below its edge too: a threshold there would be no bound)
-        if (i == 0 || j == 0 || nw > 0.75f * kListW || nx > 0.75f * kListX) continue;
-        const float cost = nw + (hist[kBins + j] > 0 ? nx + kSecondPass : 0.0f);
-        if (cost < best) {
-            best = cost;
-            tau = t;
-            sigma = bin_edge(j);
-        }
-    }
-    const float least = -block_max(-best, warps, 8);
-    if (tid == 0) hist[0] = 256;
     __syncthreads();
-    if (best == least && best < FLT_MAX) atomicMin(&hist[0], tid);
-    __syncthreads();
-    if (hist[0] == 256 || least * kDenseShare > P.C) {
-        if (tid == 0) P.t.words[0] = 1;
-    } else if (tid == hist[0]) {
-        P.t.words[kThresholdWord] = __float_as_int(tau);
-        P.t.words[kThresholdWord + 1] = __float_as_int(sigma);
+    if (t != 0) return;
+    if (best == ~0ull) {
+        P.t.words[0] = 1;
+    } else {
+        const int i = static_cast<int>(best & 0xffffffffu);
+        P.t.words[kLengthWord] = kBatch * (i / kLevelsX + 1);
+        P.t.words[kLengthWord + 1] = kBatch * (i % kLevelsX);
     }
 }
 
@@ -345,7 +387,8 @@ __global__ void __launch_bounds__(256) extreme_sample_kernel(const Problem P) {
 //
 // A lane owns a list and S outputs.  What bounds the walk is the load / store pipe: a step of 32 lists costs 4 S / 4 wavefronts
 // of shared memory and about 4.5 of list entries, hence as many rows per list as fit (S = 8) where the lists are long; the
-// samples' lists are short, and four rows leave room for two blocks, one filling its tile while the other walks.
+// samples' lists are short, and four rows leave room for two blocks, one filling its tile while the other walks.  (Times at
+// 512 x 5120 -> 5120 with index, n entries: weights' lists 44 + 0.51 n us, samples' lists 44 + 1.0 n.)
 template <bool BOUND, bool WSIDE, int S>
 __global__ void __launch_bounds__(kScanThreads, S == 4 ? 2 : 1) extreme_scan_kernel(const Problem P, int splits) {
     stream_order_begin();
@@ -359,18 +402,13 @@ __global__ void __launch_bounds__(kScanThreads, S == 4 ? 2 : 1) extreme_scan_ker
     const long long block = blockIdx.x / splits;
     const int split = static_cast<int>(blockIdx.x - block * splits);
     const long long tile_rows = WSIDE ? P.B : P.CO, list_rows = WSIDE ? P.CO : P.B;
-    const int* len = WSIDE ? P.t.w_len : P.t.x_len;
+    const int n = P.t.words[WSIDE ? kLengthWord : kLengthWord + 1];  // entries of every list
+    if (n == 0) return;
     const E* list = static_cast<const E*>(WSIDE ? P.t.w_list : P.t.x_list);
     const long long row0 = block * S;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* tile = reinterpret_cast<float*>(tile4);
     float* tile_up = tile + static_cast<size_t>(C4) * 4 * S;
-    if (!WSIDE) {
-        // nothing to do where none of the samples kept a list (then the weights are not even read)
-        int any = 0;
-        for (long long r = threadIdx.x; r < list_rows; r += kScanThreads) any |= len[r];
-        if (!__syncthreads_or(any)) return;
-    }
     auto fill = [&](const Operand& v, float* dst) {
 #pragma unroll 5
         for (int i = threadIdx.x; i < C4 * S; i += kScanThreads) {
@@ -396,8 +434,6 @@ __global__ void __launch_bounds__(kScanThreads, S == 4 ? 2 : 1) extreme_scan_ker
          chunk += static_cast<long long>(splits) * (kScanThreads / 32)) {
         const long long l = chunk * 32 + lane;
         const long long row = l < list_rows ? l : list_rows - 1;  // (lanes beyond the last list repeat it)
-        const int n = max(len[row], kBatch);
-        const int most = __reduce_max_sync(0xffffffffu, n);
         float best[S], best_up[S];
         int batch[S];  // first entry of the batch that last raised the maximum; kTie: a later batch reached it too
         constexpr int kTie = 1 << 30;
@@ -414,12 +450,9 @@ __global__ void __launch_bounds__(kScanThreads, S == 4 ? 2 : 1) extreme_scan_ker
                 v[4 * h] = t.x; v[4 * h + 1] = t.y; v[4 * h + 2] = t.z; v[4 * h + 3] = t.w;
             }
         };
-        // (lanes whose list has ended keep their last batch and work on it again without taking the result)
         auto load = [&](E (&en)[kBatch], int k0) {
-            if (k0 < n) {
 #pragma unroll
-                for (int u = 0; u < kBatch; ++u) en[u] = entries[(k0 + u) * kGroup];
-            }
+            for (int u = 0; u < kBatch; ++u) en[u] = entries[(k0 + u) * kGroup];
         };
         auto work = [&](const E (&en)[kBatch], int k0) {
             float top[S];
@@ -438,32 +471,29 @@ __global__ void __launch_bounds__(kScanThreads, S == 4 ? 2 : 1) extreme_scan_ker
                 }
             }
             if constexpr (!BOUND) {
-                if (k0 < n) {
 #pragma unroll
-                    for (int e = 0; e < S; ++e)
-                        if (top[e] >= best[e]) {
-                            batch[e] = top[e] > best[e] ? k0 : batch[e] | kTie;
-                            best[e] = top[e];
-                        }
-                }
+                for (int e = 0; e < S; ++e)
+                    if (top[e] >= best[e]) {
+                        batch[e] = top[e] > best[e] ? k0 : batch[e] | kTie;
+                        best[e] = top[e];
+                    }
             }
         };
         if constexpr (S == 4) {
             E en[kBatch];
-            for (int k0 = 0; k0 < most; k0 += kBatch) {
+            for (int k0 = 0; k0 < n; k0 += kBatch) {
                 load(en, k0);
                 work(en, k0);
             }
         } else {
             E even[kBatch], odd[kBatch];
             load(even, 0);
-#pragma unroll
-            for (int u = 0; u < kBatch; ++u) odd[u] = even[u];
-            for (int k0 = 0; k0 < most; k0 += 2 * kBatch) {
-                load(odd, k0 + kBatch);
+            for (int k0 = 0; k0 < n; k0 += 2 * kBatch) {
+                const bool more = k0 + kBatch < n;
+                if (more) load(odd, k0 + kBatch);
                 work(even, k0);
-                load(even, k0 + 2 * kBatch);
-                if (k0 + kBatch < most) work(odd, k0 + kBatch);
+                if (k0 + 2 * kBatch < n) load(even, k0 + 2 * kBatch);
+                if (more) work(odd, k0 + kBatch);
             }
         }
         if (l >= list_rows) continue;
@@ -607,12 +637,11 @@ __global__ void __launch_bounds__(256) extreme_resolve_kernel(const Problem P) {
 }
 
 unsigned most_hard_of(long long B, int CO) {
-    // a full search costs about 20 times an output's share of the dense kernel
-    const long long n = B * CO / 64;
+    // a full search costs about 20 times an output's share of the dense kernels: 1 / 32 of them more than half of all those
+    const long long n = B * CO / 32;
     return static_cast<unsigned>(n > 4096 ? n : 4096);
 }
 
-int round4(int c) { return (c + 3) & ~3; }
 template <class K>
 int allow_smem(K kernel, bool (&configured)[64], int bytes) {
     int dev = 0;
@@ -651,38 +680,56 @@ int launch_scan_s(const Problem& P, cudaStream_t st) {
 template <bool BOUND, bool WSIDE>
 int launch_scan(const Problem& P, cudaStream_t st) {
     if constexpr (WSIDE)
-        if (static_cast<long long>(round4(P.C)) * 8 * 4 * (BOUND ? 2 : 1) <= kMaxTile) return launch_scan_s<BOUND, WSIDE, 8>(P, st);
+        if (eight_rows<BOUND>(P.C)) return launch_scan_s<BOUND, WSIDE, 8>(P, st);
     return launch_scan_s<BOUND, WSIDE, 4>(P, st);
 }
 
-template <bool PAIR>
-int launch_lists(const Operand& v, const Operand& second, long long rows, int C, int cap, const float* threshold,
-                 typename EntryOf<PAIR>::type* list, int* len, float* rest, int* words, cudaStream_t st) {
-    const unsigned grid = static_cast<unsigned>(rows);
-    if (C <= 12 * kListThreads)
-        return launch_after(extreme_lists_kernel<PAIR, 12>, grid, kListThreads, 0, st, v, second, C, cap, threshold, list, len,
-                            rest, words);
-    if (C <= 20 * kListThreads)
-        return launch_after(extreme_lists_kernel<PAIR, 20>, grid, kListThreads, 0, st, v, second, C, cap, threshold, list, len,
-                            rest, words);
-    static_assert(kListKeep == 24, "the longest row");
-    return launch_after(extreme_lists_kernel<PAIR, 24>, grid, kListThreads, 0, st, v, second, C, cap, threshold, list, len,
-                        rest, words);
+// KEEP channels per thread, in steps of four: the smallest that holds a row.
+template <template <int> class Launch, class... A>
+int by_row_length(int C, const A&... args) {
+    switch ((C + 4 * kListThreads - 1) / (4 * kListThreads)) {
+        case 1: case 2: return Launch<8>::run(args...);
+        case 3: return Launch<12>::run(args...);
+        case 4: return Launch<16>::run(args...);
+        case 5: return Launch<20>::run(args...);
+        default: break;
+    }
+    static_assert(kMaxChannels == 24 * kListThreads, "the longest row");
+    return Launch<24>::run(args...);
 }
+template <bool PAIR>
+struct Lists {
+    template <int KEEP>
+    struct Launch {
+        static int run(const Operand& v, const Operand& second, long long rows, int C, int cap, int length_word,
+                       typename EntryOf<PAIR>::type* list, float* rest, int* words, cudaStream_t st) {
+            return launch_after(extreme_lists_kernel<PAIR, KEEP>, static_cast<unsigned>(rows), kListThreads, 0, st, v, second, C,
+                                cap, length_word, list, rest, words);
+        }
+    };
+};
+template <bool BOUND>
+struct Sample {
+    template <int KEEP>
+    struct Launch {
+        static int run(const Problem& P, cudaStream_t st) {
+            return launch_after(extreme_sample_kernel<BOUND, KEEP>, kSamples, kListThreads, 0, st, P);
+        }
+    };
+};
 
 template <bool BOUND>
 int run(const Problem& P, cudaStream_t st) {
     using EX = typename EntryOf<BOUND>::type;
     const cudaError_t e = cudaMemsetAsync(P.t.words, 0, kExtremeWords * sizeof(int), st);
     if (e != cudaSuccess) return cuda_status(e);
-    const float* thresholds = reinterpret_cast<const float*>(P.t.words + kThresholdWord);
-    int r = launch_after(extreme_sample_kernel<BOUND>, kSampleBlocks, 256, 0, st, P);
+    int r = by_row_length<Sample<BOUND>::template Launch>(P.C, P, st);
     if (r == kOk)
-        r = launch_lists<false>(P.w, P.w, P.CO, P.C, kListW, thresholds, static_cast<Entry1*>(P.t.w_list), P.t.w_len, P.t.w_rest,
-                                P.t.words, st);
+        r = by_row_length<Lists<false>::template Launch>(P.C, P.w, P.w, static_cast<long long>(P.CO), P.C, kListW, kLengthWord,
+                                                         static_cast<Entry1*>(P.t.w_list), P.t.w_rest, P.t.words, st);
     if (r == kOk)
-        r = launch_lists<BOUND>(P.x, P.xu, P.B, P.C, kListX, thresholds + 1, static_cast<EX*>(P.t.x_list), P.t.x_len,
-                                P.t.x_rest, P.t.words, st);
+        r = by_row_length<Lists<BOUND>::template Launch>(P.C, P.x, P.xu, P.B, P.C, kListX, kLengthWord + 1,
+                                                         static_cast<EX*>(P.t.x_list), P.t.x_rest, P.t.words, st);
     if (r == kOk) r = launch_scan<BOUND, true>(P, st);
     if (r == kOk) r = launch_scan<BOUND, false>(P, st);
     if (r == kOk) {
@@ -696,12 +743,13 @@ int run(const Problem& P, cudaStream_t st) {
 
 }  // namespace
 
-// Lines of the rule.  Below 2048 channels the lists are not a small part of a row.  Below 6.4 G pairs (values; bounds, which
-// cost the dense kernel 2.6 times as much: 2.5 G) what the path gains is not sure to cover its fixed cost, 100 us of sample,
-// lists and nine launches, and the 45 us it costs where the sample decides for dense: 128 x 3072 -> 5500 (2.2 G) takes 261 us
-// for hidden activations with index against 198 dense, 512 x 3072 -> 5120 (8.1 G) 446 against 672.  Beyond 6144 channels a
-// row no longer fits a list block's registers and four rows of both bounds no longer shared memory; narrow sides leave the
-// scan's blocks idle.
+// Lines of the rule.  Below 2048 channels the lists are not a small part of a row.  What a call pays whose data can prove
+// nothing (samples, and the launches behind them that return at once) is 35 - 45 us: under 7 % of the dense kernels' time from
+// 6.4 G pairs on (values; 512 x 3072 -> 5120, 8.1 G: 588 against 552), under 9 % of the bounds', which take them 2.6 times as
+// long, from 2.5 G on (128 x 6144 -> 3300: 519 against 474), but 11 - 25 % below (values of 512 x 2048 -> 5120, 5.4 G: 418 against
+// 378; 128 x 3072 -> 5500, 2.2 G: 195 against 163).  Data that it can be proven on gains there too: hidden activations 209
+// against 380 and 152 against 165.  Beyond 6144 channels a row no longer fits a list block's registers and four rows of both
+// bounds no longer shared memory; narrow sides leave the scan's blocks idle.
 bool extreme_applies(long long B, int CO, int C, bool bound) {
     return C >= 2048 && C <= kMaxChannels && B >= 128 && CO >= 512 && B * CO < (1LL << 31) &&
            B * CO * C >= (bound ? 2500000000LL : 6400000000LL);
@@ -710,23 +758,19 @@ bool extreme_applies(long long B, int CO, int C, bool bound) {
 size_t extreme_scratch_bytes(long long B, int CO, bool bound) {
     const size_t ex = bound ? sizeof(Entry2) : sizeof(Entry1);
     return pad256(groups_of(B) * kGroup * kListX * ex) + pad256(groups_of(CO) * kGroup * kListW * sizeof(Entry1)) +
-           2 * pad256(B * sizeof(int)) + 2 * pad256(static_cast<size_t>(CO) * sizeof(int)) +
-           pad256(static_cast<size_t>(most_hard_of(B, CO)) * sizeof(unsigned)) + pad256(kExtremeWords * sizeof(int)) +
-           pad256(kSamples * sizeof(float));
+           pad256(B * sizeof(float)) + pad256(static_cast<size_t>(CO) * sizeof(float)) +
+           pad256(static_cast<size_t>(most_hard_of(B, CO)) * sizeof(unsigned)) + pad256(kExtremeWords * sizeof(int));
 }
 
 bool extreme_take_scratch(Bump* bump, long long B, int CO, bool bound, ExtremeScratch* t) {
     const size_t ex = bound ? sizeof(Entry2) : sizeof(Entry1);
     t->x_list = bump->take<char>(groups_of(B) * kGroup * kListX * ex);
     t->w_list = bump->take<char>(groups_of(CO) * kGroup * kListW * sizeof(Entry1));
-    t->x_len = bump->take<int>(B);
-    t->w_len = bump->take<int>(CO);
     t->x_rest = bump->take<float>(B);
     t->w_rest = bump->take<float>(CO);
     t->hard = bump->take<unsigned>(most_hard_of(B, CO));
     t->words = bump->take<int>(kExtremeWords);
-    t->samples = bump->take<float>(kSamples);
-    return t->samples && t->x_list && t->w_list && t->x_len && t->w_len && t->x_rest && t->w_rest && t->hard && t->words;
+    return t->x_list && t->w_list && t->x_rest && t->w_rest && t->hard && t->words;
 }
 
 int launch_extreme(Operand x, Operand xu, Operand w, long long B, int CO, int C, bool bound, float* y, float* yu, int* pos,

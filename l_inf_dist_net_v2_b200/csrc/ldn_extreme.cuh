@@ -8,15 +8,12 @@ namespace ldn {
 struct ExtremeScratch {
     void* x_list;
     void* w_list;
-    int* x_len;
-    int* w_len;
     float* x_rest;
     float* w_rest;
     unsigned* hard;  // outputs to be searched in full
     int* words;      // kExtremeWords device words, cleared by the call; the first is the dense gate
-    float* samples;  // maxima of the sampled outputs
 };
-constexpr int kExtremeWords = 8 + 2 * 512;
+constexpr int kExtremeWords = 8 + 32 * 18;
 
 // Whether a problem of B samples, CO outputs and C channels takes this path (bound: interval bounds).
 bool extreme_applies(long long B, int CO, int C, bool bound);
