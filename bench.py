@@ -452,6 +452,20 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
     nominal_fp32 = sms * SM_LANES * max_mhz * 1e6 / 1e12
     nominal_mufu = sms * MUFU_LANES * max_mhz * 1e6 / 1e12
 
+    outcome = (ctypes.c_int * 2)()
+
+    def mark_extreme(row):
+        """Says in a p = inf forward row what its times are of, if the call just made took its outputs from the lists of
+        extreme channels: those kernels visit a few per cent of the pairs, are not bound by the FP32 pipe, and no tile kernel
+        ran."""
+        status = lib.ldn_last_extreme_outcome(torch.cuda.current_stream().cuda_stream, outcome)
+        if status == 0 and not outcome[0]:
+            row["bound"] = "load/store pipe"
+            row["note"] = ("gpair_per_s counts every pair; csrc/ldn_extreme.cu visits a few per cent of them, and searched "
+                           f"{outcome[1]} outputs in full")
+            for key in ("slots_per_pair", "tlaneop_per_s", "frac_of_ffma_probe", "frac_of_nominal"):
+                row.pop(key, None)
+
     def kernel_rows(pp, label, steps):
         fam_ = p_family(pp)
         s_f, s_x, s_w = SLOTS["inf" if fam_ == "inf" else ("8" if fam_ == "int" else "general")]
@@ -475,8 +489,7 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
             lib.ldn_enable_kernel_timing(0)
             t_tile = statistics.median(solo)
             # (a tile kernel is most of its call; anything far below that is not the kernel this row is about)
-            # (p = inf: large layers take csrc/ldn_extreme.cu, whose kernels are not timed by themselves)
-            if t_tile > 0.2 * t and fam_ != "inf":
+            if t_tile > 0.2 * t:
                 row["tile_kernel_ms"] = round(t_tile, 4)
             if fam_ == "inf" and name != "forward":
                 # scatter kernels: HBM-bound.  bytes: g + pos reads, zero-fill of the gradient, one 8-byte
@@ -489,7 +502,7 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
                             "frac_of_ffma_probe": round(ach / ffma_peak, 3),
                             "frac_of_nominal": round(ach / nominal_fp32, 3)})
                 if fam_ == "inf":
-                    row["note"] = "rates count every pair; csrc/ldn_extreme.cu visits a few per cent of them"
+                    mark_extreme(row)
                 if "tile_kernel_ms" in row:
                     ach_k = slots * pairs / (row["tile_kernel_ms"] * 1e-3) / 1e12
                     row.update({"tile_kernel_tlaneop_per_s": round(ach_k, 2),
@@ -544,6 +557,14 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
             "traffic_source": traffic_source,
             "algorithmic_bytes": (4 * (B * CO + B * CI + CO * CI) + 4 * (B * CI + CO * CI))
             if dominant["kernel"] == "backward_fused" else 4 * (B * CI + CO * CI + B * CO)}
+    elif dominant["bound"] == "load/store pipe":
+        nb = 4 * (B * CI + CO * CI + 2 * B * CO)
+        gbs = round(nb / (dominant["ms"] * 1e-3) / 1e9, 1)
+        line["roofline"] = {
+            "bound": "load/store pipe", "kernel": f"{dominant['kernel']} (p={args.p})", "achieved": gbs, "peak": hbm_peak,
+            "unit": "GB/s", "frac": round(gbs / hbm_peak, 3),
+            "note": "input, weight, output and index once each against the HBM rate; " + dominant["note"],
+            "peak_source": "MEASURED_PEAKS.json" if peaks else "fallback 6650 GB/s", "ms": dominant["ms"], "traffic": None}
     else:
         line["roofline"] = {
             "bound": "hbm", "kernel": f"{dominant['kernel']} (p={args.p})", "achieved": dominant["gb_per_s"],
@@ -563,6 +584,10 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
                           "ffma_probe_tlaneop_per_s": round(ffma_peak, 2),
                           "note": "the FFMA probe ran after this block at whatever clock the GPU then held; "
                                   "frac_of_nominal_at_sampled_clock uses the median SM clock sampled during this block"})
+        if any(r["bound"] == "load/store pipe" for r in in_step):  # (the step visits a few per cent of the pairs)
+            for key in ("slots_per_pair_per_step", "step_tlaneop_per_s", "frac_of_nominal_at_max_clock",
+                        "frac_of_nominal_at_sampled_clock"):
+                sustained.pop(key, None)
         line["sustained"] = sustained
     if model is not None:
         line["model"] = model
@@ -591,13 +616,7 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
             extra.append({"p": "inf", "kernel": name, "ms": round(t, 4), "gpair_per_s": round(pairs / (t * 1e-3) / 1e9, 1),
                           "bound": "fp32", "slots_per_pair": slots, "tlaneop_per_s": round(ach, 2),
                           "frac_of_ffma_probe": round(ach / ffma_peak, 3), "frac_of_nominal": round(ach / nominal_fp32, 3)})
-            if name != "bounds_with_indices":
-                extra[-1]["note"] = "rates count every pair; csrc/ldn_extreme.cu visits a few per cent of them"
-        for row in extra:
-            if "note" in row:  # a fraction of the dense kernels' ceiling means nothing there
-                row["bound"] = "load/store pipe"
-                for key in ("frac_of_ffma_probe", "frac_of_nominal"):
-                    row.pop(key, None)
+            mark_extreme(extra[-1])
         line["variants"] = extra
         fwd()
     C.check_status()
