@@ -4,6 +4,7 @@
 // read from the tensors as the reference does (norm_dist.cpp:44,73,127).  Differences: launches go to the
 // current stream of the tensors' device (with a device guard) and a non-zero status raises.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
@@ -192,6 +193,8 @@ void fold(Tensor& cols, Tensor& x, std::pair<int, int> kernel, int stride, int p
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
+// whether the tracer or a dispatch mode looks at the operators as they are called
+bool observed() { return torch::jit::tracer::isTracing() || c10::impl::dispatch_mode_enabled(); }
 bool plain(const Tensor& t, int64_t dim) {
     return t.is_cuda() && t.scalar_type() == at::kFloat && t.layout() == at::kStrided && t.dim() == dim && t.is_contiguous() &&
            t.numel() > 0 && t.has_storage() && !t._fw_grad(0).defined() && !t.unsafeGetTensorImpl()->is_python_dispatch();
@@ -295,7 +298,7 @@ void subtract_mean(const Tensor& x, const Tensor& running_mean, double momentum,
 
 // whether a kernel of this package may compute a linear map's gradient from this one
 bool plain_gradient(const Tensor& grad, int64_t dim) {
-    return plain(grad, dim) && !(at::GradMode::is_enabled() && grad.requires_grad());
+    return plain(grad, dim) && !observed() && !(at::GradMode::is_enabled() && grad.requires_grad());
 }
 
 struct MeanShiftFn : public torch::autograd::Function<MeanShiftFn> {
@@ -339,13 +342,13 @@ struct UnfoldFn : public torch::autograd::Function<UnfoldFn> {
 };
 
 c10::optional<Tensor> norm_dist(const Tensor& x, const Tensor& w, double p, int64_t G) {
-    if (!fits(x, w, G) || !(p > 0.0) || torch::jit::tracer::isTracing()) return c10::nullopt;
+    if (!fits(x, w, G) || !(p > 0.0) || observed()) return c10::nullopt;
     const bool need_grad = at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad());
     return NormDistFn::apply(x, w, G, p, need_grad);
 }
 
 c10::optional<std::tuple<Tensor, Tensor>> bound_inf_dist(const Tensor& xl, const Tensor& xu, const Tensor& w, int64_t G) {
-    if (!fits(xl, w, G) || !fits(xu, w, G) || xl.sizes() != xu.sizes() || torch::jit::tracer::isTracing()) return c10::nullopt;
+    if (!fits(xl, w, G) || !fits(xu, w, G) || xl.sizes() != xu.sizes() || observed()) return c10::nullopt;
     const bool need_grad = at::GradMode::is_enabled() && (xl.requires_grad() || xu.requires_grad() || w.requires_grad());
     variable_list y = BoundInfDistFn::apply(xl, xu, w, G, need_grad);
     return std::make_tuple(y[0], y[1]);
@@ -353,14 +356,14 @@ c10::optional<std::tuple<Tensor, Tensor>> bound_inf_dist(const Tensor& xl, const
 
 c10::optional<Tensor> mean_shift(const Tensor& x, const Tensor& running_mean, double momentum) {
     if (!plain(x, 3) || !plain(running_mean, 1) || x.device() != running_mean.device() || running_mean.requires_grad() ||
-        running_mean.size(0) != x.size(1) || torch::jit::tracer::isTracing())
+        running_mean.size(0) != x.size(1) || observed())
         return c10::nullopt;
     return MeanShiftFn::apply(x, running_mean, momentum);
 }
 
 c10::optional<Tensor> unfold_columns(const Tensor& x, int64_t positions, std::pair<int64_t, int64_t> kernel, int64_t stride,
                                      int64_t padding, int64_t dilation) {
-    if (!plain(x, 4) || torch::jit::tracer::isTracing()) return c10::nullopt;
+    if (!plain(x, 4) || observed()) return c10::nullopt;
     return UnfoldFn::apply(x, positions, kernel.first, kernel.second, stride, padding, dilation);
 }
 

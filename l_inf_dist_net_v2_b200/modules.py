@@ -80,11 +80,11 @@ def _unfold(x, kernel_size, dilation, padding, stride):
         out = [(s + 2 * padding - dilation * (k - 1) - 1) // stride + 1 for s, k in zip(x.shape[2:], kernel_size)]
         columns = out[0] * out[1] * kernel_size[0] * kernel_size[1]
         if min(out) > 0 and max(columns, x.size(2) * x.size(3), *(s + 2 * padding for s in x.shape[2:])) < 1 << 30:
-            if _C.native() is not None:
-                cols = _C.native().unfold_columns(x, out[0] * out[1], kernel_size, stride, padding, dilation)
-                if cols is not None:
-                    return cols
-            elif not _C.transformed() and torch.autograd.forward_ad._current_level < 0:
+            ext = _C.native()
+            cols = None if ext is None else ext.unfold_columns(x, out[0] * out[1], kernel_size, stride, padding, dilation)
+            if cols is not None:
+                return cols
+            if ext is None and not _C.transformed() and torch.autograd.forward_ad._current_level < 0:
                 return _UnfoldF.apply(x, out[0] * out[1], kernel_size, stride, padding, dilation)
     return F.unfold(x, kernel_size, dilation, padding, stride)
 

@@ -234,14 +234,17 @@ if _ext is not None:
     BINDING = "pybind11"
 
 
-def transformed():
-    """Whether something looks at the operators as they are called and would not see a kernel of this package: torch.compile,
-    a function transform (vmap, grad, jvp), a dispatch mode or the tracer."""
-    return (torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active()
-            or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing())
-
-
 def native():
     """The compiled binding when its C++ autograd functions may stand in for the Python ones, else None: it was not built, or
-    calls are being transformed, which the Python functions refuse or handle."""
-    return None if _ext is None or transformed() else _ext
+    torch.compile or a function transform (vmap, grad, jvp) is at work, which the Python functions refuse or handle.  (The
+    binding itself looks for dispatch modes and the tracer.)"""
+    if _ext is None or torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active():
+        return None
+    return _ext
+
+
+def transformed():
+    """Whether something looks at the operators as they are called and would not see a kernel of this package: torch.compile,
+    a function transform, a dispatch mode or the tracer."""
+    return (torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active()
+            or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing())
