@@ -6,6 +6,7 @@
 #include <mutex>
 
 #include "ldn_b200.h"
+#include "ldn_even.cuh"
 #include "ldn_extreme.cuh"
 #include "ldn_launch.cuh"
 #include "ldn_prep.cuh"
@@ -98,6 +99,7 @@ struct Call {
     const float* norm_rows = nullptr;  // separable normaliser of FwdPowNorm and its guard word (see TileParams)
     const float* norm_cols = nullptr;
     int* guard = nullptr;
+    CopyGate copies;                   // of the canonical copies
     const int* gate = nullptr;         // forward kernels launched while set return at once unless *gate != 0
     std::unique_lock<std::mutex> lock;  // the arena's call mutex, released when the entry point returns
 };
@@ -163,7 +165,7 @@ int get_x_view(Call& c, const float* x, const Shape& s, View* v) {
     float* xc = c.bump.take<float>(canonical_floats(s.CIg, s.M, s.G));
     if (!xc) return kWorkspace;
     *v = canonical_view(xc, s.CIg, s.M, s.G);
-    return launch_canon_x(x, xc, s, static_cast<int>(v->stride_row), c.st);
+    return launch_canon_x(x, xc, s, static_cast<int>(v->stride_row), c.copies, c.st);
 }
 int get_w_view(Call& c, const float* w, const Shape& s, View* v) {
     if (w_is_natural(w, s)) {
@@ -173,7 +175,7 @@ int get_w_view(Call& c, const float* w, const Shape& s, View* v) {
     float* wc = c.bump.take<float>(canonical_floats(s.CIg, s.COg, s.G));
     if (!wc) return kWorkspace;
     *v = canonical_view(wc, s.CIg, s.COg, s.G);
-    return launch_canon_w(w, wc, s, static_cast<int>(v->stride_row), c.st);
+    return launch_canon_w(w, wc, s, static_cast<int>(v->stride_row), c.copies, c.st);
 }
 
 // Common part of a tile-engine plan.
@@ -281,6 +283,9 @@ int int_power(float e) {
     return -1;
 }
 
+// Most scratch the matrix products of even p may take beyond the general path's (bytes).
+constexpr size_t kEvenMaxScratch = size_t(1) << 30;
+
 // One backward call on rows [0, s.B) of the given pointers.  accumulate_gw: add to grad_weight instead of
 // overwriting it (only the fused path supports that; it is how the row chunks of one call combine).
 //
@@ -320,11 +325,20 @@ int norm_dist_backward_part(const float* go, const float* x, const float* w, con
     size_t need = (tma_x ? x_scratch_bytes(x, s) : 0) + (tma_w ? w_scratch_bytes(w, s) : 0) + (iq >= 0 ? pad256(int_floats * sizeof(float)) : 0) +
                   ((iq < 0 || guarded) ? 2 * pad256(gen_floats * sizeof(float)) : 0) +
                   (guarded ? 4 : 2) * partial_bytes(cap, 1) + (fused ? pad256(side_floats * sizeof(float)) : 0);
+    // even p of large problems: both gradients from matrix products (ldn_even.cu), the kernels here gated behind them
+    const size_t even_bytes = even_power(p) && !accumulate_gx && s.co_src == s.CO && even_backward_applies(s, p, gx != nullptr, gw != nullptr, cap)
+                                  ? even_backward_bytes(s, gx != nullptr, gw != nullptr, cap)
+                                  : 0;
+    bool even = false;
     Call c;
-    if ((r = begin_call(&c, stream, need)) != kOk) return r;
+    if ((r = begin_call(&c, stream, need, even_bytes <= kEvenMaxScratch ? even_bytes : 0, &even)) != kOk) return r;
     View xv{}, wv{};
-    if (tma_x && (r = get_x_view(c, x, s, &xv)) != kOk) return r;
-    if (tma_w && (r = get_w_view(c, w, s, &wv)) != kOk) return r;
+    auto take_views = [&]() -> int {
+        int e = kOk;
+        if (tma_x && (e = get_x_view(c, x, s, &xv)) != kOk) return e;
+        return tma_w ? get_w_view(c, w, s, &wv) : kOk;
+    };
+    if (!even && (r = take_views()) != kOk) return r;
     float* side = nullptr;
     if (fused && !(side = c.bump.take<float>(side_floats))) return kWorkspace;
     // the guard's flag: a word of the arena's status block, cleared in stream order before the coefficient kernel
@@ -406,6 +420,14 @@ int norm_dist_backward_part(const float* go, const float* x, const float* w, con
         const View cv = View{c0, s.COg, s.M, s.G, int_pitch, s.M * int_pitch, 1};
         if ((r = launch_coef_int(go, y, c0, s, static_cast<int>(int_pitch), iq, flag, c.st)) != kOk) return r;
         if (!guarded) return run_family(iq, cv, cv, nullptr, nullptr);
+        const int* direct = nullptr;  // gate of the integer form behind the matrix products
+        if (even) {
+            r = launch_even_backward(c0, static_cast<int>(int_pitch), x, w, y, s, gx, gw, p, accumulate_gw, flag, c.cap, &c.bump,
+                                     c.arena->status, &direct, c.st);
+            if (r != kOk) return r;
+            c.copies = CopyGate{direct, flag};
+            if ((r = take_views()) != kOk) return r;
+        }
         // second form, gated by the flag: 1 / y and g as coefficients, 2^(q lg2(|t| / y)) per pair
         float* r0 = c.bump.take<float>(gen_floats);
         float* r1 = c.bump.take<float>(gen_floats);
@@ -413,7 +435,7 @@ int norm_dist_backward_part(const float* go, const float* x, const float* w, con
         View v0, v1;
         gen_views(r0, r1, &v0, &v1);
         const CoefJob second = coef_gen_job(go, y, r0, r1, s, static_cast<int>(gen_pitch), gen_rows, p - 1.0f, false, flag);
-        if ((r = run_family(iq, cv, cv, nullptr, &second)) != kOk) return r;
+        if ((r = run_family(iq, cv, cv, direct, &second)) != kOk) return r;
         if (!fused && (r = launch_coef_gen(second, c.st)) != kOk) return r;
         return run_family(-2, v0, v1, flag, nullptr);
     }
@@ -653,8 +675,16 @@ LDN_API int ldn_norm_dist_forward(const float* input, const float* weight, int B
     size_t need = (inplace ? 0 : x_scratch_bytes(input, s)) + w_scratch_bytes(weight, s) +
                   (bound_norm ? 3 : 2) * partial_bytes(cap_for(ctx), 1) + (normalised ? ybytes : 0) +
                   (bound_norm ? 2 * pad256(norm_floats * sizeof(float)) : 0);
+    // even p of large problems: matrix products (ldn_even.cu), the direct kernel gated behind them
+    const size_t even_bytes = even_power(p) && even_forward_applies(s, p, cap_for(ctx)) ? even_forward_bytes(s, p, cap_for(ctx)) : 0;
+    bool even = false;
     Call c;
-    if ((r = begin_call(&c, stream, need)) != kOk) return r;
+    if ((r = begin_call(&c, stream, need, even_bytes <= kEvenMaxScratch ? even_bytes : 0, &even)) != kOk) return r;
+    if (even) {
+        r = launch_even_forward(input, weight, s, output, p, c.cap, &c.bump, c.arena->status, &c.gate, c.st);
+        if (r != kOk) return r;
+        c.copies.a = c.gate;
+    }
     View xv, wv;
     if (inplace) xv = x_kmajor_view(input, s);
     else if ((r = get_x_view(c, input, s, &xv)) != kOk) return r;

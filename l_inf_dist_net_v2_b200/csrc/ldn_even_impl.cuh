@@ -1,0 +1,1532 @@
+// Even integer exponents on the tensor cores.
+//
+// For even p the distance is a polynomial:
+//   y^p            = sum_c x^p + sum_c w^p + sum_{j=1}^{p-1} (-1)^j C(p, j) sum_c x^j w^(p-j)
+//   grad_x[b, c]   = sum_j (-1)^j C(p-1, j) x^(p-1-j) sum_o A[b, o] w[o, c]^j,      A = go / y^(p-1)
+//   grad_w[o, c]   = sum_j (-1)^j C(p-1, j) w^(p-1-j) sum_b A[b, o] x[b, c]^j
+// i.e. p - 1 matrix products each.  Every factor is split into two 11-bit halves, v = hi + lo in fp16 (lo holds what hi
+// rounds off, so the pair keeps 22 - 23 bits), and a product is hi hi + hi lo + lo hi with fp32 accumulators (and lo lo for
+// p = 2): 3 x 7 multiply-adds per pair on the tensor cores for p = 8, against 4 (forward) and 8 (backward) FP32 instructions of
+// the direct kernels.  The terms do not cancel where it matters: large |x - w| come from x and w of opposite sign, for which all
+// terms of the expansion have one sign (the guards below look at every output, and at every channel).
+//
+// What is kept as precise as in the direct kernels, and how:
+//   * the tensor core's accumulator drops the bits below the largest summand instead of rounding, so it takes one stage
+//     at a time and the sums are added up in registers.  What 64 elements' products lose that way is 2.0e-7 - 2.8e-7 of
+//     their sum in the forward pass (p = 4 and 8, 128 - 3072 channels, images and zero-mean activations, against 64 bits),
+//     always towards zero: kTruncation gives it back there.  (The backward pass's sums, whose terms have either sign, show no
+//     such drift.)
+//   * powers are scaled into fp16's range: by one power of two for both operands in the forward pass (all terms of the sum
+//     share it), by one per channel and one per coefficient row in the backward pass;
+//   * forward: an output for which the terms could cancel, y^p < 2^-6 (|x|_p + |w|_p)^p, or that is small on the common
+//     scale, y^p < 2^-10 M^p with the largest magnitude M, goes to a list and is summed directly; too many of them, or a value that is not finite, and the
+//     direct kernels behind this path run instead;
+//   * backward: an output below a third of the largest |x| + |w| (its coefficient, y^-(p-1), would blow the expansion's errors
+//     up), or a channel whose values all lie close together far from zero, makes the direct kernels run.
+#pragma once
+#include <float.h>
+#include <math.h>
+
+#include <type_traits>
+
+#include "ldn_even.cuh"
+
+namespace ldn {
+namespace {
+
+constexpr int kMRows = 128;                 // rows of A per CTA = TMEM lanes
+constexpr int kNRows = 224;                 // widest B tile: 7 powers of 32 channels, or 224 rows
+constexpr int kBlockK = 32;                 // reduction elements of a block: a row of one is 32 hi | 32 lo, 128 bytes
+constexpr int kABytes = kMRows * 128;       // a block of A as shared memory holds it (128-byte swizzle)
+constexpr int kEpiWarps = 8, kConvWarps = 7;
+constexpr int kEvenThreads = 32 * (kEpiWarps + kConvWarps + 1);
+constexpr float kScaleB = 32768.0f;         // backward: powers of values below 1 as fp16 holds them best
+constexpr float kTruncation = 1.0f + 1.0f / (1 << 22);
+constexpr int kListCap = 1 << 16;
+
+// A tile is the work of a pair of CTAs: 256 rows of A, kNRows of B, half of either in each CTA.
+constexpr int kBlocks = 2;                             // blocks of 32 reduction elements per stage
+constexpr int kStageK = kBlocks * kBlockK;
+constexpr int kStages = 3;
+constexpr int kRowsB = kNRows / 2;                     // rows of B in a CTA
+constexpr int kBBytes = kRowsB * 128;
+constexpr int kStageBytes = kBlocks * (kABytes + kBBytes);  // all blocks of A, then all blocks of B
+constexpr int kEvenSmem = kStages * kStageBytes + 1024 + 256;
+
+// Channels per tile of the backward form: (p - 1) * channels rows of B, at most kNRows
+__host__ __device__ constexpr int channels_of(int np) { return np >= 5 ? 32 : (np == 3 ? 64 : 128); }
+
+__host__ __device__ constexpr float binomial(int n, int k) {
+    float r = 1.0f;
+    for (int i = 1; i <= k; ++i) r = r * (n - k + i) / i;
+    return r;
+}
+
+// An fp32 operand as the converters read it.  Element (row, k) of group g:
+//   kind 0 / 1: p[g * s_g + row * s_row + k] (s_k = 1), 0: in aligned 16-byte pieces
+//   kind 2:     p[g * s_g + (row / hw) * s_b + (row % hw) * s_row + k * s_k], without the division where hw is 0
+//   kind 3 / 4: p[g * s_g + row * s_row + (k / hw) * s_b + k % hw], 4: in aligned 16-byte pieces
+struct Source {
+    const float* p;
+    int kind, rows, k, hw;
+    long long s_row, s_k, s_b, s_g;
+};
+
+struct EvenParams {
+    int M, N, K, G;                 // per group: rows of A, rows of B (forward) or channels (backward), reduction length
+    int tiles_m, tiles_n, kt;       // kt: stages per tile
+    int blocks;                     // forward: blocks of 32 channels times powers, in this order
+    int total;                      // stages in all
+    const char* images;             // A: [g][block of rows][block of the reduction ([power], forward)], kABytes each
+    Source src;                     // B
+    OutAddr out;
+    bool swap;                      // forward: the output's row is the tile's column
+    bool vec;                       // columns n .. n + 3 (n a multiple of 4) of an output row are one aligned 16-byte piece
+    bool accumulate;
+    float* out_f;
+    // forward
+    const float *sum_a, *norm_a, *sum_b, *norm_b;  // row sums of p-th powers on the common scale and their p-th roots
+    const unsigned* scale_word;     // bits of the largest magnitude
+    int* list;                      // outputs to be summed directly
+    int* list_count;
+    int* dense;
+    // backward
+    const float* resident;          // the operand with the output's layout
+    const float* col_down;          // [g][channel, padded to whole tiles]: v = value * 2^-e
+    const int* row_exp;             // [g][row]: coefficients are scaled by 2^exp
+    const float* row_sum;           // [g][row]: sum of the scaled coefficients
+    const int *gate0, *gate1;       // run only while both words are 0 (may be null)
+    float* partials;                // [cta][2][columns][kMRows]
+    int* status;
+};
+
+// ---- tcgen05 ---------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free(uint32_t base) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory");
+}
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t desc, bool add) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(desc), "r"(static_cast<uint32_t>(add))
+        : "memory");
+}
+// arrival on the barrier of both CTAs when the products issued so far are done
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+        "h"(static_cast<uint16_t>(3))
+        : "memory");
+}
+__device__ __forceinline__ void tmem_load16(uint32_t addr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+// (the registers are operands, so that nothing that uses them moves in front of the wait)
+__device__ __forceinline__ void tmem_load_wait(float (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]),
+                   "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// arrival on the same barrier of the pair's first CTA
+__device__ __forceinline__ void mbar_arrive_first(uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\t"
+        "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+// K-major operand, rows of 128 bytes in groups of 8 (1024 bytes apart), 128-byte swizzle
+__device__ __forceinline__ uint64_t smem_desc(const void* p) {
+    return static_cast<uint64_t>((smem_u32(p) & 0x3ffffu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+// fp16 x fp16 -> fp32, both operands K-major
+__host__ __device__ constexpr uint32_t mma_desc(int m, int n) {
+    return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
+}
+
+// ---- splitting -------------------------------------------------------------------------------------------------------
+// eight values as 16 bytes of hi and 16 bytes of lo
+__device__ __forceinline__ void split8(const float2 (&v)[4], uint4* hi, uint4* lo) {
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(h[i]) : "f"(v[i].y), "f"(v[i].x));
+        float2 f;
+        asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.f32.f16 %0, a;\n\tcvt.f32.f16 %1, b;\n\t}"
+            : "=f"(f.x), "=f"(f.y)
+            : "r"(h[i]));
+        const float2 d = __ffma2_rn(f, make_float2(-1.0f, -1.0f), v[i]);
+        asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(l[i]) : "f"(d.y), "f"(d.x));
+    }
+    *hi = make_uint4(h[0], h[1], h[2], h[3]);
+    *lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+__device__ __forceinline__ float2 scale2(float2 v, float s) { return __fmul2_rn(v, make_float2(s, s)); }
+template <int E>
+__device__ __forceinline__ float2 power2(float2 v) {
+    if constexpr (E == 1) return v;
+    else if constexpr (E % 2 == 0) {
+        const float2 h = power2<E / 2>(v);
+        return __fmul2_rn(h, h);
+    } else {
+        return __fmul2_rn(power2<E - 1>(v), v);
+    }
+}
+template <int P>
+__device__ __forceinline__ float power(float v) {
+    if constexpr (P == 1) return v;
+    else if constexpr (P % 2 == 0) {
+        const float h = power<P / 2>(v);
+        return h * h;
+    } else {
+        return power<P - 1>(v) * v;
+    }
+}
+// v^(1/P), rounded (almost) once: what a square root's rounding took is carried on to the next
+template <int P>
+__device__ __forceinline__ float root(float v) {
+    if constexpr (P == 6) return cbrtf(sqrtf(v));
+    float low = 0.0f;  // v + low is the value so far
+#pragma unroll
+    for (int i = P; i > 1; i /= 2) {
+        const float inv = rsqrtf(v), r = v * inv;
+        low = 0.5f * (fmaf(-r, r, v) + low) * inv;
+        v = r;
+    }
+    return v + low;
+}
+// 2^e, |e| <= 126
+__device__ __forceinline__ float pow2i(int e) { return __int_as_float((e + 127) << 23); }
+// 2^(n e) from 2^-e, |n e| <= 126
+template <int N>
+__device__ __forceinline__ float up_of(float down) {
+    return pow2i(N * (127 - (__float_as_int(down) >> 23)));
+}
+// smallest e with 2^e > v, from the bits of |v|
+__device__ __forceinline__ int exponent_above(unsigned bits) { return static_cast<int>(bits >> 23) - 126; }
+
+__device__ __forceinline__ const float* source_row(const Source& S, int g, int row) {
+    if (row >= S.rows) return nullptr;
+    const float* p = S.p + g * S.s_g;
+    if (S.kind == 2 && S.hw > 0) {
+        const int b = row / S.hw;
+        return p + b * S.s_b + (row - b * S.hw) * S.s_row;
+    }
+    return p + row * S.s_row;
+}
+// Loads into registers that hold 0 where there is nothing to load.  (As predicated instructions on the destination itself: a
+// conditional in C++ ends in moves behind the loads, and those wait for them, a thousand cycles per prefetch.)
+__device__ __forceinline__ void load1(float* v, const float* p, bool there) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.f32 %0, [%1];\n\t}"
+                 : "+f"(*v)
+                 : "l"(p), "r"(static_cast<uint32_t>(there)));
+}
+__device__ __forceinline__ void load4(float2* v, const float* p, bool there) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+                 : "+f"(v[0].x), "+f"(v[0].y), "+f"(v[1].x), "+f"(v[1].y)
+                 : "l"(p), "r"(static_cast<uint32_t>(there)));
+}
+// elements k0 .. k0 + 7 of a row (k0 a multiple of 8); 0 outside
+__device__ __forceinline__ void fetch8(const Source& S, const float* row, int k0, float2 (&v)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = make_float2(0.0f, 0.0f);
+    const int left = row == nullptr ? 0 : S.k - k0;
+    if (S.kind == 1 || S.kind == 2) {
+        const float* p = row + k0 * S.s_k;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            load1(i % 2 ? &v[i / 2].y : &v[i / 2].x, p, left > i);
+            p += S.s_k;
+        }
+    } else if (S.kind == 0) {
+        load4(v, row + k0, left > 0);
+        load4(v + 2, row + k0 + 4, left > 4);
+    } else if (S.kind == 4) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int k = k0 + 4 * i, b = k / S.hw;
+            load4(v + 2 * i, row + b * S.s_b + (k - b * S.hw), left > 4 * i);
+        }
+    } else {
+        const int b = k0 / S.hw;
+        int r = k0 - b * S.hw;
+        const float* p = row + b * S.s_b + r;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            load1(i % 2 ? &v[i / 2].y : &v[i / 2].x, p, left > i);
+            ++p;
+            if (++r == S.hw) {
+                r = 0;
+                p += S.s_b - S.hw;
+            }
+        }
+    }
+}
+
+// ---- where results go ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ long long even_offset(const EvenParams& P, int g, int m, int n) {
+    const int r = P.swap ? n : m, c = P.swap ? m : n;
+    const int q = P.out.hw_div == 1 ? r : r / P.out.hw_div;
+    return q * P.out.s_b + (r - q * P.out.hw_div) * P.out.s_hw + g * P.out.s_g + c * P.out.s_n;
+}
+
+// Scales of the forward form, from the largest magnitude M of both operands.  With unit = 2^e > M and values v = value / unit,
+// the factors of term j are C(p, j) x^j 2^a(j) and w^(p-j) 2^b(j), both below 2^16, with a(j) + b(j) = total for all j.
+template <int PW>
+struct ForwardScale {
+    int e, total;
+    float bits, top;  // bits = log2(unit / M), top = M / unit in [0.5, 1)
+    __device__ __forceinline__ explicit ForwardScale(unsigned word) {
+        e = exponent_above(word);
+        top = __uint_as_float((word & 0x7fffffu) | 0x3f000000u);
+        bits = -log2f(top) * 0.9999f;
+        total = 1000;
+#pragma unroll
+        for (int j = 1; j < PW; ++j)
+            total = min(total, static_cast<int>(floorf(15.9f + j * bits - log2f(binomial(PW, j)))) + b(PW - j));
+    }
+    __device__ __forceinline__ int b(int exponent) const { return 15 + static_cast<int>(exponent * bits); }
+    __device__ __forceinline__ int a(int j) const { return total - b(PW - j); }
+};
+
+// A sum of the forward form -> the output value; outputs that may have lost bits go to the list.
+struct ForwardEnd {
+    float from_acc, least, unit;  // accumulated units -> sums; smallest sum that is large enough on the common scale
+};
+template <int PW>
+__device__ __forceinline__ ForwardEnd forward_end(const EvenParams& P) {
+    const ForwardScale<PW> f(*P.scale_word);
+    return ForwardEnd{pow2i(-f.total) * kTruncation, power<PW>(f.top) * (1.0f / 1024), pow2i(f.e)};
+}
+template <int PW>
+__device__ __forceinline__ float forward_value(const EvenParams& P, const ForwardEnd& E, float acc, float sa, float na, float sb,
+                                               float nb, int off) {
+    const float s = fmaf(acc, E.from_acc, sa + sb);
+    const float least = fmaxf(E.least, power<PW>(na + nb) * (1.0f / 64));
+    if (!(s >= least) && *static_cast<volatile int*>(P.dense) == 0) {
+        const int at = atomicAdd(P.list_count, 1);
+        if (at < kListCap) P.list[at] = off;
+        else *P.dense = 1;
+    }
+    return root<PW>(s) * E.unit;
+}
+
+struct Span {
+    int g, tm, tn, kt0, kt1;  // stages [kt0, kt1) of one tile
+};
+__device__ __forceinline__ Span span_at(const EvenParams& P, int it, int end) {
+    Span s;
+    const int t = it / P.kt;
+    s.kt0 = it - t * P.kt;
+    s.kt1 = min(P.kt, s.kt0 + end - it);
+    const int per_group = P.tiles_m * P.tiles_n;
+    s.g = t / per_group;
+    const int r = t - s.g * per_group;
+    s.tn = r / P.tiles_m;
+    s.tm = r - s.tn * P.tiles_m;
+    return s;
+}
+// first stage of unit (CTA or pair) i of n
+__device__ __forceinline__ int even_begin(const EvenParams& P, int n, int i) {
+    return static_cast<int>(static_cast<long long>(P.total) * i / n);
+}
+
+// The blocks of A of stage kt of a tile, for CTA `rank` of its pair.
+__device__ __forceinline__ const char* a_blocks(const EvenParams& P, const Span& s, int kt, int rank) {
+    const int row_block = (s.g * P.tiles_m + s.tm) * 2 + rank;
+    return P.images + (static_cast<long long>(row_block) * P.kt + kt) * static_cast<long long>(kBlocks * kABytes);
+}
+
+struct Bars {
+    uint64_t full[kStages], empty[kStages];
+    uint64_t peer_full[kStages];  // of the pair's first CTA: the second CTA's part of the stage is there
+    uint64_t acc_full[2], acc_empty[2];
+    uint32_t tmem;
+    int abort;
+};
+
+template <bool CLUSTER>
+__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, int* abort, int* status) {
+    for (uint32_t i = 0; i < kMaxPolls; ++i) {
+        if (CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
+        if (i >= kFastPolls) {
+            if (*static_cast<volatile int*>(abort)) return false;
+            __nanosleep(64);
+        }
+    }
+    *static_cast<volatile int*>(abort) = 1;
+    *status = kDeviceTimeout;
+    return false;
+}
+
+// FWD: powers run along the reduction (all powers of 32 channels, then of the next 32; a stage = kBlocks of these blocks),
+// B = rows of the larger operand.
+// !FWD: powers run along the tile's columns, a stage = kBlocks * 32 rows of the operand.  The columns are two halves (the rows
+// of B of the two CTAs of a pair), each p - 1 powers of CT / 2 channels.
+//
+// 16 warps and one CTA per SM, every pair with an equal share of all tiles' stages (a tile that is shared leaves partial sums
+// for the fold).  Warps 0 - 7 add up accumulators and finalise, warps 8 - 14 turn fp32 values into the powers' hi and lo and
+// ask for the blocks of A, warp 15 issues the products in the pair's first CTA (its second CTA's passes on that its part of
+// a stage is there).
+//
+// What bounds it: the products, 1344 cycles per stage at 224 columns (alone, on random data: 2.0 PFLOP/s at the clock that
+// the power limit leaves).  Measured in the middle of a tile: 1550 cycles per stage.  Why a pair: the products of one CTA read
+// 1056 x 128 bytes of shared memory per 1344 cycles, beside 256 of copies of A and 448 of stores of B; of a pair, whose CTAs
+// hold half of B each, 720, 256 and 224 (512 x 3072 -> 5120, p = 8, forward / grad_x / grad_w: 488 / 331 / 369 us with single
+// CTAs, 374 / 300 / 370 with pairs).  What made the difference after that (now 248 / 220 / 301): a remote arrival without
+// cluster-wide release (1150 cycles each), prefetching loads that nothing behind them waits for (950 cycles), loops that stay
+// in the instruction cache.
+template <int PW, bool FWD>
+__global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams P) {
+    constexpr int NP = PW - 1;
+    constexpr int CT = channels_of(NP);
+    constexpr int COLS = FWD ? kNRows : NP * CT;    // columns of the accumulator
+    constexpr int NC = COLS / 2;                    // of which a warp adds up
+    constexpr int CW = CT / 2;                      // !FWD: channels of a half, which one CTA converts
+    constexpr int UNITS = CW * kBlocks / 8;         // !FWD: converter units (32 items of 8 reduction elements) per stage
+    extern __shared__ __align__(16) char raw[];
+    char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
+    Bars* B = reinterpret_cast<Bars*>(smem + kStages * kStageBytes);
+    stream_order_begin();
+    if ((P.gate0 && *P.gate0 != 0) || (P.gate1 && *P.gate1 != 0)) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1;
+    const int workers = gridDim.x / 2, worker = blockIdx.x / 2;
+    const int it0 = even_begin(P, workers, worker), it1 = even_begin(P, workers, worker + 1);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kStages; ++i) {
+            mbar_init(&B->full[i], 1 + (FWD ? kConvWarps : UNITS));
+            mbar_init(&B->peer_full[i], 1);
+            mbar_init(&B->empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&B->acc_full[i], 1);
+            mbar_init(&B->acc_empty[i], kEpiWarps * 2);
+        }
+        B->abort = 0;
+        mbar_fence_init();
+    }
+    __syncwarp();
+    if (warp == 0) tmem_alloc(&B->tmem);
+    tmem_fence_before();
+    cluster_sync();
+    tmem_fence_after();
+    const uint32_t tmem = B->tmem;
+
+    if (warp < kEpiWarps) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+        const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane;
+        const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + half * NC;
+        const int first_tile = it0 / P.kt;
+        int buf = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int it = it0; it < it1 && ok;) {
+            const Span s = span_at(P, it, it1);
+            float2 acc[NC / 2];
+#pragma unroll
+            for (int i = 0; i < NC / 2; ++i) acc[i] = make_float2(0.0f, 0.0f);
+            for (int kt = s.kt0; kt < s.kt1; ++kt) {
+                ok = __all_sync(0xffffffffu, wait_or_abort<false>(&B->acc_full[buf], phase, &B->abort, P.status));
+                if (!ok) break;
+                tmem_fence_after();
+#pragma unroll
+                for (int q = 0; q < NC; q += 32) {
+                    float v[2][16];
+                    const bool two = q + 16 < NC;
+                    tmem_load16(taddr + buf * 256 + q, v[0]);
+                    if (two) tmem_load16(taddr + buf * 256 + q + 16, v[1]);
+                    tmem_load_wait(v[0]);
+                    if (two) tmem_load_wait(v[1]);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (i < 8 || two)
+                            acc[q / 2 + i] = __fadd2_rn(acc[q / 2 + i], make_float2(v[i / 8][2 * (i % 8)], v[i / 8][2 * (i % 8) + 1]));
+                }
+                tmem_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_first(&B->acc_empty[buf]);
+                buf ^= 1;
+                if (buf == 0) phase ^= 1;
+            }
+            if (!ok) break;
+            const bool whole = s.kt0 == 0 && s.kt1 == P.kt;
+            const int m = (s.tm * 2 + rank) * kMRows + row;
+            float* part = P.partials + (static_cast<size_t>(blockIdx.x) * 2 + (it / P.kt == first_tile ? 0 : 1)) *
+                                           static_cast<size_t>(FWD ? kNRows : CT) * kMRows + row;
+            if constexpr (FWD) {
+                if (!whole) {
+#pragma unroll
+                    for (int i = 0; i < NC / 2; ++i) {
+                        part[(half * NC + 2 * i) * kMRows] = acc[i].x;
+                        part[(half * NC + 2 * i + 1) * kMRows] = acc[i].y;
+                    }
+                } else if (m < P.M) {
+                    // the sums as they are; even_fold_kernel makes values of them (the roots and guards of a tile here would
+                    // hold its CTA up for as long as ten stages)
+#pragma unroll
+                    for (int q = 0; q < NC; q += 4) {
+                        const int n = s.tn * kNRows + half * NC + q;
+                        if (P.vec) {
+                            if (n < P.N)
+                                *reinterpret_cast<float4*>(P.out_f + even_offset(P, s.g, m, n)) =
+                                    make_float4(acc[q / 2].x, acc[q / 2].y, acc[q / 2 + 1].x, acc[q / 2 + 1].y);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                if (n + i < P.N)
+                                    P.out_f[even_offset(P, s.g, m, n + i)] = i % 2 ? acc[q / 2 + i / 2].y : acc[q / 2 + i / 2].x;
+                        }
+                    }
+                }
+            } else {
+                // Horner's scheme over the powers, four channels per trip of a rolled loop: a trip takes the first of every power's
+                // columns and moves the others down (as straight-line code, 128 x 32 outputs of a tile took 6500 cycles, most
+                // of them waiting for instructions).  Meanwhile the next tile's products run on, two accumulators long.
+                const bool in = m < P.M;
+                const int n0 = s.tn * CT + half * CW, pitch = P.tiles_n * CT;
+                const float q0 = s.kt0 == 0 && in ? P.row_sum[s.g * P.M + m] * kScaleB : 0.0f;
+                const float row_scale = in ? pow2i(-15 - P.row_exp[s.g * P.M + m]) : 0.0f;
+                const float* down = P.col_down + s.g * pitch + n0;
+                const long long off = even_offset(P, s.g, m, n0);
+                const float* res = P.resident + off;
+                float* out = P.out_f + off;
+                constexpr int AHEAD = CW < 16 ? CW / 4 : 4;
+                float2 u[AHEAD][2], d[AHEAD][2];
+                auto load_resident = [&](int c, float2* v, float2* w) {
+                    load4(w, down + c, true);
+                    v[0] = v[1] = make_float2(0.0f, 0.0f);
+                    if (P.vec) {
+                        load4(v, res + c, in && n0 + c < P.N);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            load1(i % 2 ? &v[i / 2].y : &v[i / 2].x, res + (c + i) * P.out.s_n, in && n0 + c + i < P.N);
+                    }
+                };
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i) load_resident(4 * i, u[i], d[i]);
+#pragma unroll 1
+                for (int c = 0; c < CW; c += 4) {
+                    const float2 x0 = __fmul2_rn(u[0][0], d[0][0]), x1 = __fmul2_rn(u[0][1], d[0][1]);
+                    float2 h0 = make_float2(q0, q0), h1 = h0;
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) {
+                        const float k = j % 2 == 0 ? -binomial(NP, j + 1) : binomial(NP, j + 1);
+                        h0 = __ffma2_rn(h0, x0, scale2(acc[j * (CW / 2)], k));
+                        h1 = __ffma2_rn(h1, x1, scale2(acc[j * (CW / 2) + 1], k));
+                    }
+                    if (!whole) {
+                        float* o = part + (half * CW + c) * kMRows;
+                        o[0] = h0.x; o[kMRows] = h0.y; o[2 * kMRows] = h1.x; o[3 * kMRows] = h1.y;
+                    } else if (in && n0 + c < P.N) {
+                        h0 = __fmul2_rn(scale2(h0, row_scale), make_float2(up_of<NP>(d[0][0].x), up_of<NP>(d[0][0].y)));
+                        h1 = __fmul2_rn(scale2(h1, row_scale), make_float2(up_of<NP>(d[0][1].x), up_of<NP>(d[0][1].y)));
+                        if (P.vec) {
+                            float4* o = reinterpret_cast<float4*>(out + c);
+                            const float4 old = P.accumulate ? *o : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            *o = make_float4(old.x + h0.x, old.y + h0.y, old.z + h1.x, old.w + h1.y);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                if (n0 + c + i < P.N) {
+                                    float* o = out + (c + i) * P.out.s_n;
+                                    const float h = i == 0 ? h0.x : (i == 1 ? h0.y : (i == 2 ? h1.x : h1.y));
+                                    *o = P.accumulate ? *o + h : h;
+                                }
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i + 1 < AHEAD; ++i) {
+                        u[i][0] = u[i + 1][0];
+                        u[i][1] = u[i + 1][1];
+                        d[i][0] = d[i + 1][0];
+                        d[i][1] = d[i + 1][1];
+                    }
+                    if (c + 4 * AHEAD < CW) load_resident(c + 4 * AHEAD, u[AHEAD - 1], d[AHEAD - 1]);
+#pragma unroll
+                    for (int j = 0; j < NP; ++j)
+#pragma unroll
+                        for (int i = 0; i + 2 < CW / 2; ++i) acc[j * (CW / 2) + i] = acc[j * (CW / 2) + i + 2];
+                }
+            }
+            it += s.kt1 - s.kt0;
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+        if (warp == kEpiWarps + kConvWarps) {
+            uint32_t slot = 0, phase = 0, acc_phase = 1;
+            bool ok = true;
+            if (rank == 1) {
+                const int count = it1 - it0;
+                for (int i = 0; i < count; ++i) {
+                    if (!(ok = wait_or_abort<false>(&B->full[slot], phase, &B->abort, P.status))) break;
+                    if (lane == 0) mbar_arrive_first(&B->peer_full[slot]);
+                    __syncwarp();
+                    if (++slot == kStages) {
+                        slot = 0;
+                        phase ^= 1;
+                    }
+                }
+            } else {
+                // (warp-uniform code, one elected lane issues: operands stay in uniform registers)
+                const bool lead = elect_one();
+                constexpr uint32_t desc = mma_desc(kMRows * 2, COLS);
+                const uint64_t first_slot = smem_desc(smem);
+                int buf = 0;
+                for (int it = it0; it < it1 && ok;) {
+                    const Span s = span_at(P, it, it1);
+                    const int count = s.kt1 - s.kt0;
+                    for (int i = 0; i < count; ++i) {
+                        // (a fresh barrier counts as having completed the phase before its first)
+                        if (!(ok = wait_or_abort<true>(&B->acc_empty[buf], acc_phase, &B->abort, P.status))) break;
+                        if (!(ok = wait_or_abort<false>(&B->full[slot], phase, &B->abort, P.status))) break;
+                        if (!(ok = wait_or_abort<true>(&B->peer_full[slot], phase, &B->abort, P.status))) break;
+                        tmem_fence_after();
+                        if (lead) {
+                            const uint64_t a = first_slot + slot * (kStageBytes >> 4), b = a + (kBlocks * kABytes >> 4);
+                            const uint32_t d = tmem + buf * 256;
+                            // the small products first, while the accumulator is small
+#pragma unroll
+                            for (int k = 0; k < 2 * kBlocks; ++k) {
+                                const uint64_t ak = a + (k / 2) * (kABytes >> 4) + 2 * (k % 2);
+                                const uint64_t bk = b + (k / 2) * (kBBytes >> 4) + 2 * (k % 2);
+                                mma_f16(d, ak + 4, bk, desc, k > 0);
+                                if (PW == 2) mma_f16(d, ak + 4, bk + 4, desc, true);
+                                mma_f16(d, ak, bk + 4, desc, true);
+                            }
+#pragma unroll
+                            for (int k = 0; k < 2 * kBlocks; ++k)
+                                mma_f16(d, a + (k / 2) * (kABytes >> 4) + 2 * (k % 2),
+                                              b + (k / 2) * (kBBytes >> 4) + 2 * (k % 2), desc, true);
+                            mma_commit(&B->empty[slot]);
+                            mma_commit(&B->acc_full[buf]);
+                        }
+                        __syncwarp();
+                        buf ^= 1;
+                        if (buf == 0) acc_phase ^= 1;
+                        if (++slot == kStages) {
+                            slot = 0;
+                            phase ^= 1;
+                        }
+                    }
+                    it += count;
+                }
+            }
+        } else if constexpr (FWD) {
+            // Item i of a thread: 8 channels of a row of a block.  Rows contiguous in memory: four lanes for the four pieces of
+            // a row, and lanes that store together have rows that differ in bit 2, which the swizzle turns into the other half
+            // of the banks.  Channels contiguous over rows: a lane per row.
+            constexpr int ITEMS = kRowsB * 4 / (32 * kConvWarps);
+            const int t = threadIdx.x - 32 * kEpiWarps;
+            const bool lanes_are_rows = P.src.kind == 2;
+            const int row0 = lanes_are_rows ? t % kRowsB : (t >> 4) * 8 + ((t >> 3) & 1) * 2 + ((t >> 2) & 1) * 4;
+            const int piece0 = lanes_are_rows ? t / kRowsB * ITEMS : t & 3;
+            auto row_of = [&](int i) { return lanes_are_rows ? row0 : row0 + i; };
+            const ForwardScale<PW> scales(*P.scale_word);
+            const float factor = pow2i(-scales.e);
+            float2 cur[ITEMS][4], nxt[ITEMS][4];
+            uint32_t slot = 0, phase = 1;  // (a fresh barrier counts as having completed the phase before its first)
+            bool ok = true;
+            for (int it = it0; it < it1 && ok;) {
+                const Span s = span_at(P, it, it1);
+                const int n0 = s.tn * kNRows + rank * kRowsB;
+                const int last = min(P.blocks, s.kt1 * kBlocks);  // block behind the last one of the span
+                auto load = [&](int kb) {
+#pragma unroll
+                    for (int i = 0; i < ITEMS; ++i)
+                        fetch8(P.src, source_row(P.src, s.g, n0 + row_of(i)), kb * kBlockK + 8 * (lanes_are_rows ? piece0 + i : piece0), nxt[i]);
+                };
+                // (scaled when they are needed, not when they are asked for: the loads are still under way then)
+                auto scale = [&]() {
+#pragma unroll
+                    for (int i = 0; i < ITEMS; ++i)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) cur[i][e] = scale2(nxt[i][e], factor);
+                };
+                int kb = s.kt0 * kBlocks / NP, j = s.kt0 * kBlocks - kb * NP;
+                load(kb);
+                scale();
+                if ((kb + 1) * NP < last) load(kb + 1);
+                for (int kt = s.kt0; kt < s.kt1; ++kt) {
+                    ok = __all_sync(0xffffffffu, wait_or_abort<false>(&B->empty[slot], phase, &B->abort, P.status));
+                    if (!ok) break;
+                    char* stage = smem + slot * kStageBytes;
+                    if (t == 0) {
+                        mbar_expect_tx(&B->full[slot], kBlocks * kABytes);
+                        bulk_load(stage, a_blocks(P, s, kt, rank), kBlocks * kABytes, &B->full[slot]);
+                    }
+#pragma unroll 1
+                    for (int bl = 0; bl < kBlocks; ++bl) {
+                        char* b = stage + kBlocks * kABytes + bl * kBBytes;
+                        const float lift = pow2i(scales.b(NP - j));
+                        auto put = [&](auto e_tag) {
+                            constexpr int E = decltype(e_tag)::value;
+#pragma unroll
+                            for (int i = 0; i < ITEMS; ++i) {
+                                float2 v[4];
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) v[e] = scale2(power2<E>(cur[i][e]), lift);
+                                uint4 hi, lo;
+                                split8(v, &hi, &lo);
+                                const int row = row_of(i), piece = lanes_are_rows ? piece0 + i : piece0;
+                                const uint32_t at = row * 128 + ((piece ^ (row & 7)) << 4);
+                                *reinterpret_cast<uint4*>(b + at) = hi;
+                                *reinterpret_cast<uint4*>(b + (at ^ 64)) = lo;
+                            }
+                        };
+                        switch (NP - j) {
+                            case 1: put(std::integral_constant<int, 1>()); break;
+                            case 2: if constexpr (NP >= 2) put(std::integral_constant<int, 2>()); break;
+                            case 3: if constexpr (NP >= 3) put(std::integral_constant<int, 3>()); break;
+                            case 4: if constexpr (NP >= 4) put(std::integral_constant<int, 4>()); break;
+                            case 5: if constexpr (NP >= 5) put(std::integral_constant<int, 5>()); break;
+                            case 6: if constexpr (NP >= 6) put(std::integral_constant<int, 6>()); break;
+                            default: if constexpr (NP >= 7) put(std::integral_constant<int, 7>()); break;
+                        }
+                        // (behind the last block of all there may be one that only fills the stage: A is 0 there, B finite)
+                        if (++j == NP) {
+                            j = 0;
+                            ++kb;
+                            if (kb * NP < last) scale();
+                            if ((kb + 1) * NP < last) load(kb + 1);
+                        }
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&B->full[slot]);
+                    if (++slot == kStages) {
+                        slot = 0;
+                        phase ^= 1;
+                    }
+                }
+                it += s.kt1 - s.kt0;
+            }
+        } else {
+            // unit u of the CTA's range: stage u / UNITS, 32 items of it; dealt to the warps in turn.  An item is a channel
+            // and 8 rows; neighbouring lanes have neighbouring channels.
+            const int cw = warp - kEpiWarps;
+            const int units = (it1 - it0) * UNITS;
+            Span s{};
+            int span_first = 0, span_end = 0;  // the stages of the range that s describes
+            float2 nxt[4];
+            float nxt_down = 0.0f;
+            const char* nxt_a = nullptr;
+            auto fetch = [&](int u) {
+                const int n = u / UNITS, item = (u % UNITS) * 32 + lane, cl = item % CW, chunk = item / CW;
+                while (n >= span_end) {
+                    s = span_at(P, it0 + span_end, it1);
+                    span_first = span_end;
+                    span_end += s.kt1 - s.kt0;
+                }
+                const int c = s.tn * CT + rank * CW + cl, kt = s.kt0 + n - span_first;
+                fetch8(P.src, source_row(P.src, s.g, c), kt * kStageK + 8 * chunk, nxt);
+                load1(&nxt_down, P.col_down + s.g * P.tiles_n * CT + c, true);
+                if (u % UNITS == 0) nxt_a = a_blocks(P, s, kt, rank);
+            };
+            if (cw < units) fetch(cw);
+            for (int u = cw; u < units; u += kConvWarps) {
+                const int n = u / UNITS, slot = n % kStages;
+                if (!__all_sync(0xffffffffu, wait_or_abort<false>(&B->empty[slot], (n / kStages & 1) ^ 1, &B->abort, P.status))) break;
+                char* stage = smem + slot * kStageBytes;
+                if (u % UNITS == 0 && lane == 0) {
+                    mbar_expect_tx(&B->full[slot], kBlocks * kABytes);
+                    bulk_load(stage, nxt_a, kBlocks * kABytes, &B->full[slot]);
+                }
+                float2 v[4], cur[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = scale2(nxt[e], nxt_down);
+                if (u + kConvWarps < units) fetch(u + kConvWarps);
+                // row of B: power, channel of the half
+                const int item = (u % UNITS) * 32 + lane, cl = item % CW, chunk = item / CW;
+                char* b = stage + kBlocks * kABytes + (chunk / 4) * kBBytes;
+                const uint32_t at = cl * 128 + (((chunk & 3) ^ (cl & 7)) << 4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) cur[e] = scale2(v[e], kScaleB);
+#pragma unroll 1
+                for (int j = 0; j < NP; ++j) {  // (rolled: the body stays in the instruction cache)
+                    uint4 hi, lo;
+                    split8(cur, &hi, &lo);
+                    *reinterpret_cast<uint4*>(b + j * CW * 128 + at) = hi;
+                    *reinterpret_cast<uint4*>(b + j * CW * 128 + (at ^ 64)) = lo;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) cur[e] = __fmul2_rn(cur[e], v[e]);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&B->full[slot]);
+            }
+        }
+    }
+    // (every copy has landed when its stage's products were issued; after a wait that gave up they get a while)
+    if (*static_cast<volatile int*>(&B->abort))
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    tmem_fence_before();
+    __syncwarp();
+    cluster_sync();
+    tmem_fence_after();
+    __syncwarp();
+    if (warp == 0) tmem_free(tmem);
+}
+
+// Backward: adds up the partial sums of every tile that is shared between pairs.  Such a tile holds the end of some pair's
+// range; the first boundary inside it stands for it.  blockIdx.y: eight columns, blockIdx.z: CTA of the pair.
+// Forward: makes the values, of shared tiles from their partial sums, of the others from the sums in the output array;
+// blockIdx.x: tile.
+template <int PW, bool FWD>
+__global__ void __launch_bounds__(kMRows) even_fold_kernel(const EvenParams P, const int workers) {
+    constexpr int NP = PW - 1;
+    constexpr int CT = channels_of(NP);
+    constexpr int COLS = FWD ? kNRows : CT;
+    stream_order_begin();
+    if ((P.gate0 && *P.gate0 != 0) || (P.gate1 && *P.gate1 != 0)) return;
+    const int rank = blockIdx.z, row = threadIdx.x, col0 = blockIdx.y * 8;
+    int c0, t0;
+    if constexpr (FWD) {
+        t0 = blockIdx.x * P.kt;
+        c0 = static_cast<int>((static_cast<long long>(t0 + 1) * workers - 1) / P.total);
+    } else {
+        c0 = blockIdx.x;
+        const int cut = even_begin(P, workers, c0 + 1);
+        t0 = cut / P.kt * P.kt;
+        if (cut == t0 || even_begin(P, workers, c0) > t0) return;
+    }
+    const bool second = even_begin(P, workers, c0) < t0;  // worker c0 began in an earlier tile
+    const int c1 = static_cast<int>((static_cast<long long>(t0 + P.kt) * workers - 1) / P.total);
+    const Span s = span_at(P, t0, P.total);
+    const int m = (s.tm * 2 + rank) * kMRows + row, n0 = s.tn * COLS + col0;
+    if (m >= P.M || n0 >= P.N) return;
+    float v[8];
+    if (!FWD || c0 != c1) {
+        const size_t slot = static_cast<size_t>(COLS) * kMRows;
+        const float* part = P.partials + static_cast<size_t>(c0 * 2 + rank) * 2 * slot + static_cast<size_t>(col0) * kMRows + row;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = part[(second ? slot : 0) + i * kMRows];
+        for (int c = c0 + 1; c <= c1; ++c) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] += part[static_cast<size_t>(c - c0) * 4 * slot + i * kMRows];
+        }
+    }
+    if constexpr (FWD) {
+        const ForwardEnd end = forward_end<PW>(P);
+        const float sa = P.sum_a[s.g * P.M + m], na = P.norm_a[s.g * P.M + m];
+        const float *sb = P.sum_b + s.g * P.N + n0, *nb = P.norm_b + s.g * P.N + n0;
+#pragma unroll
+        for (int q = 0; q < 8; q += 4) {
+            if (n0 + q >= P.N) break;
+            long long off[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) off[i] = i > 0 && P.vec ? off[0] + i : even_offset(P, s.g, m, min(n0 + q + i, P.N - 1));
+            if (c0 == c1) {
+                if (P.vec) {
+                    const float4 r = *reinterpret_cast<const float4*>(P.out_f + off[0]);
+                    v[q] = r.x; v[q + 1] = r.y; v[q + 2] = r.z; v[q + 3] = r.w;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[q + i] = P.out_f[off[i]];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (n0 + q + i < P.N)
+                    v[q + i] = forward_value<PW>(P, end, v[q + i], sa, na, sb[q + i], nb[q + i], static_cast<int>(off[i]));
+            if (P.vec) {
+                *reinterpret_cast<float4*>(P.out_f + off[0]) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (n0 + q + i < P.N) P.out_f[off[i]] = v[q + i];
+            }
+        }
+    } else {
+        const float row_scale = pow2i(-15 - P.row_exp[s.g * P.M + m]);
+        const float* down = P.col_down + s.g * P.tiles_n * CT + n0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (n0 + i < P.N) {
+                float* o = P.out_f + even_offset(P, s.g, m, n0 + i);
+                const float h = v[i] * row_scale * up_of<NP>(down[i]);
+                *o = P.accumulate ? *o + h : h;
+            }
+    }
+}
+
+// ---- preparation -----------------------------------------------------------------------------------------------------
+// One item of a block of A: eight reduction elements of a row, hi and lo where the swizzle puts them.
+__device__ __forceinline__ void put_item(char* block, int row, int chunk, const float2 (&v)[4]) {
+    uint4 hi, lo;
+    split8(v, &hi, &lo);
+    const uint32_t at = row * 128 + ((chunk ^ (row & 7)) << 4);
+    *reinterpret_cast<uint4*>(block + at) = hi;
+    *reinterpret_cast<uint4*>(block + (at ^ 64)) = lo;
+}
+constexpr int kPrep = 256;
+__device__ __forceinline__ void item_of(const Source& S, int i, int* row, int* chunk) {
+    const bool lanes_are_rows = S.kind == 2;  // neighbouring rows are neighbours in memory
+    *row = lanes_are_rows ? i & (kMRows - 1) : i >> 2;
+    *chunk = lanes_are_rows ? i >> 7 : i & 3;
+}
+__device__ __forceinline__ unsigned magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+
+// Sums of p-th powers of every row of both operands (64 bits: 4 us of arithmetic at 512 x 3072 -> 5120, and no error of
+// theirs reaches the result) and the largest magnitude of all.  Rows contiguous in memory: a warp per row; else 32 rows per
+// block, its warps sharing the reduction.
+template <int PW>
+__device__ __forceinline__ void row_power_sums(const Source& S, int G, int block, double* sums, unsigned* scale_word) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned top = 0;
+    double sum = 0.0;
+    auto take = [&](float v) {
+        top = max(top, magnitude(v));
+        double d = v;
+        d *= d;
+        double q = d;
+#pragma unroll
+        for (int i = 1; i < PW / 2; ++i) q *= d;
+        sum += q;
+    };
+    if (S.kind != 2) {
+        const long long r = static_cast<long long>(block) * 8 + warp;
+        if (r < static_cast<long long>(G) * S.rows) {
+            const int g = static_cast<int>(r / S.rows);
+            const float* p = source_row(S, g, static_cast<int>(r - static_cast<long long>(g) * S.rows));
+            if (S.kind == 0) {
+#pragma unroll 4
+                for (int k = 4 * lane; k < S.k; k += 128) {
+                    const float4 v = *reinterpret_cast<const float4*>(p + k);
+                    take(v.x); take(v.y); take(v.z); take(v.w);
+                }
+            } else {
+#pragma unroll 8
+                for (int k = lane; k < S.k; k += 32) take(p[k]);
+            }
+            for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+            if (lane == 0) sums[r] = sum;
+        }
+    } else {
+        __shared__ double part[8][32];
+        const int per_group = (S.rows + 31) / 32, g = block / per_group, row = (block - g * per_group) * 32 + lane;
+        const float* p = source_row(S, g, row);
+        if (p)
+#pragma unroll 4
+            for (int k = warp; k < S.k; k += 8) take(p[k * S.s_k]);
+        part[warp][lane] = sum;
+        __syncthreads();
+        if (warp == 0 && p) {
+            for (int i = 1; i < 8; ++i) sum += part[i][lane];
+            sums[static_cast<long long>(g) * S.rows + row] = sum;
+        }
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0 && top > *static_cast<volatile unsigned*>(scale_word)) atomicMax(scale_word, top);
+}
+template <int PW>
+__global__ void __launch_bounds__(kPrep) even_rows_kernel(const Source a, const Source b, int G, int blocks_a, double* sums_a,
+                                                         double* sums_b, unsigned* scale_word) {
+    stream_order_begin();
+    if (static_cast<int>(blockIdx.x) < blocks_a) row_power_sums<PW>(a, G, blockIdx.x, sums_a, scale_word);
+    else row_power_sums<PW>(b, G, blockIdx.x - blocks_a, sums_b, scale_word);
+}
+
+// The blocks of A of the forward form, C(p, j) x^j split, j = 1 .. p - 1 (seq blocks per block of rows: zeros behind the last
+// where stages need an even number); the blocks behind those put the row sums on the common scale.
+template <int PW>
+__global__ void __launch_bounds__(kPrep) even_powers_kernel(const Source a, int G, int tiles_m, int kb, int seq, char* images,
+                                                           const double* sums_a, const double* sums_b, int rows_b,
+                                                           float* sum_a, float* norm_a, float* sum_b, float* norm_b,
+                                                           const unsigned* scale_word, int* dense) {
+    constexpr int NP = PW - 1;
+    stream_order_begin();
+    const unsigned top = *scale_word;
+    const int e = exponent_above(top);
+    if (top >= 0x7f800000u || e < -100 || e > 100) {  // not finite, all zero, or hardly a number
+        if (blockIdx.x == 0 && threadIdx.x == 0) *dense = 1;
+        return;
+    }
+    const int images_blocks = G * tiles_m * kb, block = blockIdx.x;
+    if (block >= images_blocks) {
+        const int i = (block - images_blocks) * kPrep + threadIdx.x;
+        if (i >= G * (a.rows + rows_b)) return;
+        const bool is_a = i < G * a.rows;
+        const int r = is_a ? i : i - G * a.rows;
+        const float v = static_cast<float>((is_a ? sums_a : sums_b)[r] * exp2(-static_cast<double>(PW) * e));
+        (is_a ? sum_a : sum_b)[r] = v;
+        (is_a ? norm_a : norm_b)[r] = v > 0.0f ? root<PW>(v) : 0.0f;
+        return;
+    }
+    const ForwardScale<PW> scales(top);
+    const float factor = pow2i(-e);
+    const int k = block % kb, t = block / kb, tm = t % tiles_m, g = t / tiles_m;
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+        int row, chunk;
+        item_of(a, threadIdx.x + n * kPrep, &row, &chunk);
+        float2 v[4], cur[4];
+        fetch8(a, source_row(a, g, tm * kMRows + row), k * kBlockK + 8 * chunk, v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cur[i] = v[i] = scale2(v[i], factor);
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            float2 term[4];
+            const float c = (j % 2 == 0 ? -binomial(PW, j + 1) : binomial(PW, j + 1)) * pow2i(scales.a(j + 1));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) term[i] = scale2(cur[i], c);
+            put_item(images + ((static_cast<long long>(g) * tiles_m + tm) * seq + k * NP + j) * static_cast<long long>(kABytes), row,
+                     chunk, term);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) cur[i] = __fmul2_rn(cur[i], v[i]);
+        }
+        if (k == kb - 1 && seq > kb * NP) {
+            const float2 zero[4] = {};
+            put_item(images + ((static_cast<long long>(g) * tiles_m + tm) * seq + kb * NP) * static_cast<long long>(kABytes), row, chunk,
+                     zero);
+        }
+    }
+}
+
+// The listed outputs, summed directly: a warp each.
+template <int PW>
+__global__ void __launch_bounds__(kPrep) even_direct_kernel(const float* x, const float* w, Shape s, float* y, const int* list,
+                                                           const int* list_count, const int* dense) {
+    stream_order_begin();
+    if (*dense != 0) return;
+    const int count = min(*list_count, kListCap), lane = threadIdx.x & 31;
+    for (int i = blockIdx.x * (kPrep / 32) + (threadIdx.x >> 5); i < count; i += gridDim.x * (kPrep / 32)) {
+        const int off = list[i], t = off / s.HW, hw = off - t * s.HW, b = t / s.CO, o = t - b * s.CO, g = o / s.COg;
+        const float* xr = x + (static_cast<long long>(b) * s.CI + static_cast<long long>(g) * s.CIg) * s.HW + hw;
+        const float* wr = w + static_cast<long long>(o) * s.CIg;
+        float sum = 0.0f;
+        for (int c = lane; c < s.CIg; c += 32) sum += power<PW>(xr[static_cast<long long>(c) * s.HW] - wr[c]);
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (lane == 0) y[off] = powf(fmaxf(sum, FLT_MIN), 1.0f / PW);
+    }
+}
+
+// Order-preserving code of a float (0 is below all of them); a not-a-number of either sign is above infinity in the code of
+// the value or of its negative.
+__device__ __forceinline__ unsigned ordered(float v) {
+    const unsigned b = __float_as_uint(v);
+    return (b & 0x80000000u) ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float from_ordered(unsigned c) {
+    return __uint_as_float((c & 0x80000000u) ? c & 0x7fffffffu : ~c);
+}
+
+constexpr int kColumnRows = 128;  // rows per block of the column jobs
+constexpr int kMaxSplits = 64;    // row ranges of the coefficients' column sums
+constexpr int kMaxChannelExp = 17;  // channels of values beyond 2^17 or below 2^-17: 2^(7 * 17) is still a number
+
+struct BackwardStats {
+    Shape s;
+    const float *coef, *x, *w, *y;
+    int pitch;
+    int *row_exp, *out_exp;                           // rows of the coefficients, output channels
+    float *row_sum, *out_sum;
+    float *down_w, *down_x;                           // [g][channel_pitch], of the two sources
+    int channel_pitch;
+    unsigned *x_top, *x_low, *w_top, *w_low;          // per channel: codes of the largest value and of the largest negative
+    unsigned *x_all, *w_all, *y_low;                  // bits of the largest |x| and |w|, code of the largest -y
+    unsigned* part_top;                               // [split][CO]
+    double* part_sum;
+    int splits, rows_per_split;
+    int blocks_rows, blocks_cols, blocks_w, blocks_x, blocks_y; // blocks of each job, in this order
+    int blocks_channels;                              // of the second kernel
+    int* bad;                                         // data that the expansion does not suit
+    const int* range;
+    int* cond;
+};
+
+// The largest magnitude of all, from a lane's largest code of a value or of its negative.
+__device__ __forceinline__ void raise_magnitude(unsigned* all, unsigned code) {
+    code = __reduce_max_sync(0xffffffffu, code);
+    const unsigned bits = code & 0x7fffffffu;  // (the larger of the two codes is that of a positive number or of zero)
+    if ((threadIdx.x & 31) == 0 && (code & 0x80000000u) && bits > *static_cast<volatile unsigned*>(all)) atomicMax(all, bits);
+}
+
+// column extremes of rows [r0, r1) of a matrix whose columns are contiguous: 32 columns per block
+__device__ __forceinline__ void column_extremes(const float* p, long long pitch, int r0, int r1, int col, int cols, unsigned* top,
+                                                unsigned* low, unsigned* all) {
+    __shared__ unsigned tops[8][32], lows[8][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned t = 0, l = 0;
+    if (col + lane < cols)
+#pragma unroll 8
+        for (int r = r0 + warp; r < r1; r += 8) {
+            const float v = p[r * pitch + col + lane];
+            t = max(t, ordered(v));
+            l = max(l, ordered(-v));
+        }
+    tops[warp][lane] = t;
+    lows[warp][lane] = l;
+    __syncthreads();
+    if (warp == 0) {
+        for (int i = 1; i < 8; ++i) {
+            t = max(t, tops[i][lane]);
+            l = max(l, lows[i][lane]);
+        }
+        if (col + lane < cols) {
+            atomicMax(top + col + lane, t);
+            atomicMax(low + col + lane, l);
+        }
+        raise_magnitude(all, max(t, l));
+    }
+}
+
+__device__ __forceinline__ int row_scale(unsigned top) {
+    return top == 0 ? 0 : max(-100, min(100, 15 - exponent_above(top)));
+}
+
+// What the backward form needs to know of its operands: the smallest output, largest coefficient and sum of every row (over the output channels)
+// and of every output channel (over the rows, in ranges), and the range of values of every channel of x and w.
+__global__ void __launch_bounds__(kPrep) even_stats_kernel(const BackwardStats A) {
+    stream_order_begin();
+    const Shape& s = A.s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int block = blockIdx.x;
+    if (block < A.blocks_rows) {
+        const long long r = static_cast<long long>(block) * 8 + warp;
+        if (r >= static_cast<long long>(s.G) * s.M) return;
+        const float* p = A.coef + r * A.pitch;
+        unsigned top = 0;
+        double sum = 0.0;
+#pragma unroll 4
+        for (int o = lane; o < s.COg; o += 32) {
+            top = max(top, magnitude(p[o]));
+            sum += p[o];
+        }
+        top = __reduce_max_sync(0xffffffffu, top);
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (lane == 0) {
+            const int e = row_scale(top);
+            A.row_exp[r] = e;
+            A.row_sum[r] = static_cast<float>(sum * pow2i(e));
+            if (top >= 0x7f800000u) *A.bad = 1;
+        }
+        return;
+    }
+    block -= A.blocks_rows;
+    if (block < A.blocks_cols) {
+        __shared__ unsigned tops[8][32];
+        __shared__ double sums[8][32];
+        const int per_group = (s.COg + 31) / 32;
+        const int split = block / (per_group * s.G), rest = block - split * per_group * s.G, g = rest / per_group;
+        const int o = (rest - g * per_group) * 32 + lane;
+        const long long r0 = static_cast<long long>(split) * A.rows_per_split;
+        const long long r1 = r0 + A.rows_per_split < s.M ? r0 + A.rows_per_split : s.M;
+        unsigned top = 0;
+        double sum = 0.0;
+        if (o < s.COg) {
+            const float* p = A.coef + static_cast<long long>(g) * s.M * A.pitch + o;
+#pragma unroll 8
+            for (long long r = r0 + warp; r < r1; r += 8) {
+                const float v = p[r * A.pitch];
+                top = max(top, magnitude(v));
+                sum += v;
+            }
+        }
+        tops[warp][lane] = top;
+        sums[warp][lane] = sum;
+        __syncthreads();
+        if (warp == 0 && o < s.COg) {
+            for (int i = 1; i < 8; ++i) {
+                top = max(top, tops[i][lane]);
+                sum += sums[i][lane];
+            }
+            const long long at = static_cast<long long>(split) * s.CO + g * s.COg + o;
+            A.part_top[at] = top;
+            A.part_sum[at] = sum;
+        }
+        return;
+    }
+    block -= A.blocks_cols;
+    const int col_blocks = (s.CIg + 31) / 32;
+    if (block < A.blocks_w) {
+        const int cb = block % col_blocks, t = block / col_blocks, g = t % s.G, r0 = (t / s.G) * kColumnRows;
+        column_extremes(A.w + static_cast<long long>(g) * s.COg * s.CIg, s.CIg, r0, min(s.COg, r0 + kColumnRows), cb * 32, s.CIg,
+                        A.w_top + g * s.CIg, A.w_low + g * s.CIg, A.w_all);
+        return;
+    }
+    block -= A.blocks_w;
+    if (block >= A.blocks_x) {
+        const long long total = s.M * s.CO, step = static_cast<long long>(A.blocks_y) * kPrep;
+        unsigned l = 0;
+#pragma unroll 4
+        for (long long i = static_cast<long long>(block - A.blocks_x) * kPrep + threadIdx.x; i < total; i += step) l = max(l, ordered(-A.y[i]));
+        l = __reduce_max_sync(0xffffffffu, l);
+        if (lane == 0 && l > *static_cast<volatile unsigned*>(A.y_low)) atomicMax(A.y_low, l);
+        return;
+    }
+    if (s.HW == 1) {
+        const int cols = (s.CI + 31) / 32, cb = block % cols, r0 = (block / cols) * kColumnRows;
+        column_extremes(A.x, s.CI, r0, min(s.B, r0 + kColumnRows), cb * 32, s.CI, A.x_top, A.x_low, A.x_all);
+        return;
+    }
+    const long long r = static_cast<long long>(block) * 8 + warp;  // (sample, channel)
+    if (r >= static_cast<long long>(s.B) * s.CI) return;
+    const float* p = A.x + r * s.HW;
+    unsigned t = 0, l = 0;
+#pragma unroll 4
+    for (int i = lane; i < s.HW; i += 32) {
+        t = max(t, ordered(p[i]));
+        l = max(l, ordered(-p[i]));
+    }
+    t = __reduce_max_sync(0xffffffffu, t);
+    l = __reduce_max_sync(0xffffffffu, l);
+    if (lane == 0) {
+        atomicMax(A.x_top + r % s.CI, t);
+        atomicMax(A.x_low + r % s.CI, l);
+    }
+    raise_magnitude(A.x_all, max(t, l));
+}
+
+// Scales of the channels and of the output channels' coefficients; whether the expansion suits the data: the values of a
+// channel, of both operands together, have to spread over at least a quarter of the largest of them.
+__global__ void __launch_bounds__(kPrep) even_scales_kernel(const BackwardStats A) {
+    stream_order_begin();
+    const Shape& s = A.s;
+    const int i = blockIdx.x * kPrep + threadIdx.x;
+    bool bad = false;
+    if (i < s.CI && static_cast<int>(blockIdx.x) < A.blocks_channels) {
+        const float xt = from_ordered(A.x_top[i]), xl = from_ordered(A.x_low[i]);   // largest value, largest negative
+        const float wt = from_ordered(A.w_top[i]), wl = from_ordered(A.w_low[i]);
+        const float xm = fmaxf(fabsf(xt), fabsf(xl)), wm = fmaxf(fabsf(wt), fabsf(wl)), m = fmaxf(xm, wm);
+        const bool finite = xt + xl + wt + wl < INFINITY && fmaxf(xt, wt) < INFINITY && fmaxf(xl, wl) < INFINITY;
+        bad = !finite || !(4.0f * (fmaxf(xt, wt) + fmaxf(xl, wl)) >= m);
+        const unsigned fw = __float_as_uint(fmaxf(wm, xm * (1.0f / 64))), fx = __float_as_uint(fmaxf(xm, wm * (1.0f / 64)));
+        const int ew = fw == 0 ? 0 : exponent_above(fw), ex = fx == 0 ? 0 : exponent_above(fx);
+        bad |= max(abs(ew), abs(ex)) > kMaxChannelExp;
+        const int at = i / s.CIg * A.channel_pitch + i % s.CIg;
+        A.down_w[at] = pow2i(-max(-kMaxChannelExp, min(kMaxChannelExp, ew)));
+        A.down_x[at] = pow2i(-max(-kMaxChannelExp, min(kMaxChannelExp, ex)));
+    }
+    if (static_cast<int>(blockIdx.x) >= A.blocks_channels) {  // a warp per output channel
+        const int o = (static_cast<int>(blockIdx.x) - A.blocks_channels) * (kPrep / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+        unsigned top = 0;
+        double sum = 0.0;
+        for (int k = lane; k < A.splits && o < s.CO; k += 32) {
+            top = max(top, A.part_top[static_cast<long long>(k) * s.CO + o]);
+            sum += A.part_sum[static_cast<long long>(k) * s.CO + o];
+        }
+        top = __reduce_max_sync(0xffffffffu, top);
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (lane == 0 && o < s.CO) {
+            const int e = row_scale(top);
+            A.out_exp[o] = e;
+            A.out_sum[o] = static_cast<float>(sum * pow2i(e));
+        }
+        return;
+    }
+    if (i == 0) {
+        const float most = __uint_as_float(*A.x_all) + __uint_as_float(*A.w_all), least = -from_ordered(*A.y_low);
+        bad |= *A.bad != 0 || !(3.0f * least >= most);
+    }
+    if (bad && *A.range == 0) *A.cond = 1;
+}
+
+// Blocks of A of the backward form: the coefficients with rows = positions (grad_x) and with rows = output channels (grad_w).
+struct CoefImages {
+    Source src;
+    const int* exp;
+    char* images;
+    int tiles_m, kb, blocks;
+};
+__global__ void __launch_bounds__(kPrep) even_coef_kernel(const CoefImages X, const CoefImages W, const int* gate0, const int* gate1) {
+    stream_order_begin();
+    if (*gate0 != 0 || *gate1 != 0) return;
+    const bool first = static_cast<int>(blockIdx.x) < X.blocks;
+    const CoefImages& J = first ? X : W;
+    const int block = first ? blockIdx.x : blockIdx.x - X.blocks;
+    const int k = block % J.kb, t = block / J.kb, tm = t % J.tiles_m, g = t / J.tiles_m;
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+        int row, chunk;
+        item_of(J.src, threadIdx.x + n * kPrep, &row, &chunk);
+        const int r = tm * kMRows + row;
+        float2 v[4];
+        fetch8(J.src, source_row(J.src, g, r), k * kBlockK + 8 * chunk, v);
+        const float f = r < J.src.rows ? pow2i(J.exp[g * J.src.rows + r]) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = scale2(v[i], f);
+        put_item(J.images + static_cast<long long>(block) * kABytes, row, chunk, v);
+    }
+}
+
+// ---- host ------------------------------------------------------------------------------------------------------------
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline int div_up(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
+
+// x as rows = positions, reduction = channels; w as rows = output channels
+Source rows_of_x(const float* x, const Shape& s) {
+    if (s.HW == 1) return Source{x, s.CIg % 4 == 0 && aligned16(x) ? 0 : 1, static_cast<int>(s.M), s.CIg, 0, s.CI, 1, 0, s.CIg};
+    return Source{x, 2, static_cast<int>(s.M), s.CIg, s.HW, 1, s.HW, static_cast<long long>(s.CI) * s.HW,
+                  static_cast<long long>(s.CIg) * s.HW};
+}
+Source rows_of_w(const float* w, const Shape& s) {
+    return Source{w, s.CIg % 4 == 0 && aligned16(w) ? 0 : 1, s.COg, s.CIg, 0, s.CIg, 1, 0, static_cast<long long>(s.COg) * s.CIg};
+}
+// rows = channels, reduction = output channels (w) or positions (x)
+Source channels_of_w(const float* w, const Shape& s) {
+    return Source{w, 2, s.CIg, s.COg, 0, 1, s.CIg, 0, static_cast<long long>(s.COg) * s.CIg};
+}
+Source channels_of_x(const float* x, const Shape& s) {
+    if (s.HW == 1) return Source{x, 2, s.CIg, s.B, 0, 1, s.CI, 0, s.CIg};
+    return Source{x, s.HW % 4 == 0 && aligned16(x) ? 4 : 3, s.CIg, static_cast<int>(s.M), s.HW, s.HW, 1,
+                  static_cast<long long>(s.CI) * s.HW, static_cast<long long>(s.CIg) * s.HW};
+}
+
+// tiles along m rows of A and blocks of kMRows rows in them; stages along k reduction elements
+int row_tiles(long long m) { return div_up(m, 2 * kMRows); }
+int row_blocks(long long m) { return 2 * row_tiles(m); }
+int stages_of(long long k) { return div_up(k, kStageK); }
+
+// Which operand's powers are written out as A: the one for which products on padding plus the bytes of its powers take less
+// time, at 1.2 PFLOP/s and 4 TB/s.
+struct ForwardPlan {
+    bool swap;  // A = w
+    int M, N, row_blocks, tiles_n, stages;
+    size_t image_bytes;
+};
+ForwardPlan plan_forward(const Shape& s, int np) {
+    ForwardPlan best{};
+    double least = 0.0;
+    for (int swap = 0; swap < 2; ++swap) {
+        ForwardPlan f;
+        f.swap = swap != 0;
+        f.M = swap ? s.COg : static_cast<int>(s.M);
+        f.N = swap ? static_cast<int>(s.M) : s.COg;
+        f.row_blocks = row_blocks(f.M);
+        f.tiles_n = div_up(f.N, kNRows);
+        f.stages = stages_of(static_cast<long long>(div_up(s.CIg, kBlockK)) * np * kBlockK);
+        f.image_bytes = static_cast<size_t>(s.G) * f.row_blocks * f.stages * kBlocks * kABytes;
+        const double flops = 6.0 * s.G * f.stages * kStageK * (1.0 * f.row_blocks * kMRows) * (1.0 * f.tiles_n * kNRows);
+        const double t = flops / 1.2e15 + 2.0 * f.image_bytes / 4e12;
+        if (swap == 0 || t < least) {
+            least = t;
+            best = f;
+        }
+    }
+    return best;
+}
+
+size_t even_partial_floats(int cap, int cols) { return static_cast<size_t>(cap) * 2 * cols * kMRows; }
+
+template <int PW, bool FWD>
+int launch_even(const EvenParams& P, int cap, cudaStream_t st) {
+    static bool configured[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 64 && !configured[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(even_kernel<PW, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kEvenSmem);
+        if (e != cudaSuccess) return cuda_status(e);
+        configured[dev] = true;
+    }
+    const int most = cap / 2, workers = P.total < most ? P.total : most;
+    timing_before(st);
+    int r = launch_after_in_clusters(even_kernel<PW, FWD>, 2, workers * 2, kEvenThreads, kEvenSmem, st, P);
+    timing_after(st);
+    if (r != kOk) return r;
+    if (FWD) return launch_after(even_fold_kernel<PW, FWD>, dim3(P.total / P.kt, kNRows / 8, 2), kMRows, 0, st, P, workers);
+    if (workers < 2 || (P.total % workers == 0 && (P.total / workers) % P.kt == 0)) return kOk;
+    return launch_after(even_fold_kernel<PW, FWD>, dim3(workers - 1, channels_of(PW - 1) / 8, 2), kMRows, 0, st, P, workers);
+}
+
+template <int PW>
+int forward_power(const float* x, const float* w, const Shape& s, float* y, int cap, Bump* bump, int* status, const int** dense,
+                  cudaStream_t st) {
+    constexpr int NP = PW - 1;
+    const ForwardPlan f = plan_forward(s, NP);
+    const int rows_x = static_cast<int>(s.G * s.M), rows_w = s.CO;
+    const int rows_a = f.swap ? rows_w : rows_x, rows_b = f.swap ? rows_x : rows_w;
+    char* images = bump->take<char>(f.image_bytes);
+    double* sums = bump->take<double>(static_cast<size_t>(rows_a) + rows_b);
+    float* floats = bump->take<float>(2 * (static_cast<size_t>(rows_a) + rows_b));
+    int* list = bump->take<int>(kListCap);
+    int* words = bump->take<int>(4);  // largest magnitude, list length, dense
+    float* partials = bump->take<float>(even_partial_floats(cap, kNRows));
+    if (!images || !sums || !floats || !list || !words || !partials) return kWorkspace;
+    *dense = words + 2;
+    const cudaError_t e = cudaMemsetAsync(words, 0, 4 * sizeof(int), st);
+    if (e != cudaSuccess) return cuda_status(e);
+    const Source xs = rows_of_x(x, s), ws = rows_of_w(w, s);
+    const Source a = f.swap ? ws : xs, b = f.swap ? xs : ws;
+    unsigned* scale = reinterpret_cast<unsigned*>(words);
+    auto sum_blocks = [&](const Source& S) { return S.kind == 2 ? s.G * div_up(S.rows, 32) : div_up(static_cast<long long>(s.G) * S.rows, 8); };
+    const int blocks_a = sum_blocks(a);
+    int r = launch_after(even_rows_kernel<PW>, blocks_a + sum_blocks(b), kPrep, 0, st, a, b, s.G, blocks_a, sums, sums + rows_a, scale);
+    if (r != kOk) return r;
+    float *sum_a = floats, *norm_a = sum_a + rows_a, *sum_b = norm_a + rows_a, *norm_b = sum_b + rows_b;
+    const int kb = div_up(s.CIg, kBlockK);
+    const int prep = s.G * f.row_blocks * kb + div_up(static_cast<long long>(rows_a) + rows_b, kPrep);
+    r = launch_after(even_powers_kernel<PW>, prep, kPrep, 0, st, a, s.G, f.row_blocks, kb, f.stages * kBlocks, images, sums,
+                     sums + rows_a, b.rows, sum_a, norm_a, sum_b, norm_b, scale, words + 2);
+    if (r != kOk) return r;
+    EvenParams P{};
+    P.M = f.M; P.N = f.N; P.K = s.CIg; P.G = s.G;
+    P.tiles_m = row_tiles(f.M); P.tiles_n = f.tiles_n; P.kt = f.stages; P.blocks = kb * NP;
+    P.total = s.G * P.tiles_m * P.tiles_n * P.kt;
+    P.images = images;
+    P.src = b;
+    P.out = OutAddr{static_cast<long long>(s.CO) * s.HW, 1, static_cast<long long>(s.COg) * s.HW, s.HW, s.HW};
+    P.swap = f.swap;
+    // rows of four neighbours: output channels of a fully connected layer, or positions of an image
+    P.vec = aligned16(y) && (f.swap ? s.HW > 1 && s.HW % 4 == 0 : s.HW == 1 && s.COg % 4 == 0);
+    P.out_f = y;
+    P.sum_a = sum_a; P.norm_a = norm_a; P.sum_b = sum_b; P.norm_b = norm_b;
+    P.scale_word = scale;
+    P.list = list; P.list_count = words + 1; P.dense = words + 2;
+    P.gate0 = words + 2;
+    P.partials = partials;
+    P.status = status;
+    if ((r = launch_even<PW, true>(P, cap, st)) != kOk) return r;
+    return launch_after(even_direct_kernel<PW>, 148, kPrep, 0, st, x, w, s, y, static_cast<const int*>(list),
+                        static_cast<const int*>(words + 1), static_cast<const int*>(words + 2));
+}
+
+// ranges of rows for the coefficients' column sums
+int row_splits(const Shape& s) {
+    const int n = div_up(s.M, 128);
+    return n < kMaxSplits ? n : kMaxSplits;
+}
+
+template <int PW>
+int backward_power(const float* coef, int pitch, const float* x, const float* w, const float* y, const Shape& s, float* gx, float* gw,
+                   bool accumulate_gw, const int* range, int cap, Bump* bump, int* status, const int** cond, cudaStream_t st) {
+    constexpr int NP = PW - 1;
+    constexpr int CT = channels_of(NP);
+    const size_t rows = static_cast<size_t>(s.G) * s.M;
+    const int splits = row_splits(s);
+    BackwardStats A{};
+    A.s = s;
+    A.coef = coef; A.x = x; A.w = w; A.y = y; A.pitch = pitch;
+    A.row_exp = bump->take<int>(rows);
+    A.row_sum = bump->take<float>(rows);
+    A.out_exp = bump->take<int>(s.CO);
+    A.out_sum = bump->take<float>(s.CO);
+    A.channel_pitch = div_up(s.CIg, CT) * CT;
+    const size_t scales = static_cast<size_t>(s.G) * A.channel_pitch;
+    A.down_w = bump->take<float>(2 * scales);
+    A.down_x = A.down_w + scales;
+    unsigned* words = bump->take<unsigned>(4 * static_cast<size_t>(s.CI) + 8);
+    A.part_top = bump->take<unsigned>(static_cast<size_t>(splits) * s.CO);
+    A.part_sum = bump->take<double>(static_cast<size_t>(splits) * s.CO);
+    // grad_x: rows = positions, reduction = output channels; grad_w the other way round
+    const int kb_x = kBlocks * stages_of(s.COg), kb_w = kBlocks * stages_of(s.M);
+    const size_t blocks_x = static_cast<size_t>(s.G) * row_blocks(s.M) * kb_x, blocks_w = static_cast<size_t>(s.G) * row_blocks(s.COg) * kb_w;
+    char* images_x = gx ? bump->take<char>(blocks_x * kABytes) : nullptr;
+    char* images_w = gw ? bump->take<char>(blocks_w * kABytes) : nullptr;
+    float* partials = bump->take<float>(even_partial_floats(cap, CT));
+    if (!A.row_exp || !A.row_sum || !A.out_exp || !A.out_sum || !A.down_w || !words || !A.part_top ||
+        !A.part_sum || (gx && !images_x) || (gw && !images_w) || !partials)
+        return kWorkspace;
+    A.x_top = words; A.x_low = words + s.CI; A.w_top = words + 2 * s.CI; A.w_low = words + 3 * s.CI;
+    A.bad = reinterpret_cast<int*>(words + 4 * s.CI);
+    A.cond = A.bad + 1;
+    A.x_all = words + 4 * s.CI + 2; A.w_all = A.x_all + 1; A.y_low = A.x_all + 2;
+    A.range = range;
+    *cond = A.cond;
+    cudaError_t e = cudaMemsetAsync(words, 0, (4 * static_cast<size_t>(s.CI) + 8) * sizeof(unsigned), st);
+    // (scales of the padding channels are multiplied with zeros: they only have to be numbers)
+    if (e == cudaSuccess && A.channel_pitch != s.CIg) e = cudaMemsetAsync(A.down_w, 0, 2 * scales * sizeof(float), st);
+    if (e != cudaSuccess) return cuda_status(e);
+    A.splits = splits;
+    A.rows_per_split = div_up(s.M, splits);
+    A.blocks_rows = div_up(static_cast<long long>(rows), 8);
+    A.blocks_cols = splits * s.G * div_up(s.COg, 32);
+    A.blocks_w = div_up(s.CIg, 32) * s.G * div_up(s.COg, kColumnRows);
+    A.blocks_x = s.HW == 1 ? div_up(s.CI, 32) * div_up(s.B, kColumnRows) : div_up(static_cast<long long>(s.B) * s.CI, 8);
+    A.blocks_y = div_up(s.M * s.CO, 16 * kPrep);
+    if (A.blocks_y > 1184) A.blocks_y = 1184;
+    int r = launch_after(even_stats_kernel, A.blocks_rows + A.blocks_cols + A.blocks_w + A.blocks_x + A.blocks_y, kPrep, 0, st, A);
+    if (r != kOk) return r;
+    A.blocks_channels = div_up(s.CI, kPrep);
+    if ((r = launch_after(even_scales_kernel, A.blocks_channels + div_up(s.CO, kPrep / 32), kPrep, 0, st, A)) != kOk) return r;
+    CoefImages X{}, W{};
+    const long long group = static_cast<long long>(s.M) * pitch;
+    X.src = Source{coef, s.COg % 4 == 0 ? 0 : 1, static_cast<int>(s.M), s.COg, 0, pitch, 1, 0, group};
+    X.exp = A.row_exp; X.images = images_x; X.tiles_m = row_blocks(s.M); X.kb = kb_x;
+    X.blocks = gx ? static_cast<int>(blocks_x) : 0;
+    W.src = Source{coef, 2, s.COg, static_cast<int>(s.M), 0, 1, pitch, 0, group};
+    W.exp = A.out_exp; W.images = images_w; W.tiles_m = row_blocks(s.COg); W.kb = kb_w;
+    W.blocks = gw ? static_cast<int>(blocks_w) : 0;
+    if ((r = launch_after(even_coef_kernel, X.blocks + W.blocks, kPrep, 0, st, X, W, range, static_cast<const int*>(A.cond))) != kOk) return r;
+    EvenParams P{};
+    P.G = s.G;
+    P.N = s.CIg;
+    P.tiles_n = div_up(s.CIg, CT);
+    P.gate0 = range;
+    P.gate1 = A.cond;
+    P.partials = partials;
+    P.status = status;
+    if (gx) {
+        P.M = static_cast<int>(s.M); P.K = s.COg;
+        P.tiles_m = row_tiles(s.M); P.kt = stages_of(s.COg);
+        P.total = s.G * P.tiles_m * P.tiles_n * P.kt;
+        P.images = images_x;
+        P.src = channels_of_w(w, s);
+        P.out = OutAddr{static_cast<long long>(s.CI) * s.HW, 1, static_cast<long long>(s.CIg) * s.HW, s.HW, s.HW};
+        P.vec = s.HW == 1 && s.CIg % 4 == 0 && aligned16(x) && aligned16(gx);
+        P.out_f = gx;
+        P.resident = x;
+        P.col_down = A.down_w; P.row_exp = A.row_exp; P.row_sum = A.row_sum;
+        if ((r = launch_even<PW, false>(P, cap, st)) != kOk) return r;
+    }
+    if (gw) {
+        P.M = s.COg; P.K = static_cast<int>(s.M);
+        P.tiles_m = row_tiles(s.COg); P.kt = stages_of(s.M);
+        P.total = s.G * P.tiles_m * P.tiles_n * P.kt;
+        P.images = images_w;
+        P.src = channels_of_x(x, s);
+        P.out = OutAddr{s.CIg, 0, static_cast<long long>(s.COg) * s.CIg, 1, 1};
+        P.vec = s.CIg % 4 == 0 && aligned16(w) && aligned16(gw);
+        P.out_f = gw;
+        P.resident = w;
+        P.accumulate = accumulate_gw;
+        P.col_down = A.down_x; P.row_exp = A.out_exp; P.row_sum = A.out_sum;
+        if ((r = launch_even<PW, false>(P, cap, st)) != kOk) return r;
+    }
+    return kOk;
+}
+
+}  // namespace
+}  // namespace ldn

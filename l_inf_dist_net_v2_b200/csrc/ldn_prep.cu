@@ -17,8 +17,14 @@ inline unsigned blocks_for(long long n) {
     return static_cast<unsigned>(b);
 }
 
-__global__ void canon_x_kernel(const float* x, float* xc, Shape s, int pitch) {
+// Copies that only gated kernels read run when one of those will (gates: either word not 0; null, null: always).
+__device__ __forceinline__ bool copy_wanted(const CopyGate& g) {
+    return (g.a == nullptr && g.b == nullptr) || (g.a && *g.a != 0) || (g.b && *g.b != 0);
+}
+
+__global__ void canon_x_kernel(const float* x, float* xc, Shape s, int pitch, CopyGate gate) {
     stream_order_begin();
+    if (!copy_wanted(gate)) return;
     const long long total = static_cast<long long>(s.G) * s.M * s.CIg;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const CanonIdx q = canon_idx(i, s.CIg, s.M);
@@ -47,8 +53,9 @@ __global__ void canon_bounds_kernel(const float* xl, const float* xu, float* lc,
 // rows (g, m = b HW + hw, :) are contiguous in c; a 32 x 32 tile makes both sides coalesced.  grid = (ceil(HW/32),
 // ceil(CIg/32), B*G).  With `second` non-null the pair (x, second) is treated as interval bounds and sanitised.
 __global__ void canon_transpose_kernel(const float* x, const float* second,
-                                       float* xc, float* sc, Shape s, int pitch) {
+                                       float* xc, float* sc, Shape s, int pitch, CopyGate gate) {
     stream_order_begin();
+    if (!copy_wanted(gate)) return;
     __shared__ float t0[32][33], t1[32][33];
     const int bg = blockIdx.z, b = bg / s.G, g = bg % s.G;
     const int hw0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -77,8 +84,9 @@ __global__ void canon_transpose_kernel(const float* x, const float* second,
     }
 }
 
-__global__ void canon_w_kernel(const float* w, float* wc, Shape s, int pitch) {
+__global__ void canon_w_kernel(const float* w, float* wc, Shape s, int pitch, CopyGate gate) {
     stream_order_begin();
+    if (!copy_wanted(gate)) return;
     const long long total = static_cast<long long>(s.CO) * s.CIg;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const long long row = i / s.CIg;
@@ -458,24 +466,24 @@ static bool transpose_grid(const Shape& s, int channels, dim3* grid) {
     return true;
 }
 
-int launch_canon_x(const float* x, float* xc, const Shape& s, int pitch, cudaStream_t st) {
+int launch_canon_x(const float* x, float* xc, const Shape& s, int pitch, CopyGate gate, cudaStream_t st) {
     dim3 grid;
     if (transpose_grid(s, s.CIg, &grid)) {
-        return launch_after(canon_transpose_kernel, grid, dim3(32, 8), 0, st, x, nullptr, xc, nullptr, s, pitch);
+        return launch_after(canon_transpose_kernel, grid, dim3(32, 8), 0, st, x, nullptr, xc, nullptr, s, pitch, gate);
     }
-    return launch_after(canon_x_kernel, blocks_for((long long)s.G * s.M * s.CIg), kBlock, 0, st, x, xc, s, pitch);
+    return launch_after(canon_x_kernel, blocks_for((long long)s.G * s.M * s.CIg), kBlock, 0, st, x, xc, s, pitch, gate);
 }
 int launch_canon_bounds(const float* xl, const float* xu, float* lc, float* uc, const Shape& s, int pitch,
                         cudaStream_t st) {
     dim3 grid;
     if (transpose_grid(s, s.CIg, &grid)) {
-        return launch_after(canon_transpose_kernel, grid, dim3(32, 8), 0, st, xl, xu, lc, uc, s, pitch);
+        return launch_after(canon_transpose_kernel, grid, dim3(32, 8), 0, st, xl, xu, lc, uc, s, pitch, CopyGate{});
     }
     return launch_after(canon_bounds_kernel, blocks_for((long long)s.G * s.M * s.CIg), kBlock, 0, st, xl, xu, lc, uc,
                         s, pitch);
 }
-int launch_canon_w(const float* w, float* wc, const Shape& s, int pitch, cudaStream_t st) {
-    return launch_after(canon_w_kernel, blocks_for((long long)s.CO * s.CIg), kBlock, 0, st, w, wc, s, pitch);
+int launch_canon_w(const float* w, float* wc, const Shape& s, int pitch, CopyGate gate, cudaStream_t st) {
+    return launch_after(canon_w_kernel, blocks_for((long long)s.CO * s.CIg), kBlock, 0, st, w, wc, s, pitch, gate);
 }
 static bool flat_ok(const Shape& s, int pitch, const void* a, const void* b) {
     return s.HW == 1 && s.G == 1 && s.co_src == s.CO && pitch == s.COg && (s.COg & 3) == 0 &&

@@ -5,12 +5,16 @@
 namespace ldn {
 
 // xc[g][m][pitch] <- x[((b G + g) CIg + c) HW + hw],  m = b HW + hw
-int launch_canon_x(const float* x, float* xc, const Shape& s, int pitch, cudaStream_t st);
+// (only if one of the gate's words is not 0 when the kernel runs; both null: in any case)
+struct CopyGate {
+    const int *a = nullptr, *b = nullptr;
+};
+int launch_canon_x(const float* x, float* xc, const Shape& s, int pitch, CopyGate gate, cudaStream_t st);
 // same for a (lower, upper) pair; elements with lower > upper are replaced by their midpoint
 int launch_canon_bounds(const float* xl, const float* xu, float* lc, float* uc, const Shape& s, int pitch,
                         cudaStream_t st);
 // wc[g][o][pitch] <- w[(g COg + o) CIg + c]
-int launch_canon_w(const float* w, float* wc, const Shape& s, int pitch, cudaStream_t st);
+int launch_canon_w(const float* w, float* wc, const Shape& s, int pitch, CopyGate gate, cudaStream_t st);
 // integer p - 1 = iq:  coef[g][m][pitch] <- go / y^iq   (go, y in output layout).  flag (may be null): set to 1 when
 // some y^-iq is outside the range in which that coefficient times |t|^iq is accurate (cleared by the caller before).
 int launch_coef_int(const float* go, const float* y, float* coef, const Shape& s, int pitch, int iq, int* flag,
