@@ -327,7 +327,7 @@ int norm_dist_backward_part(const float* go, const float* x, const float* w, con
                   (guarded ? 4 : 2) * partial_bytes(cap, 1) + (fused ? pad256(side_floats * sizeof(float)) : 0);
     // even p of large problems: both gradients from matrix products (ldn_even.cu), the kernels here gated behind them
     const size_t even_bytes = even_power(p) && !accumulate_gx && s.co_src == s.CO && even_backward_applies(s, p, gx != nullptr, gw != nullptr, cap)
-                                  ? even_backward_bytes(s, gx != nullptr, gw != nullptr, cap)
+                                  ? even_backward_bytes(s, p, gx != nullptr, gw != nullptr, cap)
                                   : 0;
     bool even = false;
     Call c;

@@ -8,8 +8,8 @@ namespace {
 // 128 images, 256 - 4096 channels, 256 - 5120 outputs; they are within 15 % of most).  The matrix products take a fixed time
 // for preparation and launches and one per stage of 64 reduction elements, the backward pass also one per tile; the direct
 // kernels a time per pair, padding of their 128-wide tiles included.  Measured, direct -> this path, p = 8, forward / both
-// gradients: 512 x 3072 -> 5120 1045 / 2019 -> 298 / 618, 256 x 1024 -> 2048 81 / 161 -> 59 / 123, 256 x 1024 -> 1024 50 / 103
-// -> 52 / 102 (here the line lies), 64 x 784 -> 1024 20 / 71 -> 47 / 97; 32 images of 576 x 1024 -> 128 340 / 878 -> 240 / 401.
+// gradients: 512 x 3072 -> 5120 1045 / 2019 -> 281 / 612, 256 x 1024 -> 2048 81 / 161 -> 59 / 123, 256 x 1024 -> 1024 50 / 103
+// -> 52 / 102 (here the line lies), 64 x 784 -> 1024 20 / 71 -> 47 / 97; 32 images of 576 x 1024 -> 128 340 / 878 -> 219 / 409.
 constexpr double kMargin = 1.1;         // the estimate has to win by this factor
 constexpr int kLeastChannels = 192;     // below, an output's error is a few terms' error: no smaller than the direct sum's
 
@@ -28,9 +28,9 @@ bool in_range(const Shape& s, double stages) {
 
 bool even_forward_applies(const Shape& s, float p, int cap) {
     const int i = static_cast<int>(p) / 2 - 1;
-    constexpr double per_stage[4] = {3.0, 1.6, 1.4, 1.25}, per_pair[4] = {80e-9, 100e-9, 138e-9, 130e-9};
+    constexpr double per_stage[4] = {2.3, 1.35, 1.2, 1.15}, per_pair[4] = {80e-9, 100e-9, 138e-9, 130e-9};
     const ForwardPlan f = plan_forward(s, 2 * i + 1);
-    const double stages = 1.0 * s.G * (f.row_blocks / 2) * f.tiles_n * f.stages;
+    const double stages = static_cast<double>(f.total);
     const double products = 38.0 + prepare_us(s) + per_stage[i] * ceil(stages / (cap / 2));
     const double narrow = i == 3 && s.COg <= 64 ? (s.COg <= 32 ? 32.0 : 64.0) : 128.0;
     const double direct = 12.0 + per_pair[i] * direct_rows(s) * padded(s.COg, narrow) * s.G * s.CIg;
@@ -39,7 +39,7 @@ bool even_forward_applies(const Shape& s, float p, int cap) {
 
 bool even_backward_applies(const Shape& s, float p, bool gx, bool gw, int cap) {
     const int i = static_cast<int>(p) / 2 - 1, ct = channels_of(2 * i + 1);
-    constexpr double per_stage[4] = {2.6, 1.45, 1.0, 1.08}, per_tile = 3.3;
+    constexpr double per_stage[4] = {2.4, 1.3, 0.92, 1.05}, per_tile = 2.7;
     constexpr double both[4] = {139e-9, 195e-9, 223e-9, 248e-9}, one[4] = {85e-9, 134e-9, 162e-9, 190e-9};
     const double columns = div_up(s.CIg, ct), workers = cap / 2 > 0 ? cap / 2 : 1;
     double products = (gx && gw ? 70.0 : 58.0) + prepare_us(s), most = 0.0;
@@ -49,16 +49,19 @@ bool even_backward_applies(const Shape& s, float p, bool gx, bool gw, int cap) {
         products += per_stage[i] * ceil(stages / workers) + per_tile * ceil(tiles / workers);
         most = stages > most ? stages : most;
     }
-    const double pairs = direct_rows(s) * padded(s.CIg, 128.0) * s.CO;
+    // tiles of the direct kernels: rows x channels, over the outputs; for grad_w alone outputs x channels, over the rows
+    const double columns_d = s.G * padded(s.CIg, 128.0), out_rows = s.COg <= 64 ? 64.0 : padded(s.COg, 128.0);
+    const double pairs = columns_d * (gx ? direct_rows(s) * padded(s.COg, 32.0) : out_rows * padded(static_cast<double>(s.M), 32.0));
     const double direct = gx && gw ? 35.0 + both[i] * pairs : 30.0 + one[i] * pairs;
     return cap >= 2 && in_range(s, most) && products * kMargin < direct;
 }
 
 size_t even_forward_bytes(const Shape& s, float p, int cap) {
     const size_t rows = static_cast<size_t>(s.G) * s.M + s.CO;
-    return pad256(plan_forward(s, static_cast<int>(p) - 1).image_bytes) + pad256(rows * sizeof(double)) +
+    const ForwardPlan f = plan_forward(s, static_cast<int>(p) - 1);
+    return pad256(f.image_bytes) + pad256(rows * sizeof(double)) +
            pad256(2 * rows * sizeof(float)) + pad256(kListCap * sizeof(int)) + 256 +
-           pad256(even_partial_floats(cap, kNRows) * sizeof(float));
+           pad256(part_floats(f.M, f.total, f.stages, cap, kNRows) * sizeof(float));
 }
 
 int launch_even_forward(const float* x, const float* w, const Shape& s, float* y, float p, int cap, Bump* bump, int* status,
@@ -71,15 +74,15 @@ int launch_even_forward(const float* x, const float* w, const Shape& s, float* y
     }
 }
 
-size_t even_backward_bytes(const Shape& s, bool gx, bool gw, int cap) {
+size_t even_backward_bytes(const Shape& s, float p, bool gx, bool gw, int cap) {
+    const int ct = channels_of(static_cast<int>(p) - 1);
     const int splits = row_splits(s);
     const size_t rows = static_cast<size_t>(s.G) * s.M;
     return 2 * pad256(rows * 4) + 2 * pad256(4 * static_cast<size_t>(s.CO)) + pad256(8 * static_cast<size_t>(s.G) * (s.CIg + 128)) +
            pad256(4 * (4 * static_cast<size_t>(s.CI) + 8)) + pad256(static_cast<size_t>(splits) * s.CO * sizeof(unsigned)) +
            pad256(static_cast<size_t>(splits) * s.CO * sizeof(double)) +
-           (gx ? pad256(static_cast<size_t>(s.G) * row_blocks(s.M) * kBlocks * stages_of(s.COg) * kABytes) : 0) +
-           (gw ? pad256(static_cast<size_t>(s.G) * row_blocks(s.COg) * kBlocks * stages_of(s.M) * kABytes) : 0) +
-           pad256(even_partial_floats(cap, channels_of(1)) * sizeof(float));
+           (gx ? pad256(plan_gradient(s, false, ct).image_bytes) : 0) + (gw ? pad256(plan_gradient(s, true, ct).image_bytes) : 0) +
+           pad256(gradient_part_floats(s, gx, gw, ct, cap) * sizeof(float));
 }
 
 int launch_even_backward(const float* coef, int pitch, const float* x, const float* w, const float* y, const Shape& s, float* gx, float* gw,

@@ -17,7 +17,7 @@ size_t even_forward_bytes(const Shape& s, float p, int cap);
 int launch_even_forward(const float* x, const float* w, const Shape& s, float* y, float p, int cap, Bump* bump, int* status,
                         const int** dense, cudaStream_t st);
 
-size_t even_backward_bytes(const Shape& s, bool gx, bool gw, int cap);
+size_t even_backward_bytes(const Shape& s, float p, bool gx, bool gw, int cap);
 // Gradients from the coefficients coef[g][m][pitch] = go / y^(p-1); range: the word that the coefficient kernel raises.  *cond:
 // the same for data that the expansion does not suit; neither word set: gx / gw hold the result.  (cond is left alone when
 // range is set.)  gx or gw may be null; gw is added to when accumulate_gw.

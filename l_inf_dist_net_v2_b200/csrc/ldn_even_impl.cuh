@@ -27,8 +27,6 @@
 #include <float.h>
 #include <math.h>
 
-#include <type_traits>
-
 #include "ldn_even.cuh"
 
 namespace ldn {
@@ -49,12 +47,20 @@ constexpr int kBlocks = 2;                             // blocks of 32 reduction
 constexpr int kStageK = kBlocks * kBlockK;
 constexpr int kStages = 3;
 constexpr int kRowsB = kNRows / 2;                     // rows of B in a CTA
-constexpr int kBBytes = kRowsB * 128;
-constexpr int kStageBytes = kBlocks * (kABytes + kBBytes);  // all blocks of A, then all blocks of B
-constexpr int kEvenSmem = kStages * kStageBytes + 1024 + 256;
+// bytes of a block of B in a CTA; of a stage: all blocks of A, then all blocks of B
+__host__ __device__ constexpr int b_bytes(bool fwd, int np);
+__host__ __device__ constexpr int stage_bytes(bool fwd, int np) { return kBlocks * (kABytes + b_bytes(fwd, np)); }
+// backward: the resident operand of a tile (32 kEpiWarps threads, half of the tile's channels each) and the channels' scales
+__host__ __device__ constexpr int resident_bytes(int ct) { return 32 * kEpiWarps * (ct / 2) * 4; }
+__host__ __device__ constexpr int even_smem(bool fwd, int np);
 
 // Channels per tile of the backward form: (p - 1) * channels rows of B, at most kNRows
 __host__ __device__ constexpr int channels_of(int np) { return np >= 5 ? 32 : (np == 3 ? 64 : 128); }
+
+__host__ __device__ constexpr int b_bytes(bool fwd, int np) { return (fwd ? kRowsB : np * channels_of(np) / 2) * 128; }
+__host__ __device__ constexpr int even_smem(bool fwd, int np) {
+    return kStages * stage_bytes(fwd, np) + 1024 + 256 + (fwd ? 0 : resident_bytes(channels_of(np)) + kEpiWarps * (channels_of(np) / 2) * 4);
+}
 
 __host__ __device__ constexpr float binomial(int n, int k) {
     float r = 1.0f;
@@ -80,6 +86,8 @@ struct EvenParams {
     const char* images;             // A: [g][block of rows][block of the reduction ([power], forward)], kABytes each
     Source src;                     // B
     OutAddr out;
+    bool split;                     // at most 128 rows of A: the pair's first CTA has their hi, the second their lo
+    int slots;                      // partial sums that a CTA may have to keep (split: one per tile that its range touches)
     bool swap;                      // forward: the output's row is the tile's column
     bool vec;                       // columns n .. n + 3 (n a multiple of 4) of an output row are one aligned 16-byte piece
     bool accumulate;
@@ -96,7 +104,7 @@ struct EvenParams {
     const int* row_exp;             // [g][row]: coefficients are scaled by 2^exp
     const float* row_sum;           // [g][row]: sum of the scaled coefficients
     const int *gate0, *gate1;       // run only while both words are 0 (may be null)
-    float* partials;                // [cta][2][columns][kMRows]
+    float* partials;                // [cta][slots][columns][kMRows]
     int* status;
 };
 
@@ -203,16 +211,6 @@ __device__ __forceinline__ void split8(const float2 (&v)[4], uint4* hi, uint4* l
     *lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 __device__ __forceinline__ float2 scale2(float2 v, float s) { return __fmul2_rn(v, make_float2(s, s)); }
-template <int E>
-__device__ __forceinline__ float2 power2(float2 v) {
-    if constexpr (E == 1) return v;
-    else if constexpr (E % 2 == 0) {
-        const float2 h = power2<E / 2>(v);
-        return __fmul2_rn(h, h);
-    } else {
-        return __fmul2_rn(power2<E - 1>(v), v);
-    }
-}
 template <int P>
 __device__ __forceinline__ float power(float v) {
     if constexpr (P == 1) return v;
@@ -261,6 +259,14 @@ __device__ __forceinline__ void load1(float* v, const float* p, bool there) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.f32 %0, [%1];\n\t}"
                  : "+f"(*v)
                  : "l"(p), "r"(static_cast<uint32_t>(there)));
+}
+// BYTES of global memory into shared memory, in the background; zeros where there is nothing to load
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const float* src, bool there) {
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(there ? 4 : 0) : "memory");
 }
 __device__ __forceinline__ void load4(float2* v, const float* p, bool there) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
@@ -374,7 +380,7 @@ __device__ __forceinline__ int even_begin(const EvenParams& P, int n, int i) {
 
 // The blocks of A of stage kt of a tile, for CTA `rank` of its pair.
 __device__ __forceinline__ const char* a_blocks(const EvenParams& P, const Span& s, int kt, int rank) {
-    const int row_block = (s.g * P.tiles_m + s.tm) * 2 + rank;
+    const int row_block = (s.g * P.tiles_m + s.tm) * 2 + rank;  // (split: of the same rows, with hi and lo exchanged)
     return P.images + (static_cast<long long>(row_block) * P.kt + kt) * static_cast<long long>(kBlocks * kABytes);
 }
 
@@ -410,13 +416,18 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, in
 // ask for the blocks of A, warp 15 issues the products in the pair's first CTA (its second CTA's passes on that its part of
 // a stage is there).
 //
+// Problems of at most 128 rows of A (128 output channels of a convolution, small batches) are split otherwise: both CTAs take the
+// same rows, the first their hi, the second their lo, so that a product is two passes, A hi and lo times B lo and B hi, instead
+// of three with half of the rows empty; both leave partial sums, which the fold adds.
+//
 // What bounds it: the products, 1344 cycles per stage at 224 columns (alone, on random data: 2.0 PFLOP/s at the clock that
 // the power limit leaves).  Measured in the middle of a tile: 1550 cycles per stage.  Why a pair: the products of one CTA read
 // 1056 x 128 bytes of shared memory per 1344 cycles, beside 256 of copies of A and 448 of stores of B; of a pair, whose CTAs
 // hold half of B each, 720, 256 and 224 (512 x 3072 -> 5120, p = 8, forward / grad_x / grad_w: 488 / 331 / 369 us with single
-// CTAs, 374 / 300 / 370 with pairs).  What made the difference after that (now 248 / 220 / 301): a remote arrival without
+// CTAs, 374 / 300 / 370 with pairs).  What made the difference after that (now 232 / 222 / 286): a remote arrival without
 // cluster-wide release (1150 cycles each), prefetching loads that nothing behind them waits for (950 cycles), loops that stay
-// in the instruction cache.
+// in the instruction cache, forward powers from one another instead of from the value (248 -> 232).  The forward form's
+// converters, 2080 cycles per stage, are what bounds it now; 222 us are 1.5 PFLOP/s.
 template <int PW, bool FWD>
 __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams P) {
     constexpr int NP = PW - 1;
@@ -424,7 +435,11 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
     constexpr int COLS = FWD ? kNRows : NP * CT;    // columns of the accumulator
     constexpr int NC = COLS / 2;                    // of which a warp adds up
     constexpr int CW = CT / 2;                      // !FWD: channels of a half, which one CTA converts
+    constexpr int kBBytes = b_bytes(FWD, NP), kStageBytes = stage_bytes(FWD, NP);
     constexpr int UNITS = CW * kBlocks / 8;         // !FWD: converter units (32 items of 8 reduction elements) per stage
+    // (A barrier's parity tells a phase from its neighbours only: a converter warp's units have to lie less than kStages stages
+    // apart, or it may take the phase before for the one that it waits for.)
+    static_assert(FWD || kConvWarps < kStages * UNITS, "units of a warp too far apart");
     extern __shared__ __align__(16) char raw[];
     char* smem = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
     Bars* B = reinterpret_cast<Bars*>(smem + kStages * kStageBytes);
@@ -459,6 +474,8 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
         const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane;
         const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + half * NC;
         const int first_tile = it0 / P.kt;
+        [[maybe_unused]] char* resident = reinterpret_cast<char*>(B) + 256;  // [piece of 4 channels][thread], 16 bytes each
+        [[maybe_unused]] char* scales = resident + resident_bytes(CT) + warp * CW * 4;
         int buf = 0;
         uint32_t phase = 0;
         bool ok = true;
@@ -467,6 +484,30 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
             float2 acc[NC / 2];
 #pragma unroll
             for (int i = 0; i < NC / 2; ++i) acc[i] = make_float2(0.0f, 0.0f);
+            const int m = (P.split ? s.tm : s.tm * 2 + rank) * kMRows + row;
+            const bool in = m < P.M;
+            [[maybe_unused]] const int n0 = s.tn * CT + half * CW;  // backward: first channel
+            [[maybe_unused]] long long off = 0;
+            [[maybe_unused]] float q0 = 0.0f, row_exp = 0.0f;
+            if constexpr (!FWD) {
+                // what the end of the tile needs, fetched meanwhile (each thread reads back what it copied, a warp its scales)
+                off = even_offset(P, s.g, in ? m : 0, n0);
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < CW; c += 4) {
+                    if (P.vec) {
+                        copy_async<16>(resident + (c / 4 * 32 * kEpiWarps + threadIdx.x) * 16, P.resident + off + c, in && n0 + c < P.N);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            copy_async<4>(resident + (c / 4 * 32 * kEpiWarps + threadIdx.x) * 16 + 4 * i, P.resident + off + (c + i) * P.out.s_n,
+                                          in && n0 + c + i < P.N);
+                    }
+                }
+                if (lane < CW / 4) copy_async<16>(scales + lane * 16, P.col_down + s.g * P.tiles_n * CT + n0 + 4 * lane, true);
+                load1(&row_exp, reinterpret_cast<const float*>(P.row_exp) + s.g * P.M + m, in);
+                load1(&q0, P.row_sum + s.g * P.M + m, s.kt0 == 0 && in && !(P.split && rank == 1));
+            }
             for (int kt = s.kt0; kt < s.kt1; ++kt) {
                 ok = __all_sync(0xffffffffu, wait_or_abort<false>(&B->acc_full[buf], phase, &B->abort, P.status));
                 if (!ok) break;
@@ -481,8 +522,16 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                     if (two) tmem_load_wait(v[1]);
 #pragma unroll
                     for (int i = 0; i < 16; ++i)
-                        if (i < 8 || two)
-                            acc[q / 2 + i] = __fadd2_rn(acc[q / 2 + i], make_float2(v[i / 8][2 * (i % 8)], v[i / 8][2 * (i % 8) + 1]));
+                        if (i < 8 || two) {
+                            const float2 sum = make_float2(v[i / 8][2 * (i % 8)], v[i / 8][2 * (i % 8) + 1]);
+                            if constexpr (FWD) {
+                                acc[q / 2 + i] = __fadd2_rn(acc[q / 2 + i], sum);
+                            } else {  // the power's coefficient (-1)^j C(p - 1, j) in the same instruction
+                                const int j = (q + 2 * i) / CW + 1;
+                                const float k = j % 2 ? -binomial(NP, j) : binomial(NP, j);
+                                acc[q / 2 + i] = __ffma2_rn(sum, make_float2(k, k), acc[q / 2 + i]);
+                            }
+                        }
                 }
                 tmem_fence_before();
                 __syncwarp();
@@ -491,10 +540,9 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                 if (buf == 0) phase ^= 1;
             }
             if (!ok) break;
-            const bool whole = s.kt0 == 0 && s.kt1 == P.kt;
-            const int m = (s.tm * 2 + rank) * kMRows + row;
-            float* part = P.partials + (static_cast<size_t>(blockIdx.x) * 2 + (it / P.kt == first_tile ? 0 : 1)) *
-                                           static_cast<size_t>(FWD ? kNRows : CT) * kMRows + row;
+            const bool whole = s.kt0 == 0 && s.kt1 == P.kt && !P.split;
+            const int slot = P.split ? it / P.kt - first_tile : (it / P.kt == first_tile ? 0 : 1);
+            float* part = P.partials + (static_cast<size_t>(blockIdx.x) * P.slots + slot) * static_cast<size_t>(FWD ? kNRows : CT) * kMRows + row;
             if constexpr (FWD) {
                 if (!whole) {
 #pragma unroll
@@ -502,7 +550,7 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                         part[(half * NC + 2 * i) * kMRows] = acc[i].x;
                         part[(half * NC + 2 * i + 1) * kMRows] = acc[i].y;
                     }
-                } else if (m < P.M) {
+                } else if (in) {
                     // the sums as they are; even_fold_kernel makes values of them (the roots and guards of a tile here would
                     // hold its CTA up for as long as ten stages)
 #pragma unroll
@@ -521,48 +569,33 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                     }
                 }
             } else {
-                // Horner's scheme over the powers, four channels per trip of a rolled loop: a trip takes the first of every power's
-                // columns and moves the others down (as straight-line code, 128 x 32 outputs of a tile took 6500 cycles, most
-                // of them waiting for instructions).  Meanwhile the next tile's products run on, two accumulators long.
-                const bool in = m < P.M;
-                const int n0 = s.tn * CT + half * CW, pitch = P.tiles_n * CT;
-                const float q0 = s.kt0 == 0 && in ? P.row_sum[s.g * P.M + m] * kScaleB : 0.0f;
-                const float row_scale = in ? pow2i(-15 - P.row_exp[s.g * P.M + m]) : 0.0f;
-                const float* down = P.col_down + s.g * pitch + n0;
-                const long long off = even_offset(P, s.g, m, n0);
-                const float* res = P.resident + off;
+                // Horner's scheme over the powers.  The next tile's products run on meanwhile, but only for two accumulators, 2700
+                // cycles, so a tile's end has to be short: the coefficients came with the sums, the resident operand waits in
+                // shared memory.  (512 x 3072 -> 5120, weight gradient, tiles of 8 stages: 7500 cycles and 297 us with a rolled
+                // loop that loaded and multiplied them here, 5400 and 286 now.)
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncwarp();
+                const float row_scale = pow2i(-15 - __float_as_int(row_exp));
+                const float2 start = scale2(make_float2(q0, q0), kScaleB);
                 float* out = P.out_f + off;
-                constexpr int AHEAD = CW < 16 ? CW / 4 : 4;
-                float2 u[AHEAD][2], d[AHEAD][2];
-                auto load_resident = [&](int c, float2* v, float2* w) {
-                    load4(w, down + c, true);
-                    v[0] = v[1] = make_float2(0.0f, 0.0f);
-                    if (P.vec) {
-                        load4(v, res + c, in && n0 + c < P.N);
-                    } else {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            load1(i % 2 ? &v[i / 2].y : &v[i / 2].x, res + (c + i) * P.out.s_n, in && n0 + c + i < P.N);
-                    }
-                };
-#pragma unroll
-                for (int i = 0; i < AHEAD; ++i) load_resident(4 * i, u[i], d[i]);
-#pragma unroll 1
                 for (int c = 0; c < CW; c += 4) {
-                    const float2 x0 = __fmul2_rn(u[0][0], d[0][0]), x1 = __fmul2_rn(u[0][1], d[0][1]);
-                    float2 h0 = make_float2(q0, q0), h1 = h0;
+                    const float4 u = *reinterpret_cast<const float4*>(resident + (c / 4 * 32 * kEpiWarps + threadIdx.x) * 16);
+                    const float4 d = *reinterpret_cast<const float4*>(scales + c * 4);
+                    const float2 x0 = __fmul2_rn(make_float2(u.x, u.y), make_float2(d.x, d.y));
+                    const float2 x1 = __fmul2_rn(make_float2(u.z, u.w), make_float2(d.z, d.w));
+                    float2 h0 = start, h1 = start;
 #pragma unroll
                     for (int j = 0; j < NP; ++j) {
-                        const float k = j % 2 == 0 ? -binomial(NP, j + 1) : binomial(NP, j + 1);
-                        h0 = __ffma2_rn(h0, x0, scale2(acc[j * (CW / 2)], k));
-                        h1 = __ffma2_rn(h1, x1, scale2(acc[j * (CW / 2) + 1], k));
+                        h0 = __ffma2_rn(h0, x0, acc[(j * CW + c) / 2]);
+                        h1 = __ffma2_rn(h1, x1, acc[(j * CW + c) / 2 + 1]);
                     }
                     if (!whole) {
                         float* o = part + (half * CW + c) * kMRows;
                         o[0] = h0.x; o[kMRows] = h0.y; o[2 * kMRows] = h1.x; o[3 * kMRows] = h1.y;
                     } else if (in && n0 + c < P.N) {
-                        h0 = __fmul2_rn(scale2(h0, row_scale), make_float2(up_of<NP>(d[0][0].x), up_of<NP>(d[0][0].y)));
-                        h1 = __fmul2_rn(scale2(h1, row_scale), make_float2(up_of<NP>(d[0][1].x), up_of<NP>(d[0][1].y)));
+                        h0 = __fmul2_rn(scale2(h0, row_scale), make_float2(up_of<NP>(d.x), up_of<NP>(d.y)));
+                        h1 = __fmul2_rn(scale2(h1, row_scale), make_float2(up_of<NP>(d.z), up_of<NP>(d.w)));
                         if (P.vec) {
                             float4* o = reinterpret_cast<float4*>(out + c);
                             const float4 old = P.accumulate ? *o : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -577,18 +610,6 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                                 }
                         }
                     }
-#pragma unroll
-                    for (int i = 0; i + 1 < AHEAD; ++i) {
-                        u[i][0] = u[i + 1][0];
-                        u[i][1] = u[i + 1][1];
-                        d[i][0] = d[i + 1][0];
-                        d[i][1] = d[i + 1][1];
-                    }
-                    if (c + 4 * AHEAD < CW) load_resident(c + 4 * AHEAD, u[AHEAD - 1], d[AHEAD - 1]);
-#pragma unroll
-                    for (int j = 0; j < NP; ++j)
-#pragma unroll
-                        for (int i = 0; i + 2 < CW / 2; ++i) acc[j * (CW / 2) + i] = acc[j * (CW / 2) + i + 2];
                 }
             }
             it += s.kt1 - s.kt0;
@@ -627,19 +648,17 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                         if (lead) {
                             const uint64_t a = first_slot + slot * (kStageBytes >> 4), b = a + (kBlocks * kABytes >> 4);
                             const uint32_t d = tmem + buf * 256;
+                            auto at = [](int k, int step) { return (k / 2) * (step >> 4) + 2 * (k % 2); };
                             // the small products first, while the accumulator is small
 #pragma unroll
                             for (int k = 0; k < 2 * kBlocks; ++k) {
-                                const uint64_t ak = a + (k / 2) * (kABytes >> 4) + 2 * (k % 2);
-                                const uint64_t bk = b + (k / 2) * (kBBytes >> 4) + 2 * (k % 2);
-                                mma_f16(d, ak + 4, bk, desc, k > 0);
-                                if (PW == 2) mma_f16(d, ak + 4, bk + 4, desc, true);
-                                mma_f16(d, ak, bk + 4, desc, true);
+                                const uint64_t ak = a + at(k, kABytes), bk = b + at(k, kBBytes);
+                                mma_f16(d, ak, bk + 4, desc, k > 0);
+                                if (!P.split) mma_f16(d, ak + 4, bk, desc, true);
+                                if (PW == 2 && !P.split) mma_f16(d, ak + 4, bk + 4, desc, true);
                             }
 #pragma unroll
-                            for (int k = 0; k < 2 * kBlocks; ++k)
-                                mma_f16(d, a + (k / 2) * (kABytes >> 4) + 2 * (k % 2),
-                                              b + (k / 2) * (kBBytes >> 4) + 2 * (k % 2), desc, true);
+                            for (int k = 0; k < 2 * kBlocks; ++k) mma_f16(d, a + at(k, kABytes), b + at(k, kBBytes), desc, true);
                             mma_commit(&B->empty[slot]);
                             mma_commit(&B->acc_full[buf]);
                         }
@@ -666,7 +685,7 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
             auto row_of = [&](int i) { return lanes_are_rows ? row0 : row0 + i; };
             const ForwardScale<PW> scales(*P.scale_word);
             const float factor = pow2i(-scales.e);
-            float2 cur[ITEMS][4], nxt[ITEMS][4];
+            float2 base[ITEMS][4], cur[ITEMS][4], nxt[ITEMS][4];  // values, their power of this block, values of the next channels
             uint32_t slot = 0, phase = 1;  // (a fresh barrier counts as having completed the phase before its first)
             bool ok = true;
             for (int it = it0; it < it1 && ok;) {
@@ -679,15 +698,27 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                         fetch8(P.src, source_row(P.src, s.g, n0 + row_of(i)), kb * kBlockK + 8 * (lanes_are_rows ? piece0 + i : piece0), nxt[i]);
                 };
                 // (scaled when they are needed, not when they are asked for: the loads are still under way then)
-                auto scale = [&]() {
+                auto first_power = [&]() {
+                    const float lift = pow2i(scales.b(1));
 #pragma unroll
                     for (int i = 0; i < ITEMS; ++i)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) cur[i][e] = scale2(nxt[i][e], factor);
+                        for (int e = 0; e < 4; ++e) {
+                            base[i][e] = scale2(nxt[i][e], factor);
+                            cur[i][e] = scale2(base[i][e], lift);
+                        }
                 };
-                int kb = s.kt0 * kBlocks / NP, j = s.kt0 * kBlocks - kb * NP;
+                auto next_power = [&](int exponent) {
+                    const float step = pow2i(scales.b(exponent) - scales.b(exponent - 1));
+#pragma unroll
+                    for (int i = 0; i < ITEMS; ++i)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) cur[i][e] = __fmul2_rn(cur[i][e], scale2(base[i][e], step));
+                };
+                int kb = s.kt0 * kBlocks / NP, j = s.kt0 * kBlocks - kb * NP;  // block: channels 32 kb .., exponent j + 1
                 load(kb);
-                scale();
+                first_power();
+                for (int e = 2; e <= j + 1; ++e) next_power(e);
                 if ((kb + 1) * NP < last) load(kb + 1);
                 for (int kt = s.kt0; kt < s.kt1; ++kt) {
                     ok = __all_sync(0xffffffffu, wait_or_abort<false>(&B->empty[slot], phase, &B->abort, P.status));
@@ -700,36 +731,22 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
 #pragma unroll 1
                     for (int bl = 0; bl < kBlocks; ++bl) {
                         char* b = stage + kBlocks * kABytes + bl * kBBytes;
-                        const float lift = pow2i(scales.b(NP - j));
-                        auto put = [&](auto e_tag) {
-                            constexpr int E = decltype(e_tag)::value;
 #pragma unroll
-                            for (int i = 0; i < ITEMS; ++i) {
-                                float2 v[4];
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) v[e] = scale2(power2<E>(cur[i][e]), lift);
-                                uint4 hi, lo;
-                                split8(v, &hi, &lo);
-                                const int row = row_of(i), piece = lanes_are_rows ? piece0 + i : piece0;
-                                const uint32_t at = row * 128 + ((piece ^ (row & 7)) << 4);
-                                *reinterpret_cast<uint4*>(b + at) = hi;
-                                *reinterpret_cast<uint4*>(b + (at ^ 64)) = lo;
-                            }
-                        };
-                        switch (NP - j) {
-                            case 1: put(std::integral_constant<int, 1>()); break;
-                            case 2: if constexpr (NP >= 2) put(std::integral_constant<int, 2>()); break;
-                            case 3: if constexpr (NP >= 3) put(std::integral_constant<int, 3>()); break;
-                            case 4: if constexpr (NP >= 4) put(std::integral_constant<int, 4>()); break;
-                            case 5: if constexpr (NP >= 5) put(std::integral_constant<int, 5>()); break;
-                            case 6: if constexpr (NP >= 6) put(std::integral_constant<int, 6>()); break;
-                            default: if constexpr (NP >= 7) put(std::integral_constant<int, 7>()); break;
+                        for (int i = 0; i < ITEMS; ++i) {
+                            uint4 hi, lo;
+                            split8(cur[i], &hi, &lo);
+                            const int row = row_of(i), piece = lanes_are_rows ? piece0 + i : piece0;
+                            const uint32_t at = row * 128 + ((piece ^ (row & 7)) << 4);
+                            *reinterpret_cast<uint4*>(b + at) = hi;
+                            *reinterpret_cast<uint4*>(b + (at ^ 64)) = lo;
                         }
                         // (behind the last block of all there may be one that only fills the stage: A is 0 there, B finite)
-                        if (++j == NP) {
+                        if (++j < NP) {
+                            next_power(j + 1);
+                        } else {
                             j = 0;
                             ++kb;
-                            if (kb * NP < last) scale();
+                            if (kb * NP < last) first_power();
                             if ((kb + 1) * NP < last) load(kb + 1);
                         }
                     }
@@ -810,10 +827,10 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
     if (warp == 0) tmem_free(tmem);
 }
 
-// Backward: adds up the partial sums of every tile that is shared between pairs.  Such a tile holds the end of some pair's
-// range; the first boundary inside it stands for it.  blockIdx.y: eight columns, blockIdx.z: CTA of the pair.
-// Forward: makes the values, of shared tiles from their partial sums, of the others from the sums in the output array;
-// blockIdx.x: tile.
+// Adds up the partial sums of tiles that are shared between pairs (or by the CTAs of one, split).  blockIdx.y: eight columns,
+// blockIdx.z: CTA of the pair (one block for both where they have the same rows).  Forward and split: a tile per blockIdx.x, and
+// in the forward pass the values are made here, of tiles that one pair had from the sums in the output array.  Backward: a shared
+// tile holds the end of some pair's range; the first boundary inside it stands for it.
 template <int PW, bool FWD>
 __global__ void __launch_bounds__(kMRows) even_fold_kernel(const EvenParams P, const int workers) {
     constexpr int NP = PW - 1;
@@ -823,7 +840,7 @@ __global__ void __launch_bounds__(kMRows) even_fold_kernel(const EvenParams P, c
     if ((P.gate0 && *P.gate0 != 0) || (P.gate1 && *P.gate1 != 0)) return;
     const int rank = blockIdx.z, row = threadIdx.x, col0 = blockIdx.y * 8;
     int c0, t0;
-    if constexpr (FWD) {
+    if (FWD || P.split) {
         t0 = blockIdx.x * P.kt;
         c0 = static_cast<int>((static_cast<long long>(t0 + 1) * workers - 1) / P.total);
     } else {
@@ -832,20 +849,30 @@ __global__ void __launch_bounds__(kMRows) even_fold_kernel(const EvenParams P, c
         t0 = cut / P.kt * P.kt;
         if (cut == t0 || even_begin(P, workers, c0) > t0) return;
     }
-    const bool second = even_begin(P, workers, c0) < t0;  // worker c0 began in an earlier tile
     const int c1 = static_cast<int>((static_cast<long long>(t0 + P.kt) * workers - 1) / P.total);
     const Span s = span_at(P, t0, P.total);
-    const int m = (s.tm * 2 + rank) * kMRows + row, n0 = s.tn * COLS + col0;
+    const int m = (P.split ? s.tm : s.tm * 2 + rank) * kMRows + row, n0 = s.tn * COLS + col0;
     if (m >= P.M || n0 >= P.N) return;
     float v[8];
-    if (!FWD || c0 != c1) {
-        const size_t slot = static_cast<size_t>(COLS) * kMRows;
-        const float* part = P.partials + static_cast<size_t>(c0 * 2 + rank) * 2 * slot + static_cast<size_t>(col0) * kMRows + row;
+    const bool parts = P.split || !FWD || c0 != c1;
+    if (parts) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = part[(second ? slot : 0) + i * kMRows];
+        for (int i = 0; i < 8; ++i) v[i] = 0.0f;
+        // a worker's slot of this tile is its first, unless it began in an earlier one, as only c0 can have
+        int slot = t0 / P.kt - even_begin(P, workers, c0) / P.kt;
+        if (!P.split) slot = min(slot, 1);
+        const size_t size = static_cast<size_t>(COLS) * kMRows, step = P.slots * size;  // of a partial sum, of a CTA's
+        const float* part = P.partials + (P.split ? 2 * c0 : 2 * c0 + rank) * step + static_cast<size_t>(col0) * kMRows + row;
+        auto add = [&](const float* p) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] += p[i * kMRows];
+        };
+        add(part + slot * size);
+        if (P.split) add(part + step + slot * size);
+#pragma unroll 4
         for (int c = c0 + 1; c <= c1; ++c) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] += part[static_cast<size_t>(c - c0) * 4 * slot + i * kMRows];
+            add(part + static_cast<size_t>(c - c0) * 2 * step);
+            if (P.split) add(part + (static_cast<size_t>(c - c0) * 2 + 1) * step);
         }
     }
     if constexpr (FWD) {
@@ -858,7 +885,7 @@ __global__ void __launch_bounds__(kMRows) even_fold_kernel(const EvenParams P, c
             long long off[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) off[i] = i > 0 && P.vec ? off[0] + i : even_offset(P, s.g, m, min(n0 + q + i, P.N - 1));
-            if (c0 == c1) {
+            if (!parts) {
                 if (P.vec) {
                     const float4 r = *reinterpret_cast<const float4*>(P.out_f + off[0]);
                     v[q] = r.x; v[q + 1] = r.y; v[q + 2] = r.z; v[q + 3] = r.w;
@@ -894,12 +921,17 @@ __global__ void __launch_bounds__(kMRows) even_fold_kernel(const EvenParams P, c
 
 // ---- preparation -----------------------------------------------------------------------------------------------------
 // One item of a block of A: eight reduction elements of a row, hi and lo where the swizzle puts them.
-__device__ __forceinline__ void put_item(char* block, int row, int chunk, const float2 (&v)[4]) {
+// twin: not 0 if the block of the pair's second CTA, which takes lo for hi, is that many bytes behind this one.
+__device__ __forceinline__ void put_item(char* block, int row, int chunk, const float2 (&v)[4], long long twin) {
     uint4 hi, lo;
     split8(v, &hi, &lo);
     const uint32_t at = row * 128 + ((chunk ^ (row & 7)) << 4);
     *reinterpret_cast<uint4*>(block + at) = hi;
     *reinterpret_cast<uint4*>(block + (at ^ 64)) = lo;
+    if (twin != 0) {
+        *reinterpret_cast<uint4*>(block + twin + at) = lo;
+        *reinterpret_cast<uint4*>(block + twin + (at ^ 64)) = hi;
+    }
 }
 constexpr int kPrep = 256;
 __device__ __forceinline__ void item_of(const Source& S, int i, int* row, int* chunk) {
@@ -972,7 +1004,7 @@ __global__ void __launch_bounds__(kPrep) even_rows_kernel(const Source a, const 
 // The blocks of A of the forward form, C(p, j) x^j split, j = 1 .. p - 1 (seq blocks per block of rows: zeros behind the last
 // where stages need an even number); the blocks behind those put the row sums on the common scale.
 template <int PW>
-__global__ void __launch_bounds__(kPrep) even_powers_kernel(const Source a, int G, int tiles_m, int kb, int seq, char* images,
+__global__ void __launch_bounds__(kPrep) even_powers_kernel(const Source a, int G, int tiles_m, int kb, int seq, bool split, char* images,
                                                            const double* sums_a, const double* sums_b, int rows_b,
                                                            float* sum_a, float* norm_a, float* sum_b, float* norm_b,
                                                            const unsigned* scale_word, int* dense) {
@@ -998,6 +1030,8 @@ __global__ void __launch_bounds__(kPrep) even_powers_kernel(const Source a, int 
     const ForwardScale<PW> scales(top);
     const float factor = pow2i(-e);
     const int k = block % kb, t = block / kb, tm = t % tiles_m, g = t / tiles_m;
+    const long long first_block = (static_cast<long long>(g) * tiles_m + tm) * (split ? 2 : 1);  // block of rows in the images
+    const long long twin = split ? static_cast<long long>(seq) * kABytes : 0;
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
         int row, chunk;
@@ -1012,15 +1046,14 @@ __global__ void __launch_bounds__(kPrep) even_powers_kernel(const Source a, int 
             const float c = (j % 2 == 0 ? -binomial(PW, j + 1) : binomial(PW, j + 1)) * pow2i(scales.a(j + 1));
 #pragma unroll
             for (int i = 0; i < 4; ++i) term[i] = scale2(cur[i], c);
-            put_item(images + ((static_cast<long long>(g) * tiles_m + tm) * seq + k * NP + j) * static_cast<long long>(kABytes), row,
-                     chunk, term);
+            // (in the order in which B's exponent, p less this one, rises)
+            put_item(images + (first_block * seq + k * NP + NP - 1 - j) * static_cast<long long>(kABytes), row, chunk, term, twin);
 #pragma unroll
             for (int i = 0; i < 4; ++i) cur[i] = __fmul2_rn(cur[i], v[i]);
         }
         if (k == kb - 1 && seq > kb * NP) {
             const float2 zero[4] = {};
-            put_item(images + ((static_cast<long long>(g) * tiles_m + tm) * seq + kb * NP) * static_cast<long long>(kABytes), row, chunk,
-                     zero);
+            put_item(images + (first_block * seq + kb * NP) * static_cast<long long>(kABytes), row, chunk, zero, twin);
         }
     }
 }
@@ -1270,6 +1303,7 @@ struct CoefImages {
     const int* exp;
     char* images;
     int tiles_m, kb, blocks;
+    bool split;
 };
 __global__ void __launch_bounds__(kPrep) even_coef_kernel(const CoefImages X, const CoefImages W, const int* gate0, const int* gate1) {
     stream_order_begin();
@@ -1288,7 +1322,8 @@ __global__ void __launch_bounds__(kPrep) even_coef_kernel(const CoefImages X, co
         const float f = r < J.src.rows ? pow2i(J.exp[g * J.src.rows + r]) : 0.0f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] = scale2(v[i], f);
-        put_item(J.images + static_cast<long long>(block) * kABytes, row, chunk, v);
+        put_item(J.images + (static_cast<long long>(t) * (J.split ? 2 : 1) * J.kb + k) * kABytes, row, chunk, v,
+                 J.split ? static_cast<long long>(J.kb) * kABytes : 0);
     }
 }
 
@@ -1315,9 +1350,22 @@ Source channels_of_x(const float* x, const Shape& s) {
                   static_cast<long long>(s.CI) * s.HW, static_cast<long long>(s.CIg) * s.HW};
 }
 
-// tiles along m rows of A and blocks of kMRows rows in them; stages along k reduction elements
+// Tiles along m rows of A, and blocks of kMRows rows in them that are prepared; stages along k reduction elements.
+// Split tiles take two passes per product instead of three: worth it up to 128 rows, where a pair would be half empty (32 x 64 x
+// 32 x 32 convolution to 128 channels, p = 8, forward and weight gradient: 172 and 133 us with half-empty pairs, 162 and 129
+// split, all else equal: the converters bound the forward form there, 2200 cycles per stage against 896 of products).
+bool split_rows(long long m) { return m <= kMRows; }
 int row_tiles(long long m) { return div_up(m, 2 * kMRows); }
-int row_blocks(long long m) { return 2 * row_tiles(m); }
+int row_blocks(long long m) { return split_rows(m) ? 1 : 2 * row_tiles(m); }
+// partial sums that a CTA may have to keep: of the tiles that its range touches (split), or of its first and last
+int part_slots(long long m, long long total, int kt, int workers) {
+    return split_rows(m) ? static_cast<int>(((total + workers - 1) / workers + kt - 2) / kt) + 1 : 2;
+}
+int workers_of(long long total, int cap) { return static_cast<int>(total < cap / 2 ? total : cap / 2); }
+size_t part_floats(long long m, long long total, int kt, int cap, int cols) {
+    const int workers = workers_of(total, cap);
+    return 2 * static_cast<size_t>(workers) * part_slots(m, total, kt, workers) * cols * kMRows;
+}
 int stages_of(long long k) { return div_up(k, kStageK); }
 
 // Which operand's powers are written out as A: the one for which products on padding plus the bytes of its powers take less
@@ -1326,6 +1374,7 @@ struct ForwardPlan {
     bool swap;  // A = w
     int M, N, row_blocks, tiles_n, stages;
     size_t image_bytes;
+    long long total;
 };
 ForwardPlan plan_forward(const Shape& s, int np) {
     ForwardPlan best{};
@@ -1338,8 +1387,10 @@ ForwardPlan plan_forward(const Shape& s, int np) {
         f.row_blocks = row_blocks(f.M);
         f.tiles_n = div_up(f.N, kNRows);
         f.stages = stages_of(static_cast<long long>(div_up(s.CIg, kBlockK)) * np * kBlockK);
-        f.image_bytes = static_cast<size_t>(s.G) * f.row_blocks * f.stages * kBlocks * kABytes;
-        const double flops = 6.0 * s.G * f.stages * kStageK * (1.0 * f.row_blocks * kMRows) * (1.0 * f.tiles_n * kNRows);
+        f.total = static_cast<long long>(s.G) * row_tiles(f.M) * f.tiles_n * f.stages;
+        f.image_bytes = static_cast<size_t>(s.G) * 2 * row_tiles(f.M) * f.stages * kBlocks * kABytes;
+        // (split: four operations per pair of halves and row of the pair instead of six)
+        const double flops = (split_rows(f.M) ? 4.0 : 6.0) * f.total * kStageK * (2.0 * kMRows) * kNRows;
         const double t = flops / 1.2e15 + 2.0 * f.image_bytes / 4e12;
         if (swap == 0 || t < least) {
             least = t;
@@ -1349,26 +1400,27 @@ ForwardPlan plan_forward(const Shape& s, int np) {
     return best;
 }
 
-size_t even_partial_floats(int cap, int cols) { return static_cast<size_t>(cap) * 2 * cols * kMRows; }
-
 template <int PW, bool FWD>
 int launch_even(const EvenParams& P, int cap, cudaStream_t st) {
     static bool configured[64] = {};
+    constexpr int smem = even_smem(FWD, PW - 1);
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(even_kernel<PW, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kEvenSmem);
+        const cudaError_t e = cudaFuncSetAttribute(even_kernel<PW, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return cuda_status(e);
         configured[dev] = true;
     }
-    const int most = cap / 2, workers = P.total < most ? P.total : most;
+    const int workers = workers_of(P.total, cap);
     timing_before(st);
-    int r = launch_after_in_clusters(even_kernel<PW, FWD>, 2, workers * 2, kEvenThreads, kEvenSmem, st, P);
+    int r = launch_after_in_clusters(even_kernel<PW, FWD>, 2, workers * 2, kEvenThreads, smem, st, P);
     timing_after(st);
     if (r != kOk) return r;
-    if (FWD) return launch_after(even_fold_kernel<PW, FWD>, dim3(P.total / P.kt, kNRows / 8, 2), kMRows, 0, st, P, workers);
+    constexpr unsigned pieces = (FWD ? kNRows : channels_of(PW - 1)) / 8;
+    if (FWD || P.split)
+        return launch_after(even_fold_kernel<PW, FWD>, dim3(P.total / P.kt, pieces, P.split ? 1 : 2), kMRows, 0, st, P, workers);
     if (workers < 2 || (P.total % workers == 0 && (P.total / workers) % P.kt == 0)) return kOk;
-    return launch_after(even_fold_kernel<PW, FWD>, dim3(workers - 1, channels_of(PW - 1) / 8, 2), kMRows, 0, st, P, workers);
+    return launch_after(even_fold_kernel<PW, FWD>, dim3(workers - 1, pieces, 2), kMRows, 0, st, P, workers);
 }
 
 template <int PW>
@@ -1383,7 +1435,7 @@ int forward_power(const float* x, const float* w, const Shape& s, float* y, int 
     float* floats = bump->take<float>(2 * (static_cast<size_t>(rows_a) + rows_b));
     int* list = bump->take<int>(kListCap);
     int* words = bump->take<int>(4);  // largest magnitude, list length, dense
-    float* partials = bump->take<float>(even_partial_floats(cap, kNRows));
+    float* partials = bump->take<float>(part_floats(f.M, f.total, f.stages, cap, kNRows));
     if (!images || !sums || !floats || !list || !words || !partials) return kWorkspace;
     *dense = words + 2;
     const cudaError_t e = cudaMemsetAsync(words, 0, 4 * sizeof(int), st);
@@ -1398,13 +1450,15 @@ int forward_power(const float* x, const float* w, const Shape& s, float* y, int 
     float *sum_a = floats, *norm_a = sum_a + rows_a, *sum_b = norm_a + rows_a, *norm_b = sum_b + rows_b;
     const int kb = div_up(s.CIg, kBlockK);
     const int prep = s.G * f.row_blocks * kb + div_up(static_cast<long long>(rows_a) + rows_b, kPrep);
-    r = launch_after(even_powers_kernel<PW>, prep, kPrep, 0, st, a, s.G, f.row_blocks, kb, f.stages * kBlocks, images, sums,
+    r = launch_after(even_powers_kernel<PW>, prep, kPrep, 0, st, a, s.G, f.row_blocks, kb, f.stages * kBlocks, split_rows(f.M), images, sums,
                      sums + rows_a, b.rows, sum_a, norm_a, sum_b, norm_b, scale, words + 2);
     if (r != kOk) return r;
     EvenParams P{};
     P.M = f.M; P.N = f.N; P.K = s.CIg; P.G = s.G;
     P.tiles_m = row_tiles(f.M); P.tiles_n = f.tiles_n; P.kt = f.stages; P.blocks = kb * NP;
-    P.total = s.G * P.tiles_m * P.tiles_n * P.kt;
+    P.total = static_cast<int>(f.total);
+    P.split = split_rows(f.M);
+    P.slots = part_slots(f.M, f.total, P.kt, workers_of(f.total, cap));
     P.images = images;
     P.src = b;
     P.out = OutAddr{static_cast<long long>(s.CO) * s.HW, 1, static_cast<long long>(s.COg) * s.HW, s.HW, s.HW};
@@ -1421,6 +1475,32 @@ int forward_power(const float* x, const float* w, const Shape& s, float* y, int 
     if ((r = launch_even<PW, true>(P, cap, st)) != kOk) return r;
     return launch_after(even_direct_kernel<PW>, 148, kPrep, 0, st, x, w, s, y, static_cast<const int*>(list),
                         static_cast<const int*>(words + 1), static_cast<const int*>(words + 2));
+}
+
+// one gradient: rows of A (positions for grad_x, output channels for grad_w), reduction length
+struct GradientPlan {
+    int M, K, kt;
+    long long total;
+    size_t image_bytes;
+};
+GradientPlan plan_gradient(const Shape& s, bool weights, int ct) {
+    GradientPlan g;
+    g.M = weights ? s.COg : static_cast<int>(s.M);
+    g.K = weights ? static_cast<int>(s.M) : s.COg;
+    g.kt = stages_of(g.K);
+    g.total = static_cast<long long>(s.G) * row_tiles(g.M) * div_up(s.CIg, ct) * g.kt;
+    g.image_bytes = static_cast<size_t>(s.G) * 2 * row_tiles(g.M) * kBlocks * g.kt * kABytes;
+    return g;
+}
+size_t gradient_part_floats(const Shape& s, bool gx, bool gw, int ct, int cap) {
+    size_t most = 0;
+    for (int k = 0; k < 2; ++k) {
+        if (!(k == 0 ? gx : gw)) continue;
+        const GradientPlan g = plan_gradient(s, k == 1, ct);
+        const size_t n = part_floats(g.M, g.total, g.kt, cap, ct);
+        most = n > most ? n : most;
+    }
+    return most;
 }
 
 // ranges of rows for the coefficients' column sums
@@ -1450,12 +1530,10 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
     unsigned* words = bump->take<unsigned>(4 * static_cast<size_t>(s.CI) + 8);
     A.part_top = bump->take<unsigned>(static_cast<size_t>(splits) * s.CO);
     A.part_sum = bump->take<double>(static_cast<size_t>(splits) * s.CO);
-    // grad_x: rows = positions, reduction = output channels; grad_w the other way round
-    const int kb_x = kBlocks * stages_of(s.COg), kb_w = kBlocks * stages_of(s.M);
-    const size_t blocks_x = static_cast<size_t>(s.G) * row_blocks(s.M) * kb_x, blocks_w = static_cast<size_t>(s.G) * row_blocks(s.COg) * kb_w;
-    char* images_x = gx ? bump->take<char>(blocks_x * kABytes) : nullptr;
-    char* images_w = gw ? bump->take<char>(blocks_w * kABytes) : nullptr;
-    float* partials = bump->take<float>(even_partial_floats(cap, CT));
+    const GradientPlan px = plan_gradient(s, false, CT), pw = plan_gradient(s, true, CT);
+    char* images_x = gx ? bump->take<char>(px.image_bytes) : nullptr;
+    char* images_w = gw ? bump->take<char>(pw.image_bytes) : nullptr;
+    float* partials = bump->take<float>(gradient_part_floats(s, gx != nullptr, gw != nullptr, CT, cap));
     if (!A.row_exp || !A.row_sum || !A.out_exp || !A.out_sum || !A.down_w || !words || !A.part_top ||
         !A.part_sum || (gx && !images_x) || (gw && !images_w) || !partials)
         return kWorkspace;
@@ -1484,11 +1562,18 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
     CoefImages X{}, W{};
     const long long group = static_cast<long long>(s.M) * pitch;
     X.src = Source{coef, s.COg % 4 == 0 ? 0 : 1, static_cast<int>(s.M), s.COg, 0, pitch, 1, 0, group};
-    X.exp = A.row_exp; X.images = images_x; X.tiles_m = row_blocks(s.M); X.kb = kb_x;
-    X.blocks = gx ? static_cast<int>(blocks_x) : 0;
+    auto blocks_of = [&](CoefImages& J, const GradientPlan& g, char* images) {
+        J.images = images;
+        J.split = split_rows(g.M);
+        J.tiles_m = row_blocks(g.M);
+        J.kb = kBlocks * g.kt;
+        J.blocks = images ? s.G * J.tiles_m * J.kb : 0;
+    };
+    blocks_of(X, px, images_x);
+    X.exp = A.row_exp;
     W.src = Source{coef, 2, s.COg, static_cast<int>(s.M), 0, 1, pitch, 0, group};
-    W.exp = A.out_exp; W.images = images_w; W.tiles_m = row_blocks(s.COg); W.kb = kb_w;
-    W.blocks = gw ? static_cast<int>(blocks_w) : 0;
+    blocks_of(W, pw, images_w);
+    W.exp = A.out_exp;
     if ((r = launch_after(even_coef_kernel, X.blocks + W.blocks, kPrep, 0, st, X, W, range, static_cast<const int*>(A.cond))) != kOk) return r;
     EvenParams P{};
     P.G = s.G;
@@ -1498,10 +1583,17 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
     P.gate1 = A.cond;
     P.partials = partials;
     P.status = status;
+    auto rows_of = [&](const GradientPlan& g) {
+        P.M = g.M;
+        P.K = g.K;
+        P.kt = g.kt;
+        P.tiles_m = row_tiles(g.M);
+        P.total = static_cast<int>(g.total);
+        P.split = split_rows(g.M);
+        P.slots = part_slots(g.M, g.total, g.kt, workers_of(g.total, cap));
+    };
     if (gx) {
-        P.M = static_cast<int>(s.M); P.K = s.COg;
-        P.tiles_m = row_tiles(s.M); P.kt = stages_of(s.COg);
-        P.total = s.G * P.tiles_m * P.tiles_n * P.kt;
+        rows_of(px);
         P.images = images_x;
         P.src = channels_of_w(w, s);
         P.out = OutAddr{static_cast<long long>(s.CI) * s.HW, 1, static_cast<long long>(s.CIg) * s.HW, s.HW, s.HW};
@@ -1512,9 +1604,7 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
         if ((r = launch_even<PW, false>(P, cap, st)) != kOk) return r;
     }
     if (gw) {
-        P.M = s.COg; P.K = static_cast<int>(s.M);
-        P.tiles_m = row_tiles(s.COg); P.kt = stages_of(s.M);
-        P.total = s.G * P.tiles_m * P.tiles_n * P.kt;
+        rows_of(pw);
         P.images = images_w;
         P.src = channels_of_x(x, s);
         P.out = OutAddr{s.CIg, 0, static_cast<long long>(s.COg) * s.CIg, 1, 1};
