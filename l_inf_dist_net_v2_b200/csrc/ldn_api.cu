@@ -9,6 +9,7 @@
 #include "ldn_even.cuh"
 #include "ldn_extreme.cuh"
 #include "ldn_launch.cuh"
+#include "ldn_power_lists.cuh"
 #include "ldn_prep.cuh"
 
 namespace ldn {
@@ -677,10 +678,18 @@ LDN_API int ldn_norm_dist_forward(const float* input, const float* weight, int B
                   (bound_norm ? 2 * pad256(norm_floats * sizeof(float)) : 0);
     // even p of large problems: matrix products (ldn_even.cu), the direct kernel gated behind them
     const size_t even_bytes = even_power(p) && even_forward_applies(s, p, cap_for(ctx)) ? even_forward_bytes(s, p, cap_for(ctx)) : 0;
-    bool even = false;
+    // large fully connected layers at general p: from the channels whose terms count (ldn_power_lists.cu), likewise
+    const bool lists = bound_norm && power_lists_apply(s, p);
+    const size_t more = lists ? power_lists_bytes(s) : even_bytes;
+    bool granted = false;
     Call c;
-    if ((r = begin_call(&c, stream, need, even_bytes <= kEvenMaxScratch ? even_bytes : 0, &even)) != kOk) return r;
-    if (even) {
+    if ((r = begin_call(&c, stream, need, more <= kEvenMaxScratch ? more : 0, &granted)) != kOk) return r;
+    PowerLists listed{};
+    if (granted && lists) {
+        r = launch_power_lists(input, weight, s, output, p, c.cap, &c.bump, &listed, c.st);
+        if (r != kOk) return r;
+        c.gate = c.copies.a = listed.dense;
+    } else if (granted) {
         r = launch_even_forward(input, weight, s, output, p, c.cap, &c.bump, c.arena->status, &c.gate, c.st);
         if (r != kOk) return r;
         c.copies.a = c.gate;
@@ -695,19 +704,26 @@ LDN_API int ldn_norm_dist_forward(const float* input, const float* weight, int B
     float* mbuf = c.bump.take<float>(static_cast<size_t>(B) * CO * HW);
     if (!mbuf) return kWorkspace;
     if (bound_norm) {
-        float* xa = c.bump.take<float>(static_cast<size_t>(xrows * xgroups));
-        float* wa = c.bump.take<float>(static_cast<size_t>(s.CO));
-        if (!xa || !wa) return kWorkspace;
+        float* xa = nullptr;
+        float* wa = nullptr;
         // the guard word (a word of the arena's status block): cleared by the first row reduction, raised by the sum
         // kernel, read by the gated kernels behind it -- all in stream order
         int* flag = c.arena->status + 2;
+        if (listed.dense) {
+            const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), c.st);
+            if (e != cudaSuccess) return cuda_status(e);
+        } else {
+            xa = c.bump.take<float>(static_cast<size_t>(xrows * xgroups));
+            wa = c.bump.take<float>(static_cast<size_t>(s.CO));
+            if (!xa || !wa) return kWorkspace;
+        }
         const Operand xop = inplace ? Operand{input, 1, static_cast<long long>(s.CIg) * s.HW} : as_operand(xv);
-        if ((r = launch_row_absmax(xop, xrows, s.CIg, static_cast<int>(xgroups), inplace ? s.HW : 1, xa, flag,
-                                   c.st)) != kOk)
+        if (!listed.dense && (r = launch_row_absmax(xop, xrows, s.CIg, static_cast<int>(xgroups), inplace ? s.HW : 1, xa, flag,
+                                                    c.st)) != kOk)
             return r;
-        if ((r = launch_row_absmax(as_operand(wv), s.COg, s.CIg, s.G, 1, wa, nullptr, c.st)) != kOk) return r;
-        c.norm_rows = xa;
-        c.norm_cols = wa;
+        if (!listed.dense && (r = launch_row_absmax(as_operand(wv), s.COg, s.CIg, s.G, 1, wa, nullptr, c.st)) != kOk) return r;
+        c.norm_rows = listed.dense ? listed.norm_rows : xa;
+        c.norm_cols = listed.dense ? listed.norm_cols : wa;
         c.guard = flag;
         r = run_forward(c, FwdKind::PowNorm, -1, xv, nullptr, wv, s, output, nullptr, nullptr, nullptr, nullptr, p, inplace);
         if (r != kOk) return r;
