@@ -9,6 +9,7 @@
 #include "ldn_even.cuh"
 #include "ldn_extreme.cuh"
 #include "ldn_launch.cuh"
+#include "ldn_positions.cuh"
 #include "ldn_power_lists.cuh"
 #include "ldn_prep.cuh"
 
@@ -504,6 +505,13 @@ int inf_forward(const float* x, const float* w, const Shape& s, float* y, int* p
     c.col_sub = col_sub;
     c.col_add = col_add;
     View xv, wv;
+    if (cap_for(ctx) == ctx->sm_count && inf_positions_apply(s, pos != nullptr, false)) {
+        // (one launch, of the scratch only a copy of the weights; the call still asks for what the tile kernels take, so that a
+        // stream prepared for one is prepared for both)
+        timing_forget();  // (no tile kernel is launched)
+        if ((r = get_w_view(c, w, s, &wv)) != kOk) return r;
+        return launch_inf_positions(x, nullptr, as_operand(wv), s, y, nullptr, pos, col_sub, col_add, c.st);
+    }
     if (inplace) xv = x_kmajor_view(x, s);
     else if ((r = get_x_view(c, x, s, &xv)) != kOk) return r;
     if ((r = get_w_view(c, w, s, &wv)) != kOk) return r;
@@ -540,6 +548,12 @@ int bound_forward(const float* xl, const float* xu, const float* w, const Shape&
     if ((r = begin_call(&c, stream, need, pl ? 0 : extreme_path_bytes(ctx, s, true), &extreme)) != kOk) return r;
     c.col_sub = col_sub;
     c.col_add = col_add;
+    if (!pl && cap_for(ctx) == ctx->sm_count && inf_positions_apply(s, false, true)) {
+        View wv;
+        timing_forget();  // (no tile kernel is launched)
+        if ((r = get_w_view(c, w, s, &wv)) != kOk) return r;
+        return launch_inf_positions(xl, xu, as_operand(wv), s, yl, yu, nullptr, col_sub, col_add, c.st);
+    }
     float* lc = c.bump.take<float>(xfloats);
     float* uc = c.bump.take<float>(xfloats);
     if (!lc || !uc) return kWorkspace;
