@@ -452,6 +452,14 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
     nominal_fp32 = sms * SM_LANES * max_mhz * 1e6 / 1e12
     nominal_mufu = sms * MUFU_LANES * max_mhz * 1e6 / 1e12
 
+    peaks = {}
+    try:
+        peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
+    except Exception:
+        pass
+    hbm_peak = peaks.get("hbm_gbs", 6650.0)
+    gemm_peak = peaks.get("bf16_tflops", 1590.0)  # the 16-bit types of the tensor cores share one rate
+
     outcome = (ctypes.c_int * 2)()
 
     def mark_extreme(row):
@@ -491,7 +499,18 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
             # (a tile kernel is most of its call; anything far below that is not the kernel this row is about)
             if t_tile > 0.2 * t:
                 row["tile_kernel_ms"] = round(t_tile, 4)
-            if fam_ == "inf" and name != "forward":
+            if "tile_kernel_ms" not in row and pp in (2.0, 4.0, 6.0, 8.0):
+                # even p of large problems: sums of powers as matrix products (csrc/ldn_even.cu), three products of 16-bit halves
+                # for each of the p - 1 mixed terms; no tile kernel ran
+                flops = 6 * (pp - 1) * pairs * (2 if name == "backward_fused" else 1)
+                row.update({"bound": "tensor", "gflop": round(flops / 1e9, 1),
+                            "tflop_per_s": round(flops / (t * 1e-3) / 1e12, 1),
+                            "frac_of_measured_gemm": round(flops / (t * 1e-3) / 1e12 / gemm_peak, 3)})
+            elif "tile_kernel_ms" not in row and fam_ == "general" and name == "forward":
+                # from the channels whose terms count (csrc/ldn_power_lists.cu): no tile kernel ran
+                row.update({"bound": "load/store pipe", "note": "gpair_per_s counts every pair; csrc/ldn_power_lists.cu visits "
+                                                                "the few per cent whose terms count"})
+            elif fam_ == "inf" and name != "forward":
                 # scatter kernels: HBM-bound.  bytes: g + pos reads, zero-fill of the gradient, one 8-byte
                 # read-modify-write per scattered element
                 nb = 8 * B * CO + 4 * (B * CI if name == "grad_input" else CO * CI) + 8 * B * CO
@@ -532,13 +551,17 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
     in_step = [r for r in rows if r["kernel"] in (("forward", "grad_input", "grad_weight") if fam == "inf"
                                                  else ("forward", "backward_fused"))]
     dominant = max(in_step, key=lambda r: r["ms"])
-    peaks = {}
-    try:
-        peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
-    except Exception:
-        pass
-    hbm_peak = peaks.get("hbm_gbs", 6650.0)
-    if dominant["bound"] == "fp32":
+    if dominant["bound"] == "tensor":
+        line["roofline"] = {
+            "bound": "tensor", "kernel": f"{dominant['kernel']} (p={args.p})", "achieved": dominant["tflop_per_s"],
+            "peak": gemm_peak, "unit": "TFLOP/s", "frac": dominant["frac_of_measured_gemm"], "gflop": dominant["gflop"],
+            "note": "products of 16-bit halves that the sums of powers take, over the whole call (preparation of the operands and "
+                    "the folds included), against the measured bf16 matrix product",
+            "peak_source": "MEASURED_PEAKS.json" if peaks else "fallback 1590 TFLOP/s", "ms": dominant["ms"],
+            "fp32_lane_bound_ms": round((SLOTS["8"][0] if dominant["kernel"] == "forward" else SLOTS_FUSED) * pairs
+                                        / (ffma_peak * 1e12) * 1e3, 3),
+            "traffic": None}
+    elif dominant["bound"] == "fp32":
         line["roofline"] = {
             "bound": "fp32", "kernel": f"{dominant['kernel']} (p={args.p})",
             "achieved": dominant.get("tile_kernel_tlaneop_per_s", dominant["tlaneop_per_s"]),
@@ -584,7 +607,12 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
                           "ffma_probe_tlaneop_per_s": round(ffma_peak, 2),
                           "note": "the FFMA probe ran after this block at whatever clock the GPU then held; "
                                   "frac_of_nominal_at_sampled_clock uses the median SM clock sampled during this block"})
-        if any(r["bound"] == "load/store pipe" for r in in_step):  # (the step visits a few per cent of the pairs)
+        if all(r["bound"] == "tensor" for r in in_step):
+            gflop = sum(r["gflop"] for r in in_step)
+            rate = gflop / sustained["ms_per_step"]
+            sustained.update({"gflop_per_step": round(gflop, 1), "tflop_per_s": round(rate, 1),
+                              "frac_of_measured_sustained_gemm": round(rate / peaks.get("bf16_tflops_sustained", 1400.0), 3)})
+        if any(r["bound"] != "fp32" for r in in_step):  # (the step is no lane-instruction per pair)
             for key in ("slots_per_pair_per_step", "step_tlaneop_per_s", "frac_of_nominal_at_max_clock",
                         "frac_of_nominal_at_sampled_clock"):
                 sustained.pop(key, None)
