@@ -148,6 +148,21 @@ LDN_API int ldn_fold(const float* cols, int B, int C, int H, int W, int kh, int 
                      ldn_stream_t stream);
 
 /*
+ * Margins of a classifier's last distance layer while it trains, and the hinge loss on them (ell_inf_models.py:30-45,
+ * main.py:304-318).  dist, logits, margin and their gradients are [B][classes], at most 2^24 elements:
+ *   logits = -dist;  margin[b][j] = ((dist[b][t] + eps) - (dist[b][j] - eps)) * inv, 0 for the target t = targets[b];
+ *   loss = (1 - mix) mean_b max_j max(margin, 0) + mix mean_bj max(margin, 0);  first[b]: where row b's maximum stands first.
+ * dist_target[b] = dist[b][targets[b]].  The gradient of either output may be NULL (zero).  Status 1 for other sizes.
+ */
+LDN_API int ldn_margins(const float* dist, const float* dist_target, const long long* targets, int B, int classes, float eps,
+                        float inv, float* logits, float* margin, ldn_stream_t stream);
+LDN_API int ldn_margins_backward(const float* grad_logits, const float* grad_margin, const long long* targets, int B, int classes,
+                                 float inv, float* grad, ldn_stream_t stream);
+LDN_API int ldn_hinge(const float* margin, int B, int classes, double mix, float* loss, int* first, ldn_stream_t stream);
+LDN_API int ldn_hinge_backward(const float* grad_loss, const float* margin, const int* first, int B, int classes, double mix,
+                               float* grad, ldn_stream_t stream);
+
+/*
  * Pipe-throughput probe for roofline denominators (no counterpart in the reference).  kind 0 runs a loop
  * of independent FFMA chains, kind 2 the same chains issued as packed fma.rn.f32x2, kind 1 a loop of
  * independent ex2(lg2(x)) chains, kind 3 eight such MUFU chains beside eight packed-FMA chains (16 FMAs per step;

@@ -39,6 +39,10 @@ SIGNATURES = {
     "ldn_mean_shift_planes": [_c_float_p, _i, _i, _i, _c_float_p, _f, _c_float_p, _s],
     "ldn_unfold": [_c_float_p] + [_i] * 9 + [_c_float_p, _s],
     "ldn_fold": [_c_float_p] + [_i] * 9 + [_c_float_p, _s],
+    "ldn_margins": [_c_float_p, _c_float_p, ctypes.c_void_p, _i, _i, _f, _f, _c_float_p, _c_float_p, _s],
+    "ldn_margins_backward": [_c_float_p, _c_float_p, ctypes.c_void_p, _i, _i, _f, _c_float_p, _s],
+    "ldn_hinge": [_c_float_p, _i, _i, ctypes.c_double, _c_float_p, _c_int_p, _s],
+    "ldn_hinge_backward": [_c_float_p, _c_float_p, _c_int_p, _i, _i, ctypes.c_double, _c_float_p, _s],
     "ldn_adam_update": [_i, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                         _f, _f, _f, _f, _i, _f, _s],
     "ldn_adam_update_device_step": [_i, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,

@@ -341,6 +341,97 @@ struct UnfoldFn : public torch::autograd::Function<UnfoldFn> {
     }
 };
 
+// Margins behind the last layer (models.py) and the hinge loss (losses.py).  Both replace torch operators that can be
+// differentiated in any way; where a gradient is itself to be differentiated or is not plain memory, their backward steps are
+// those operators.
+const long long* lptr(const Tensor& t) { return reinterpret_cast<const long long*>(t.data_ptr<int64_t>()); }
+
+struct MarginsFn : public torch::autograd::Function<MarginsFn> {
+    static variable_list forward(AutogradContext* ctx, Tensor dist, Tensor targets, double eps) {
+        ctx->set_materialize_grads(false);
+        ctx->saved_data["eps"] = eps;
+        ctx->save_for_backward({targets});
+        Tensor of_target = at::gather(dist, 1, targets.view({-1, 1}));  // (it checks the targets)
+        Tensor logits = at::empty_like(dist), margin = at::empty_like(dist);
+        const c10::cuda::CUDAGuard guard(dist.device());
+        check(ldn_margins(fptr(dist, "dist"), fptr(of_target, "dist"), lptr(targets), dist.size(0), dist.size(1),
+                          static_cast<float>(eps), 1.0f / static_cast<float>(2 * eps), fptr_mut(logits, "logits"),
+                          fptr_mut(margin, "margin"), stream()),
+              "margins");
+        return {logits, margin};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        if (!grads[0].defined() && !grads[1].defined()) return {Tensor(), Tensor(), Tensor()};
+        const double eps = ctx->saved_data["eps"].toDouble();
+        const Tensor targets = ctx->get_saved_variables()[0];
+        const Tensor gl = grads[0].defined() ? grads[0].contiguous() : Tensor();
+        const Tensor gm = grads[1].defined() ? grads[1].contiguous() : Tensor();
+        if ((gl.defined() && !plain_gradient(gl, 2)) || (gm.defined() && !plain_gradient(gm, 2))) {
+            Tensor g;
+            if (gm.defined()) {
+                const Tensor col = targets.view({-1, 1}), m = (gm / (2 * eps)).scatter(1, col, 0);
+                g = (-m).scatter_add(1, col, m.sum(1, true));
+            }
+            if (gl.defined()) g = g.defined() ? g - gl : -gl;
+            return {g, Tensor(), Tensor()};
+        }
+        Tensor g = at::empty_like(gl.defined() ? gl : gm);
+        const c10::cuda::CUDAGuard guard(g.device());
+        check(ldn_margins_backward(gl.defined() ? fptr(gl, "grad") : nullptr, gm.defined() ? fptr(gm, "grad") : nullptr,
+                                   lptr(targets), g.size(0), g.size(1), 1.0f / static_cast<float>(2 * eps), fptr_mut(g, "grad"),
+                                   stream()),
+              "margins_backward");
+        return {g, Tensor(), Tensor()};
+    }
+};
+
+struct HingeFn : public torch::autograd::Function<HingeFn> {
+    static Tensor forward(AutogradContext* ctx, Tensor margin, double mix) {
+        ctx->saved_data["mix"] = mix;
+        Tensor loss = at::empty({}, margin.options()), first = at::empty({margin.size(0)}, margin.options().dtype(at::kInt));
+        const c10::cuda::CUDAGuard guard(margin.device());
+        check(ldn_hinge(fptr(margin, "margin"), margin.size(0), margin.size(1), mix, fptr_mut(loss, "loss"), iptr(first, "first"),
+                        stream()),
+              "hinge");
+        ctx->save_for_backward({margin, first});
+        return loss;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const double mix = ctx->saved_data["mix"].toDouble();
+        variable_list saved = ctx->get_saved_variables();
+        const Tensor &margin = saved[0], &g = grads[0];
+        if (!plain_gradient(g, 0)) {
+            const Tensor part = at::full_like(margin, mix / margin.numel())
+                                    .scatter_add(1, saved[1].to(at::kLong).view({-1, 1}),
+                                                 at::full({margin.size(0), 1}, (1 - mix) / margin.size(0), margin.options()));
+            return {at::where(margin.detach() >= 0, g * part, at::zeros({}, margin.options())), Tensor()};
+        }
+        Tensor grad = at::empty_like(margin);
+        const c10::cuda::CUDAGuard guard(margin.device());
+        check(ldn_hinge_backward(fptr(g, "grad"), fptr(margin, "margin"), iptr(saved[1], "first"), margin.size(0), margin.size(1),
+                                 mix, fptr_mut(grad, "grad"), stream()),
+              "hinge_backward");
+        return {grad, Tensor()};
+    }
+};
+
+constexpr int64_t kMostLogits = 1 << 20;  // (beyond, the operators are as fast, and one block is not enough for the loss)
+
+c10::optional<std::tuple<Tensor, Tensor>> margins(const Tensor& dist, const Tensor& targets, double eps) {
+    if (!plain(dist, 2) || dist.numel() > kMostLogits || !targets.is_cuda() || targets.scalar_type() != at::kLong ||
+        targets.layout() != at::kStrided || targets.dim() != 1 || !targets.is_contiguous() || targets.size(0) != dist.size(0) ||
+        targets.device() != dist.device() || !targets.has_storage() || targets.unsafeGetTensorImpl()->is_python_dispatch() ||
+        !(eps > 0) || !std::isnormal(static_cast<float>(2 * eps)) || observed())
+        return c10::nullopt;
+    variable_list out = MarginsFn::apply(dist, targets, eps);
+    return std::make_tuple(out[0], out[1]);
+}
+
+c10::optional<Tensor> hinge(const Tensor& margin, double mix) {
+    if (!plain(margin, 2) || margin.numel() > kMostLogits || !std::isfinite(mix) || observed()) return c10::nullopt;
+    return HingeFn::apply(margin, mix);
+}
+
 c10::optional<Tensor> norm_dist(const Tensor& x, const Tensor& w, double p, int64_t G) {
     if (!fits(x, w, G) || !(p > 0.0) || observed()) return c10::nullopt;
     const bool need_grad = at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad());
@@ -413,6 +504,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("bound_inf_dist", &bound_inf_dist);
     m.def("mean_shift", &mean_shift);
     m.def("unfold_columns", &unfold_columns);
+    m.def("margins", &margins);
+    m.def("hinge", &hinge);
     m.def("inf_dist_forward_nograd_shifted", &inf_dist_forward_nograd_shifted);
     m.def("bound_inf_dist_forward_nograd_shifted", &bound_inf_dist_forward_nograd_shifted);
     m.def("check_status", &check_status);
