@@ -499,10 +499,12 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
             # (a tile kernel is most of its call; anything far below that is not the kernel this row is about)
             if t_tile > 0.2 * t:
                 row["tile_kernel_ms"] = round(t_tile, 4)
-            if "tile_kernel_ms" not in row and pp in (2.0, 4.0, 6.0, 8.0):
-                # even p of large problems: sums of powers as matrix products (csrc/ldn_even.cu), three products of 16-bit halves
-                # for each of the p - 1 mixed terms; no tile kernel ran
+            if pp in (2.0, 4.0, 6.0, 8.0) and slots * pairs / (t * 1e-3) / 1e12 > ffma_peak:
+                # beyond what the FP32 pipe can do.  Even p of large problems: sums of powers as matrix products
+                # (csrc/ldn_even.cu), three products of 16-bit halves for each of the p - 1 mixed terms
                 flops = 6 * (pp - 1) * pairs * (2 if name == "backward_fused" else 1)
+                if "tile_kernel_ms" in row:  # (of two gradients: the second's products)
+                    row["products_kernel_ms"] = row.pop("tile_kernel_ms")
                 row.update({"bound": "tensor", "gflop": round(flops / 1e9, 1),
                             "tflop_per_s": round(flops / (t * 1e-3) / 1e12, 1),
                             "frac_of_measured_gemm": round(flops / (t * 1e-3) / 1e12 / gemm_peak, 3)})
