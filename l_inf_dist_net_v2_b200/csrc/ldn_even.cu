@@ -78,9 +78,13 @@ size_t even_backward_bytes(const Shape& s, float p, bool gx, bool gw, int cap) {
     const int ct = channels_of(static_cast<int>(p) - 1);
     const int splits = row_splits(s);
     const size_t rows = static_cast<size_t>(s.G) * s.M;
-    return 2 * pad256(rows * 4) + 2 * pad256(4 * static_cast<size_t>(s.CO)) + pad256(8 * static_cast<size_t>(s.G) * (s.CIg + 128)) +
-           pad256(4 * (4 * static_cast<size_t>(s.CI) + 8)) + pad256(static_cast<size_t>(splits) * s.CO * sizeof(unsigned)) +
-           pad256(static_cast<size_t>(splits) * s.CO * sizeof(double)) +
+    int x_ranges, w_ranges, in_each;
+    channel_ranges(s.B, s.HW == 1, &x_ranges, &in_each);
+    channel_ranges(s.COg, true, &w_ranges, &in_each);
+    return 2 * pad256(rows * 4) + 2 * pad256(4 * static_cast<size_t>(s.CO)) + pad256(4 * 4 * static_cast<size_t>(s.G) * (s.CIg + 128)) +
+           pad256(channel_words(s) * sizeof(unsigned)) + 2 * pad256(static_cast<size_t>(splits) * s.CO * 4) +
+           pad256(static_cast<size_t>(splits) * s.CO * sizeof(double)) + pad256(x_ranges * static_cast<size_t>(s.CI) * sizeof(double2)) +
+           pad256(w_ranges * static_cast<size_t>(s.CI) * sizeof(double2)) + pad256(s.G * static_cast<size_t>(div_up(s.CIg, 32)) * sizeof(double)) +
            (gx ? pad256(plan_gradient(s, false, ct).image_bytes) : 0) + (gw ? pad256(plan_gradient(s, true, ct).image_bytes) : 0) +
            pad256(gradient_part_floats(s, gx, gw, ct, cap) * sizeof(float));
 }

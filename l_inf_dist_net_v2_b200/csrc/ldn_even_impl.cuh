@@ -2,13 +2,19 @@
 //
 // For even p the distance is a polynomial:
 //   y^p            = sum_c x^p + sum_c w^p + sum_{j=1}^{p-1} (-1)^j C(p, j) sum_c x^j w^(p-j)
-//   grad_x[b, c]   = sum_j (-1)^j C(p-1, j) x^(p-1-j) sum_o A[b, o] w[o, c]^j,      A = go / y^(p-1)
-//   grad_w[o, c]   = sum_j (-1)^j C(p-1, j) w^(p-1-j) sum_b A[b, o] x[b, c]^j
-// i.e. p - 1 matrix products each.  Every factor is split into two 11-bit halves, v = hi + lo in fp16 (lo holds what hi
+//   grad_x[b, c]   = sum_j (-1)^j C(p-1, j) d^(p-1-j) sum_o A[b, o] u[o, c]^j,      A = go / y^(p-1)
+//   grad_w[o, c]   = sum_j (-1)^j C(p-1, j) d^(p-1-j) sum_b A[b, o] u[b, c]^j
+// with u = w - m, d = x - m for grad_x and u = x - m, d = w - m for grad_w, m[c] the mean of the channel in the operand that
+// is summed over.  That is p - 1 matrix products each.  Every factor is split into two 11-bit halves, v = hi + lo in fp16 (lo holds what hi
 // rounds off, so the pair keeps 22 - 23 bits), and a product is hi hi + hi lo + lo hi with fp32 accumulators (and lo lo for
 // p = 2): 3 x 7 multiply-adds per pair on the tensor cores for p = 8, against 4 (forward) and 8 (backward) FP32 instructions of
-// the direct kernels.  The terms do not cancel where it matters: large |x - w| come from x and w of opposite sign, for which all
-// terms of the expansion have one sign (the guards below look at every output, and at every channel).
+// the direct kernels.  In the forward pass the terms do not cancel where it matters: large |x - w| come from x and w of opposite
+// sign, for which all terms of the expansion have one sign (a guard looks at every output).  In the backward pass the errors go
+// with E = sum |A| (|d| + |u|)^(p-1) and the direct kernels' with D = sum |A| |d - u|^(p-1).  Around the mean the two are close
+// whatever the channel holds: |m - x| <= ||d - u|| in the (p-1)-norm over the rows, so ||d| + |u|| <= 3 ||d - u|| at worst, and
+// E is about 2 D for channels of any offset or spread, a few of the rows far from the others, or values that hardly differ.
+// (Around zero, p = 8: entries of grad_w at pixels 0.5 +- 0.02 were wrong by 1.3e-2 at the 90th percentile, channels of offset
+// 1.5 by 4e-3 in 2-norm.)  What may still go wrong is that the coefficients prefer rows near x: the guards below.
 //
 // What is kept as precise as in the direct kernels, and how:
 //   * the tensor core's accumulator drops the bits below the largest summand instead of rounding, so it takes one stage
@@ -21,8 +27,17 @@
 //   * forward: an output for which the terms could cancel, y^p < 2^-6 (|x|_p + |w|_p)^p, or that is small on the common
 //     scale, y^p < 2^-10 M^p with the largest magnitude M, goes to a list and is summed directly; too many of them, or a value that is not finite, and the
 //     direct kernels behind this path run instead;
-//   * backward: an output below a third of the largest |x| + |w| (its coefficient, y^-(p-1), would blow the expansion's errors
-//     up), or a channel whose values all lie close together far from zero, makes the direct kernels run.
+//   * backward: the direct kernels run if the coefficients of a row (of x, or of w) sit on few of its terms, sum |A| < 4 max |A|;
+//     if they prefer small differences in all channels at once, as within clusters: an output below kLeastOfSpread (by p) of
+//     (sum_c s^p)^(1/p), s[c] the root mean square of x - w over all pairs; if an output is below a third of the largest |d| + |u|
+//     of a channel (rows of different scales: powers of the small ones would leave fp16's range); or if a channel's u are
+//     below 2^-12 of its d without being 0.
+//     Errors against 64 bits in a restatement of this arithmetic, 256 x 1024 -> 1200, p = 8, expansion / direct kernels, 2-norm
+//     (99th percentile of the entries' relative errors): grad_w of images 1.7e-7 / 3.7e-7 (4.9e-6 / 1.7e-5), of pixels 0.5 +-
+//     0.02 2.1e-7 / 4.2e-7 (1.7e-6 / 2.0e-5); grad_x 1.9e-7 / 5.8e-7 (8.3e-6 / 1.9e-5).  Two clusters of Gaussian rows, as far apart as
+//     they are wide, 1.03 (sum_c s^p)^(1/p), pass: 3.1e-7 / 3.6e-7 and 5.1e-7 / 5.5e-7; at half that width, 0.59, it would be 3.0e-6 /
+//     3.4e-7.  Rows whose channels are independent of one another lie at 1.24 and above (192 - 1024 channels, uniform, normal,
+//     of zeros and ones).
 #pragma once
 #include <float.h>
 #include <math.h>
@@ -41,6 +56,12 @@ constexpr int kEvenThreads = 32 * (kEpiWarps + kConvWarps + 1);
 constexpr float kScaleB = 32768.0f;         // backward: powers of values below 1 as fp16 holds them best
 constexpr float kTruncation = 1.0f + 1.0f / (1 << 22);
 constexpr int kListCap = 1 << 16;
+// guards of the backward form
+constexpr float kLeastSpread = 4.0f;       // sum of |A| over its largest, per row
+__device__ __forceinline__ double least_of_spread(int p) { return p == 8 ? 0.95 : (p == 6 ? 0.85 : (p == 4 ? 0.5 : 0.25)); }
+constexpr float kMostOfOutput = 3.0f;      // largest |d| + |u| of a channel over y
+constexpr float kLeastChannel = 1.0f / 4096;   // largest |u| over largest |d|
+constexpr float kChannelFloor = 1.0f / 512;    // scales: d stays below 512, d^7 times the sums below 2^127
 
 // A tile is the work of a pair of CTAs: 256 rows of A, kNRows of B, half of either in each CTA.
 constexpr int kBlocks = 2;                             // blocks of 32 reduction elements per stage
@@ -50,7 +71,7 @@ constexpr int kRowsB = kNRows / 2;                     // rows of B in a CTA
 // bytes of a block of B in a CTA; of a stage: all blocks of A, then all blocks of B
 __host__ __device__ constexpr int b_bytes(bool fwd, int np);
 __host__ __device__ constexpr int stage_bytes(bool fwd, int np) { return kBlocks * (kABytes + b_bytes(fwd, np)); }
-// backward: the resident operand of a tile (32 kEpiWarps threads, half of the tile's channels each) and the channels' scales
+// backward: the resident operand of a tile (32 kEpiWarps threads, half of the tile's channels each), the channels' scales and shifts
 __host__ __device__ constexpr int resident_bytes(int ct) { return 32 * kEpiWarps * (ct / 2) * 4; }
 __host__ __device__ constexpr int even_smem(bool fwd, int np);
 
@@ -59,7 +80,7 @@ __host__ __device__ constexpr int channels_of(int np) { return np >= 5 ? 32 : (n
 
 __host__ __device__ constexpr int b_bytes(bool fwd, int np) { return (fwd ? kRowsB : np * channels_of(np) / 2) * 128; }
 __host__ __device__ constexpr int even_smem(bool fwd, int np) {
-    return kStages * stage_bytes(fwd, np) + 1024 + 256 + (fwd ? 0 : resident_bytes(channels_of(np)) + kEpiWarps * (channels_of(np) / 2) * 4);
+    return kStages * stage_bytes(fwd, np) + 1024 + 256 + (fwd ? 0 : resident_bytes(channels_of(np)) + kEpiWarps * (channels_of(np) / 2) * 8);
 }
 
 __host__ __device__ constexpr float binomial(int n, int k) {
@@ -100,7 +121,7 @@ struct EvenParams {
     int* dense;
     // backward
     const float* resident;          // the operand with the output's layout
-    const float* col_down;          // [g][channel, padded to whole tiles]: v = value * 2^-e
+    const float *col_down, *col_shift; // [g][channel, padded to whole tiles]: v = (value - m) 2^-e = value * down + shift
     const int* row_exp;             // [g][row]: coefficients are scaled by 2^exp
     const float* row_sum;           // [g][row]: sum of the scaled coefficients
     const int *gate0, *gate1;       // run only while both words are 0 (may be null)
@@ -475,7 +496,7 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
         const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + half * NC;
         const int first_tile = it0 / P.kt;
         [[maybe_unused]] char* resident = reinterpret_cast<char*>(B) + 256;  // [piece of 4 channels][thread], 16 bytes each
-        [[maybe_unused]] char* scales = resident + resident_bytes(CT) + warp * CW * 4;
+        [[maybe_unused]] char* scales = resident + resident_bytes(CT) + warp * CW * 8;  // 2^-e, then shifts
         int buf = 0;
         uint32_t phase = 0;
         bool ok = true;
@@ -504,7 +525,10 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                                           in && n0 + c + i < P.N);
                     }
                 }
-                if (lane < CW / 4) copy_async<16>(scales + lane * 16, P.col_down + s.g * P.tiles_n * CT + n0 + 4 * lane, true);
+                if (lane < CW / 2) {
+                    const int q = lane % (CW / 4);
+                    copy_async<16>(scales + lane * 16, (lane < CW / 4 ? P.col_down : P.col_shift) + s.g * P.tiles_n * CT + n0 + 4 * q, true);
+                }
                 load1(&row_exp, reinterpret_cast<const float*>(P.row_exp) + s.g * P.M + m, in);
                 load1(&q0, P.row_sum + s.g * P.M + m, s.kt0 == 0 && in && !(P.split && rank == 1));
             }
@@ -582,8 +606,9 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                 for (int c = 0; c < CW; c += 4) {
                     const float4 u = *reinterpret_cast<const float4*>(resident + (c / 4 * 32 * kEpiWarps + threadIdx.x) * 16);
                     const float4 d = *reinterpret_cast<const float4*>(scales + c * 4);
-                    const float2 x0 = __fmul2_rn(make_float2(u.x, u.y), make_float2(d.x, d.y));
-                    const float2 x1 = __fmul2_rn(make_float2(u.z, u.w), make_float2(d.z, d.w));
+                    const float4 t = *reinterpret_cast<const float4*>(scales + (CW + c) * 4);
+                    const float2 x0 = __ffma2_rn(make_float2(u.x, u.y), make_float2(d.x, d.y), make_float2(t.x, t.y));
+                    const float2 x1 = __ffma2_rn(make_float2(u.z, u.w), make_float2(d.z, d.w), make_float2(t.z, t.w));
                     float2 h0 = start, h1 = start;
 #pragma unroll
                     for (int j = 0; j < NP; ++j) {
@@ -768,7 +793,8 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
             Span s{};
             int span_first = 0, span_end = 0;  // the stages of the range that s describes
             float2 nxt[4];
-            float nxt_down = 0.0f;
+            float nxt_down = 0.0f, nxt_shift = 0.0f;
+            int nxt_left = 0;  // elements of the item that there are
             const char* nxt_a = nullptr;
             auto fetch = [&](int u) {
                 const int n = u / UNITS, item = (u % UNITS) * 32 + lane, cl = item % CW, chunk = item / CW;
@@ -779,7 +805,9 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                 }
                 const int c = s.tn * CT + rank * CW + cl, kt = s.kt0 + n - span_first;
                 fetch8(P.src, source_row(P.src, s.g, c), kt * kStageK + 8 * chunk, nxt);
+                nxt_left = P.src.k - kt * kStageK - 8 * chunk;
                 load1(&nxt_down, P.col_down + s.g * P.tiles_n * CT + c, true);
+                load1(&nxt_shift, P.col_shift + s.g * P.tiles_n * CT + c, true);
                 if (u % UNITS == 0) nxt_a = a_blocks(P, s, kt, rank);
             };
             if (cw < units) fetch(cw);
@@ -793,7 +821,14 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
                 }
                 float2 v[4], cur[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) v[e] = scale2(nxt[e], nxt_down);
+                for (int e = 0; e < 4; ++e) v[e] = __ffma2_rn(nxt[e], make_float2(nxt_down, nxt_down), make_float2(nxt_shift, nxt_shift));
+                if (nxt_left < 8) {  // (the powers of a shift alone could leave fp16's range)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (nxt_left <= 2 * e) v[e].x = 0.0f;
+                        if (nxt_left <= 2 * e + 1) v[e].y = 0.0f;
+                    }
+                }
                 if (u + kConvWarps < units) fetch(u + kConvWarps);
                 // row of B: power, channel of the half
                 const int item = (u % UNITS) * 32 + lane, cl = item % CW, chunk = item / CW;
@@ -1086,7 +1121,8 @@ __device__ __forceinline__ float from_ordered(unsigned c) {
     return __uint_as_float((c & 0x80000000u) ? c & 0x7fffffffu : ~c);
 }
 
-constexpr int kColumnRows = 128;  // rows per block of the column jobs
+constexpr int kColumnRows = 128;  // least rows per block of the column jobs
+constexpr int kMaxRanges = 64;
 constexpr int kMaxSplits = 64;    // row ranges of the coefficients' column sums
 constexpr int kMaxChannelExp = 17;  // channels of values beyond 2^17 or below 2^-17: 2^(7 * 17) is still a number
 
@@ -1096,13 +1132,20 @@ struct BackwardStats {
     int pitch;
     int *row_exp, *out_exp;                           // rows of the coefficients, output channels
     float *row_sum, *out_sum;
-    float *down_w, *down_x;                           // [g][channel_pitch], of the two sources
+    // [g][channel_pitch], of the two operands that are summed over (w: grad_x, x: grad_w): 2^-e, -mean 2^-e
+    float *down_w, *down_x, *shift_w, *shift_x;
     int channel_pitch;
     unsigned *x_top, *x_low, *w_top, *w_low;          // per channel: codes of the largest value and of the largest negative
-    unsigned *x_all, *w_all, *y_low;                  // bits of the largest |x| and |w|, code of the largest -y
+    double2 *x_part, *w_part;                         // [range of rows][channel]: sums of values and of squares
+    int x_ranges, w_ranges, x_rows, w_rows;           // ranges, and rows (samples, of images) in each
+    unsigned *y_low, *most;                           // code of the largest -y, bits of the largest |d| + |u| of a channel
+    double* spread_part;                              // [channel block]: sum of s^p
+    int p;
     unsigned* part_top;                               // [split][CO]
     double* part_sum;
+    float* part_abs;
     int splits, rows_per_split;
+    bool need_x, need_w;                              // grad_x / grad_w is wanted
     int blocks_rows, blocks_cols, blocks_w, blocks_x, blocks_y; // blocks of each job, in this order
     int blocks_channels;                              // of the second kernel
     int* bad;                                         // data that the expansion does not suit
@@ -1110,39 +1153,44 @@ struct BackwardStats {
     int* cond;
 };
 
-// The largest magnitude of all, from a lane's largest code of a value or of its negative.
-__device__ __forceinline__ void raise_magnitude(unsigned* all, unsigned code) {
-    code = __reduce_max_sync(0xffffffffu, code);
-    const unsigned bits = code & 0x7fffffffu;  // (the larger of the two codes is that of a positive number or of zero)
-    if ((threadIdx.x & 31) == 0 && (code & 0x80000000u) && bits > *static_cast<volatile unsigned*>(all)) atomicMax(all, bits);
+__device__ __forceinline__ void add_moments(double2* sum, float v) {
+    const double d = v;
+    sum->x += d;
+    sum->y += d * d;
 }
 
-// column extremes of rows [r0, r1) of a matrix whose columns are contiguous: 32 columns per block
+// column extremes and sums of rows [r0, r1) of a matrix whose columns are contiguous: 32 columns per block
 __device__ __forceinline__ void column_extremes(const float* p, long long pitch, int r0, int r1, int col, int cols, unsigned* top,
-                                                unsigned* low, unsigned* all) {
+                                                unsigned* low, double2* part) {
     __shared__ unsigned tops[8][32], lows[8][32];
+    __shared__ double2 sums[8][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned t = 0, l = 0;
+    double2 sum = make_double2(0.0, 0.0);
     if (col + lane < cols)
 #pragma unroll 8
         for (int r = r0 + warp; r < r1; r += 8) {
             const float v = p[r * pitch + col + lane];
             t = max(t, ordered(v));
             l = max(l, ordered(-v));
+            add_moments(&sum, v);
         }
     tops[warp][lane] = t;
     lows[warp][lane] = l;
+    sums[warp][lane] = sum;
     __syncthreads();
     if (warp == 0) {
         for (int i = 1; i < 8; ++i) {
             t = max(t, tops[i][lane]);
             l = max(l, lows[i][lane]);
+            sum.x += sums[i][lane].x;
+            sum.y += sums[i][lane].y;
         }
         if (col + lane < cols) {
             atomicMax(top + col + lane, t);
             atomicMax(low + col + lane, l);
+            part[col + lane] = sum;
         }
-        raise_magnitude(all, max(t, l));
     }
 }
 
@@ -1150,8 +1198,8 @@ __device__ __forceinline__ int row_scale(unsigned top) {
     return top == 0 ? 0 : max(-100, min(100, 15 - exponent_above(top)));
 }
 
-// What the backward form needs to know of its operands: the smallest output, largest coefficient and sum of every row (over the output channels)
-// and of every output channel (over the rows, in ranges), and the range of values of every channel of x and w.
+// What the backward form needs to know of its operands: largest coefficient and sums of every row (over the output channels)
+// and of every output channel (over the rows, in ranges), range and mean of the values of every channel of x and w.
 __global__ void __launch_bounds__(kPrep) even_stats_kernel(const BackwardStats A) {
     stream_order_begin();
     const Shape& s = A.s;
@@ -1163,18 +1211,23 @@ __global__ void __launch_bounds__(kPrep) even_stats_kernel(const BackwardStats A
         const float* p = A.coef + r * A.pitch;
         unsigned top = 0;
         double sum = 0.0;
+        float abs = 0.0f;
 #pragma unroll 4
         for (int o = lane; o < s.COg; o += 32) {
             top = max(top, magnitude(p[o]));
             sum += p[o];
+            abs += fabsf(p[o]);
         }
         top = __reduce_max_sync(0xffffffffu, top);
-        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        for (int d = 16; d > 0; d >>= 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, d);
+            abs += __shfl_xor_sync(0xffffffffu, abs, d);
+        }
         if (lane == 0) {
             const int e = row_scale(top);
             A.row_exp[r] = e;
             A.row_sum[r] = static_cast<float>(sum * pow2i(e));
-            if (top >= 0x7f800000u) *A.bad = 1;
+            if (top >= 0x7f800000u || (A.need_x && !(abs >= kLeastSpread * __uint_as_float(top)))) *A.bad = 1;
         }
         return;
     }
@@ -1182,6 +1235,7 @@ __global__ void __launch_bounds__(kPrep) even_stats_kernel(const BackwardStats A
     if (block < A.blocks_cols) {
         __shared__ unsigned tops[8][32];
         __shared__ double sums[8][32];
+        __shared__ float abses[8][32];
         const int per_group = (s.COg + 31) / 32;
         const int split = block / (per_group * s.G), rest = block - split * per_group * s.G, g = rest / per_group;
         const int o = (rest - g * per_group) * 32 + lane;
@@ -1189,6 +1243,7 @@ __global__ void __launch_bounds__(kPrep) even_stats_kernel(const BackwardStats A
         const long long r1 = r0 + A.rows_per_split < s.M ? r0 + A.rows_per_split : s.M;
         unsigned top = 0;
         double sum = 0.0;
+        float abs = 0.0f;
         if (o < s.COg) {
             const float* p = A.coef + static_cast<long long>(g) * s.M * A.pitch + o;
 #pragma unroll 8
@@ -1196,28 +1251,32 @@ __global__ void __launch_bounds__(kPrep) even_stats_kernel(const BackwardStats A
                 const float v = p[r * A.pitch];
                 top = max(top, magnitude(v));
                 sum += v;
+                abs += fabsf(v);
             }
         }
         tops[warp][lane] = top;
         sums[warp][lane] = sum;
+        abses[warp][lane] = abs;
         __syncthreads();
         if (warp == 0 && o < s.COg) {
             for (int i = 1; i < 8; ++i) {
                 top = max(top, tops[i][lane]);
                 sum += sums[i][lane];
+                abs += abses[i][lane];
             }
             const long long at = static_cast<long long>(split) * s.CO + g * s.COg + o;
             A.part_top[at] = top;
             A.part_sum[at] = sum;
+            A.part_abs[at] = abs;
         }
         return;
     }
     block -= A.blocks_cols;
     const int col_blocks = (s.CIg + 31) / 32;
     if (block < A.blocks_w) {
-        const int cb = block % col_blocks, t = block / col_blocks, g = t % s.G, r0 = (t / s.G) * kColumnRows;
-        column_extremes(A.w + static_cast<long long>(g) * s.COg * s.CIg, s.CIg, r0, min(s.COg, r0 + kColumnRows), cb * 32, s.CIg,
-                        A.w_top + g * s.CIg, A.w_low + g * s.CIg, A.w_all);
+        const int cb = block % col_blocks, t = block / col_blocks, g = t % s.G, range = t / s.G, r0 = range * A.w_rows;
+        column_extremes(A.w + static_cast<long long>(g) * s.COg * s.CIg, s.CIg, r0, min(s.COg, r0 + A.w_rows), cb * 32, s.CIg,
+                        A.w_top + g * s.CIg, A.w_low + g * s.CIg, A.w_part + static_cast<long long>(range) * s.CI + g * s.CIg);
         return;
     }
     block -= A.blocks_w;
@@ -1231,70 +1290,152 @@ __global__ void __launch_bounds__(kPrep) even_stats_kernel(const BackwardStats A
         return;
     }
     if (s.HW == 1) {
-        const int cols = (s.CI + 31) / 32, cb = block % cols, r0 = (block / cols) * kColumnRows;
-        column_extremes(A.x, s.CI, r0, min(s.B, r0 + kColumnRows), cb * 32, s.CI, A.x_top, A.x_low, A.x_all);
+        const int cols = (s.CI + 31) / 32, cb = block % cols, range = block / cols, r0 = range * A.x_rows;
+        column_extremes(A.x, s.CI, r0, min(s.B, r0 + A.x_rows), cb * 32, s.CI, A.x_top, A.x_low, A.x_part + static_cast<long long>(range) * s.CI);
         return;
     }
-    const long long r = static_cast<long long>(block) * 8 + warp;  // (sample, channel)
-    if (r >= static_cast<long long>(s.B) * s.CI) return;
-    const float* p = A.x + r * s.HW;
+    const long long r = static_cast<long long>(block) * 8 + warp;  // (range of samples, channel)
+    if (r >= static_cast<long long>(A.x_ranges) * s.CI) return;
+    const int range = static_cast<int>(r / s.CI), c = static_cast<int>(r - static_cast<long long>(range) * s.CI);
     unsigned t = 0, l = 0;
+    double2 sum = make_double2(0.0, 0.0);
+    for (int b = range * A.x_rows; b < min(s.B, (range + 1) * A.x_rows); ++b) {
+        const float* p = A.x + (static_cast<long long>(b) * s.CI + c) * s.HW;
 #pragma unroll 4
-    for (int i = lane; i < s.HW; i += 32) {
-        t = max(t, ordered(p[i]));
-        l = max(l, ordered(-p[i]));
+        for (int i = lane; i < s.HW; i += 32) {
+            t = max(t, ordered(p[i]));
+            l = max(l, ordered(-p[i]));
+            add_moments(&sum, p[i]);
+        }
     }
     t = __reduce_max_sync(0xffffffffu, t);
     l = __reduce_max_sync(0xffffffffu, l);
-    if (lane == 0) {
-        atomicMax(A.x_top + r % s.CI, t);
-        atomicMax(A.x_low + r % s.CI, l);
+    for (int d = 16; d > 0; d >>= 1) {
+        sum.x += __shfl_xor_sync(0xffffffffu, sum.x, d);
+        sum.y += __shfl_xor_sync(0xffffffffu, sum.y, d);
     }
-    raise_magnitude(A.x_all, max(t, l));
+    if (lane == 0) {
+        atomicMax(A.x_top + c, t);
+        atomicMax(A.x_low + c, l);
+        A.x_part[r] = sum;
+    }
 }
 
-// Scales of the channels and of the output channels' coefficients; whether the expansion suits the data: the values of a
-// channel, of both operands together, have to spread over at least a quarter of the largest of them.
+// 2^-e and shift of a channel that is summed over, its values in [u_low, u_top], the other operand's in [d_low, d_top]; the largest
+// |d| + |u|.
+__device__ __forceinline__ float channel_scale(float mean, float u_low, float u_top, float d_low, float d_top, float* down, float* shift,
+                                               bool* bad) {
+    const float u = fmaxf(u_top - mean, mean - u_low), d = fmaxf(d_top - mean, mean - d_low);
+    const float m = u > 0.0f ? fmaxf(u, d * kChannelFloor) : d;
+    const int e = m > 0.0f ? exponent_above(__float_as_uint(m)) : 0;
+    *bad |= abs(e) > kMaxChannelExp || (u > 0.0f && !(u >= d * kLeastChannel));
+    *down = pow2i(-max(-kMaxChannelExp, min(kMaxChannelExp, e)));
+    *shift = -mean * *down;
+    return u + d;
+}
+
+// Scales of the channels and of the output channels' coefficients; guards on both.  Blocks of channels: 32 of a group, whose
+// warps share the ranges of rows.
 __global__ void __launch_bounds__(kPrep) even_scales_kernel(const BackwardStats A) {
     stream_order_begin();
     const Shape& s = A.s;
-    const int i = blockIdx.x * kPrep + threadIdx.x;
     bool bad = false;
-    if (i < s.CI && static_cast<int>(blockIdx.x) < A.blocks_channels) {
-        const float xt = from_ordered(A.x_top[i]), xl = from_ordered(A.x_low[i]);   // largest value, largest negative
-        const float wt = from_ordered(A.w_top[i]), wl = from_ordered(A.w_low[i]);
-        const float xm = fmaxf(fabsf(xt), fabsf(xl)), wm = fmaxf(fabsf(wt), fabsf(wl)), m = fmaxf(xm, wm);
-        const bool finite = xt + xl + wt + wl < INFINITY && fmaxf(xt, wt) < INFINITY && fmaxf(xl, wl) < INFINITY;
-        bad = !finite || !(4.0f * (fmaxf(xt, wt) + fmaxf(xl, wl)) >= m);
-        const unsigned fw = __float_as_uint(fmaxf(wm, xm * (1.0f / 64))), fx = __float_as_uint(fmaxf(xm, wm * (1.0f / 64)));
-        const int ew = fw == 0 ? 0 : exponent_above(fw), ex = fx == 0 ? 0 : exponent_above(fx);
-        bad |= max(abs(ew), abs(ex)) > kMaxChannelExp;
-        const int at = i / s.CIg * A.channel_pitch + i % s.CIg;
-        A.down_w[at] = pow2i(-max(-kMaxChannelExp, min(kMaxChannelExp, ew)));
-        A.down_x[at] = pow2i(-max(-kMaxChannelExp, min(kMaxChannelExp, ex)));
+    if (static_cast<int>(blockIdx.x) < A.blocks_channels) {
+        __shared__ double2 parts[2][8][32];
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int per_group = (s.CIg + 31) / 32, g = blockIdx.x / per_group, c = (blockIdx.x - g * per_group) * 32 + lane, i = g * s.CIg + c;
+        double2 sx = make_double2(0.0, 0.0), sw = sx;
+        if (c < s.CIg) {
+#pragma unroll 4
+            for (int k = warp; k < A.x_ranges; k += 8) {
+                const double2 v = A.x_part[static_cast<long long>(k) * s.CI + i];
+                sx.x += v.x;
+                sx.y += v.y;
+            }
+#pragma unroll 4
+            for (int k = warp; k < A.w_ranges; k += 8) {
+                const double2 v = A.w_part[static_cast<long long>(k) * s.CI + i];
+                sw.x += v.x;
+                sw.y += v.y;
+            }
+        }
+        parts[0][warp][lane] = sx;
+        parts[1][warp][lane] = sw;
+        __syncthreads();
+        if (warp != 0) return;
+        float most = 0.0f;
+        double spread = 0.0;
+        if (c < s.CIg) {
+            for (int k = 1; k < 8; ++k) {
+                sx.x += parts[0][k][lane].x;
+                sx.y += parts[0][k][lane].y;
+                sw.x += parts[1][k][lane].x;
+                sw.y += parts[1][k][lane].y;
+            }
+            const float xt = from_ordered(A.x_top[i]), xl = -from_ordered(A.x_low[i]);
+            const float wt = from_ordered(A.w_top[i]), wl = -from_ordered(A.w_low[i]);
+            bad = !(fmaxf(fabsf(xt), fabsf(wt)) < INFINITY) || !(fmaxf(fabsf(xl), fabsf(wl)) < INFINITY) || isnan(xt + xl + wt + wl);
+            const double nx = static_cast<double>(s.M), nw = s.COg, ex = sx.x / nx, ew = sw.x / nw;
+            const double square = fmax(sx.y / nx - ex * ex, 0.0) + fmax(sw.y / nw - ew * ew, 0.0) + (ex - ew) * (ex - ew);
+            spread = square;
+            for (int k = 1; k < A.p / 2; ++k) spread *= square;
+            const int at = g * A.channel_pitch + c;
+            bool bad_x = false, bad_w = false;
+            const float mean_w = fminf(fmaxf(static_cast<float>(ew), wl), wt), mean_x = fminf(fmaxf(static_cast<float>(ex), xl), xt);
+            const float most_x = channel_scale(mean_w, wl, wt, xl, xt, A.down_w + at, A.shift_w + at, &bad_x);
+            const float most_w = channel_scale(mean_x, xl, xt, wl, wt, A.down_x + at, A.shift_x + at, &bad_w);
+            bad |= (A.need_x && bad_x) || (A.need_w && bad_w);
+            most = bad ? 0.0f : fmaxf(A.need_x ? most_x : 0.0f, A.need_w ? most_w : 0.0f);
+        }
+        for (int d = 16; d > 0; d >>= 1) spread += __shfl_xor_sync(0xffffffffu, spread, d);
+        const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(most));
+        if (lane == 0) {
+            A.spread_part[blockIdx.x] = spread;
+            atomicMax(A.most, bits);
+            bad |= blockIdx.x == 0 && *A.bad != 0;
+        }
+        if (bad && *A.range == 0) *A.cond = 1;
+        return;
     }
     if (static_cast<int>(blockIdx.x) >= A.blocks_channels) {  // a warp per output channel
         const int o = (static_cast<int>(blockIdx.x) - A.blocks_channels) * (kPrep / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
         unsigned top = 0;
         double sum = 0.0;
+        float abs = 0.0f;
         for (int k = lane; k < A.splits && o < s.CO; k += 32) {
             top = max(top, A.part_top[static_cast<long long>(k) * s.CO + o]);
             sum += A.part_sum[static_cast<long long>(k) * s.CO + o];
+            abs += A.part_abs[static_cast<long long>(k) * s.CO + o];
         }
         top = __reduce_max_sync(0xffffffffu, top);
-        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        for (int d = 16; d > 0; d >>= 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, d);
+            abs += __shfl_xor_sync(0xffffffffu, abs, d);
+        }
         if (lane == 0 && o < s.CO) {
+            if (A.need_w && !(abs >= kLeastSpread * __uint_as_float(top)) && *A.range == 0) *A.cond = 1;
             const int e = row_scale(top);
             A.out_exp[o] = e;
             A.out_sum[o] = static_cast<float>(sum * pow2i(e));
         }
-        return;
     }
-    if (i == 0) {
-        const float most = __uint_as_float(*A.x_all) + __uint_as_float(*A.w_all), least = -from_ordered(*A.y_low);
-        bad |= *A.bad != 0 || !(3.0f * least >= most);
+}
+
+// The guards on the smallest output, by one warp.
+__device__ __forceinline__ void guard_outputs(const BackwardStats& A) {
+    const int lane = threadIdx.x & 31, per_group = (A.s.CIg + 31) / 32;
+    double most = 0.0;
+    for (int g = 0; g < A.s.G; ++g) {
+        double sum = 0.0;
+        for (int k = lane; k < per_group; k += 32) sum += A.spread_part[g * per_group + k];
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        most = fmax(most, sum);
     }
-    if (bad && *A.range == 0) *A.cond = 1;
+    const float y = -from_ordered(*A.y_low);
+    const double scaled = y / least_of_spread(A.p), square = scaled * scaled;
+    double power = square;
+    for (int k = 1; k < A.p / 2; ++k) power *= square;
+    if (lane == 0 && (!(kMostOfOutput * y >= __uint_as_float(*A.most)) || !(power >= most))) *A.cond = 1;
 }
 
 // Blocks of A of the backward form: the coefficients with rows = positions (grad_x) and with rows = output channels (grad_w).
@@ -1305,9 +1446,11 @@ struct CoefImages {
     int tiles_m, kb, blocks;
     bool split;
 };
-__global__ void __launch_bounds__(kPrep) even_coef_kernel(const CoefImages X, const CoefImages W, const int* gate0, const int* gate1) {
+// (and, beside the first of them, the last guard: the products, not the images, wait for it)
+__global__ void __launch_bounds__(kPrep) even_coef_kernel(const BackwardStats A, const CoefImages X, const CoefImages W) {
     stream_order_begin();
-    if (*gate0 != 0 || *gate1 != 0) return;
+    if (*A.range != 0 || *A.cond != 0) return;
+    if (blockIdx.x == 0 && threadIdx.x < 32) guard_outputs(A);
     const bool first = static_cast<int>(blockIdx.x) < X.blocks;
     const CoefImages& J = first ? X : W;
     const int block = first ? blockIdx.x : blockIdx.x - X.blocks;
@@ -1509,6 +1652,15 @@ int row_splits(const Shape& s) {
     return n < kMaxSplits ? n : kMaxSplits;
 }
 
+// words that a backward call clears: codes of the extremes of the channels of x and w, and single ones
+inline size_t channel_words(const Shape& s) { return 4 * static_cast<size_t>(s.CI) + 8; }
+// ranges of rows for the channels' sums: at most kMaxRanges, of kColumnRows rows or more (images: of any number of samples)
+inline void channel_ranges(int rows, bool columns, int* ranges, int* in_each) {
+    *in_each = div_up(rows, kMaxRanges);
+    if (columns && *in_each < kColumnRows) *in_each = kColumnRows;
+    *ranges = div_up(rows, *in_each);
+}
+
 template <int PW>
 int backward_power(const float* coef, int pitch, const float* x, const float* w, const float* y, const Shape& s, float* gx, float* gw,
                    bool accumulate_gw, const int* range, int cap, Bump* bump, int* status, const int** cond, cudaStream_t st) {
@@ -1525,39 +1677,51 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
     A.out_sum = bump->take<float>(s.CO);
     A.channel_pitch = div_up(s.CIg, CT) * CT;
     const size_t scales = static_cast<size_t>(s.G) * A.channel_pitch;
-    A.down_w = bump->take<float>(2 * scales);
-    A.down_x = A.down_w + scales;
-    unsigned* words = bump->take<unsigned>(4 * static_cast<size_t>(s.CI) + 8);
+    float* channels = bump->take<float>(4 * scales);
+    const size_t words_size = channel_words(s);
+    unsigned* words = bump->take<unsigned>(words_size);
     A.part_top = bump->take<unsigned>(static_cast<size_t>(splits) * s.CO);
     A.part_sum = bump->take<double>(static_cast<size_t>(splits) * s.CO);
+    A.part_abs = bump->take<float>(static_cast<size_t>(splits) * s.CO);
+    channel_ranges(s.B, s.HW == 1, &A.x_ranges, &A.x_rows);
+    channel_ranges(s.COg, true, &A.w_ranges, &A.w_rows);
+    A.x_part = bump->take<double2>(static_cast<size_t>(A.x_ranges) * s.CI);
+    A.w_part = bump->take<double2>(static_cast<size_t>(A.w_ranges) * s.CI);
+    A.blocks_channels = s.G * div_up(s.CIg, 32);
+    A.spread_part = bump->take<double>(A.blocks_channels);
     const GradientPlan px = plan_gradient(s, false, CT), pw = plan_gradient(s, true, CT);
     char* images_x = gx ? bump->take<char>(px.image_bytes) : nullptr;
     char* images_w = gw ? bump->take<char>(pw.image_bytes) : nullptr;
     float* partials = bump->take<float>(gradient_part_floats(s, gx != nullptr, gw != nullptr, CT, cap));
-    if (!A.row_exp || !A.row_sum || !A.out_exp || !A.out_sum || !A.down_w || !words || !A.part_top ||
-        !A.part_sum || (gx && !images_x) || (gw && !images_w) || !partials)
+    if (!A.row_exp || !A.row_sum || !A.out_exp || !A.out_sum || !channels || !words || !A.part_top || !A.part_sum || !A.part_abs ||
+        !A.x_part || !A.w_part || !A.spread_part || (gx && !images_x) || (gw && !images_w) || !partials)
         return kWorkspace;
-    A.x_top = words; A.x_low = words + s.CI; A.w_top = words + 2 * s.CI; A.w_low = words + 3 * s.CI;
-    A.bad = reinterpret_cast<int*>(words + 4 * s.CI);
+    A.p = PW;
+    A.down_w = channels; A.down_x = channels + scales;
+    A.shift_w = channels + 2 * scales; A.shift_x = channels + 3 * scales;
+    A.x_top = words; A.x_low = A.x_top + s.CI; A.w_top = A.x_low + s.CI; A.w_low = A.w_top + s.CI;
+    unsigned* single = A.w_low + s.CI;
+    A.bad = reinterpret_cast<int*>(single);
     A.cond = A.bad + 1;
-    A.x_all = words + 4 * s.CI + 2; A.w_all = A.x_all + 1; A.y_low = A.x_all + 2;
+    A.y_low = single + 2; A.most = single + 3;
     A.range = range;
+    A.need_x = gx != nullptr;
+    A.need_w = gw != nullptr;
     *cond = A.cond;
-    cudaError_t e = cudaMemsetAsync(words, 0, (4 * static_cast<size_t>(s.CI) + 8) * sizeof(unsigned), st);
-    // (scales of the padding channels are multiplied with zeros: they only have to be numbers)
-    if (e == cudaSuccess && A.channel_pitch != s.CIg) e = cudaMemsetAsync(A.down_w, 0, 2 * scales * sizeof(float), st);
+    cudaError_t e = cudaMemsetAsync(words, 0, words_size * sizeof(unsigned), st);
+    // (scales and shifts of the padding channels are multiplied with zeros: they only have to be numbers)
+    if (e == cudaSuccess && A.channel_pitch != s.CIg) e = cudaMemsetAsync(channels, 0, 4 * scales * sizeof(float), st);
     if (e != cudaSuccess) return cuda_status(e);
     A.splits = splits;
     A.rows_per_split = div_up(s.M, splits);
     A.blocks_rows = div_up(static_cast<long long>(rows), 8);
     A.blocks_cols = splits * s.G * div_up(s.COg, 32);
-    A.blocks_w = div_up(s.CIg, 32) * s.G * div_up(s.COg, kColumnRows);
-    A.blocks_x = s.HW == 1 ? div_up(s.CI, 32) * div_up(s.B, kColumnRows) : div_up(static_cast<long long>(s.B) * s.CI, 8);
+    A.blocks_w = div_up(s.CIg, 32) * s.G * A.w_ranges;
+    A.blocks_x = s.HW == 1 ? div_up(s.CI, 32) * A.x_ranges : div_up(static_cast<long long>(A.x_ranges) * s.CI, 8);
     A.blocks_y = div_up(s.M * s.CO, 16 * kPrep);
     if (A.blocks_y > 1184) A.blocks_y = 1184;
     int r = launch_after(even_stats_kernel, A.blocks_rows + A.blocks_cols + A.blocks_w + A.blocks_x + A.blocks_y, kPrep, 0, st, A);
     if (r != kOk) return r;
-    A.blocks_channels = div_up(s.CI, kPrep);
     if ((r = launch_after(even_scales_kernel, A.blocks_channels + div_up(s.CO, kPrep / 32), kPrep, 0, st, A)) != kOk) return r;
     CoefImages X{}, W{};
     const long long group = static_cast<long long>(s.M) * pitch;
@@ -1574,7 +1738,7 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
     W.src = Source{coef, 2, s.COg, static_cast<int>(s.M), 0, 1, pitch, 0, group};
     blocks_of(W, pw, images_w);
     W.exp = A.out_exp;
-    if ((r = launch_after(even_coef_kernel, X.blocks + W.blocks, kPrep, 0, st, X, W, range, static_cast<const int*>(A.cond))) != kOk) return r;
+    if ((r = launch_after(even_coef_kernel, X.blocks + W.blocks, kPrep, 0, st, A, X, W)) != kOk) return r;
     EvenParams P{};
     P.G = s.G;
     P.N = s.CIg;
@@ -1600,7 +1764,7 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
         P.vec = s.HW == 1 && s.CIg % 4 == 0 && aligned16(x) && aligned16(gx);
         P.out_f = gx;
         P.resident = x;
-        P.col_down = A.down_w; P.row_exp = A.row_exp; P.row_sum = A.row_sum;
+        P.col_down = A.down_w; P.col_shift = A.shift_w; P.row_exp = A.row_exp; P.row_sum = A.row_sum;
         if ((r = launch_even<PW, false>(P, cap, st)) != kOk) return r;
     }
     if (gw) {
@@ -1612,7 +1776,7 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
         P.out_f = gw;
         P.resident = w;
         P.accumulate = accumulate_gw;
-        P.col_down = A.down_x; P.row_exp = A.out_exp; P.row_sum = A.out_sum;
+        P.col_down = A.down_x; P.col_shift = A.shift_x; P.row_exp = A.out_exp; P.row_sum = A.out_sum;
         if ((r = launch_even<PW, false>(P, cap, st)) != kOk) return r;
     }
     return kOk;
