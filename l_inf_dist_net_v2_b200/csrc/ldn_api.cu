@@ -328,7 +328,7 @@ int norm_dist_backward_part(const float* go, const float* x, const float* w, con
                   ((iq < 0 || guarded) ? 2 * pad256(gen_floats * sizeof(float)) : 0) +
                   (guarded ? 4 : 2) * partial_bytes(cap, 1) + (fused ? pad256(side_floats * sizeof(float)) : 0);
     // even p of large problems: both gradients from matrix products (ldn_even.cu), the kernels here gated behind them
-    const size_t even_bytes = even_power(p) && !accumulate_gx && s.co_src == s.CO && even_backward_applies(s, p, gx != nullptr, gw != nullptr, cap)
+    const size_t even_bytes = even_power(p) && !accumulate_gx && s.co_src == s.CO && even_backward_applies(s, p, gx != nullptr, gw != nullptr, cap, ctx->sm_count)
                                   ? even_backward_bytes(s, p, gx != nullptr, gw != nullptr, cap)
                                   : 0;
     bool even = false;
@@ -691,7 +691,7 @@ LDN_API int ldn_norm_dist_forward(const float* input, const float* weight, int B
                   (bound_norm ? 3 : 2) * partial_bytes(cap_for(ctx), 1) + (normalised ? ybytes : 0) +
                   (bound_norm ? 2 * pad256(norm_floats * sizeof(float)) : 0);
     // even p of large problems: matrix products (ldn_even.cu), the direct kernel gated behind them
-    const size_t even_bytes = even_power(p) && even_forward_applies(s, p, cap_for(ctx)) ? even_forward_bytes(s, p, cap_for(ctx)) : 0;
+    const size_t even_bytes = even_power(p) && even_forward_applies(s, p, cap_for(ctx), ctx->sm_count) ? even_forward_bytes(s, p, cap_for(ctx)) : 0;
     // large fully connected layers at general p: from the channels whose terms count (ldn_power_lists.cu), likewise
     const bool lists = bound_norm && power_lists_apply(s, p);
     const size_t more = lists ? power_lists_bytes(s) : even_bytes;

@@ -7,7 +7,9 @@ namespace {
 // Which path is the faster one: estimated times in microseconds, from fits to measured calls of either (32 - 512 rows or 8 -
 // 128 images, 256 - 4096 channels, 256 - 5120 outputs; they are within 15 % of most).  The matrix products take a fixed time
 // for preparation and launches and one per stage of 64 reduction elements, the backward pass also one per tile; the direct
-// kernels a time per pair, padding of their 128-wide tiles included.  Measured, direct -> this path, p = 8, forward / both
+// kernels a time per pair, padding of their 128-wide tiles included.  Either runs on the CTAs it may have: the fits' times per
+// stage and per pair go up as those go down (512 x 1536 -> 2048, p = 8, 37 of 148: 842 / 1614 us direct,
+// 212 / 434 on the products).  Measured, direct -> this path, p = 8, forward / both
 // gradients: 512 x 3072 -> 5120 1045 / 2019 -> 281 / 612, 256 x 1024 -> 2048 81 / 161 -> 59 / 123, 256 x 1024 -> 1024 50 / 103
 // -> 52 / 102 (here the line lies), 64 x 784 -> 1024 20 / 71 -> 47 / 97; 32 images of 576 x 1024 -> 128 340 / 878 -> 219 / 409.
 constexpr double kMargin = 1.1;         // the estimate has to win by this factor
@@ -26,18 +28,18 @@ bool in_range(const Shape& s, double stages) {
 
 }  // namespace
 
-bool even_forward_applies(const Shape& s, float p, int cap) {
+bool even_forward_applies(const Shape& s, float p, int cap, int sm_count) {
     const int i = static_cast<int>(p) / 2 - 1;
     constexpr double per_stage[4] = {2.3, 1.35, 1.2, 1.15}, per_pair[4] = {80e-9, 100e-9, 138e-9, 130e-9};
     const ForwardPlan f = plan_forward(s, 2 * i + 1);
     const double stages = static_cast<double>(f.total);
     const double products = 38.0 + prepare_us(s) + per_stage[i] * ceil(stages / (cap / 2));
     const double narrow = i == 3 && s.COg <= 64 ? (s.COg <= 32 ? 32.0 : 64.0) : 128.0;
-    const double direct = 12.0 + per_pair[i] * direct_rows(s) * padded(s.COg, narrow) * s.G * s.CIg;
+    const double direct = 12.0 + per_pair[i] * direct_rows(s) * padded(s.COg, narrow) * s.G * s.CIg * sm_count / (cap > 0 ? cap : 1);
     return cap >= 2 && in_range(s, stages) && products * kMargin < direct;
 }
 
-bool even_backward_applies(const Shape& s, float p, bool gx, bool gw, int cap) {
+bool even_backward_applies(const Shape& s, float p, bool gx, bool gw, int cap, int sm_count) {
     const int i = static_cast<int>(p) / 2 - 1, ct = channels_of(2 * i + 1);
     constexpr double per_stage[4] = {2.4, 1.3, 0.92, 1.05}, per_tile = 2.7;
     constexpr double both[4] = {139e-9, 195e-9, 223e-9, 248e-9}, one[4] = {85e-9, 134e-9, 162e-9, 190e-9};
@@ -51,7 +53,8 @@ bool even_backward_applies(const Shape& s, float p, bool gx, bool gw, int cap) {
     }
     // tiles of the direct kernels: rows x channels, over the outputs; for grad_w alone outputs x channels, over the rows
     const double columns_d = s.G * padded(s.CIg, 128.0), out_rows = s.COg <= 64 ? 64.0 : padded(s.COg, 128.0);
-    const double pairs = columns_d * (gx ? direct_rows(s) * padded(s.COg, 32.0) : out_rows * padded(static_cast<double>(s.M), 32.0));
+    double pairs = columns_d * (gx ? direct_rows(s) * padded(s.COg, 32.0) : out_rows * padded(static_cast<double>(s.M), 32.0));
+    pairs *= static_cast<double>(sm_count) / (cap > 0 ? cap : 1);
     const double direct = gx && gw ? 35.0 + both[i] * pairs : 30.0 + one[i] * pairs;
     return cap >= 2 && in_range(s, most) && products * kMargin < direct;
 }

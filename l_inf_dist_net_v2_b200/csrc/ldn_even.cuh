@@ -6,9 +6,9 @@ namespace ldn {
 
 inline bool even_power(float p) { return p == 2.0f || p == 4.0f || p == 6.0f || p == 8.0f; }
 
-// Whether a problem is large enough for this path to be the faster one, forward and backward.
-bool even_forward_applies(const Shape& s, float p, int cap);
-bool even_backward_applies(const Shape& s, float p, bool gx, bool gw, int cap);
+// Whether a problem is large enough for this path to be the faster one, forward and backward, on `cap` of the device's CTAs.
+bool even_forward_applies(const Shape& s, float p, int cap, int sm_count);
+bool even_backward_applies(const Shape& s, float p, bool gx, bool gw, int cap, int sm_count);
 
 // Scratch of a forward call; launch_even_forward takes it from the bump allocator.
 size_t even_forward_bytes(const Shape& s, float p, int cap);
