@@ -20,7 +20,10 @@
 //   * the tensor core's accumulator drops the bits below the largest summand instead of rounding, so it takes one stage
 //     at a time and the sums are added up in registers.  What 64 elements' products lose that way is 2.0e-7 - 2.8e-7 of
 //     their sum in the forward pass (p = 4 and 8, 128 - 3072 channels, images and zero-mean activations, against 64 bits),
-//     always towards zero: kTruncation gives it back there.  (The backward pass's sums, whose terms have either sign, show no
+//     always towards zero: kTruncation gives it back there.  What is left of it in the values, on average: between -5e-9 and 1.5e-8
+//     of them for p = 2, 4, 6 and 8, 256 - 3000 channels, pairs' tiles and split ones, images, activations and operands of opposite
+//     signs.  (Root mean square errors 2.0e-8 - 4.3e-8, direct kernels 4e-8 - 4e-7; the largest of one output of 4 M 1.1e-6 at
+//     p = 8 and 256 channels, where direct ones have 2.6e-7, 1e-7 - 6e-7 from 576 channels on, 2e-7 - 2.3e-6.)  (The backward pass's sums, whose terms have either sign, show no
 //     such drift.)
 //   * powers are scaled into fp16's range: by one power of two for both operands in the forward pass (all terms of the sum
 //     share it), by one per channel and one per coefficient row in the backward pass;
@@ -100,7 +103,7 @@ struct Source {
 };
 
 struct EvenParams {
-    int M, N, K, G;                 // per group: rows of A, rows of B (forward) or channels (backward), reduction length
+    int M, N, G;                    // per group: rows of A, rows of B (forward) or channels (backward)
     int tiles_m, tiles_n, kt;       // kt: stages per tile
     int blocks;                     // forward: blocks of 32 channels times powers, in this order
     int total;                      // stages in all
@@ -1042,7 +1045,7 @@ template <int PW>
 __global__ void __launch_bounds__(kPrep) even_powers_kernel(const Source a, int G, int tiles_m, int kb, int seq, bool split, char* images,
                                                            const double* sums_a, const double* sums_b, int rows_b,
                                                            float* sum_a, float* norm_a, float* sum_b, float* norm_b,
-                                                           const unsigned* scale_word, int* dense) {
+                                                           const unsigned* scale_word, int* dense, int* small) {
     constexpr int NP = PW - 1;
     stream_order_begin();
     const unsigned top = *scale_word;
@@ -1053,13 +1056,32 @@ __global__ void __launch_bounds__(kPrep) even_powers_kernel(const Source a, int 
     }
     const int images_blocks = G * tiles_m * kb, block = blockIdx.x;
     if (block >= images_blocks) {
-        const int i = (block - images_blocks) * kPrep + threadIdx.x;
-        if (i >= G * (a.rows + rows_b)) return;
-        const bool is_a = i < G * a.rows;
-        const int r = is_a ? i : i - G * a.rows;
-        const float v = static_cast<float>((is_a ? sums_a : sums_b)[r] * exp2(-static_cast<double>(PW) * e));
-        (is_a ? sum_a : sum_b)[r] = v;
-        (is_a ? norm_a : norm_b)[r] = v > 0.0f ? root<PW>(v) : 0.0f;
+        // An output is at most the sum of its rows' norms.  Where rows of either operand lie below half of what an output has to
+        // reach (ForwardEnd::least), their outputs go to the list for certain: more of them than it holds, and there is no
+        // point in the products (512 x 3072 -> 5120, p = 8, one value of 100: 1594 -> 1089 us; the
+        // direct kernels take 1045).  small: rows of a, rows of b, blocks done.
+        const int i = (block - images_blocks) * kPrep + threadIdx.x, rows = G * (a.rows + rows_b);
+        const float half = 0.5f * __uint_as_float((top & 0x7fffffu) | 0x3f000000u) * exp2f(-10.0f / PW);
+        bool small_a = false, small_b = false;
+        if (i < rows) {
+            const bool is_a = i < G * a.rows;
+            const int r = is_a ? i : i - G * a.rows;
+            const float v = static_cast<float>((is_a ? sums_a : sums_b)[r] * exp2(-static_cast<double>(PW) * e));
+            const float norm = v > 0.0f ? root<PW>(v) : 0.0f;
+            (is_a ? sum_a : sum_b)[r] = v;
+            (is_a ? norm_a : norm_b)[r] = norm;
+            (is_a ? small_a : small_b) = norm < 0.999f * half;
+        }
+        const int count_a = __syncthreads_count(small_a), count_b = __syncthreads_count(small_b);
+        if (threadIdx.x == 0) {
+            if (count_a) atomicAdd(small, count_a);
+            if (count_b) atomicAdd(small + 1, count_b);
+            __threadfence();
+            if (atomicAdd(small + 2, 1) == (rows + kPrep - 1) / kPrep - 1) {
+                const double pairs = static_cast<double>(atomicAdd(small, 0)) * atomicAdd(small + 1, 0);
+                if (pairs > static_cast<double>(kListCap) * G) *dense = 1;  // (of G groups: as many on average)
+            }
+        }
         return;
     }
     const ForwardScale<PW> scales(top);
@@ -1577,11 +1599,11 @@ int forward_power(const float* x, const float* w, const Shape& s, float* y, int 
     double* sums = bump->take<double>(static_cast<size_t>(rows_a) + rows_b);
     float* floats = bump->take<float>(2 * (static_cast<size_t>(rows_a) + rows_b));
     int* list = bump->take<int>(kListCap);
-    int* words = bump->take<int>(4);  // largest magnitude, list length, dense
+    int* words = bump->take<int>(8);  // largest magnitude, list length, dense, three counts of even_powers_kernel
     float* partials = bump->take<float>(part_floats(f.M, f.total, f.stages, cap, kNRows));
     if (!images || !sums || !floats || !list || !words || !partials) return kWorkspace;
     *dense = words + 2;
-    const cudaError_t e = cudaMemsetAsync(words, 0, 4 * sizeof(int), st);
+    const cudaError_t e = cudaMemsetAsync(words, 0, 8 * sizeof(int), st);
     if (e != cudaSuccess) return cuda_status(e);
     const Source xs = rows_of_x(x, s), ws = rows_of_w(w, s);
     const Source a = f.swap ? ws : xs, b = f.swap ? xs : ws;
@@ -1594,10 +1616,10 @@ int forward_power(const float* x, const float* w, const Shape& s, float* y, int 
     const int kb = div_up(s.CIg, kBlockK);
     const int prep = s.G * f.row_blocks * kb + div_up(static_cast<long long>(rows_a) + rows_b, kPrep);
     r = launch_after(even_powers_kernel<PW>, prep, kPrep, 0, st, a, s.G, f.row_blocks, kb, f.stages * kBlocks, split_rows(f.M), images, sums,
-                     sums + rows_a, b.rows, sum_a, norm_a, sum_b, norm_b, scale, words + 2);
+                     sums + rows_a, b.rows, sum_a, norm_a, sum_b, norm_b, scale, words + 2, words + 3);
     if (r != kOk) return r;
     EvenParams P{};
-    P.M = f.M; P.N = f.N; P.K = s.CIg; P.G = s.G;
+    P.M = f.M; P.N = f.N; P.G = s.G;
     P.tiles_m = row_tiles(f.M); P.tiles_n = f.tiles_n; P.kt = f.stages; P.blocks = kb * NP;
     P.total = static_cast<int>(f.total);
     P.split = split_rows(f.M);
@@ -1749,7 +1771,6 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
     P.status = status;
     auto rows_of = [&](const GradientPlan& g) {
         P.M = g.M;
-        P.K = g.K;
         P.kt = g.kt;
         P.tiles_m = row_tiles(g.M);
         P.total = static_cast<int>(g.total);
