@@ -460,7 +460,7 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
     hbm_peak = peaks.get("hbm_gbs", 6650.0)
     gemm_peak = peaks.get("bf16_tflops", 1590.0)  # the 16-bit types of the tensor cores share one rate
 
-    outcome = (ctypes.c_int * 2)()
+    outcome, power_outcome = (ctypes.c_int * 2)(), ctypes.c_int()
 
     def mark_extreme(row):
         """Says in a p = inf forward row what its times are of, if the call just made took its outputs from the lists of
@@ -473,6 +473,11 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
                            f"{outcome[1]} outputs in full")
             for key in ("slots_per_pair", "tlaneop_per_s", "frac_of_ffma_probe", "frac_of_nominal"):
                 row.pop(key, None)
+
+    def fast_power_path():
+        """Whether the matrix products of an even p, or power lists, gave the result of the call just made."""
+        stream = torch.cuda.current_stream().cuda_stream
+        return lib.ldn_last_power_outcome(stream, ctypes.byref(power_outcome)) == 0 and not power_outcome.value
 
     def kernel_rows(pp, label, steps):
         fam_ = p_family(pp)
@@ -499,19 +504,20 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
             # (a tile kernel is most of its call; anything far below that is not the kernel this row is about)
             if t_tile > 0.2 * t:
                 row["tile_kernel_ms"] = round(t_tile, 4)
-            if pp in (2.0, 4.0, 6.0, 8.0) and slots * pairs / (t * 1e-3) / 1e12 > ffma_peak:
-                # beyond what the FP32 pipe can do.  Even p of large problems: sums of powers as matrix products
-                # (csrc/ldn_even.cu), three products of 16-bit halves for each of the p - 1 mixed terms
+            fast = fast_power_path()
+            if fast and pp in (2.0, 4.0, 6.0, 8.0):
+                # Even p of large problems: sums of powers as matrix products (csrc/ldn_even.cu), three products of 16-bit
+                # halves for each of the p - 1 mixed terms
                 flops = 6 * (pp - 1) * pairs * (2 if name == "backward_fused" else 1)
                 if "tile_kernel_ms" in row:  # (of two gradients: the second's products)
                     row["products_kernel_ms"] = row.pop("tile_kernel_ms")
                 row.update({"bound": "tensor", "gflop": round(flops / 1e9, 1),
                             "tflop_per_s": round(flops / (t * 1e-3) / 1e12, 1),
                             "frac_of_measured_gemm": round(flops / (t * 1e-3) / 1e12 / gemm_peak, 3)})
-            elif "tile_kernel_ms" not in row and fam_ == "general" and name == "forward":
+            elif fast:
                 # from the channels whose terms count (csrc/ldn_power_lists.cu): no tile kernel ran
-                row.update({"bound": "load/store pipe", "note": "gpair_per_s counts every pair; csrc/ldn_power_lists.cu visits "
-                                                                "the few per cent whose terms count"})
+                row.update({"bound": "logarithm / exponential mix", "note": "gpair_per_s counts every pair; csrc/ldn_power_lists.cu "
+                                                                            "visits those whose terms count"})
             elif fam_ == "inf" and name != "forward":
                 # scatter kernels: HBM-bound.  bytes: g + pos reads, zero-fill of the gradient, one 8-byte
                 # read-modify-write per scattered element
@@ -582,11 +588,11 @@ def run_ours(args, rank, world, local_rank, comm_group=None):
             "traffic_source": traffic_source,
             "algorithmic_bytes": (4 * (B * CO + B * CI + CO * CI) + 4 * (B * CI + CO * CI))
             if dominant["kernel"] == "backward_fused" else 4 * (B * CI + CO * CI + B * CO)}
-    elif dominant["bound"] == "load/store pipe":
+    elif dominant["bound"] in ("load/store pipe", "logarithm / exponential mix"):
         nb = 4 * (B * CI + CO * CI + 2 * B * CO)
         gbs = round(nb / (dominant["ms"] * 1e-3) / 1e9, 1)
         line["roofline"] = {
-            "bound": "load/store pipe", "kernel": f"{dominant['kernel']} (p={args.p})", "achieved": gbs, "peak": hbm_peak,
+            "bound": dominant["bound"], "kernel": f"{dominant['kernel']} (p={args.p})", "achieved": gbs, "peak": hbm_peak,
             "unit": "GB/s", "frac": round(gbs / hbm_peak, 3),
             "note": "input, weight, output and index once each against the HBM rate; " + dominant["note"],
             "peak_source": "MEASURED_PEAKS.json" if peaks else "fallback 6650 GB/s", "ms": dominant["ms"], "traffic": None}

@@ -99,8 +99,8 @@ LDN_API unsigned long long ldn_kernel_launches(void);
  * Per-kernel timing (no counterpart in the reference): while enabled, every launch of a tile kernel is bracketed by
  * a CUDA-event pair on its stream, but for launches that run or return at once by a word in device memory;
  * ldn_last_tile_kernel_ms waits for the latest pair and returns the duration of that one kernel in milliseconds.  It
- * returns -1 if nothing was recorded since timing was enabled, or after a large p = inf call that starts from the
- * extreme channels, whose tile kernels are of that kind.  One pair per process: use from one thread, one device.
+ * returns -1 if nothing was recorded since timing was enabled, or after a large call that starts from the extreme
+ * channels (p = inf) or from power lists (32 <= p <= 100), whose tile kernels are of that kind.  One pair per process: use from one thread, one device.
  */
 LDN_API void ldn_enable_kernel_timing(int enabled);
 LDN_API float ldn_last_tile_kernel_ms(void);
@@ -112,6 +112,13 @@ LDN_API float ldn_last_tile_kernel_ms(void);
  * last call was another one.  Not during a capture.
  */
 LDN_API int ldn_last_extreme_outcome(ldn_stream_t stream, int outcome[2]);
+
+/*
+ * The same for the last call on the stream if it began with the matrix products of an even p or with power lists (no
+ * counterpart in the reference): waits for the stream and writes *outcome = 1 if the data made the general kernels give the
+ * result, else 0 (a backward pass in chunks: of the last one).  Status 1 if the last call was another one.  Not during a capture.
+ */
+LDN_API int ldn_last_power_outcome(ldn_stream_t stream, int* outcome);
 
 /*
  * Tracing hook (no counterpart in the reference): while a non-null device buffer is set, every CTA of every

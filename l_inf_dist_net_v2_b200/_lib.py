@@ -54,6 +54,7 @@ SIGNATURES = {
     "ldn_release_scratch": [],
     "ldn_reserve_scratch": [_s, ctypes.c_ulonglong],
     "ldn_last_extreme_outcome": [_s, ctypes.c_void_p],
+    "ldn_last_power_outcome": [_s, ctypes.c_void_p],
     "ldn_probe_pipe": [_i, _i, _c_float_p, ctypes.c_void_p, _s],
 }
 OTHER_SYMBOLS = ["ldn_status_string", "ldn_version", "ldn_set_max_ctas", "ldn_kernel_launches", "ldn_set_trace_buffer",

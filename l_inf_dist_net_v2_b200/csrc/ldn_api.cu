@@ -119,7 +119,8 @@ int begin_call(Call* c, ldn_stream_t stream, size_t scratch_bytes, size_t more =
     if (granted) *granted = extended;
     if (!extended && (r = ensure_arena(c->arena, c->st, scratch_bytes)) != kOk) return r;
     c->bump = Bump{c->arena->base, 0, c->arena->capacity};
-    c->arena->extreme_words = nullptr;  // (the scratch that held them is this call's now)
+    // (the scratch that held them is this call's now)
+    c->arena->extreme_words = c->arena->power_words[0] = c->arena->power_words[1] = nullptr;
     return kOk;
 }
 
@@ -428,6 +429,8 @@ int norm_dist_backward_part(const float* go, const float* x, const float* w, con
                                      c.arena->status, &direct, c.st);
             if (r != kOk) return r;
             c.copies = CopyGate{direct, flag};
+            c.arena->power_words[0] = direct;
+            c.arena->power_words[1] = flag;
             if ((r = take_views()) != kOk) return r;
         }
         // second form, gated by the flag: 1 / y and g as coefficients, 2^(q lg2(|t| / y)) per pair
@@ -665,6 +668,26 @@ LDN_API int ldn_last_extreme_outcome(ldn_stream_t stream, int* outcome) {
     return kOk;
 }
 
+LDN_API int ldn_last_power_outcome(ldn_stream_t stream, int* outcome) {
+    if (!outcome) return kBadArgument;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    Arena* arena;
+    int r = find_arena(st, &arena);
+    if (r != kOk) return r;
+    std::lock_guard<std::mutex> lock(*static_cast<std::mutex*>(arena->call_mutex));
+    if (!arena->power_words[0]) return kBadArgument;
+    int words[2] = {};
+    for (int i = 0; i < 2; ++i) {
+        if (!arena->power_words[i]) continue;
+        const cudaError_t e = cudaMemcpyAsync(words + i, arena->power_words[i], sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess) return cuda_status(e);
+    }
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_status(e);
+    *outcome = words[0] != 0 || words[1] != 0;
+    return kOk;
+}
+
 LDN_API int ldn_norm_dist_forward(const float* input, const float* weight, int B, int CO, int CI, int G, int HW,
                           float* output, float p, ldn_stream_t stream) {
     Shape s;
@@ -702,11 +725,12 @@ LDN_API int ldn_norm_dist_forward(const float* input, const float* weight, int B
     if (granted && lists) {
         r = launch_power_lists(input, weight, s, output, p, c.cap, &c.bump, &listed, c.st);
         if (r != kOk) return r;
-        c.gate = c.copies.a = listed.dense;
+        c.gate = c.copies.a = c.arena->power_words[0] = listed.dense;
+        timing_forget();  // (the tile kernel behind the lists is gated)
     } else if (granted) {
         r = launch_even_forward(input, weight, s, output, p, c.cap, &c.bump, c.arena->status, &c.gate, c.st);
         if (r != kOk) return r;
-        c.copies.a = c.gate;
+        c.copies.a = c.arena->power_words[0] = c.gate;
     }
     View xv, wv;
     if (inplace) xv = x_kmajor_view(input, s);

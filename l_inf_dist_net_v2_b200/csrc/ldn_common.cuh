@@ -200,6 +200,8 @@ struct Arena {
     void* retired;     // std::vector<void*>*: earlier blocks that captured graphs may still refer to
     bool reserved = false;  // the caller chose the size (ldn_reserve_scratch): it grows only for what a call cannot do without
     const int* extreme_words = nullptr;  // device words of the last call, if that started from the extreme channels
+    const int* power_words[2] = {};  // device words of the last call, if that began with the matrix products of an even p or with
+                                     // power lists: one that is not 0 (either may be null) says that the general kernels ran
     size_t refused = 0;     // not 0: the smallest size that could not be had for a growth that a call can do without
 };
 int find_arena(cudaStream_t stream, Arena** out);

@@ -108,7 +108,7 @@ static void drop_block(Arena* arena, cudaStream_t stream) {
     }
     arena->base = nullptr;
     arena->capacity = 0;
-    arena->extreme_words = nullptr;
+    arena->extreme_words = arena->power_words[0] = arena->power_words[1] = nullptr;
 }
 
 // Makes the arena's block at least `bytes` large.  The caller holds the arena's call mutex, so no other host thread

@@ -3,6 +3,8 @@ sample, and data on either side of the guards.  The yardstick is the direct kern
 outputs: what the products give may be at most twice as far off, as a whole, in the worst channel, and at the 99th percentile
 of the entries' relative errors.  (Each is a rounding error's size times a constant: the margin of 1e-7 is that of a result
 rounded once to 32 bits, its seven powers 1e-6 for a single entry.)"""
+import ctypes
+
 import pytest
 import torch
 
@@ -104,12 +106,14 @@ def test_entries_of_both_gradients(lib, kind, p):
     before = lib.ldn_kernel_launches()
     got = torch.autograd.grad(y, (x, w), g, retain_graph=True)
     assert lib.ldn_kernel_launches() - before > 8  # (more than the direct kernels make)
+    direct_ran = ctypes.c_int(-1)
+    assert lib.ldn_last_power_outcome(torch.cuda.current_stream().cuda_stream, ctypes.byref(direct_ran)) == 0
+    if kind in SUITED or p == 8.0:
+        assert direct_ran.value == (kind in UNSUITED)
     lib.ldn_set_max_ctas(1)  # the direct kernels
     direct = torch.autograd.grad(y, (x, w), g, retain_graph=True)
     want = _exact(x, w, g, y.detach(), p)
     for a, d, b in zip(got, direct, want):
-        if p == 8.0 and kind in SUITED and kind != "wide clusters":
-            assert not torch.equal(a, d)
         for mine, theirs, margin in zip(_errors(a, b), _errors(d, b), (1e-7, 1e-7, 1e-6)):
             assert mine < 2 * theirs + margin
 
