@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace ldn {
 
 // ---------------------------------------------------------------------------------------------
@@ -170,6 +172,25 @@ __device__ __forceinline__ unsigned sm_id() {
     return s;
 }
 
+// `bytes` of BYTES (4 or 16) from global into shared memory, in the background; zeros for the rest
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src, int bytes) {
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+// Order-preserving code of a float (0 is below all of them); a not-a-number of either sign is above infinity in the code of
+// the value or of its negative.
+__device__ __forceinline__ unsigned ordered(float v) {
+    const unsigned b = __float_as_uint(v);
+    return (b & 0x80000000u) ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float from_ordered(unsigned c) {
+    return __uint_as_float((c & 0x80000000u) ? c & 0x7fffffffu : ~c);
+}
+
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -240,6 +261,27 @@ unsigned long long* trace_buffer();
 void count_launches(int n);
 
 inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? kOk : kCudaBase + static_cast<int>(e); }
+
+// What a launcher sets up once per device (static in it), such as its kernels' shared memory: by whichever thread comes first, or
+// by several (it does no harm).
+class OncePerDevice {
+    std::atomic<bool> done_[64] = {};
+
+public:
+    template <class F>
+    int operator()(F set_up) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev < 64 && done_[dev].load(std::memory_order_acquire)) return kOk;
+        const cudaError_t e = set_up();
+        if (e == cudaSuccess && dev < 64) done_[dev].store(true, std::memory_order_release);
+        return cuda_status(e);
+    }
+};
+template <class K>
+cudaError_t allow_smem(K* kernel, int bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
 
 // Launches a kernel that begins with stream_order_begin(): its blocks may be placed on the SMs that the kernel in front of it
 // on the stream leaves, instead of after that kernel's end and a launch's latency.

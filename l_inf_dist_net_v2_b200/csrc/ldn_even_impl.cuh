@@ -284,14 +284,6 @@ __device__ __forceinline__ void load1(float* v, const float* p, bool there) {
                  : "+f"(*v)
                  : "l"(p), "r"(static_cast<uint32_t>(there)));
 }
-// BYTES of global memory into shared memory, in the background; zeros where there is nothing to load
-template <int BYTES>
-__device__ __forceinline__ void copy_async(void* dst, const float* src, bool there) {
-    if (BYTES == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(there ? 4 : 0) : "memory");
-}
 __device__ __forceinline__ void load4(float2* v, const float* p, bool there) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
                  : "+f"(v[0].x), "+f"(v[0].y), "+f"(v[1].x), "+f"(v[1].y)
@@ -520,17 +512,17 @@ __global__ void __launch_bounds__(kEvenThreads, 1) even_kernel(const EvenParams 
 #pragma unroll
                 for (int c = 0; c < CW; c += 4) {
                     if (P.vec) {
-                        copy_async<16>(resident + (c / 4 * 32 * kEpiWarps + threadIdx.x) * 16, P.resident + off + c, in && n0 + c < P.N);
+                        copy_async<16>(resident + (c / 4 * 32 * kEpiWarps + threadIdx.x) * 16, P.resident + off + c, in && n0 + c < P.N ? 16 : 0);
                     } else {
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
                             copy_async<4>(resident + (c / 4 * 32 * kEpiWarps + threadIdx.x) * 16 + 4 * i, P.resident + off + (c + i) * P.out.s_n,
-                                          in && n0 + c + i < P.N);
+                                          in && n0 + c + i < P.N ? 4 : 0);
                     }
                 }
                 if (lane < CW / 2) {
                     const int q = lane % (CW / 4);
-                    copy_async<16>(scales + lane * 16, (lane < CW / 4 ? P.col_down : P.col_shift) + s.g * P.tiles_n * CT + n0 + 4 * q, true);
+                    copy_async<16>(scales + lane * 16, (lane < CW / 4 ? P.col_down : P.col_shift) + s.g * P.tiles_n * CT + n0 + 4 * q, 16);
                 }
                 load1(&row_exp, reinterpret_cast<const float*>(P.row_exp) + s.g * P.M + m, in);
                 load1(&q0, P.row_sum + s.g * P.M + m, s.kt0 == 0 && in && !(P.split && rank == 1));
@@ -1133,16 +1125,6 @@ __global__ void __launch_bounds__(kPrep) even_direct_kernel(const float* x, cons
     }
 }
 
-// Order-preserving code of a float (0 is below all of them); a not-a-number of either sign is above infinity in the code of
-// the value or of its negative.
-__device__ __forceinline__ unsigned ordered(float v) {
-    const unsigned b = __float_as_uint(v);
-    return (b & 0x80000000u) ? ~b : b | 0x80000000u;
-}
-__device__ __forceinline__ float from_ordered(unsigned c) {
-    return __uint_as_float((c & 0x80000000u) ? c & 0x7fffffffu : ~c);
-}
-
 constexpr int kColumnRows = 128;  // least rows per block of the column jobs
 constexpr int kMaxRanges = 64;
 constexpr int kMaxSplits = 64;    // row ranges of the coefficients' column sums
@@ -1567,18 +1549,13 @@ ForwardPlan plan_forward(const Shape& s, int np) {
 
 template <int PW, bool FWD>
 int launch_even(const EvenParams& P, int cap, cudaStream_t st) {
-    static bool configured[64] = {};
+    static OncePerDevice once;
     constexpr int smem = even_smem(FWD, PW - 1);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 64 && !configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(even_kernel<PW, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return cuda_status(e);
-        configured[dev] = true;
-    }
+    int r = once([] { return allow_smem(even_kernel<PW, FWD>, smem); });
+    if (r != kOk) return r;
     const int workers = workers_of(P.total, cap);
     timing_before(st);
-    int r = launch_after_in_clusters(even_kernel<PW, FWD>, 2, workers * 2, kEvenThreads, smem, st, P);
+    r = launch_after_in_clusters(even_kernel<PW, FWD>, 2, workers * 2, kEvenThreads, smem, st, P);
     timing_after(st);
     if (r != kOk) return r;
     constexpr unsigned pieces = (FWD ? kNRows : channels_of(PW - 1)) / 8;

@@ -642,21 +642,10 @@ unsigned most_hard_of(long long B, int CO) {
     return static_cast<unsigned>(n > 4096 ? n : 4096);
 }
 
-template <class K>
-int allow_smem(K kernel, bool (&configured)[64], int bytes) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 64 && configured[dev]) return kOk;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return cuda_status(e);
-    if (dev < 64) configured[dev] = true;
-    return kOk;
-}
-
 template <bool BOUND, bool WSIDE, int S>
 int launch_scan_s(const Problem& P, cudaStream_t st) {
-    static bool configured[64] = {};
-    int r = allow_smem(extreme_scan_kernel<BOUND, WSIDE, S>, configured, kMaxTile);
+    static OncePerDevice once;
+    int r = once([] { return allow_smem(extreme_scan_kernel<BOUND, WSIDE, S>, kMaxTile); });
     if (r != kOk) return r;
     const int smem = round4(P.C) * S * 4 * (BOUND && WSIDE ? 2 : 1);
     const long long tiles = ((WSIDE ? P.B : P.CO) + S - 1) / S;

@@ -35,12 +35,6 @@ inline int smem_bytes(const Shape& s, int warps, int mode) {
            static_cast<int>(sizeof(float));
 }
 
-template <int BYTES>
-__device__ __forceinline__ void copy_async(void* dst, const void* src, int bytes) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int PENDING>
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }

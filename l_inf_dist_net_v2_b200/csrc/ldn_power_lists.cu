@@ -75,12 +75,7 @@ struct ListParams {
     float* y;
 };
 
-__device__ __forceinline__ unsigned code_of(float v) {
-    const unsigned b = __float_as_uint(v);
-    return (b & 0x80000000u) ? ~b : b | 0x80000000u;
-}
-__device__ __forceinline__ float value_of(unsigned c) { return __uint_as_float((c & 0x80000000u) ? c & 0x7fffffffu : ~c); }
-__device__ __forceinline__ float center_of(const Words* W) { return 0.5f * (value_of(W->x_top) - value_of(W->x_low)); }
+__device__ __forceinline__ float center_of(const Words* W) { return 0.5f * (from_ordered(W->x_top) - from_ordered(W->x_low)); }
 
 __global__ void __launch_bounds__(kBlock) lists_range_kernel(const ListParams P) {
     stream_order_begin();
@@ -89,8 +84,8 @@ __global__ void __launch_bounds__(kBlock) lists_range_kernel(const ListParams P)
 #pragma unroll 4
     for (long long i = blockIdx.x * static_cast<long long>(kBlock) + threadIdx.x; i < total; i += static_cast<long long>(gridDim.x) * kBlock) {
         const float v = P.x[i];
-        t = max(t, code_of(v));
-        l = max(l, code_of(-v));
+        t = max(t, ordered(v));
+        l = max(l, ordered(-v));
     }
     t = __reduce_max_sync(0xffffffffu, t);
     l = __reduce_max_sync(0xffffffffu, l);
@@ -571,20 +566,17 @@ inline int x_cap_of(const Shape& s) { return whole_trips(0.35 * s.CI / (32 / til
 
 template <int ROWS>
 int launch_lists(const ListParams& P, int sm_count, cudaStream_t st) {
-    static bool configured[64] = {};
+    static OncePerDevice once;
     constexpr int classes = 32 / ROWS;
     const int smem = ((P.CI + classes - 1) / classes * classes + classes) * ROWS * 4;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 64 && !configured[dev]) {
-        constexpr int most = ((ROWS == 16 ? kMaxWide : kMaxChannels) + 2 * classes) * ROWS * 4;
-        cudaError_t e = cudaFuncSetAttribute(lists_walk_kernel<ROWS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(lists_walk_kernel<ROWS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e != cudaSuccess) return cuda_status(e);
-        configured[dev] = true;
-    }
+    int r = once([] {
+        constexpr int most = ((ROWS == 16 ? kMaxWide : kMaxChannels) + 2 * (32 / ROWS)) * ROWS * 4;
+        const cudaError_t e = allow_smem(lists_walk_kernel<ROWS, false>, most);
+        return e == cudaSuccess ? allow_smem(lists_walk_kernel<ROWS, true>, most) : e;
+    });
+    if (r != kOk) return r;
     const int row_blocks = (P.B + P.CO + kBlock / 32 - 1) / (kBlock / 32);
-    int r = launch_after(lists_range_kernel, 2 * sm_count, kBlock, 0, st, P);
+    r = launch_after(lists_range_kernel, 2 * sm_count, kBlock, 0, st, P);
     if (r == kOk) r = launch_after(lists_rows_kernel, row_blocks, kBlock, 0, st, P);
     if (r == kOk) r = launch_after(lists_sample_kernel, kSamples, kBlock, 0, st, P, 0.5f);
     if (r == kOk) r = launch_after(lists_build_kernel<ROWS>, row_blocks, kBlock, 0, st, P);

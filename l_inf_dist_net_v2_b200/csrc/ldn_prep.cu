@@ -344,16 +344,10 @@ __global__ void __launch_bounds__(kBlock) rescan_inplace_kernel(Operand a0, Oper
 
 template <int P>
 int launch_rescan_inplace(Operand a0, Operand b, const float* y, int* pos, const Shape& s, cudaStream_t st) {
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
+    static OncePerDevice once;
     const int smem = s.CIg * P * static_cast<int>(sizeof(float));
-    if (dev >= 64 || !configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(rescan_inplace_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   kRescanInplaceMaxSmem);
-        if (e != cudaSuccess) return cuda_status(e);
-        if (dev < 64) configured[dev] = true;
-    }
+    const int r = once([] { return allow_smem(rescan_inplace_kernel<P>, kRescanInplaceMaxSmem); });
+    if (r != kOk) return r;
     const dim3 grid(static_cast<unsigned>(static_cast<long long>(s.B) * s.G), static_cast<unsigned>((s.HW + P - 1) / P));
     return launch_after(rescan_inplace_kernel<P>, grid, kBlock, smem, st, a0, b, y, pos, s);
 }

@@ -700,25 +700,19 @@ struct TileLaunch {
 
 template <class Op>
 int launch_tile(const TileLaunch& L, cudaStream_t stream) {
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
+    static OncePerDevice once;
     constexpr int SMEM = TileSmem<Op>::kTotal;
     // ops whose rows are batch rows also exist with half of the register rows, for problems of at most 64 rows
     constexpr bool HALF = Op::LA == Layout::RowMajor;
-    if (dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(tile_kernel<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e == cudaSuccess && HALF)
-            e = cudaFuncSetAttribute(tile_kernel<Op, (HALF ? kRegM / 2 : kRegM)>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) return cuda_status(e);
-        configured[dev] = true;
-    }
+    int r = once([] {
+        const cudaError_t e = allow_smem(tile_kernel<Op>, SMEM);
+        return e == cudaSuccess && HALF ? allow_smem(tile_kernel<Op, (HALF ? kRegM / 2 : kRegM)>, SMEM) : e;
+    });
+    if (r != kOk) return r;
     // (a gated launch usually returns at once: the optional timing brackets the ungated kernels only)
     const bool timed = L.params.gate == nullptr;
     if (timed) timing_before(stream);
     const bool half = HALF && L.params.M <= kTileM / 2;
-    int r;
     if (half)
         r = launch_after(tile_kernel<Op, (HALF ? kRegM / 2 : kRegM)>, L.grid, kThreads, SMEM, stream, L.map_a0, L.map_a1,
                          L.map_b, L.params);
