@@ -156,9 +156,11 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
 // early.  (Pointers of these kernels carry no __restrict__: a load that is known not to change could be moved up across it.)
 // A launch behind another costs 1 us less: 200 x 1001 -> 777, p = 3, forward + input gradient (10 launches) 121 -> 107 us,
 // 128 x 64 x 16 x 16 convolution step at p = inf 400 -> 391, 512 x 3072 -> 5120 certification 1982 -> 1972.
+__device__ __forceinline__ void stream_order_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void stream_order_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void stream_order_begin() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    stream_order_release();
+    stream_order_wait();
 }
 
 __device__ __forceinline__ unsigned long long global_timer_ns() {

@@ -27,9 +27,10 @@
 //     such drift.)
 //   * powers are scaled into fp16's range: by one power of two for both operands in the forward pass (all terms of the sum
 //     share it), by one per channel and one per coefficient row in the backward pass;
-//   * forward: an output for which the terms could cancel, y^p < 2^-6 (|x|_p + |w|_p)^p, or that is small on the common
-//     scale, y^p < 2^-10 M^p with the largest magnitude M, goes to a list and is summed directly; too many of them, or a value that is not finite, and the
-//     direct kernels behind this path run instead;
+//   * forward: an output for which the terms could cancel, y^p < r (|x|_p + |w|_p)^p (least_of_norms says with which r), or that is
+//     small on the common scale, y^p < 2^-10 M^p with the largest magnitude M, goes to a list and is summed directly; too many of
+//     them, or a value that is not finite, and the direct kernels behind this path run instead.  Where that is to be expected it is
+//     known before the products: from sampled outputs, and from rows whose norms are small on the common scale;
 //   * backward: the direct kernels run if the coefficients of a row (of x, or of w) sit on few of its terms, sum |A| < 4 max |A|;
 //     if they prefer small differences in all channels at once, as within clusters: an output below kLeastOfSpread (by p) of
 //     (sum_c s^p)^(1/p), s[c] the root mean square of x - w over all pairs; if an output is below a third of the largest |d| + |u|
@@ -59,6 +60,8 @@ constexpr int kEvenThreads = 32 * (kEpiWarps + kConvWarps + 1);
 constexpr float kScaleB = 32768.0f;         // backward: powers of values below 1 as fp16 holds them best
 constexpr float kTruncation = 1.0f + 1.0f / (1 << 22);
 constexpr int kListCap = 1 << 16;
+constexpr int kGuardSamples = 64;  // sampled outputs of the forward form, and how many of them below the line say that the list
+constexpr int kMostBelow = 8;      // will not do (it holds a 40th of 512 x 5120 outputs: 8 of 64 then by chance 3 times in 10^4)
 // guards of the backward form
 constexpr float kLeastSpread = 4.0f;       // sum of |A| over its largest, per row
 __device__ __forceinline__ double least_of_spread(int p) { return p == 8 ? 0.95 : (p == 6 ? 0.85 : (p == 4 ? 0.5 : 0.25)); }
@@ -119,6 +122,7 @@ struct EvenParams {
     // forward
     const float *sum_a, *norm_a, *sum_b, *norm_b;  // row sums of p-th powers on the common scale and their p-th roots
     const unsigned* scale_word;     // bits of the largest magnitude
+    float least;                    // of the guard on the norms (least_of_norms)
     int* list;                      // outputs to be summed directly
     int* list_count;
     int* dense;
@@ -365,7 +369,7 @@ template <int PW>
 __device__ __forceinline__ float forward_value(const EvenParams& P, const ForwardEnd& E, float acc, float sa, float na, float sb,
                                                float nb, int off) {
     const float s = fmaf(acc, E.from_acc, sa + sb);
-    const float least = fmaxf(E.least, power<PW>(na + nb) * (1.0f / 64));
+    const float least = fmaxf(E.least, power<PW>(na + nb) * P.least);
     if (!(s >= least) && *static_cast<volatile int*>(P.dense) == 0) {
         const int at = atomicAdd(P.list_count, 1);
         if (at < kListCap) P.list[at] = off;
@@ -1023,6 +1027,52 @@ __device__ __forceinline__ void row_power_sums(const Source& S, int G, int block
     top = __reduce_max_sync(0xffffffffu, top);
     if (lane == 0 && top > *static_cast<volatile unsigned*>(scale_word)) atomicMax(scale_word, top);
 }
+// One of the sampled outputs: whether it is below the guard's line.  The last block to know decides.  counts: outputs below, blocks.
+// It runs beside the kernel in front of it, whose results it does not need, and waits for that at its end (in one kernel with the
+// row sums these took 72 us instead of 31 for 32 images of 576 x 1024; behind them it would add 9).
+// That kernel starts behind a memset, which nothing overtakes: whatever was queued before the memset is done when blocks of either
+// kernel start, so that only the kernels behind this one depend on the wait.
+template <int PW>
+__global__ void __launch_bounds__(kPrep) even_sample_kernel(const Source a, const Source b, int G, float least, int* counts, int* dense) {
+    stream_order_release();
+    const int sample = blockIdx.x;
+    __shared__ double part[3][8];
+    const int g = sample % G;
+    // (spread over both operands; coprime strides)
+    const float* pa = source_row(a, g, static_cast<int>(static_cast<long long>(sample) * a.rows / kGuardSamples));
+    const float* pb = source_row(b, g, static_cast<int>((sample * 7919LL + 13) % b.rows));
+    double sum[3] = {};
+#pragma unroll 4
+    for (int k = threadIdx.x; k < a.k; k += kPrep) {
+        const double v[3] = {pa[k * a.s_k], pb[k * b.s_k], static_cast<double>(pa[k * a.s_k]) - pb[k * b.s_k]};
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double d = v[i] * v[i];
+            double q = d;
+#pragma unroll
+            for (int e = 1; e < PW / 2; ++e) q *= d;
+            sum[i] += q;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        for (int d = 16; d > 0; d >>= 1) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], d);
+        if ((threadIdx.x & 31) == 0) part[i][threadIdx.x >> 5] = sum[i];
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) {
+        stream_order_wait();
+        return;
+    }
+    for (int w = 1; w < kPrep / 32; ++w)
+        for (int i = 0; i < 3; ++i) sum[i] += part[i][w];
+    const double most = fmax(sum[0], sum[1]);
+    const float na = static_cast<float>(sum[0] / most), nb = static_cast<float>(sum[1] / most);
+    if (static_cast<float>(sum[2] / most) < least * power<PW>(powf(na, 1.0f / PW) + powf(nb, 1.0f / PW))) atomicAdd(counts, 1);
+    __threadfence();
+    if (atomicAdd(counts + 1, 1) == kGuardSamples - 1 && atomicAdd(counts, 0) >= kMostBelow) *dense = 1;
+    stream_order_wait();
+}
 template <int PW>
 __global__ void __launch_bounds__(kPrep) even_rows_kernel(const Source a, const Source b, int G, int blocks_a, double* sums_a,
                                                          double* sums_b, unsigned* scale_word) {
@@ -1042,6 +1092,7 @@ __global__ void __launch_bounds__(kPrep) even_powers_kernel(const Source a, int 
     stream_order_begin();
     const unsigned top = *scale_word;
     const int e = exponent_above(top);
+    if (*static_cast<volatile int*>(dense) != 0) return;
     if (top >= 0x7f800000u || e < -100 || e > 100) {  // not finite, all zero, or hardly a number
         if (blockIdx.x == 0 && threadIdx.x == 0) *dense = 1;
         return;
@@ -1119,6 +1170,7 @@ __global__ void __launch_bounds__(kPrep) even_direct_kernel(const float* x, cons
         const float* xr = x + (static_cast<long long>(b) * s.CI + static_cast<long long>(g) * s.CIg) * s.HW + hw;
         const float* wr = w + static_cast<long long>(o) * s.CIg;
         float sum = 0.0f;
+#pragma unroll 8
         for (int c = lane; c < s.CIg; c += 32) sum += power<PW>(xr[static_cast<long long>(c) * s.HW] - wr[c]);
         for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
         if (lane == 0) y[off] = powf(fmaxf(sum, FLT_MIN), 1.0f / PW);
@@ -1565,6 +1617,17 @@ int launch_even(const EvenParams& P, int cap, cudaStream_t st) {
     return launch_after(even_fold_kernel<PW, FWD>, dim3(workers - 1, pieces, 2), kMRows, 0, st, P, workers);
 }
 
+// r of the forward guard: what an output may be, to the p-th power, of its rows' norms.  The expansion's error of a value goes with
+// 1 / (p r), the direct kernels' with the root of the channels.  Measured with r = 2^-6 for all, operands with a common offset,
+// products / direct kernels, in 1e-8 of the values: root mean square at p = 2 133 / 26 (1536 channels) and 93 / 12 (256), p = 4 17 / 16
+// and 19 / 6.5; the largest at p = 6 and 8 and 256 channels 103 / 27 and 111 / 26, from 576 channels on 40 - 65 / 36.  With these
+// of what passes at most 26 / 30 and 14 / 11, 6 / 16 and 5 / 7; the largest 63 / 27 (p = 6, 256 channels).  Images and activations
+// with N(0, 1) weights lie at 2^-0.9 (p = 2) to 2^-3.4 (p = 8), their smallest outputs at 2^-5.5 and above from 576 channels on.
+inline float least_of_norms(int p, int channels) {
+    const float base = p == 2 ? 0.0625f : (p == 4 ? 0.0221f : 0.015625f);
+    return channels < 1024 ? base * sqrtf(1024.0f / channels) : base;
+}
+
 template <int PW>
 int forward_power(const float* x, const float* w, const Shape& s, float* y, int cap, Bump* bump, int* status, const int** dense,
                   cudaStream_t st) {
@@ -1576,7 +1639,7 @@ int forward_power(const float* x, const float* w, const Shape& s, float* y, int 
     double* sums = bump->take<double>(static_cast<size_t>(rows_a) + rows_b);
     float* floats = bump->take<float>(2 * (static_cast<size_t>(rows_a) + rows_b));
     int* list = bump->take<int>(kListCap);
-    int* words = bump->take<int>(8);  // largest magnitude, list length, dense, three counts of even_powers_kernel
+    int* words = bump->take<int>(8);  // largest magnitude, list length, dense, three counts of even_powers_kernel, two of samples
     float* partials = bump->take<float>(part_floats(f.M, f.total, f.stages, cap, kNRows));
     if (!images || !sums || !floats || !list || !words || !partials) return kWorkspace;
     *dense = words + 2;
@@ -1588,6 +1651,9 @@ int forward_power(const float* x, const float* w, const Shape& s, float* y, int 
     auto sum_blocks = [&](const Source& S) { return S.kind == 2 ? s.G * div_up(S.rows, 32) : div_up(static_cast<long long>(s.G) * S.rows, 8); };
     const int blocks_a = sum_blocks(a);
     int r = launch_after(even_rows_kernel<PW>, blocks_a + sum_blocks(b), kPrep, 0, st, a, b, s.G, blocks_a, sums, sums + rows_a, scale);
+    const float least = least_of_norms(PW, s.CIg);
+    if (r == kOk && static_cast<double>(s.M) * s.CO * kMostBelow > 2.0 * kListCap * kGuardSamples)
+        r = launch_after(even_sample_kernel<PW>, kGuardSamples, kPrep, 0, st, a, b, s.G, least, words + 6, words + 2);
     if (r != kOk) return r;
     float *sum_a = floats, *norm_a = sum_a + rows_a, *sum_b = norm_a + rows_a, *norm_b = sum_b + rows_b;
     const int kb = div_up(s.CIg, kBlockK);
@@ -1610,6 +1676,7 @@ int forward_power(const float* x, const float* w, const Shape& s, float* y, int 
     P.out_f = y;
     P.sum_a = sum_a; P.norm_a = norm_a; P.sum_b = sum_b; P.norm_b = norm_b;
     P.scale_word = scale;
+    P.least = least;
     P.list = list; P.list_count = words + 1; P.dense = words + 2;
     P.gate0 = words + 2;
     P.partials = partials;
