@@ -10,8 +10,8 @@ namespace {
 // kernels a time per pair, padding of their 128-wide tiles included.  Either runs on the CTAs it may have: the fits' times per
 // stage and per pair go up as those go down (512 x 1536 -> 2048, p = 8, 37 of 148: 842 / 1614 us direct,
 // 212 / 434 on the products).  Measured, direct -> this path, p = 8, forward / both
-// gradients: 512 x 3072 -> 5120 1045 / 2019 -> 281 / 612, 256 x 1024 -> 2048 81 / 161 -> 59 / 123, 256 x 1024 -> 1024 50 / 103
-// -> 52 / 102 (here the line lies), 64 x 784 -> 1024 20 / 71 -> 47 / 97; 32 images of 576 x 1024 -> 128 340 / 878 -> 219 / 409.
+// gradients: 512 x 3072 -> 5120 1045 / 2019 -> 285 / 640, 256 x 1024 -> 2048 81 / 161 -> 70 / 128, 256 x 1024 -> 1024 50 / 103
+// -> 52 / 102 (here the line lies), 64 x 784 -> 1024 20 / 71 -> 47 / 97; 32 images of 576 x 1024 -> 128 340 / 878 -> 232 / 426.
 constexpr double kMargin = 1.1;         // the estimate has to win by this factor
 constexpr int kLeastChannels = 192;     // below, an output's error is a few terms' error: no smaller than the direct sum's
 
