@@ -4,8 +4,8 @@
 //   y^p            = sum_c x^p + sum_c w^p + sum_{j=1}^{p-1} (-1)^j C(p, j) sum_c x^j w^(p-j)
 //   grad_x[b, c]   = sum_j (-1)^j C(p-1, j) d^(p-1-j) sum_o A[b, o] u[o, c]^j,      A = go / y^(p-1)
 //   grad_w[o, c]   = sum_j (-1)^j C(p-1, j) d^(p-1-j) sum_b A[b, o] u[b, c]^j
-// with u = w - m, d = x - m for grad_x and u = x - m, d = w - m for grad_w, m[c] the mean of the channel in the operand that
-// is summed over.  That is p - 1 matrix products each.  Every factor is split into two 11-bit halves, v = hi + lo in fp16 (lo holds what hi
+// with u = w - m, d = x - m for grad_x and u = x - m, d = w - m for grad_w, m[c] about the mean of the channel in the operand
+// that is summed over.  That is p - 1 matrix products each.  Every factor is split into two 11-bit halves, v = hi + lo in fp16 (lo holds what hi
 // rounds off, so the pair keeps 22 - 23 bits), and a product is hi hi + hi lo + lo hi with fp32 accumulators (and lo lo for
 // p = 2): 3 x 7 multiply-adds per pair on the tensor cores for p = 8, against 4 (forward) and 8 (backward) FP32 instructions of
 // the direct kernels.  In the forward pass the terms do not cancel where it matters: large |x - w| come from x and w of opposite
@@ -37,8 +37,8 @@
 //     of a channel (rows of different scales: powers of the small ones would leave fp16's range); or if a channel's u are
 //     below 2^-12 of its d without being 0.
 //     Errors against 64 bits, 512 x 1536 -> 2048, p = 8, products / direct kernels, 2-norm (99th percentile of the entries'
-//     relative errors): grad_x of images 2.8e-7 / 7.6e-7 (1.4e-5 / 2.6e-5), grad_w 2.6e-7 / 2.8e-7 (1.2e-5 / 1.7e-5), of pixels
-//     0.5 +- 0.02 2.5e-7 / 2.7e-7 (1.1e-5 / 1.7e-5), both operands in [1, 2) 2.4e-7 / 2.3e-7 (1.4e-5 / 1.4e-5).  Two clusters of
+//     relative errors): grad_x of images 2.4e-7 / 7.6e-7 (1.2e-5 / 2.6e-5), grad_w 2.4e-7 / 2.8e-7 (1.2e-5 / 1.7e-5), of pixels
+//     0.5 +- 0.02 2.3e-7 / 2.7e-7 (1.1e-5 / 1.7e-5), both operands in [1, 2) 2.4e-7 / 2.3e-7 (1.4e-5 / 1.4e-5).  Two clusters of
 //     Gaussian rows, as far apart as they are wide, lie at 1.03 (sum_c s^p)^(1/p) and would have 6.2e-7 / 2.9e-7; at half that width,
 //     0.59, 3.0e-6 / 3.4e-7.  Rows whose channels are independent of one another lie at 1.24 and above (192 - 1024 channels, uniform,
 //     normal, of zeros and ones).
@@ -1188,7 +1188,7 @@ struct BackwardStats {
     int pitch;
     int *row_exp, *out_exp;                           // rows of the coefficients, output channels
     float *row_sum, *out_sum;
-    // [g][channel_pitch], of the two operands that are summed over (w: grad_x, x: grad_w): 2^-e, -mean 2^-e
+    // [g][channel_pitch], of the two operands that are summed over (w: grad_x, x: grad_w): 2^-e, -m 2^-e
     float *down_w, *down_x, *shift_w, *shift_x;
     int channel_pitch;
     unsigned *x_top, *x_low, *w_top, *w_low;          // per channel: codes of the largest value and of the largest negative
@@ -1196,6 +1196,7 @@ struct BackwardStats {
     int x_ranges, w_ranges, x_rows, w_rows;           // ranges, and rows (samples, of images) in each
     unsigned *y_low, *most;                           // code of the largest -y, bits of the largest |d| + |u| of a channel
     double* spread_part;                              // [channel block]: sum of s^p
+    double per_x, per_w;                              // 1 / rows
     int p;
     unsigned* part_top;                               // [split][CO]
     double* part_sum;
@@ -1377,16 +1378,26 @@ __global__ void __launch_bounds__(kPrep) even_stats_kernel(const BackwardStats A
     }
 }
 
+// What a channel is taken relative to: its mean, to a sixteenth of half its range (the value itself where there is but one).  With
+// so few bits the other operand less the centre is exact for all but small values of it, and zero-mean channels are left as they
+// are; the mean itself, with its rounding in every d, made gradients 10 % worse (3.0e-7 -> 3.3e-7, p = 8).
+__device__ __forceinline__ float center_of(double mean, float least, float most) {
+    const float half = 0.5f * most - 0.5f * least;
+    if (!(half > 0.0f)) return most;
+    const int e = max(-120, min(120, exponent_above(__float_as_uint(half)) - 4));
+    return static_cast<float>(rint(mean * pow2i(-e)) * pow2i(e));
+}
+
 // 2^-e and shift of a channel that is summed over, its values in [u_low, u_top], the other operand's in [d_low, d_top]; the largest
 // |d| + |u|.
-__device__ __forceinline__ float channel_scale(float mean, float u_low, float u_top, float d_low, float d_top, float* down, float* shift,
+__device__ __forceinline__ float channel_scale(float center, float u_low, float u_top, float d_low, float d_top, float* down, float* shift,
                                                bool* bad) {
-    const float u = fmaxf(u_top - mean, mean - u_low), d = fmaxf(d_top - mean, mean - d_low);
+    const float u = fmaxf(u_top - center, center - u_low), d = fmaxf(d_top - center, center - d_low);
     const float m = u > 0.0f ? fmaxf(u, d * kChannelFloor) : d;
     const int e = m > 0.0f ? exponent_above(__float_as_uint(m)) : 0;
     *bad |= abs(e) > kMaxChannelExp || (u > 0.0f && !(u >= d * kLeastChannel));
     *down = pow2i(-max(-kMaxChannelExp, min(kMaxChannelExp, e)));
-    *shift = -mean * *down;
+    *shift = -center * *down;
     return u + d;
 }
 
@@ -1401,6 +1412,10 @@ __global__ void __launch_bounds__(kPrep) even_scales_kernel(const BackwardStats 
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const int per_group = (s.CIg + 31) / 32, g = blockIdx.x / per_group, c = (blockIdx.x - g * per_group) * 32 + lane, i = g * s.CIg + c;
         double2 sx = make_double2(0.0, 0.0), sw = sx;
+        unsigned codes[4] = {};
+        if (warp == 0 && c < s.CIg) {
+            codes[0] = A.x_top[i]; codes[1] = A.x_low[i]; codes[2] = A.w_top[i]; codes[3] = A.w_low[i];
+        }
         if (c < s.CIg) {
 #pragma unroll 4
             for (int k = warp; k < A.x_ranges; k += 8) {
@@ -1428,18 +1443,17 @@ __global__ void __launch_bounds__(kPrep) even_scales_kernel(const BackwardStats 
                 sw.x += parts[1][k][lane].x;
                 sw.y += parts[1][k][lane].y;
             }
-            const float xt = from_ordered(A.x_top[i]), xl = -from_ordered(A.x_low[i]);
-            const float wt = from_ordered(A.w_top[i]), wl = -from_ordered(A.w_low[i]);
+            const float xt = from_ordered(codes[0]), xl = -from_ordered(codes[1]);
+            const float wt = from_ordered(codes[2]), wl = -from_ordered(codes[3]);
             bad = !(fmaxf(fabsf(xt), fabsf(wt)) < INFINITY) || !(fmaxf(fabsf(xl), fabsf(wl)) < INFINITY) || isnan(xt + xl + wt + wl);
-            const double nx = static_cast<double>(s.M), nw = s.COg, ex = sx.x / nx, ew = sw.x / nw;
-            const double square = fmax(sx.y / nx - ex * ex, 0.0) + fmax(sw.y / nw - ew * ew, 0.0) + (ex - ew) * (ex - ew);
+            const double ex = sx.x * A.per_x, ew = sw.x * A.per_w;
+            const double square = fmax(sx.y * A.per_x - ex * ex, 0.0) + fmax(sw.y * A.per_w - ew * ew, 0.0) + (ex - ew) * (ex - ew);
             spread = square;
             for (int k = 1; k < A.p / 2; ++k) spread *= square;
             const int at = g * A.channel_pitch + c;
             bool bad_x = false, bad_w = false;
-            const float mean_w = fminf(fmaxf(static_cast<float>(ew), wl), wt), mean_x = fminf(fmaxf(static_cast<float>(ex), xl), xt);
-            const float most_x = channel_scale(mean_w, wl, wt, xl, xt, A.down_w + at, A.shift_w + at, &bad_x);
-            const float most_w = channel_scale(mean_x, xl, xt, wl, wt, A.down_x + at, A.shift_x + at, &bad_w);
+            const float most_x = channel_scale(center_of(ew, wl, wt), wl, wt, xl, xt, A.down_w + at, A.shift_w + at, &bad_x);
+            const float most_w = channel_scale(center_of(ex, xl, xt), xl, xt, wl, wt, A.down_x + at, A.shift_x + at, &bad_w);
             bad |= (A.need_x && bad_x) || (A.need_w && bad_w);
             most = bad ? 0.0f : fmaxf(A.need_x ? most_x : 0.0f, A.need_w ? most_w : 0.0f);
         }
@@ -1502,11 +1516,14 @@ struct CoefImages {
     int tiles_m, kb, blocks;
     bool split;
 };
-// (and, beside the first of them, the last guard: the products, not the images, wait for it)
+// (and, in a block behind theirs, the last guard: the products, not the images, wait for it)
 __global__ void __launch_bounds__(kPrep) even_coef_kernel(const BackwardStats A, const CoefImages X, const CoefImages W) {
     stream_order_begin();
     if (*A.range != 0 || *A.cond != 0) return;
-    if (blockIdx.x == 0 && threadIdx.x < 32) guard_outputs(A);
+    if (static_cast<int>(blockIdx.x) == X.blocks + W.blocks) {
+        if (threadIdx.x < 32) guard_outputs(A);
+        return;
+    }
     const bool first = static_cast<int>(blockIdx.x) < X.blocks;
     const CoefImages& J = first ? X : W;
     const int block = first ? blockIdx.x : blockIdx.x - X.blocks;
@@ -1763,6 +1780,8 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
         !A.x_part || !A.w_part || !A.spread_part || (gx && !images_x) || (gw && !images_w) || !partials)
         return kWorkspace;
     A.p = PW;
+    A.per_x = 1.0 / static_cast<double>(s.M);
+    A.per_w = 1.0 / s.COg;
     A.down_w = channels; A.down_x = channels + scales;
     A.shift_w = channels + 2 * scales; A.shift_x = channels + 3 * scales;
     A.x_top = words; A.x_low = A.x_top + s.CI; A.w_top = A.x_low + s.CI; A.w_low = A.w_top + s.CI;
@@ -1804,7 +1823,7 @@ int backward_power(const float* coef, int pitch, const float* x, const float* w,
     W.src = Source{coef, 2, s.COg, static_cast<int>(s.M), 0, 1, pitch, 0, group};
     blocks_of(W, pw, images_w);
     W.exp = A.out_exp;
-    if ((r = launch_after(even_coef_kernel, X.blocks + W.blocks, kPrep, 0, st, A, X, W)) != kOk) return r;
+    if ((r = launch_after(even_coef_kernel, X.blocks + W.blocks + 1, kPrep, 0, st, A, X, W)) != kOk) return r;
     EvenParams P{};
     P.G = s.G;
     P.N = s.CIg;
