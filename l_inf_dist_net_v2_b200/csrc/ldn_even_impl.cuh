@@ -40,8 +40,8 @@
 //     relative errors): grad_x of images 2.4e-7 / 7.6e-7 (1.2e-5 / 2.6e-5), grad_w 2.4e-7 / 2.8e-7 (1.2e-5 / 1.7e-5), of pixels
 //     0.5 +- 0.02 2.3e-7 / 2.7e-7 (1.1e-5 / 1.7e-5), both operands in [1, 2) 2.4e-7 / 2.3e-7 (1.4e-5 / 1.4e-5).  Two clusters of
 //     Gaussian rows, as far apart as they are wide, lie at 1.03 (sum_c s^p)^(1/p) and would have 6.2e-7 / 2.9e-7; at half that width,
-//     0.59, 3.0e-6 / 3.4e-7.  Rows whose channels are independent of one another lie at 1.24 and above (192 - 1024 channels, uniform,
-//     normal, of zeros and ones).
+//     0.59, 3.0e-6 / 3.4e-7.  Rows whose channels are independent of one another lie at 1.24 and above (1.14, 1.0, 0.78 at
+//     p = 6, 4, 2; 192 - 1024 channels, uniform, normal, of zeros and ones).
 #pragma once
 #include <float.h>
 #include <math.h>
